@@ -59,13 +59,9 @@ def lookup(R: int, k: int, dense: bool = False) -> dict | None:
 
 
 def candidate_shapes_dense():
-    # the two-kernel cell-mask pass (what the automatic variant runs on dense
-    # DBs): ring stages (tiles in flight per SM) and consumer warps, a
-    # multiple of the stages (warps per stage split its tiles' chunks), 24 at
-    # most; then a few shapes of the one-kernel pass for comparison
-    for st, cpt in itertools.product((4, 6, 8, 10, 12, 16), (1, 2, 3, 4)):
-        if st * cpt <= 24:
-            yield dict(variant=5, stages=st, consumers=st * cpt)
+    # the grouped records' filter (no launch shape to choose), then a few shapes
+    # of the one-kernel cell-mask pass for comparison
+    yield dict(variant=5)
     for q, cons in itertools.product((0, 1), (8, 12)):
         yield dict(variant=4, consumers=cons, cell_queue=q)
 

@@ -436,6 +436,127 @@ __device__ __forceinline__ void process(const CmpArgs &a, const Spots sp, int c,
   }
 }
 
+// The j-th set bit of m (j < popcount).
+__device__ __forceinline__ int nth_bit(unsigned long long m, int j) {
+  unsigned w = (unsigned)m;
+  int base = 0;
+  const int p = __popc(w);
+  if (j >= p) {
+    j -= p;
+    w = (unsigned)(m >> 32);
+    base = 32;
+  }
+#pragma unroll
+  for (int s = 16; s; s >>= 1) {
+    const int t = __popc(w & ((1u << s) - 1u));
+    if (j >= t) {
+      j -= t;
+      w >>= s;
+      base += s;
+    }
+  }
+  return base;
+}
+
+// The per-record logic of process() for 32 records whose on-detector pixels lie
+// in the warp's shared-memory rows (lane l's c pixels at rows + l * SP).  The
+// sums are shared out by (record, slot) pair over all lanes: a warp with many
+// candidates on one record, or in many slots, takes a round per 32 pairs
+// instead of one per slot, and its counter updates go out together.
+template <int B>
+__device__ __forceinline__ void process_rows(const CmpArgs &a, const uint32_t *rows, uint32_t SP, int c,
+                                             unsigned long long oid, uint64_t pol, bool valid) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t *my = rows + (uint32_t)lane * SP;
+  const int n = (!a.full_gather && c < a.min_spots) ? 0 : c;  // cannot pass: not gathered
+  unsigned long long cnt[B];
+#pragma unroll
+  for (int b = 0; b < B; b++) cnt[b] = 0ull;
+  for (int s0 = 0; s0 < n; s0 += kGather) {
+    unsigned long long m[kGather];
+#pragma unroll
+    for (int j = 0; j < kGather; j++) m[j] = s0 + j < n ? ld_nc_hint(a.occ + my[s0 + j], pol) : 0ull;
+#pragma unroll
+    for (int j = 0; j < kGather; j++) {
+      unsigned long long v = m[j] & a.active;
+      if (v) {
+#pragma unroll
+        for (int b = 0; b < B; b++) {
+          const unsigned long long t = cnt[b] & v;
+          cnt[b] ^= v;
+          v = t;
+        }
+      }
+    }
+  }
+  unsigned long long gt = 0ull, eq = ~0ull;  // count >= min_spots, bit-sliced
+#pragma unroll
+  for (int b = B - 1; b >= 0; b--) {
+    if ((a.min_spots >> b) & 1) {
+      eq &= cnt[b];
+    } else {
+      gt |= eq & cnt[b];
+      eq &= ~cnt[b];
+    }
+  }
+  const unsigned long long cand = valid ? ((gt | eq) & a.active) : 0ull;
+  const int np = __popcll(cand);
+  int x = np;  // inclusive prefix sum of the pairs over the warp
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  const int total = __shfl_sync(0xffffffffu, x, 31);
+  __syncwarp();  // every lane's row is complete before another lane reads it
+  for (int q0 = 0; q0 < total; q0 += 32) {
+    const int q = q0 + lane;
+    int o = 0;  // the lane that owns pair q: the first with x > q
+#pragma unroll
+    for (int s = 16; s; s >>= 1) {
+      const int v = __shfl_sync(0xffffffffu, x, o + s - 1);
+      if (v <= q) o += s;
+    }
+    const int before = __shfl_sync(0xffffffffu, x - np, o);
+    const unsigned long long mask = __shfl_sync(0xffffffffu, cand, o);
+    const int co = __shfl_sync(0xffffffffu, c, o);
+    const unsigned long long id = __shfl_sync(0xffffffffu, oid, o);
+    int k = 0, ns = 0, su = 0;
+    bool pass = false, surv = false;
+    double tot = 0.0, score = 0.0;
+    if (q < total) {
+      k = nth_bit(mask, q - before);
+      ns = slot_sum_body(a, ListSpots{rows + (uint32_t)o * SP}, co, k, tot, su);
+      pass = ns >= a.min_spots && tot >= a.min_int;
+      if (pass) {
+        score = dmul(tot, dsqrt((double)ns));
+        surv = score != 0.0;  // collection skips zero scores (LaueMatchingCPU.c:783)
+      }
+    }
+    if (!__any_sync(0xffffffffu, pass)) continue;
+    const unsigned same_p = __match_any_sync(0xffffffffu, pass ? k : -1);
+    const unsigned same_s = __match_any_sync(0xffffffffu, surv ? k : -1);
+    if (pass && lane == __ffs(same_p) - 1) atomicAdd(&a.pass_cnt[k], (unsigned)__popc(same_p));
+    const int lead = __ffs(same_s) - 1;
+    unsigned base = 0;
+    if (surv && lane == lead) base = atomicAdd(&a.surv_cnt[k], (unsigned)__popc(same_s));
+    base = __shfl_sync(0xffffffffu, base, lead);
+    if (surv) {
+      const unsigned pos = base + __popc(same_s & ((1u << lane) - 1u));
+      if (pos < a.cap) {
+        lmb_survivor sv;
+        sv.id = id;
+        sv.n_spots = ns;
+        sv.sum_u8 = su;
+        sv.tot_int = tot;
+        sv.score = score;
+        a.surv[(size_t)k * a.cap + pos] = sv;
+      }
+    }
+  }
+  __syncwarp();  // the rows may be overwritten
+}
+
 // One record of the reference layout.
 template <int B>
 __device__ __forceinline__ void process_rec(const CmpArgs &a, const uint16_t *rec, uint64_t oid,
@@ -980,239 +1101,254 @@ __global__ void __launch_bounds__(32 * 13, 1) compare_cell_kernel(const __grid_c
 }
 
 // ----------------------------------------------------------------------------
-// Variant 5: the cell-mask filter and the counting of its candidates as two
-// kernels.
+// Filter over the grouped records (glist.cu): which of the records with at least
+// MinNrSpots spots can reach that count in some slot?
 //
-// In one kernel (variant 4) the per-record counting logic rides along with
-// the spot filter: its registers and branches weigh on every chunk, and the
-// chunks of a tile are dealt out across all consumer warps, so each warp
-// walks every chunk of every tile.  Here the filter kernel only streams and
-// filters: one ring stage per consumer warp, the warp takes whole tiles (the
-// producer prefetches the warp's next tile into L2 while the warp works),
-// tests each spot's cell 64 spots at a time, and appends the records that can
-// still pass (at least MinNrSpots spots on marked cells) with their marked
-// pixels, in record order, to its block's region of a candidate buffer.  The
-// counting kernel then runs the per-record logic of the other variants on
-// full warps of candidates.  Survivors and pass counts are those of the other
-// variants (the candidate set and each candidate's nonzero spots are the
-// same; order is restored by the ordering kernel).
+// The pass's slots are split into up to 16 groups (one slot each up to 16 slots,
+// up to four at 64), and every cell of the detector (8 x 8 pixels at 2048^2) has a
+// 16-bit mask word: bit g says that a pixel of the cell is positive in a slot of
+// group g.  The words of all cells (at most 128 KiB) lie in each block's shared
+// memory.  A lane owns a record: it looks up the word of each of its spots and
+// counts the 16 groups at once with bit-sliced adders, two words side by side in a
+// register.  A spot counted in a slot has its cell marked in the slot's group, so
+// a record whose counts stay below MinNrSpots in every group passes in no slot;
+// the others go to the counting kernel below.  Finer groups with coarser cells
+// beat one group with fine cells: 64 frames of the tilted detector leave 1.6 % of
+// the records with 8 x 8 cells in 16 groups, 14.7 % with 4 x 1 cells in one.
 // ----------------------------------------------------------------------------
-__global__ void __launch_bounds__(32 * 25, 1) cell_filter_kernel(const __grid_constant__ CmpArgs a) {
-  extern __shared__ __align__(128) unsigned char smem[];
-  // consumers / stages warps share a ring stage (its tiles), splitting each
-  // tile's chunks between them
-  const int ST = a.stages;
-  const int CPT = a.consumers / a.stages;
-  uint64_t *full = reinterpret_cast<uint64_t *>(smem);
-  uint64_t *empty = full + 16;
-  uint32_t *ctr = reinterpret_cast<uint32_t *>(smem + 256);  // entries, pixels, warps done
-  uint32_t *cm = reinterpret_cast<uint32_t *>(smem + 384);
-  unsigned char *ring = smem + 384 + a.cm_bytes;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int NC = a.consumers;
-  const uint64_t G = gridDim.x;
-  const uint64_t my_tiles = (a.ntiles > blockIdx.x) ? (a.ntiles - 1 - blockIdx.x) / G + 1 : 0;
-  {  // the pass's cell mask into shared memory
-    const uint4 *src = reinterpret_cast<const uint4 *>(a.cellmask);
-    uint4 *dst = reinterpret_cast<uint4 *>(cm);
-    for (uint32_t i = threadIdx.x; i < a.cm_bytes / 16; i += blockDim.x) dst[i] = src[i];
+GroupCells group_cells(int W, int H) {
+  GroupCells best{};
+  long cost = -1;
+  for (int cw = 1; cw <= 256; cw++) {
+    const int nx = (W + cw - 1) / cw;
+    const int rows = 65536 / nx;  // W <= 65535, so nx <= 65536
+    if (rows < 1) continue;
+    const int ch = (H + rows - 1) / rows;
+    // cells that a spot of about 10 x 10 pixels marks, in pixels
+    const long c = (long)(cw + 9) * (ch + 9);
+    if (cost < 0 || c < cost) {
+      const int ny = (H + ch - 1) / ch;
+      best = GroupCells{cw, ch, nx, ny, (uint32_t)nx * (uint32_t)ny};
+      cost = c;
+    }
   }
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < ST; s++) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], CPT);
+  return best;
+}
+
+// Four threads per cell take its rows in turn.
+__global__ void __launch_bounds__(256) groupmask_kernel(const __grid_constant__ FilterArgs f) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t cell = t >> 2;
+  unsigned long long any = 0ull;
+  if (cell < f.cells.n) {
+    const int cy = (int)(cell / (uint32_t)f.cells.nx), cx = (int)(cell % (uint32_t)f.cells.nx);
+    const int x0 = cx * f.cells.cw, x1 = min(x0 + f.cells.cw, f.W);
+    const int y1 = min((cy + 1) * f.cells.ch, f.H);
+    for (int y = cy * f.cells.ch + (int)(t & 3u); y < y1; y += 4) {
+      const unsigned long long *row = f.occ + (size_t)y * f.W;
+#pragma unroll 8
+      for (int x = x0; x < x1; x++) any |= __ldg(row + x);
     }
-    ctr[0] = ctr[1] = ctr[2] = 0u;
-    fence_mbar_init();
   }
-  __syncthreads();
-  if (warp == 0) {
-    if (lane != 0) return;
-    const uint64_t pol_db = l2_evict_first();
-    uint64_t issued = 0;
-    int ps = 0;
-    uint32_t pr = 0;
-    for (uint64_t i = 0; i < my_tiles; i++, ring_next(ps, pr, ST)) {
-      const int s = ps;
-      if (pr > 0 && !mbar_wait_bounded(&empty[s], (pr - 1) & 1u, kWaitNs)) {
-        atomicExch(a.err, DEV_TIMEOUT_TMA);
-        break;
-      }
-      const uint64_t t = blockIdx.x + i * G;
-      mbar_expect_tx(&full[s], a.tile_bytes);
-      bulk_g2s_hint(ring + (size_t)s * a.tile_bytes, a.cl + t * a.tile_bytes, a.tile_bytes,
-                    &full[s], pol_db);
-      // the stage's next tile, into L2 while this one is worked on
-      if (i + ST < my_tiles) bulk_prefetch_l2(a.cl + (t + ST * G) * a.tile_bytes, a.tile_bytes);
-      issued = i + 1;
-    }
-    {
-      const uint64_t j0 = issued > (uint64_t)ST ? issued - ST : 0;
-      int ds = (int)(j0 % ST);
-      uint32_t dr = (uint32_t)(j0 / ST);
-      for (uint64_t j = j0; j < issued; j++, ring_next(ds, dr, ST))
-        mbar_wait_bounded(&full[ds], dr & 1u, kWaitNs);
-    }
-    return;
-  }
-  const int cw = warp - 1;
-  if (cw >= NC) return;
-  const uint32_t QS = (uint32_t)(a.qS < 1 ? 1 : a.qS);
-  uint32_t *wm = reinterpret_cast<uint32_t *>(ring + (size_t)ST * a.tile_bytes +
-                                              (size_t)cw * filter_warp_bytes(a.qS));
-  const unsigned lt = (1u << lane) - 1u;
-  const int need = a.full_gather ? 0 : a.min_spots;
-  const int sh = a.cm_shift;
-  const uint64_t e_base = a.cq_ebase[blockIdx.x], e_cap = a.cq_ebase[blockIdx.x + 1] - e_base;
-  const uint64_t p_base = a.cq_pbase[blockIdx.x], p_cap = a.cq_pbase[blockIdx.x + 1] - p_base;
-  CandEntry *E = a.cq_e + e_base;
-  uint32_t *P = a.cq_pix + p_base;
-  const int s = cw / CPT, sub = cw % CPT;  // this warp's ring stage, its share of the chunks
-  uint32_t rd = 0;  // round of tile i (i / ST)
-  for (uint64_t i = (uint64_t)s; i < my_tiles; i += (uint64_t)ST, rd++) {
-    const bool ok = mbar_wait_bounded(&full[s], rd & 1u, kWaitNs);
-    if (!__all_sync(0xffffffffu, ok)) {
-      if (lane == 0) atomicExch(a.err, DEV_TIMEOUT_TMA);
-      break;
-    }
-    const unsigned char *tb = ring + (size_t)s * a.tile_bytes;
-    const uint64_t first = *reinterpret_cast<const uint64_t *>(tb);
-    const uint32_t nch = *reinterpret_cast<const uint32_t *>(tb + 8);
-    const unsigned char *cmax = tb + 16;
-    const unsigned char *cnt = tb + clist_cnt_offset(nch);
-    const uint32_t *base = reinterpret_cast<const uint32_t *>(tb + clist_base_offset(nch));
-    const uint32_t *spots = reinterpret_cast<const uint32_t *>(tb + clist_spot_offset(nch));
-    uint32_t turn = 0;  // the k-th chunk that can pass goes to sub-warp k mod CPT
-    for (uint32_t j0 = 0; j0 < nch; j0 += 32) {
-      unsigned m = __ballot_sync(0xffffffffu, j0 + lane < nch && cmax[j0 + lane] >= need);
-      while (m) {
-        const uint32_t ch = j0 + (uint32_t)(__ffs(m) - 1);
-        m &= m - 1;
-        const bool take = turn == (uint32_t)sub;
-        turn = (turn + 1 == (uint32_t)CPT) ? 0 : turn + 1;
-        if (!take) continue;
-        const uint64_t oid = first + ch * 32 + lane;
-        const bool valid = oid < a.n;
-        const int c = valid ? cnt[ch * 32 + lane] : 0;
-        if (valid && c > a.qS) atomicExch(a.err, DEV_BAD_QUEUE);  // cannot come from this layout
-        int x = c;  // inclusive prefix sum of the counts over the warp
+  any |= __shfl_xor_sync(0xffffffffu, any, 1);
+  any |= __shfl_xor_sync(0xffffffffu, any, 2);
+  if (cell < f.cells.n && (t & 3u) == 0) {
+    unsigned w = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int y = __shfl_up_sync(0xffffffffu, x, o);
-          if (lane >= o) x += y;
-        }
-        const uint32_t total = min((uint32_t)__shfl_sync(0xffffffffu, x, 31), 32u * QS);
-        const uint32_t *sp = spots + base[ch];
-        // hit bits of the chunk's spots, four 32-spot windows per step
-        for (uint32_t w0 = 0; w0 < total; w0 += 128) {
-          bool h[4];
-#pragma unroll
-          for (int u = 0; u < 4; u++) {
-            const uint32_t k = w0 + 32u * (uint32_t)u + (uint32_t)lane;
-            h[u] = false;
-            if (k < total) {
-              const uint32_t q = sp[k] >> sh;
-              h[u] = (cm[q >> 5] >> (q & 31u)) & 1u;
-            }
-          }
-          unsigned bw[4];
-#pragma unroll
-          for (int u = 0; u < 4; u++) bw[u] = __ballot_sync(0xffffffffu, h[u]);
-          if (lane == 0) {
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-              if (w0 + 32u * (uint32_t)u < total) wm[(w0 >> 5) + (uint32_t)u] = bw[u];
-          }
-        }
-        __syncwarp();
-        // this record's spots are [xs, xe) of the chunk: its marked ones
-        const uint32_t xe = min((uint32_t)x, total), xs = min((uint32_t)(x - c), total);
-        int ub = 0;
-        for (uint32_t w = xs >> 5; xe > xs && w <= (xe - 1) >> 5; w++) {
-          unsigned mw = wm[w];
-          const int lo = (int)xs - (int)(w << 5), hi = (int)xe - (int)(w << 5);
-          if (lo > 0) mw &= ~0u << lo;
-          if (hi < 32) mw &= (1u << hi) - 1u;
-          ub += __popc(mw);
-        }
-        const bool cand = valid && c <= a.qS && ub >= need;
-        const unsigned cmk = __ballot_sync(0xffffffffu, cand);
-        if (cmk) {
-          // the warp's places in the block's region, one reservation per
-          // chunk: an entry per candidate, and pixel room for all the chunk's
-          // spots, so a candidate's pixels go where its spots sit in the chunk
-          // (its count prefix; the room a region holds covers every spot)
-          uint32_t e0 = 0, p0 = 0;
-          if (lane == 0) {
-            e0 = atomicAdd(&ctr[0], (uint32_t)__popc(cmk));
-            p0 = atomicAdd(&ctr[1], total);
-          }
-          e0 = __shfl_sync(0xffffffffu, e0, 0);
-          p0 = __shfl_sync(0xffffffffu, p0, 0);
-          if (cand) {
-            const uint64_t e = (uint64_t)e0 + (uint64_t)__popc(cmk & lt);
-            const uint64_t off = (uint64_t)p0 + (uint64_t)xs;
-            if (e < e_cap && off + (uint64_t)ub <= p_cap) {
-              CandEntry ce;
-              ce.oid = oid;
-              ce.off = (uint32_t)off;
-              ce.n = (uint32_t)ub;
-              E[e] = ce;
-              uint32_t k = 0;  // its marked pixels in record order (none when xe == xs)
-              for (uint32_t w = xs >> 5; xe > xs && w <= (xe - 1) >> 5; w++) {
-                unsigned mw = wm[w];
-                const int lo = (int)xs - (int)(w << 5), hi = (int)xe - (int)(w << 5);
-                if (lo > 0) mw &= ~0u << lo;
-                if (hi < 32) mw &= (1u << hi) - 1u;
-                while (mw) {
-                  const int b = __ffs(mw) - 1;
-                  mw &= mw - 1;
-                  P[off + k++] = sp[(w << 5) + (uint32_t)b];
-                }
-              }
-            } else {
-              atomicExch(a.err, DEV_BAD_QUEUE);  // regions hold every record: cannot happen
-            }
-          }
-        }
-        __syncwarp();
-      }
-    }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[s]);
-  }
-  // the last consumer warp to finish publishes the block's counts
-  __syncwarp();
-  if (lane == 0) {
-    __threadfence_block();
-    if (atomicAdd(&ctr[2], 1u) == (uint32_t)NC - 1) {
-      a.cq_count[2 * blockIdx.x] = atomicAdd(&ctr[0], 0u);
-      a.cq_count[2 * blockIdx.x + 1] = atomicAdd(&ctr[1], 0u);
-    }
+    for (int g = 0; g < kMaskGroups; g++) w |= (any & f.group[g]) ? 1u << g : 0u;
+    f.mask[cell] = (uint16_t)w;
   }
 }
 
-// The filter's candidates, 32 per warp: the per-record logic of the other
-// variants over each candidate's marked pixels.  blockIdx.y = the filter
-// block whose region is read.
-template <int B>
-__global__ void __launch_bounds__(256) cell_count_kernel(const __grid_constant__ CmpArgs a) {
-  const uint32_t b = blockIdx.y;
-  const uint64_t cap = a.cq_ebase[b + 1] - a.cq_ebase[b];
-  const uint64_t n = min((uint64_t)a.cq_count[2 * b], cap);
-  const CandEntry *E = a.cq_e + a.cq_ebase[b];
-  const uint32_t *P = a.cq_pix + a.cq_pbase[b];
-  const int lane = threadIdx.x & 31;
-  const uint64_t wpb = blockDim.x >> 5;
-  const uint64_t nw = gridDim.x * wpb;
-  const uint64_t pol_occ = l2_evict_last();
-  for (uint64_t g = (blockIdx.x * wpb + (threadIdx.x >> 5)) * 32; g < n; g += nw * 32) {
-    const uint64_t e = g + lane;
-    const bool v = e < n;
-    CandEntry ce{0ull, 0u, 0u};
-    if (v) ce = E[e];
-    process<B, ListSpots, 1>(a, ListSpots{P + ce.off}, v ? (int)ce.n : 0, ce.oid, pol_occ, v);
+__device__ __forceinline__ uint2 ld_stream8(const uint2 *p) {
+  uint2 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  return v;
+}
+
+// NB counter bits per half word: 5 hold 16 spots a half (records of up to 32
+// spots), 8 hold 128 (up to 255).
+template <int NB>
+struct SlicedCount {
+  unsigned z[NB];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int b = 0; b < NB; b++) z[b] = 0u;
   }
+  // a full adder of z[0], p and q, its carry through the rest
+  __device__ __forceinline__ void add2(unsigned p, unsigned q) {
+    unsigned c = (z[0] & p) | (z[0] & q) | (p & q);
+    z[0] ^= p ^ q;
+#pragma unroll
+    for (int b = 1; b < NB; b++) {
+      const unsigned t = z[b] & c;
+      z[b] ^= c;
+      c = t;
+    }
+  }
+  // groups whose two halves add up to at least need (bits 0..15)
+  __device__ __forceinline__ unsigned reached(unsigned need) const {
+    unsigned s[NB + 1], c = 0u;
+#pragma unroll
+    for (int b = 0; b < NB; b++) {
+      const unsigned x = z[b], y = z[b] >> 16;
+      s[b] = x ^ y ^ c;
+      c = (x & y) | (c & (x | y));
+    }
+    s[NB] = c;
+    unsigned gt = 0u, eq = ~0u;
+#pragma unroll
+    for (int b = NB; b >= 0; b--) {
+      const unsigned n = (need >> b) & 1u ? ~0u : 0u;
+      gt |= eq & s[b] & ~n;
+      eq &= ~(s[b] ^ n);
+    }
+    return (gt | eq) & 0xFFFFu;
+  }
+};
+
+constexpr int kFilterWarps = 32;
+constexpr int kAhead = 8;  // groups of four spots held in registers (32 spots)
+
+// Persistent: one block per SM, its warps take every grid-th chunk of 32 records
+// and load the next chunk's codes before they count the present one's.
+template <int NB>
+__global__ void __launch_bounds__(32 * kFilterWarps, 1)
+    group_filter_kernel(const __grid_constant__ FilterArgs f) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ uint32_t found;
+  const uint32_t mask_bytes = (f.cells.n * 2u + 15u) & ~15u;
+  const uint16_t *cm = reinterpret_cast<const uint16_t *>(smem);
+  const GroupBucket *tab = reinterpret_cast<const GroupBucket *>(smem + mask_bytes);
+  {
+    const uint4 *src = reinterpret_cast<const uint4 *>(f.mask);  // padded to 16 bytes
+    uint4 *dst = reinterpret_cast<uint4 *>(smem);
+    for (uint32_t i = threadIdx.x; i < mask_bytes / 16; i += blockDim.x) dst[i] = src[i];
+    const uint4 *ts = reinterpret_cast<const uint4 *>(f.tab);
+    uint4 *td = reinterpret_cast<uint4 *>(smem + mask_bytes);
+    for (uint32_t i = threadIdx.x; i < (uint32_t)f.nb * 2u; i += blockDim.x) td[i] = ts[i];
+    if (threadIdx.x == 0) found = 0u;
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const uint32_t step = gridDim.x * kFilterWarps;
+  uint32_t ch = blockIdx.x * kFilterWarps + (threadIdx.x >> 5);
+  uint32_t *out = f.cand + (uint64_t)blockIdx.x * filter_region(f.nchunks, gridDim.x);
+  int bi = 0;
+  uint2 next[kAhead];
+  GroupBucket nb{};
+  auto load = [&]() {
+    while (ch >= tab[bi].chunk_end) bi++;
+    nb = tab[bi];
+    const int groups = (int)(nb.c + 3) / 4;
+    const uint2 *src = f.codes + nb.code0 + (uint64_t)(ch - nb.chunk0) * groups * 32 + lane;
+#pragma unroll
+    for (int g = 0; g < kAhead; g++)
+      if (g < groups) next[g] = ld_stream8(src + g * 32);
+  };
+  if (ch < f.nchunks) load();
+  while (ch < f.nchunks) {
+    uint2 v[kAhead];
+#pragma unroll
+    for (int g = 0; g < kAhead; g++) v[g] = next[g];
+    const uint32_t at = (ch - nb.chunk0) * 32u + (uint32_t)lane;
+    const uint32_t nrec = nb.nrec, pos0 = nb.pos0;
+    const int c = (int)nb.c, groups = (c + 3) / 4;
+    const uint2 *src = f.codes + nb.code0 + (uint64_t)(ch - nb.chunk0) * groups * 32 + lane;
+    ch += step;
+    if (ch < f.nchunks) load();
+    SlicedCount<NB> sc;
+    sc.clear();
+    auto four = [&](uint2 u, int g) {
+      unsigned p = __byte_perm(cm[u.x & 0xFFFFu], cm[u.x >> 16], 0x5410);
+      unsigned q = __byte_perm(cm[u.y & 0xFFFFu], cm[u.y >> 16], 0x5410);
+      if (g == groups - 1) {  // spots past the record's last one
+        const int r = c - 4 * g;
+        if (r < 2) p &= 0xFFFFu;
+        q = r < 3 ? 0u : r < 4 ? q & 0xFFFFu : q;
+      }
+      sc.add2(p, q);
+    };
+#pragma unroll
+    for (int g = 0; g < kAhead; g++) {
+      if (g >= groups) break;
+      four(v[g], g);
+    }
+    if (NB > 5)
+      for (int g = kAhead; g < groups; g++) four(ld_stream8(src + (uint64_t)g * 32), g);
+    const bool keep = at < nrec && sc.reached(f.need) != 0u;
+    const unsigned km = __ballot_sync(0xffffffffu, keep);
+    if (km) {
+      uint32_t base = 0;
+      if (lane == 0) base = atomicAdd(&found, (uint32_t)__popc(km));
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (keep) out[base + __popc(km & ((1u << lane) - 1u))] = pos0 + at;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) f.cand_cnt[blockIdx.x] = found;
+}
+
+template <int NB>
+static int launch_filter(const FilterArgs &f, size_t smem, cudaStream_t st) {
+  const int rc = ensure_smem((const void *)group_filter_kernel<NB>, (int)smem);
+  if (rc) return rc;
+  group_filter_kernel<NB><<<f.grid, 32 * kFilterWarps, smem, st>>>(f);
+  LMB_CUDA(cudaGetLastError());
+  return LMB_OK;
+}
+
+int filter_launch(const FilterArgs &f, cudaStream_t st) {
+  LMB_REQUIRE(f.cells.n >= 1 && f.cells.n <= 65536 && f.need >= 1 && f.grid >= 1 && f.nb >= 1,
+              "group filter: malformed arguments");
+  groupmask_kernel<<<(f.cells.n * 4 + 255) / 256, 256, 0, st>>>(f);
+  LMB_CUDA(cudaGetLastError());
+  const size_t smem = ((f.cells.n * 2u + 15u) & ~15u) + (size_t)f.nb * sizeof(GroupBucket);
+  return f.most_spots <= 32 ? launch_filter<5>(f, smem, st) : launch_filter<8>(f, smem, st);
+}
+
+// ----------------------------------------------------------------------------
+// Listed pass: the records perm[0, nlist), those with at least MinNrSpots
+// on-detector spots, or the filter's candidates, 32 per warp.  Each lane copies
+// its record's on-detector pixels into the warp's shared-memory rows (odd stride:
+// conflict-free), then the warp runs the per-record logic of the other variants
+// on them.
+// ----------------------------------------------------------------------------
+template <int B>
+__global__ void __launch_bounds__(256) listed_kernel(const __grid_constant__ CmpArgs a) {
+  extern __shared__ __align__(128) uint32_t rows[];
+  const int lane = threadIdx.x & 31;
+  const uint32_t SP = clist_queue_stride(a.qS);
+  uint32_t *wrows = rows + (threadIdx.x >> 5) * 32u * SP;
+  uint32_t *my = wrows + (uint32_t)lane * SP;
+  const uint64_t pol_occ = l2_evict_last();
+  const uint32_t *cand = a.cand ? a.cand + blockIdx.y * a.cand_region : nullptr;
+  const uint64_t n = a.cand ? a.cand_cnt[blockIdx.y] : a.nlist;
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); g < n; g += step) {
+    const bool v = g + lane < n;
+    const uint64_t oid = v ? a.perm[cand ? cand[g + lane] : g + lane] : 0;
+    int c = 0;
+    if (v) {
+      const uint16_t *rec = a.db + oid * (uint64_t)a.R;
+      const int stored = min((int)rec[0], a.S);
+#pragma unroll 4
+      for (int s = 0; s < stored; s++) {
+        const uint32_t x = rec[1 + 2 * s], y = rec[2 + 2 * s];
+        if (x < (uint32_t)a.W && y < (uint32_t)a.H && c < a.qS) my[c++] = y * (uint32_t)a.W + x;
+      }
+    }
+    process_rows<B>(a, wrows, SP, c, oid, pol_occ, v);
+  }
+}
+
+template <int B>
+static int launch_listed(const CmpArgs &a, dim3 grid, int threads, size_t smem, cudaStream_t st) {
+  const int rc = ensure_smem((const void *)listed_kernel<B>, (int)smem);
+  if (rc) return rc;
+  listed_kernel<B><<<grid, threads, smem, st>>>(a);
+  LMB_CUDA(cudaGetLastError());
+  return LMB_OK;
 }
 
 // ----------------------------------------------------------------------------
@@ -1347,21 +1483,7 @@ static int counter_bits(int S) {
 CompareTuning compare_config(int R, const CompareTuning &req) {
   CompareTuning c = req;
   const size_t rb = (size_t)R * 2;
-  if (c.variant == 5) {  // cell-mask filter + counting kernel: one filter block per SM
-    c.tile_sub = 0;
-    // stages (tiles in flight) and consumer warps, a multiple of them: the
-    // warps of a stage split its tiles' chunks; 25 warps at most
-    // (__launch_bounds__ of the kernel)
-    if (c.stages <= 0) c.stages = 12;
-    c.stages = std::max(1, std::min(c.stages, 16));
-    if (c.consumers <= 0) c.consumers = 2 * c.stages;
-    int cpt = std::max(1, c.consumers / c.stages);
-    while (cpt > 1 && c.stages * cpt > 24) cpt--;
-    c.consumers = c.stages * cpt;
-    c.blocks_per_sm = 1;
-    c.grid_mult = 1;
-    return c;
-  }
+  if (c.variant == 5) return c;  // grouped records: no launch shape to choose
   if (c.variant == 4) {  // compact layout + cell mask: one block per SM
     c.tile_sub = 0;
     if (c.consumers <= 0) c.consumers = 12;
@@ -1414,14 +1536,7 @@ static int launch_clist_bounded(const CmpArgs &a, unsigned grid, size_t smem, cu
 template <int B>
 static int launch_b(const CmpArgs &a, const CompareTuning &c, unsigned grid, size_t smem,
                     int nblk, cudaStream_t st) {
-  if (c.variant == 5) {
-    int rc = ensure_smem((const void *)cell_filter_kernel, (int)smem);
-    if (rc) return rc;
-    cell_filter_kernel<<<grid, 32 * (1 + c.consumers), smem, st>>>(a);
-    LMB_CUDA(cudaGetLastError());
-    // the counting kernel: four 256-thread blocks per filter block's region
-    cell_count_kernel<B><<<dim3(4, grid), 256, 0, st>>>(a);
-  } else if (c.variant == 4) {
+  if (c.variant == 4) {
     const int rc = ensure_smem((const void *)compare_cell_kernel<B>, (int)smem);
     if (rc) return rc;
     compare_cell_kernel<B><<<grid, 32 * (1 + c.consumers), smem, st>>>(a);
@@ -1451,30 +1566,12 @@ static int launch_b(const CmpArgs &a, const CompareTuning &c, unsigned grid, siz
 int compare_launch(CmpArgs a, const CompareTuning &req, int num_sms, cudaStream_t st) {
   LMB_REQUIRE((reinterpret_cast<uintptr_t>(a.db) & 15) == 0,
               "DB device pointer must be 16-byte aligned");
+  LMB_REQUIRE(req.variant != 5, "variant 5 runs over the grouped records");
   CompareTuning c = compare_config(a.R, req);
   a.test_consumer_wait_ns = (uint64_t)std::max(0, c.test_consumer_wait_us) * 1000ull;
   LMB_REQUIRE(!a.test_consumer_wait_ns || c.variant == 2 || c.variant == 4,
               "the test wait applies to variants 2 and 4");
   size_t fixed = 256;  // barriers
-  if (c.variant == 5) {
-    // barriers and block counters, the cell mask, and per consumer warp one
-    // ring stage (set below) and its window words
-    LMB_REQUIRE(a.cellmask && a.cm_bytes > 0 && a.cm_bytes % 128 == 0 &&
-                    a.cm_bytes <= kCellMaskBytes && (reinterpret_cast<uintptr_t>(a.cellmask) & 15) == 0,
-                "cell mask missing or malformed");
-    LMB_REQUIRE(a.cq_e && a.cq_pix && a.cq_ebase && a.cq_pbase && a.cq_count,
-                "candidate buffer missing");
-    LMB_REQUIRE(a.qS >= 1 && a.qS <= a.S, "filter windows for %d spots per record", a.qS);
-    LMB_REQUIRE(!c.test_consumer_wait_us, "the test wait applies to variants 2 and 4");
-    // fewer stages (keeping the warps per stage) until the ring fits
-    const int cpt = c.consumers / c.stages;
-    while (c.stages > 1 && 384 + (size_t)a.cm_bytes + (size_t)c.stages * a.tile_bytes +
-                                   (size_t)c.stages * cpt * filter_warp_bytes(a.qS) >
-                               227 * 1024)
-      c.stages--;
-    c.consumers = c.stages * cpt;
-    fixed = 384 + a.cm_bytes + (size_t)c.consumers * filter_warp_bytes(a.qS);
-  }
   if (c.variant == 4) {
     // the cell mask, and per consumer warp its hit list and window words; as
     // many consumer warps as leave room for a two-stage ring
@@ -1491,7 +1588,7 @@ int compare_launch(CmpArgs a, const CompareTuning &req, int num_sms, cudaStream_
     fixed += a.cm_bytes + (size_t)c.consumers * per_warp;
   }
   a.consumers = c.consumers;
-  if (c.variant == 2 || c.variant == 4 || c.variant == 5) {
+  if (c.variant == 2 || c.variant == 4) {
     // a.cl_tiles tiles of a.tile_bytes come from the compact layout; every
     // tile, the last included, is one bulk copy
     LMB_REQUIRE(a.cl && a.cl_tiles > 0 && a.tile_bytes > 0 && a.tile_bytes % 128 == 0,
@@ -1507,13 +1604,8 @@ int compare_launch(CmpArgs a, const CompareTuning &req, int num_sms, cudaStream_
     const size_t room = 227 * 1024 > 256 + qbytes ? 227 * 1024 - 256 - qbytes : 0;
     // barrier 15 is the test wait's when one is set
     const int fit = (int)std::min<size_t>(a.test_consumer_wait_ns ? 15 : 16, room / a.tile_bytes);
-    if (c.variant == 5) {  // one stage per consumer warp, sized above
-      LMB_REQUIRE(c.stages >= 1 && c.stages <= fit && c.stages <= 16,
-                  "compact tiles of %u bytes leave no room for the filter's stages", a.tile_bytes);
-    } else {
-      LMB_REQUIRE(fit >= 2, "compact tiles of %u bytes leave no room for a ring", a.tile_bytes);
-      c.stages = c.stages > 0 ? std::min(c.stages, fit) : fit;
-    }
+    LMB_REQUIRE(fit >= 2, "compact tiles of %u bytes leave no room for a ring", a.tile_bytes);
+    c.stages = c.stages > 0 ? std::min(c.stages, fit) : fit;
   } else {
     a.tile_sub = c.tile_sub;
     a.tile = (uint32_t)c.tile_sub * 32;
@@ -1530,8 +1622,6 @@ int compare_launch(CmpArgs a, const CompareTuning &req, int num_sms, cudaStream_
   const int mult = c.grid_mult > 0 ? c.grid_mult : 1;
   const unsigned grid = (unsigned)std::min<uint64_t>(
       a.ntiles, (uint64_t)num_sms * c.blocks_per_sm * (uint64_t)mult);
-  LMB_REQUIRE(c.variant != 5 || grid == a.cq_blocks,
-              "candidate regions laid out for %u filter blocks, grid of %u", a.cq_blocks, grid);
   const int B = counter_bits(a.S);
   // six to eight 128-thread compact-pass blocks per SM (the tuned shapes) get
   // a kernel whose registers are bounded for that occupancy
@@ -1543,6 +1633,22 @@ int compare_launch(CmpArgs a, const CompareTuning &req, int num_sms, cudaStream_
   if (B <= 9) return launch_b<9>(a, c, grid, smem, nblk, st);
   if (B <= 11) return launch_b<11>(a, c, grid, smem, nblk, st);
   return launch_b<16>(a, c, grid, smem, nblk, st);
+}
+
+int listed_launch(CmpArgs a, int num_sms, cudaStream_t st) {
+  LMB_REQUIRE(a.qS >= 1 && a.qS <= 255, "listed pass rows of %d spots", a.qS);
+  if ((a.nlist == 0 && !a.cand) || a.active == 0) return LMB_OK;
+  // 8 warps' rows per block (255 spots: 4 warps), at most 32 KiB at 30 spots
+  const int threads = a.qS <= 127 ? 256 : 128;
+  const size_t smem = (size_t)threads * clist_queue_stride(a.qS) * sizeof(uint32_t);
+  // candidates: eight blocks share the region of one filter block
+  const dim3 grid = a.cand ? dim3(8, a.cand_blocks)
+                           : dim3((unsigned)std::min<uint64_t>((a.nlist + threads - 1) / threads,
+                                                               (uint64_t)num_sms * 8));
+  const int B = counter_bits(a.qS);
+  if (B <= 3) return launch_listed<3>(a, grid, threads, smem, st);
+  if (B <= 5) return launch_listed<5>(a, grid, threads, smem, st);
+  return launch_listed<8>(a, grid, threads, smem, st);
 }
 
 // Zero the survivor and pass counters of the pass's slots only: the counters

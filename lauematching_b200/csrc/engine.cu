@@ -46,9 +46,12 @@ struct PassKey {
   int min_spots = 0;
   double min_int = 0;
   int mode = 0;
+  bool listed = false;  // over the listed records that can pass, not a layout of all
+  bool filter = false;  // ... of those the ones that the filter keeps
   CompareTuning tuning{};
   bool operator==(const PassKey &o) const {
-    return mask == o.mask && min_spots == o.min_spots &&
+    return mask == o.mask && min_spots == o.min_spots && listed == o.listed &&
+           filter == o.filter &&
            memcmp(&min_int, &o.min_int, sizeof(double)) == 0 && mode == o.mode &&
            memcmp(&tuning, &o.tuning, sizeof(CompareTuning)) == 0;
   }
@@ -77,17 +80,22 @@ struct lmb_engine {
   int cl_state = 0;  // 0 not built, 1 built, -1 this DB cannot use it
   unsigned long long cl_hist[256] = {};  // records per on-detector spot count
   int cl_qs = 0;  // largest on-detector spot count of a record (sizes the pass's queues)
-  // per tile of the compact layout: its chunks and its spots (sizes the
-  // variant-5 candidate regions: at most every record and spot of a tile)
-  std::vector<uint32_t> cl_tile_nch;
-  std::vector<uint64_t> cl_tile_spots;
-  // variant 5: candidate buffer, per filter block a region of entries and one
-  // of pixels (bases [G+1] each, in one allocation), counts written per block
-  CandEntry *d_cq_e = nullptr;
-  uint32_t *d_cq_pix = nullptr;
-  uint64_t *d_cq_base = nullptr;
-  uint32_t *d_cq_count = nullptr;
-  uint32_t cq_blocks = 0;
+  // records grouped by falling on-detector spot count (built on first use)
+  uint32_t *d_perm = nullptr;
+  int gl_state = 0;  // 0 not built, 1 built, -1 this DB cannot use it
+  unsigned long long gl_hist[256] = {};  // records per on-detector spot count
+  int gl_qs = 0;                         // largest on-detector spot count
+  bool on_detector = false;  // every stored spot is on the detector (a DB built here)
+  // variant 5 (built on first use): cell codes of the grouped records, their
+  // buckets by falling count (host and device), the mask of a pass, the filter's
+  // candidates (a region per block) and their counts
+  std::vector<GroupBucket> gl_tab;
+  uint2 *d_codes = nullptr;
+  GroupBucket *d_gl_tab = nullptr;
+  uint16_t *d_group_mask = nullptr;
+  uint32_t *d_cand = nullptr, *d_cand_cnt = nullptr;
+  GroupCells cells{};
+  uint64_t gl_bytes = 0;  // perm and codes
   // image slots
   uint8_t *d_u8 = nullptr;
   double *d_f64 = nullptr;  // allocated on first keep_f64 load
@@ -149,54 +157,23 @@ struct lmb_engine {
 
 namespace {
 
-void free_candidates(lmb_engine *e) {
-  cudaFree(e->d_cq_e);
-  cudaFree(e->d_cq_pix);
-  cudaFree(e->d_cq_base);
-  cudaFree(e->d_cq_count);
-  e->d_cq_e = nullptr;
-  e->d_cq_pix = nullptr;
-  e->d_cq_base = nullptr;
-  e->d_cq_count = nullptr;
-  e->cq_blocks = 0;
-}
-
-// The variant-5 candidate buffer for a filter grid of G blocks (block b takes
-// tiles b, b + G, ...): per block room for every record and every spot of its
-// tiles, so the filter cannot run out of room whatever the frames.  Made
-// before the first such pass (never inside a captured pass).
-int ensure_candidates(lmb_engine *e, uint32_t G) {
-  if (e->d_cq_e && e->cq_blocks == G) return LMB_OK;
-  free_candidates(e);
-  std::vector<uint64_t> base(2 * ((size_t)G + 1), 0);
-  uint64_t *eb = base.data(), *pb = base.data() + G + 1;
-  for (uint64_t t = 0; t < e->cl_tiles; t++) {
-    const uint64_t b = t % G;
-    eb[b + 1] += 32ull * e->cl_tile_nch[t];
-    pb[b + 1] += e->cl_tile_spots[t];
-  }
-  for (uint32_t b = 0; b < G; b++) {
-    eb[b + 1] += eb[b];
-    pb[b + 1] += pb[b];
-  }
-  LMB_REQUIRE(pb[G] < (1ull << 40), "candidate pixel buffer too large");
-  for (uint32_t b = 0; b < G; b++)
-    LMB_REQUIRE(pb[b + 1] - pb[b] < (1ull << 32), "candidate region of block %u too large", b);
-  cudaError_t ce = cudaMalloc(&e->d_cq_e, std::max<uint64_t>(eb[G], 1) * sizeof(CandEntry));
-  if (ce == cudaSuccess)
-    ce = cudaMalloc(&e->d_cq_pix, std::max<uint64_t>(pb[G], 1) * sizeof(uint32_t));
-  if (ce == cudaSuccess) ce = cudaMalloc(&e->d_cq_base, base.size() * sizeof(uint64_t));
-  if (ce == cudaSuccess) ce = cudaMalloc(&e->d_cq_count, 2ull * G * sizeof(uint32_t));
-  if (ce == cudaSuccess)
-    ce = cudaMemcpy(e->d_cq_base, base.data(), base.size() * sizeof(uint64_t),
-                    cudaMemcpyHostToDevice);
-  if (ce == cudaSuccess) ce = cudaMemset(e->d_cq_count, 0, 2ull * G * sizeof(uint32_t));
-  if (ce != cudaSuccess) {
-    free_candidates(e);
-    return cuda_fail(ce, "variant-5 candidate buffer", __FILE__, __LINE__);
-  }
-  e->cq_blocks = G;
-  return LMB_OK;
+void free_grouped(lmb_engine *e) {
+  cudaFree(e->d_perm);
+  cudaFree(e->d_codes);
+  cudaFree(e->d_gl_tab);
+  cudaFree(e->d_group_mask);
+  cudaFree(e->d_cand);
+  cudaFree(e->d_cand_cnt);
+  e->d_perm = nullptr;
+  e->d_codes = nullptr;
+  e->d_gl_tab = nullptr;
+  e->d_group_mask = nullptr;
+  e->d_cand = nullptr;
+  e->d_cand_cnt = nullptr;
+  e->gl_tab.clear();
+  e->gl_state = 0;
+  e->gl_qs = 0;
+  e->gl_bytes = 0;
 }
 
 int check_engine(lmb_engine *e) {
@@ -215,10 +192,7 @@ void free_engine(lmb_engine *e) {
   if (e->ld) cudaStreamSynchronize(e->ld);
   cudaFree(e->d_db);
   cudaFree(e->d_cl);
-  cudaFree(e->d_cq_e);
-  cudaFree(e->d_cq_pix);
-  cudaFree(e->d_cq_base);
-  cudaFree(e->d_cq_count);
+  free_grouped(e);
   cudaFree(e->d_u8);
   cudaFree(e->d_f64);
   cudaFree(e->d_occ);
@@ -320,7 +294,8 @@ int alloc_db(lmb_engine *e, uint64_t n) {
   e->cl_state = 0;
   e->cl_bytes = 0;
   e->cl_qs = 0;
-  free_candidates(e);
+  free_grouped(e);
+  e->on_detector = false;
   const size_t bytes = (size_t)n * e->R * 2;
   const size_t alloc = ((bytes + 255) / 256) * 256 + 256;
   LMB_CUDA(cudaMalloc(&e->d_db, alloc));
@@ -442,22 +417,30 @@ int try_sparse(lmb_engine *e, const T *px, int slot, int dtype, bool *sparse) {
   return LMB_OK;
 }
 
-// Automatic variant.  Each spot the pass gathers costs the same in both
-// layouts; what the compact layout saves is the stream of the records'
-// padding.  Measured on B200 at 1e8 records (two detector geometries, K=64),
-// the compact pass is as fast or faster while the records that can pass
-// (at least min_spots on-detector spots) hold up to ~3 spots per DB record
-// on average, and up to 1.4x slower beyond (dense records, where the
-// reference records' stream is no longer the cost).
+// Automatic variant over the grouped records: a pass whose listed records hold
+// more spots than this filters them first.  Measured on B200 (compare stage, one
+// slot, 64 within 2 us of it), listed / filtered: 1.05 M spots 16.4 / 26.6 us,
+// 1.5 M (15 per record) 20.4 / 28.7, 2.1 M (4 per record) 30.7 / 26.6, 3.0 M 30.7 to
+// 41.0 / 28.6 to 30.7; at 113 M (1e8 hexagonal orientations, 32 slots) 920 / 184.
+constexpr double kFilterSpots = 2e6;
+// What last_variant reports for the automatic variant: 2 while the records that
+// can pass hold at most this many spots per DB record, 5 beyond.  Without grouped
+// records it is also where the compact layout's pass gives way to the reference
+// records' (1e8 records, K = 64, 3.1 spots per record: 4.74 / 4.90 ms; 6.7: 6.55 /
+// 5.34 ms).
 constexpr double kAutoGather = 3.0;
-// the cell-mask pass the automatic variant runs beyond that
-constexpr int kAutoCellVariant = 5;
 
-double gathered_per_record(const lmb_engine *e, int min_spots) {
+double gathered_per_record(const lmb_engine *e, const unsigned long long *hist, int min_spots) {
   const int m = std::max(0, min_spots);
   double g = 0;
-  for (int c = m; c < 256; c++) g += (double)c * (double)e->cl_hist[c];
+  for (int c = m; c < 256; c++) g += (double)c * (double)hist[c];
   return e->n ? g / (double)e->n : 0.0;
+}
+// Records with at least min_spots on-detector spots: the first of d_perm.
+uint64_t listed_records(const lmb_engine *e, int min_spots) {
+  uint64_t k = 0;
+  for (int c = std::max(0, min_spots); c < 256; c++) k += e->gl_hist[c];
+  return k;
 }
 
 // Tile size of the compact layout of a dense DB (one whose passes run the
@@ -508,7 +491,7 @@ int build_compact(lmb_engine *e, int min_spots) {
   auto round128 = [](uint64_t b) { return ((b + 127) / 128) * 128; };
   const uint64_t avg_chunk = 36 + (4 * total_spots + nch - 1) / nch;
   uint64_t TB = std::min<uint64_t>(24 * 1024, std::max<uint64_t>(4096, round128(64 * avg_chunk)));
-  if (gathered_per_record(e, min_spots) > kAutoGather) {
+  if (gathered_per_record(e, e->cl_hist, min_spots) > kAutoGather) {
     // the automatic variant will run the cell-mask filter over it: its tile
     // size, whatever the tuning of this pass
     TB = kCellTileBytes;
@@ -571,20 +554,143 @@ int build_compact(lmb_engine *e, int min_spots) {
   e->cl_stage = (uint32_t)TB;
   e->cl_bytes = total;
   e->cl_state = 1;
-  e->cl_tile_nch = tnch;
-  e->cl_tile_spots.assign(nt, 0);
-  for (uint64_t c = 0; c < nch; c++) e->cl_tile_spots[ctile[c]] += cs[c];
   return LMB_OK;
 }
 
 
-// The cell-mask pass needs its mask, a hit list per consumer warp and a
-// two-stage ring of the layout's tiles in one block's shared memory.
-bool cell_pass_fits(const lmb_engine *e) {
-  const size_t need = 256 + (size_t)e->cm_bytes +
-                      cell_warp_bytes(e->cl_qs > 0 ? e->cl_qs : e->S, e->tuning.cell_queue) +
-                      2 * (size_t)e->cl_stage;
-  return e->d_cellmask && need <= 227 * 1024;
+// Group the resident records by on-detector spot count (glist.cu), on the
+// device alone.  A DB that cannot be grouped (S > 255, 2^32 records or more, no
+// memory for 4 bytes per record) keeps the other layouts.
+int build_grouped(lmb_engine *e) {
+  e->gl_state = -1;
+  if (e->S > 255 || e->n == 0 || e->n >= (1ull << 32)) return LMB_OK;
+  const uint64_t n = e->n, nt = glist_tiles(n);
+  const size_t hist_bytes = 256 * sizeof(unsigned long long);
+  unsigned char *d_aux = nullptr;  // histogram, per-tile counts, counts
+  cudaError_t ce = cudaMalloc(&d_aux, hist_bytes + nt * 256 * sizeof(uint32_t) + n);
+  if (ce == cudaSuccess) ce = cudaMalloc(&e->d_perm, n * sizeof(uint32_t));
+  if (ce != cudaSuccess) {
+    cudaGetLastError();
+    cudaFree(d_aux);
+    e->d_perm = nullptr;
+    return ce == cudaErrorMemoryAllocation ? LMB_OK
+                                           : cuda_fail(ce, "grouped records", __FILE__, __LINE__);
+  }
+  unsigned long long *d_hist = reinterpret_cast<unsigned long long *>(d_aux);
+  uint32_t *d_bh = reinterpret_cast<uint32_t *>(d_aux + hist_bytes);
+  uint8_t *d_cnt = d_aux + hist_bytes + nt * 256 * sizeof(uint32_t);
+  int rc = glist_count_launch(e->d_db, n, e->R, e->S, e->geo.nr_px_x, e->geo.nr_px_y, e->on_detector,
+                              d_cnt, d_bh, d_hist, e->st);
+  if (rc == LMB_OK) rc = glist_scatter_launch(d_cnt, n, d_bh, e->d_perm, e->st);
+  if (rc == LMB_OK) {
+    ce = cudaMemcpyAsync(e->gl_hist, d_hist, hist_bytes, cudaMemcpyDeviceToHost, e->st);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->st);
+    if (ce != cudaSuccess) rc = cuda_fail(ce, "grouped records", __FILE__, __LINE__);
+  }
+  cudaFree(d_aux);
+  if (rc) {
+    cudaFree(e->d_perm);
+    e->d_perm = nullptr;
+    return rc;
+  }
+  e->gl_qs = 1;
+  for (int c = 255; c >= 1; c--)
+    if (e->gl_hist[c]) {
+      e->gl_qs = c;
+      break;
+    }
+  e->gl_bytes = n * sizeof(uint32_t);
+  e->gl_state = 1;
+  return LMB_OK;
+}
+
+// What variant 5 needs besides the grouped records: buckets, cell codes, mask
+// and room for every record as a candidate (4 bytes each).  false: no memory.
+int ensure_filter(lmb_engine *e, bool *ok) {
+  *ok = e->d_codes != nullptr;
+  if (*ok) return LMB_OK;
+  e->cells = group_cells(e->geo.nr_px_x, e->geo.nr_px_y);
+  e->gl_tab.clear();
+  uint32_t chunk = 0, pos = 0;
+  uint64_t code = 0;
+  for (int c = e->gl_qs; c >= 1; c--) {
+    const uint32_t nrec = (uint32_t)e->gl_hist[c], nch = (nrec + 31) / 32;
+    if (!nrec) continue;
+    e->gl_tab.push_back(GroupBucket{chunk + nch, chunk, pos, nrec, code, (uint32_t)c, 0});
+    chunk += nch;
+    pos += nrec;
+    code += (uint64_t)nch * ((c + 3) / 4) * 32;
+  }
+  if (e->gl_tab.empty()) return LMB_OK;  // no record has a spot
+  const uint32_t grid = (uint32_t)e->num_sms;
+  cudaError_t ce = cudaMalloc(&e->d_cand, grid * filter_region(chunk, grid) * sizeof(uint32_t));
+  if (ce == cudaSuccess) ce = cudaMalloc(&e->d_codes, code * sizeof(uint2));
+  if (ce == cudaSuccess) ce = cudaMalloc(&e->d_cand_cnt, grid * sizeof(uint32_t));
+  if (ce == cudaSuccess) ce = cudaMalloc(&e->d_group_mask, 65536 * sizeof(uint16_t));
+  if (ce == cudaSuccess) ce = cudaMalloc(&e->d_gl_tab, e->gl_tab.size() * sizeof(GroupBucket));
+  if (ce == cudaSuccess)
+    ce = cudaMemcpyAsync(e->d_gl_tab, e->gl_tab.data(), e->gl_tab.size() * sizeof(GroupBucket),
+                         cudaMemcpyHostToDevice, e->st);
+  int rc = LMB_OK;
+  for (size_t i = 0; i < e->gl_tab.size() && ce == cudaSuccess && rc == LMB_OK; i++)
+    rc = glist_code_launch(e->d_db, e->R, e->S, e->geo.nr_px_x, e->geo.nr_px_y, e->d_perm,
+                           e->gl_tab[i], e->cells, e->d_codes, e->st);
+  if (ce == cudaSuccess && rc == LMB_OK) ce = cudaStreamSynchronize(e->st);
+  if (ce != cudaSuccess || rc) {
+    cudaFree(e->d_cand);
+    cudaFree(e->d_codes);
+    cudaFree(e->d_cand_cnt);
+    cudaFree(e->d_group_mask);
+    cudaFree(e->d_gl_tab);
+    e->d_cand = e->d_cand_cnt = nullptr;
+    e->d_codes = nullptr;
+    e->d_group_mask = nullptr;
+    e->d_gl_tab = nullptr;
+    if (rc) return rc;
+    if (ce != cudaErrorMemoryAllocation) return cuda_fail(ce, "cell codes", __FILE__, __LINE__);
+    cudaGetLastError();
+    return LMB_OK;
+  }
+  e->gl_bytes += code * sizeof(uint2);
+  *ok = true;
+  return LMB_OK;
+}
+
+// The filter of one pass over the records with at least min_spots (>= 1) spots.
+int enqueue_filter(lmb_engine *e, const PassKey &k, CmpArgs *a) {
+  FilterArgs f{};
+  f.occ = e->d_occ;
+  f.W = e->geo.nr_px_x;
+  f.H = e->geo.nr_px_y;
+  f.cells = e->cells;
+  f.mask = e->d_group_mask;
+  // the pass's slots in turn into groups of equal size, give or take one
+  const int ns = __builtin_popcountll(k.mask);
+  for (int i = 0, r = 0; i < LMB_MAX_SLOTS; i++)
+    if (k.mask >> i & 1) {
+      f.group[ns <= kMaskGroups ? r : r * kMaskGroups / ns] |= 1ull << i;
+      r++;
+    }
+  f.codes = e->d_codes;
+  f.tab = e->d_gl_tab;
+  for (const GroupBucket &b : e->gl_tab)
+    if ((int)b.c >= k.min_spots) {
+      f.nb++;
+      f.nchunks = b.chunk_end;
+    }
+  f.need = (uint32_t)k.min_spots;
+  f.most_spots = e->gl_qs;
+  f.cand = e->d_cand;
+  f.cand_cnt = e->d_cand_cnt;
+  f.grid = std::min<uint32_t>((uint32_t)e->num_sms, (f.nchunks + 31) / 32);
+  const int rc = filter_launch(f, e->st);
+  if (rc) return rc;
+  a->nlist = 0;
+  a->cand = e->d_cand;
+  a->cand_cnt = e->d_cand_cnt;
+  a->cand_region = filter_region(f.nchunks, f.grid);
+  a->cand_blocks = f.grid;
+  return LMB_OK;
 }
 
 int enqueue_pass(lmb_engine *e, const PassKey &k, bool capturing) {
@@ -620,31 +726,33 @@ int enqueue_pass(lmb_engine *e, const PassKey &k, bool capturing) {
   a.pass_cnt = e->d_status + LMB_MAX_SLOTS;
   a.err = reinterpret_cast<int *>(e->d_status + 2 * LMB_MAX_SLOTS);
   a.full_gather = k.tuning.full_gather;
-  if (k.tuning.variant == 2 || k.tuning.variant >= 4) {
+  if (k.tuning.variant == 2 || k.tuning.variant == 4) {
     a.cl = e->d_cl;
     a.cl_tiles = e->cl_tiles;
     a.tile_bytes = e->cl_stage;
   }
-  if (k.tuning.variant >= 4) {
+  if (k.tuning.variant == 4) {
     a.cellmask = e->d_cellmask;
     a.cm_bytes = e->cm_bytes;
     a.cm_shift = e->cm_shift;
   }
-  if (k.tuning.variant == 5) {
-    a.cq_e = e->d_cq_e;
-    a.cq_pix = e->d_cq_pix;
-    a.cq_ebase = e->d_cq_base;
-    a.cq_pbase = e->d_cq_base + e->cq_blocks + 1;
-    a.cq_count = e->d_cq_count;
-    a.cq_blocks = e->cq_blocks;
-  }
   if (k.min_spots <= e->S && !std::isnan(k.min_int)) {
-    if (k.tuning.variant >= 4) {  // the cell mask of this pass's slots, then the pass
+    if (k.tuning.variant == 4) {  // the cell mask of this pass's slots, then the pass
       const int rc = cellmask_launch(e->d_occ, e->npx, k.mask, e->cm_shift, e->cm_bytes,
                                      e->d_cellmask, e->num_sms, e->st);
       if (rc) return rc;
     }
-    const int rc = compare_launch(a, k.tuning, e->num_sms, e->st);
+    if (k.listed) {  // nothing can pass when no record has that many spots
+      a.qS = e->gl_qs;
+      a.perm = e->d_perm;
+      a.nlist = k.min_spots <= e->gl_qs ? listed_records(e, a.full_gather ? 0 : k.min_spots) : 0;
+      if (k.filter && a.nlist) {
+        const int rc = enqueue_filter(e, k, &a);
+        if (rc) return rc;
+      }
+    }
+    const int rc = k.listed ? listed_launch(a, e->num_sms, e->st)
+                            : compare_launch(a, k.tuning, e->num_sms, e->st);
     if (rc) return rc;
   }
   LMB_CUDA(cudaEventRecordWithFlags(e->ev[1], e->st, evf));
@@ -818,6 +926,7 @@ static int db_build_common(lmb_engine *e, const double *orients, uint64_t seed, 
   }
   cudaFree(d_om);
   cudaFree(d_hkl);
+  e->on_detector = rc == LMB_OK;
   return rc;
 }
 
@@ -1169,32 +1278,42 @@ int lmb_match(lmb_engine *e, uint64_t slot_mask, int32_t min_nr_spots, double mi
   LMB_REQUIRE(value_mode == LMB_VALUE_U8 || (slot_mask & ~e->f64_mask) == 0,
               "float64 pass needs images loaded with keep_f64");
   CompareTuning tun = e->tuning;
-  if (tun.variant >= 2) {  // compact layout: derive it once per DB
+  // Grouped records: the automatic variant's form (and variant 5's) whenever a
+  // record needs spots to pass.  It lists the records that can pass, and filters
+  // the list by the frames' cells when it is long (variant 5: always).
+  bool listed = false, filter = false;
+  const bool some = min_nr_spots >= 1 && !tun.full_gather;
+  if (tun.variant == 5 || (tun.variant == 3 && some && !tun.test_consumer_wait_us)) {
+    LMB_REQUIRE(!tun.test_consumer_wait_us, "the test wait applies to variants 2 and 4");
+    if (e->gl_state == 0) {
+      rc = build_grouped(e);
+      if (rc) return rc;
+    }
+    listed = e->gl_state == 1;
+    if (listed) {
+      const double per_record = gathered_per_record(e, e->gl_hist, min_nr_spots);
+      if (some && (tun.variant == 5 || per_record * (double)e->n > kFilterSpots)) {
+        rc = ensure_filter(e, &filter);
+        if (rc) return rc;
+      }
+      // reported: 2 while the records that can pass hold few spots, 5 beyond
+      if (tun.variant == 3) tun.variant = per_record <= kAutoGather ? 2 : 5;
+    }
+  }
+  if (tun.variant >= 2 && !listed) {  // compact layout: derive it once per DB
     if (e->cl_state == 0) {
       rc = build_compact(e, min_nr_spots);
       if (rc) return rc;
     }
-    // variant 3 (automatic): the compact layout alone while the records that
-    // can pass hold few spots; beyond that, the compact layout filtered by
-    // the batch's cell mask (variant 4) when its hit lists fit a block, the
-    // reference records otherwise
-    bool compact = e->cl_state == 1;
+    // variant 3 (automatic) without grouped records: the compact layout while
+    // the records that can pass hold few spots, the reference records beyond
+    bool compact = e->cl_state == 1 && tun.variant != 5;
     if (compact && tun.variant == 3) {
-      if (gathered_per_record(e, tun.full_gather ? 0 : min_nr_spots) <= kAutoGather)
-        tun.variant = 2;
-      else if (!tun.full_gather && min_nr_spots >= 1 && cell_pass_fits(e))
-        tun = CompareTuning{kAutoCellVariant, 0, tun.cell_stages, tun.cell_consumers, 1, 1, 0,
-                            tun.test_consumer_wait_us, 0, 0, tun.cell_queue};  // cell-mask pass
-      else
-        compact = false;
+      tun.variant = 2;
+      compact = gathered_per_record(e, e->cl_hist, tun.full_gather ? 0 : min_nr_spots) <= kAutoGather;
     }
     if (!compact)  // warp-specialised over the reference records
       tun = CompareTuning{1, 0, 0, 0, 0, 0, tun.full_gather, tun.test_consumer_wait_us, 0, 0, 0};
-  }
-  if (tun.variant == 5) {  // its candidate regions, for the filter grid it will launch
-    const uint32_t G = (uint32_t)std::min<uint64_t>(e->cl_tiles, (uint64_t)e->num_sms);
-    rc = ensure_candidates(e, std::max<uint32_t>(G, 1));
-    if (rc) return rc;
   }
   e->last_variant = tun.variant;
   for (int k = 0; k < LMB_MAX_SLOTS; k++)
@@ -1207,6 +1326,8 @@ int lmb_match(lmb_engine *e, uint64_t slot_mask, int32_t min_nr_spots, double mi
   key.min_spots = min_nr_spots;
   key.min_int = min_intensity;
   key.mode = value_mode;
+  key.listed = listed;
+  key.filter = filter;
   key.tuning = tun;
   PassGraph *pg = nullptr;
   for (auto &g : e->graphs)
@@ -1417,8 +1538,9 @@ int lmb_engine_set_tuning(lmb_engine *e, const int32_t *fields, int32_t n_fields
 int lmb_engine_layout_info(lmb_engine *e, int32_t *compact, uint64_t *compact_bytes,
                            int32_t *tiles, int32_t *tile_bytes) {
   LMB_REQUIRE(e, "null engine");
-  if (compact) *compact = e->cl_state;
-  if (compact_bytes) *compact_bytes = e->cl_bytes;
+  const bool built = e->cl_state == 1 || e->gl_state == 1;
+  if (compact) *compact = built ? 1 : std::min(e->cl_state, e->gl_state);
+  if (compact_bytes) *compact_bytes = e->cl_bytes + e->gl_bytes;
   if (tiles) *tiles = (int32_t)e->cl_tiles;
   if (tile_bytes) *tile_bytes = (int32_t)e->cl_stage;
   return LMB_OK;

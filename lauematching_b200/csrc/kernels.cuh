@@ -6,15 +6,6 @@
 
 namespace lmb {
 
-// A record the cell filter kept: its id and its marked pixels (n of them at
-// offset off of its block's pixel region).
-struct CandEntry {
-  unsigned long long oid;
-  uint32_t off;
-  uint32_t n;
-};
-static_assert(sizeof(CandEntry) == 16, "candidate entry layout");
-
 // One batched DB pass (compare.cu).
 struct CmpArgs {
   const uint16_t *db;  // n records of R uint16, 16-byte aligned
@@ -55,17 +46,15 @@ struct CmpArgs {
   // spots) into a per-warp queue and counted 32 at a time; 0 = counted in
   // place, chunk by chunk
   int cell_queue;
-  // variant 5: records that can still pass after the cell mask, appended by
-  // the filter kernel to its block's region (entries at cq_e + cq_ebase[b],
-  // their marked pixels at cq_pix + cq_pbase[b]); cq_count[2b], [2b + 1] =
-  // entries and pixels the block wrote; the regions hold every record and
-  // spot of the block's tiles, so they cannot overflow
-  struct CandEntry *cq_e;
-  uint32_t *cq_pix;
-  const uint64_t *cq_ebase;
-  const uint64_t *cq_pbase;
-  uint32_t *cq_count;
-  uint32_t cq_blocks;  // the filter grid the regions were laid out for
+  // listed pass: the records perm[0, nlist) (grouped by falling spot count); or,
+  // after the filter (nlist = 0), perm[cand[b * cand_region + k]] for k below
+  // cand_cnt[b], b = blockIdx.y
+  const uint32_t *perm;
+  uint64_t nlist;
+  const uint32_t *cand;
+  const uint32_t *cand_cnt;
+  uint64_t cand_region;
+  uint32_t cand_blocks;
   // filled by compare_launch
   uint64_t full_tiles, ntiles;
   uint32_t tile_bytes;
@@ -79,7 +68,7 @@ struct CmpArgs {
 struct CompareTuning {
   int variant;        // 0 = block-barrier ring, 1 = warp-specialised, 2 = compact layout,
                       // 3 = automatic, 4 = compact layout + the batch's cell mask,
-                      // 5 = cell-mask filter kernel + candidate counting kernel
+                      // 5 = grouped records: filter by group masks, then count
   int tile_sub;       // 32-orientation sub-tiles per tile
   int stages;         // ring depth
   int consumers;      // consumer warps (variant 1)
@@ -227,14 +216,59 @@ __host__ __device__ __forceinline__ uint32_t cell_warp_bytes(int qS) {
 __host__ __device__ __forceinline__ uint32_t cell_warp_bytes(int qS, int queue) {
   return cell_warp_bytes(qS) + (queue ? clist_queue_bytes(qS) : 0u);
 }
-// Variant 5's filter kernel: per consumer warp the hit bits of up to qS
-// 32-spot windows.
-__host__ __device__ __forceinline__ uint32_t filter_warp_bytes(int qS) {
-  const uint32_t q = (uint32_t)(qS < 1 ? 1 : qS);
-  return (4u * q + 15u) / 16u * 16u;
-}
 int cellmask_launch(const unsigned long long *d_occ, uint64_t npx, unsigned long long active,
                     int shift, uint32_t cm_bytes, uint32_t *d_mask, int num_sms, cudaStream_t st);
+// Records grouped by on-detector spot count (glist.cu).
+constexpr uint32_t kGlTile = 4096;  // records per tile of the counting sort
+__host__ __device__ __forceinline__ uint32_t glist_tiles(uint64_t n) {
+  return (uint32_t)((n + kGlTile - 1) / kGlTile);
+}
+int glist_count_launch(const uint16_t *d_db, uint64_t n, int R, int S, int W, int H, bool on_detector,
+                       uint8_t *d_cnt, uint32_t *d_bh, unsigned long long *d_hist, cudaStream_t st);
+int glist_scatter_launch(const uint8_t *d_cnt, uint64_t n, const uint32_t *d_bh, uint32_t *d_perm,
+                         cudaStream_t st);
+int listed_launch(CmpArgs a, int num_sms, cudaStream_t st);
+
+// Cells of the group masks: cw x ch pixels, nx per row, n in all (at most 65536).
+struct GroupCells {
+  int cw, ch, nx, ny;
+  uint32_t n;
+};
+// The records of one spot count: perm[pos0, pos0 + nrec), chunks [chunk0,
+// chunk_end) of 32 of them, their codes from code0 on.  Ordered by falling count.
+struct GroupBucket {
+  uint32_t chunk_end, chunk0, pos0, nrec;
+  uint64_t code0;
+  uint32_t c, pad;
+};
+static_assert(sizeof(GroupBucket) == 32, "bucket layout");
+constexpr int kMaskGroups = 16;  // image groups of a mask word
+GroupCells group_cells(int W, int H);
+int glist_code_launch(const uint16_t *d_db, int R, int S, int W, int H, const uint32_t *d_perm,
+                      const GroupBucket &b, const GroupCells &cells, uint2 *d_codes, cudaStream_t st);
+
+// The filter over the grouped records (compare.cu).
+struct FilterArgs {
+  const unsigned long long *occ;
+  int W, H;
+  GroupCells cells;
+  uint16_t *mask;  // one 16-bit word per cell: bit g = a pixel of it is positive in a slot of group g
+  unsigned long long group[kMaskGroups];  // slots of each group
+  const uint2 *codes;
+  const GroupBucket *tab;
+  int nb;            // buckets of the records that can pass
+  uint32_t nchunks;  // their chunks
+  uint32_t need;     // MinNrSpots (>= 1)
+  int most_spots;    // largest count
+  uint32_t *cand;    // per block a region of positions in perm
+  uint32_t *cand_cnt;
+  uint32_t grid;     // blocks
+};
+// Positions a filter block can keep: its 32 warps' chunks of 32 records.
+__host__ __device__ __forceinline__ uint64_t filter_region(uint32_t nchunks, uint32_t grid) {
+  return 1024ull * ((nchunks + 32ull * grid - 1) / (32ull * grid));
+}
+int filter_launch(const FilterArgs &f, cudaStream_t st);
 int clist_fill_launch(const uint16_t *d_db, uint64_t n, int R, int S, int W, int H, uint32_t TB,
                       const uint32_t *d_ctile, const uint32_t *d_cpos, const uint32_t *d_cbase,
                       const uint32_t *d_tnch, unsigned char *d_cl, cudaStream_t st);
