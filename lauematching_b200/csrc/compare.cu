@@ -1105,7 +1105,7 @@ __global__ void __launch_bounds__(32 * 13, 1) compare_cell_kernel(const __grid_c
 // MinNrSpots spots can reach that count in some slot?
 //
 // The pass's slots are split into up to 16 groups (one slot each up to 16 slots,
-// up to four at 64), and every cell of the detector (8 x 8 pixels at 2048^2) has a
+// up to four at 64), and every cell of the detector (8 x 9 pixels at 2048^2) has a
 // 16-bit mask word: bit g says that a pixel of the cell is positive in a slot of
 // group g.  The words of all cells (at most 128 KiB) lie in each block's shared
 // memory.  A lane owns a record: it looks up the word of each of its spots and
@@ -1121,7 +1121,7 @@ GroupCells group_cells(int W, int H) {
   long cost = -1;
   for (int cw = 1; cw <= 256; cw++) {
     const int nx = (W + cw - 1) / cw;
-    const int rows = 65536 / nx;  // W <= 65535, so nx <= 65536
+    const int rows = 65535 / nx;  // W <= 65535; one 16-bit code is left for "no spot"
     if (rows < 1) continue;
     const int ch = (H + rows - 1) / rows;
     // cells that a spot of about 10 x 10 pixels marks, in pixels
@@ -1152,6 +1152,7 @@ __global__ void __launch_bounds__(256) groupmask_kernel(const __grid_constant__ 
   }
   any |= __shfl_xor_sync(0xffffffffu, any, 1);
   any |= __shfl_xor_sync(0xffffffffu, any, 2);
+  if (t == 0) f.mask[f.cells.n] = 0;  // the code of "no spot"
   if (cell < f.cells.n && (t & 3u) == 0) {
     unsigned w = 0;
 #pragma unroll
@@ -1166,58 +1167,59 @@ __device__ __forceinline__ uint2 ld_stream8(const uint2 *p) {
   return v;
 }
 
-// NB counter bits per half word: 5 hold 16 spots a half (records of up to 32
-// spots), 8 hold 128 (up to 255).
+__device__ __forceinline__ unsigned majority(unsigned x, unsigned y, unsigned z) {
+  return (x & y) | (x & z) | (y & z);
+}
+
+// Counts of 32 groups side by side, bit b of each in z[b]: the 16 groups of the
+// mask words in the low half, and again in the high half, which takes every other
+// spot.  The low half starts at 2^NB - need, so both halves together reach 2^NB
+// exactly when need spots have been counted: their carry out is the answer.
+// NB = 5 for records of up to 32 spots, 8 for up to 255.
 template <int NB>
 struct SlicedCount {
-  unsigned z[NB];
-  __device__ __forceinline__ void clear() {
+  unsigned z[NB + 1];
+  __device__ __forceinline__ void start(unsigned need) {
+    const unsigned from = (1u << NB) - need;
 #pragma unroll
-    for (int b = 0; b < NB; b++) z[b] = 0u;
+    for (int b = 0; b < NB; b++) z[b] = (from >> b) & 1u ? 0xFFFFu : 0u;
+    z[NB] = 0u;
   }
-  // a full adder of z[0], p and q, its carry through the rest
-  __device__ __forceinline__ void add2(unsigned p, unsigned q) {
-    unsigned c = (z[0] & p) | (z[0] & q) | (p & q);
-    z[0] ^= p ^ q;
-#pragma unroll
-    for (int b = 1; b < NB; b++) {
-      const unsigned t = z[b] & c;
-      z[b] ^= c;
-      c = t;
-    }
+  // full adder at weight 2^b
+  __device__ __forceinline__ unsigned add(int b, unsigned p, unsigned q) {
+    const unsigned c = majority(z[b], p, q);
+    z[b] ^= p ^ q;
+    return c;
   }
-  // groups whose two halves add up to at least need (bits 0..15)
-  __device__ __forceinline__ unsigned reached(unsigned need) const {
-    unsigned s[NB + 1], c = 0u;
+  // a carry of weight 2^b and up
+  __device__ __forceinline__ void ripple(int b, unsigned c) {
 #pragma unroll
-    for (int b = 0; b < NB; b++) {
-      const unsigned x = z[b], y = z[b] >> 16;
-      s[b] = x ^ y ^ c;
-      c = (x & y) | (c & (x | y));
-    }
-    s[NB] = c;
-    unsigned gt = 0u, eq = ~0u;
+    for (int k = 0; k <= NB; k++)
+      if (k >= b) {
+        const unsigned t = z[k] & c;
+        z[k] ^= c;
+        c = t;
+      }
+  }
+  __device__ __forceinline__ bool reached() const {
+    unsigned c = 0u;
 #pragma unroll
-    for (int b = NB; b >= 0; b--) {
-      const unsigned n = (need >> b) & 1u ? ~0u : 0u;
-      gt |= eq & s[b] & ~n;
-      eq &= ~(s[b] ^ n);
-    }
-    return (gt | eq) & 0xFFFFu;
+    for (int b = 0; b < NB; b++) c = majority(z[b], z[b] >> 16, c);
+    return ((z[NB] ^ c) & 0xFFFFu) != 0u;
   }
 };
 
 constexpr int kFilterWarps = 32;
 constexpr int kAhead = 8;  // groups of four spots held in registers (32 spots)
 
-// Persistent: one block per SM, its warps take every grid-th chunk of 32 records
-// and load the next chunk's codes before they count the present one's.
+// Persistent: one block per SM, its warps take every grid-th chunk of 32 records,
+// with two chunks' codes in registers: one being counted, the next on its way.
 template <int NB>
 __global__ void __launch_bounds__(32 * kFilterWarps, 1)
     group_filter_kernel(const __grid_constant__ FilterArgs f) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ uint32_t found;
-  const uint32_t mask_bytes = (f.cells.n * 2u + 15u) & ~15u;
+  const uint32_t mask_bytes = filter_mask_bytes(f.cells.n);
   const uint16_t *cm = reinterpret_cast<const uint16_t *>(smem);
   const GroupBucket *tab = reinterpret_cast<const GroupBucket *>(smem + mask_bytes);
   {
@@ -1232,58 +1234,76 @@ __global__ void __launch_bounds__(32 * kFilterWarps, 1)
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const uint32_t step = gridDim.x * kFilterWarps;
-  uint32_t ch = blockIdx.x * kFilterWarps + (threadIdx.x >> 5);
-  uint32_t *out = f.cand + (uint64_t)blockIdx.x * filter_region(f.nchunks, gridDim.x);
-  int bi = 0;
-  uint2 next[kAhead];
-  GroupBucket nb{};
-  auto load = [&]() {
-    while (ch >= tab[bi].chunk_end) bi++;
-    nb = tab[bi];
-    const int groups = (int)(nb.c + 3) / 4;
-    const uint2 *src = f.codes + nb.code0 + (uint64_t)(ch - nb.chunk0) * groups * 32 + lane;
+  const uint32_t out = blockIdx.x * (uint32_t)filter_region(f.nchunks, gridDim.x);
+  // the next chunk to load, its bucket and where its codes and records are
+  uint32_t ch = blockIdx.x * kFilterWarps + (threadIdx.x >> 5), chunk_end = 0, next_pos = 0;
+  int bi = -1, next_groups = 0;
+  uint32_t next = 0;  // 8-byte words of codes fit 32 bits (ensure_filter)
+  struct Chunk {
+    uint2 v[kAhead];
+    uint32_t src, pos;
+    int groups;  // 0: no more chunks
+  };
+  auto fetch = [&](Chunk &c) {
+    c.groups = 0;
+    if (ch >= f.nchunks) return;
+    if (ch >= chunk_end) {
+      do bi++;
+      while (ch >= tab[bi].chunk_end);
+      const GroupBucket b = tab[bi];
+      chunk_end = b.chunk_end;
+      next_groups = (int)(b.c + 3) / 4;
+      next = (uint32_t)b.code0 + (ch - b.chunk0) * (uint32_t)next_groups * 32u + (uint32_t)lane;
+      next_pos = b.pos0 + (ch - b.chunk0) * 32u + (uint32_t)lane;
+    }
+    c.groups = next_groups;
+    c.src = next;
+    c.pos = next_pos;
 #pragma unroll
     for (int g = 0; g < kAhead; g++)
-      if (g < groups) next[g] = ld_stream8(src + g * 32);
-  };
-  if (ch < f.nchunks) load();
-  while (ch < f.nchunks) {
-    uint2 v[kAhead];
-#pragma unroll
-    for (int g = 0; g < kAhead; g++) v[g] = next[g];
-    const uint32_t at = (ch - nb.chunk0) * 32u + (uint32_t)lane;
-    const uint32_t nrec = nb.nrec, pos0 = nb.pos0;
-    const int c = (int)nb.c, groups = (c + 3) / 4;
-    const uint2 *src = f.codes + nb.code0 + (uint64_t)(ch - nb.chunk0) * groups * 32 + lane;
+      if (g < next_groups) c.v[g] = ld_stream8(f.codes + next + g * 32);
     ch += step;
-    if (ch < f.nchunks) load();
+    next += step * (uint32_t)next_groups * 32u;
+    next_pos += step * 32u;
+  };
+  auto count = [&](const Chunk &c) {
     SlicedCount<NB> sc;
-    sc.clear();
-    auto four = [&](uint2 u, int g) {
-      unsigned p = __byte_perm(cm[u.x & 0xFFFFu], cm[u.x >> 16], 0x5410);
-      unsigned q = __byte_perm(cm[u.y & 0xFFFFu], cm[u.y >> 16], 0x5410);
-      if (g == groups - 1) {  // spots past the record's last one
-        const int r = c - 4 * g;
-        if (r < 2) p &= 0xFFFFu;
-        q = r < 3 ? 0u : r < 4 ? q & 0xFFFFu : q;
-      }
-      sc.add2(p, q);
+    sc.start(f.need);
+    auto four = [&](uint2 u) {
+      const unsigned p = __byte_perm(cm[u.x & 0xFFFFu], cm[u.x >> 16], 0x5410);
+      const unsigned q = __byte_perm(cm[u.y & 0xFFFFu], cm[u.y >> 16], 0x5410);
+      return sc.add(0, p, q);
     };
 #pragma unroll
-    for (int g = 0; g < kAhead; g++) {
-      if (g >= groups) break;
-      four(v[g], g);
+    for (int g = 0; g < kAhead; g += 4) {
+      if (g >= c.groups) break;
+      const unsigned c0 = four(c.v[g]);
+      const unsigned c1 = g + 1 < c.groups ? four(c.v[g + 1]) : 0u;
+      const unsigned c2 = g + 2 < c.groups ? four(c.v[g + 2]) : 0u;
+      const unsigned c3 = g + 3 < c.groups ? four(c.v[g + 3]) : 0u;
+      const unsigned d0 = sc.add(1, c0, c1), d1 = sc.add(1, c2, c3);
+      sc.ripple(3, sc.add(2, d0, d1));
     }
     if (NB > 5)
-      for (int g = kAhead; g < groups; g++) four(ld_stream8(src + (uint64_t)g * 32), g);
-    const bool keep = at < nrec && sc.reached(f.need) != 0u;
+      for (int g = kAhead; g < c.groups; g++) sc.ripple(1, four(ld_stream8(f.codes + c.src + g * 32)));
+    const bool keep = sc.reached();  // never for a lane past the last record: no spots
     const unsigned km = __ballot_sync(0xffffffffu, keep);
     if (km) {
       uint32_t base = 0;
       if (lane == 0) base = atomicAdd(&found, (uint32_t)__popc(km));
       base = __shfl_sync(0xffffffffu, base, 0);
-      if (keep) out[base + __popc(km & ((1u << lane) - 1u))] = pos0 + at;
+      if (keep) f.cand[out + base + __popc(km & ((1u << lane) - 1u))] = c.pos;
     }
+  };
+  Chunk a, b;
+  fetch(a);
+  for (;;) {
+    fetch(b);
+    if (!a.groups) break;
+    count(a);
+    fetch(a);
+    if (!b.groups) break;
+    count(b);
   }
   __syncthreads();
   if (threadIdx.x == 0) f.cand_cnt[blockIdx.x] = found;
@@ -1299,11 +1319,11 @@ static int launch_filter(const FilterArgs &f, size_t smem, cudaStream_t st) {
 }
 
 int filter_launch(const FilterArgs &f, cudaStream_t st) {
-  LMB_REQUIRE(f.cells.n >= 1 && f.cells.n <= 65536 && f.need >= 1 && f.grid >= 1 && f.nb >= 1,
+  LMB_REQUIRE(f.cells.n >= 1 && f.cells.n <= 65535 && f.need >= 1 && f.grid >= 1 && f.nb >= 1,
               "group filter: malformed arguments");
   groupmask_kernel<<<(f.cells.n * 4 + 255) / 256, 256, 0, st>>>(f);
   LMB_CUDA(cudaGetLastError());
-  const size_t smem = ((f.cells.n * 2u + 15u) & ~15u) + (size_t)f.nb * sizeof(GroupBucket);
+  const size_t smem = filter_mask_bytes(f.cells.n) + (size_t)f.nb * sizeof(GroupBucket);
   return f.most_spots <= 32 ? launch_filter<5>(f, smem, st) : launch_filter<8>(f, smem, st);
 }
 

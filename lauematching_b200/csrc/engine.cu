@@ -623,6 +623,8 @@ int ensure_filter(lmb_engine *e, bool *ok) {
   }
   if (e->gl_tab.empty()) return LMB_OK;  // no record has a spot
   const uint32_t grid = (uint32_t)e->num_sms;
+  // the filter addresses codes and candidates with 32 bits
+  if (code >= (1ull << 32) || grid * filter_region(chunk, grid) >= (1ull << 32)) return LMB_OK;
   cudaError_t ce = cudaMalloc(&e->d_cand, grid * filter_region(chunk, grid) * sizeof(uint32_t));
   if (ce == cudaSuccess) ce = cudaMalloc(&e->d_codes, code * sizeof(uint2));
   if (ce == cudaSuccess) ce = cudaMalloc(&e->d_cand_cnt, grid * sizeof(uint32_t));

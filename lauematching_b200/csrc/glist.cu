@@ -125,12 +125,13 @@ __global__ void __launch_bounds__(256) glist_scatter_kernel(const uint8_t *__res
 // of cw x ch pixels, 16 bits each.  32 records make a chunk; a lane's codes are
 // stored four at a time, [chunk][ceil(c / 4)][lane][4], so that a warp reads a
 // group of four spots of its 32 records with one 8-byte load per lane.  Codes
-// past the last spot or record are 0 (their reader leaves them out).
+// past the last spot or record are `none`, the code of a cell that is never marked.
 __global__ void __launch_bounds__(256) glist_code_kernel(const uint16_t *__restrict__ db, int R, int S,
                                                          int W, int H,
                                                          const uint32_t *__restrict__ perm,
                                                          uint32_t nrec, int c, int cw, int ch,
-                                                         int cells_x, uint2 *__restrict__ codes) {
+                                                         int cells_x, uint32_t none,
+                                                         uint2 *__restrict__ codes) {
   const uint32_t chunk = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (chunk >= (nrec + 31) / 32) return;
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(256) glist_code_kernel(const uint16_t *__restr
   const uint32_t at = chunk * 32 + lane;
   const uint16_t *rec = db + (at < nrec ? (uint64_t)perm[at] * R : 0);
   const int stored = at < nrec ? min((int)rec[0], S) : 0;
-  uint32_t four[4] = {0u, 0u, 0u, 0u};
+  uint32_t four[4] = {none, none, none, none};
   int k = 0, g = 0;
   for (int s = 0; s < stored && k < c; s++) {
     const uint32_t x = rec[1 + 2 * s], y = rec[2 + 2 * s];
@@ -151,13 +152,13 @@ __global__ void __launch_bounds__(256) glist_code_kernel(const uint16_t *__restr
     if ((++k & 3) == 0) {
       out[(uint64_t)g++ * 32] = make_uint2(four[0] | four[1] << 16, four[2] | four[3] << 16);
 #pragma unroll
-      for (int j = 0; j < 4; j++) four[j] = 0u;
+      for (int j = 0; j < 4; j++) four[j] = none;
     }
   }
   for (; g < groups; g++) {
     out[(uint64_t)g * 32] = make_uint2(four[0] | four[1] << 16, four[2] | four[3] << 16);
 #pragma unroll
-    for (int j = 0; j < 4; j++) four[j] = 0u;
+    for (int j = 0; j < 4; j++) four[j] = none;
   }
 }
 
@@ -167,7 +168,7 @@ int glist_code_launch(const uint16_t *d_db, int R, int S, int W, int H, const ui
   const uint32_t chunks = (b.nrec + 31) / 32;
   glist_code_kernel<<<(chunks + 7) / 8, 256, 0, st>>>(d_db, R, S, W, H, d_perm + b.pos0, b.nrec,
                                                       (int)b.c, cells.cw, cells.ch, cells.nx,
-                                                      d_codes + b.code0);
+                                                      cells.n, d_codes + b.code0);
   LMB_CUDA(cudaGetLastError());
   return LMB_OK;
 }

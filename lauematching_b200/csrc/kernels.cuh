@@ -229,7 +229,8 @@ int glist_scatter_launch(const uint8_t *d_cnt, uint64_t n, const uint32_t *d_bh,
                          cudaStream_t st);
 int listed_launch(CmpArgs a, int num_sms, cudaStream_t st);
 
-// Cells of the group masks: cw x ch pixels, nx per row, n in all (at most 65536).
+// Cells of the group masks: cw x ch pixels, nx per row, n in all (at most 65535;
+// code n stands for no spot).
 struct GroupCells {
   int cw, ch, nx, ny;
   uint32_t n;
@@ -267,6 +268,9 @@ struct FilterArgs {
 // Positions a filter block can keep: its 32 warps' chunks of 32 records.
 __host__ __device__ __forceinline__ uint64_t filter_region(uint32_t nchunks, uint32_t grid) {
   return 1024ull * ((nchunks + 32ull * grid - 1) / (32ull * grid));
+}
+__host__ __device__ __forceinline__ uint32_t filter_mask_bytes(uint32_t cells) {
+  return ((cells + 1u) * 2u + 15u) & ~15u;
 }
 int filter_launch(const FilterArgs &f, cudaStream_t st);
 int clist_fill_launch(const uint16_t *d_db, uint64_t n, int R, int S, int W, int H, uint32_t TB,
