@@ -126,15 +126,23 @@ __global__ void __launch_bounds__(256) glist_scatter_kernel(const uint8_t *__res
 // stored four at a time, [chunk][ceil(c / 4)][lane][4], so that a warp reads a
 // group of four spots of its 32 records with one 8-byte load per lane.  Codes
 // past the last spot or record are `none`, the code of a cell that is never marked.
+//
+// The order of a record's codes is free, and the filter's lanes look up their
+// k-th codes together: for records of up to 32 spots the k-th codes of a chunk are
+// chosen to lie in different shared-memory banks (two cells per 4-byte word).  A
+// lane offers the banks of the spots it has left, three rounds hand every free bank
+// to one lane that asks for it, and the lanes that got none take any spot.
 __global__ void __launch_bounds__(256) glist_code_kernel(const uint16_t *__restrict__ db, int R, int S,
                                                          int W, int H,
                                                          const uint32_t *__restrict__ perm,
                                                          uint32_t nrec, int c, int cw, int ch,
                                                          int cells_x, uint32_t none,
                                                          uint2 *__restrict__ codes) {
+  constexpr int kMost = 32;  // spots of a record whose codes are ordered
+  __shared__ uint16_t held[8][kMost][33];
   const uint32_t chunk = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (chunk >= (nrec + 31) / 32) return;
+  if (chunk >= (nrec + 31) / 32) return;  // whole warps
   const int groups = (c + 3) / 4;
   uint2 *out = codes + (uint64_t)chunk * groups * 32 + lane;
   const uint32_t at = chunk * 32 + lane;
@@ -142,10 +150,7 @@ __global__ void __launch_bounds__(256) glist_code_kernel(const uint16_t *__restr
   const int stored = at < nrec ? min((int)rec[0], S) : 0;
   uint32_t four[4] = {none, none, none, none};
   int k = 0, g = 0;
-  for (int s = 0; s < stored && k < c; s++) {
-    const uint32_t x = rec[1 + 2 * s], y = rec[2 + 2 * s];
-    if (x >= (uint32_t)W || y >= (uint32_t)H) continue;
-    const uint32_t q = (y / (uint32_t)ch) * (uint32_t)cells_x + x / (uint32_t)cw;
+  auto put = [&](uint32_t q) {
 #pragma unroll
     for (int j = 0; j < 4; j++)
       if ((k & 3) == j) four[j] = q;
@@ -153,6 +158,53 @@ __global__ void __launch_bounds__(256) glist_code_kernel(const uint16_t *__restr
       out[(uint64_t)g++ * 32] = make_uint2(four[0] | four[1] << 16, four[2] | four[3] << 16);
 #pragma unroll
       for (int j = 0; j < 4; j++) four[j] = none;
+    }
+  };
+  uint16_t(*mine)[33] = held[threadIdx.x >> 5];
+  int n = 0;
+  for (int s = 0; s < stored && n < c; s++) {
+    const uint32_t x = rec[1 + 2 * s], y = rec[2 + 2 * s];
+    if (x >= (uint32_t)W || y >= (uint32_t)H) continue;
+    const uint32_t q = (y / (uint32_t)ch) * (uint32_t)cells_x + x / (uint32_t)cw;
+    if (c <= kMost)
+      mine[n][lane] = (uint16_t)q;
+    else
+      put(q);
+    n++;
+  }
+  if (c <= kMost) {
+    unsigned left = n >= 32 ? ~0u : (1u << n) - 1u, banks = 0u;
+    for (int j = 0; j < n; j++) banks |= 1u << ((mine[j][lane] >> 1) & 31);
+    const unsigned all = 0xffffffffu;
+    for (int step = 0; step < c; step++) {
+      unsigned taken = 0u;
+      int bank = -1;
+      const int turn = (lane + 11 * step) & 31;  // where a lane starts looking
+      for (int round = 0; round < 3; round++) {
+        const unsigned free = bank < 0 ? banks & ~taken : 0u;
+        const int ask = free ? (__ffs(__funnelshift_r(free, free, turn)) - 1 + turn) & 31 : -1;
+        const unsigned same = __match_any_sync(all, ask);
+        const bool mine_now = ask >= 0 && lane == __ffs(same) - 1;
+        if (mine_now) bank = ask;
+        taken |= __reduce_or_sync(all, mine_now ? 1u << ask : 0u);
+      }
+      if (bank < 0 && banks) bank = (__ffs(__funnelshift_r(banks, banks, turn)) - 1 + turn) & 31;
+      if (bank >= 0) {  // the lane's spot of that bank; the banks of the others
+        int pick = -1;
+        banks = 0u;
+        for (unsigned m = left; m; m &= m - 1u) {
+          const int j = __ffs(m) - 1;
+          const int b = (mine[j][lane] >> 1) & 31;
+          if (pick < 0 && b == bank)
+            pick = j;
+          else
+            banks |= 1u << b;
+        }
+        left &= ~(1u << pick);
+        put(mine[pick][lane]);
+      } else {
+        put(none);
+      }
     }
   }
   for (; g < groups; g++) {
