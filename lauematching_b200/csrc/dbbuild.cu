@@ -6,22 +6,48 @@
 // walks the HKL list in file order, appending on-detector, in-band,
 // not-yet-seen pixels until MaxNrLaueSpots are taken.
 //
-// Arithmetic.  Each (orientation, HKL) pair is first screened in FP32 with
-// FMA.  The screen only REJECTS: a pair is dropped when, with an error
-// margin far above the FP32 error of the chain, it is certainly behind the
-// detector, off the detector or outside the energy band.  Every other pair
-// is recomputed in FP64 with the reference's exact operation order and
-// rounding (no FMA; C truncation of the pixel coordinate as x86 performs
-// it), and that result alone decides acceptance and the pixel.  The records
-// are therefore identical to the reference's, byte for byte; a build flag
-// (exact_all) runs the FP64 path for every pair to check the screen.
+// Arithmetic.  FP64 in the reference's exact operation order and rounding (no
+// FMA; C truncation of the pixel coordinate as x86 performs it) alone decides
+// acceptance and the pixel, so the records are the reference's, byte for byte.
+// FP32 screens before it only REJECT, with margins above their error bounds:
 //
-// Layout.  Blocks of TB orientations; the HKL list is staged through shared
-// memory in chunks (broadcast reads); accepted pixels live in shared memory
-// as [spot][thread] so the de-duplication scan is bank-conflict free; the
-// block's records (contiguous in the DB) are written with coalesced stores.
+//   band      E = (hc / 4 pi) |q|^2 / (-q_z) and sin(theta) = -q_z / |q|, and |q| of
+//             an HKL is the same for every rotation: the energy band and the
+//             scattering angles that the detector covers are an interval of |q_z|
+//             per HKL, known on the host.  HKLs whose interval is empty are left
+//             out of the build (of 1240 fcc HKLs at 5-30 keV a detector normal to
+//             the beam at 500 mm can see 88, of 7790 hexagonal ones 256); the
+//             others cost three FMAs and two comparisons, one test for h and -h
+//             together (they differ in the sign of q_z, which says which of the two
+//             has a positive energy; both reflect the same way).
+//   detector  of those: z > 0 and the pixel inside the frame as linear
+//             inequalities in the unnormalised direction, without a division or a
+//             square root.
+//
+// The HKLs that can be seen are taken in chunks of file order.  Each thread owns one orientation
+// and keeps a bit per unit (a pair h, -h of the chunk, or a single HKL) that
+// passed the band test, then a bit per HKL that passed both; it walks its own
+// set bits, so the lanes of a warp stay busy over a whole chunk although they
+// keep different HKLs.  FP64 then takes an orientation's HKLs in file order.
+// The band test is bound by instruction issue (about 10 per unit and warp), the
+// other two by the lane with the most bits of its warp.  Measured on B200 at 1e8
+// synthetic orientations (whole build, one warp-wide FP32 test of energy and
+// detector per HKL before): fcc beam-normal 644 -> 39 ms, tilted 34-ID-E detector
+// 890 -> 234 ms, hexagonal beam-normal 3250 -> 66 ms.  A build flag
+// (exact_all), an orientation that is no rotation, and geometry outside the
+// screens' assumptions take FP64 for every HKL.
+//
+// Layout.  Blocks of TB orientations; accepted pixels live in shared memory as
+// [spot][thread] so the de-duplication scan is bank-conflict free; the block's
+// records (contiguous in the DB) are written with coalesced stores.
+#include <algorithm>
 #include <climits>
 #include <cmath>
+#include <cstring>
+#include <limits>
+#include <map>
+#include <tuple>
+#include <vector>
 
 #include "kernels.cuh"
 
@@ -31,60 +57,27 @@ struct BuildGeo {
   double recip[9], rt[9];
   double p0, p1, p2, px_x, px_y, cx, cy, elo, ehi;
   int W, H, S, R;
-  float rtf[9];
-  float p0f, p1f, p2f, inv_pxxf, inv_pyf, cxf, cyf, elof, ehif, hc4pif;
-  float tolx, toly;  // FP32 pixel-error scale: 1e-4 * p2 / |px|
+  // detector screen: pixel * z = a * x + b * z, and its margins
+  float rt2[3];
+  float ax, bx0, bx1, ay, by0, by1, tolx, toly;
 };
 
 static constexpr double kHcKeVnm = 1.2398419739;              // LaueMatchingHeaders.h:41
 static constexpr double kFourPi = 4.0 * 3.14159265358979323846;  // 4 * M_PI as C folds it
-static constexpr int kHklChunk = 512;
+static constexpr int kHklChunk = 512;                // HKLs per chunk
+static constexpr int kChunkWords = kHklChunk / 32;
+static constexpr double kRotTol = 1e-4;  // a rotation: |OM^T OM - 1| below this
+static constexpr double kBandTol = 4e-4;  // relative margin of the energy band (3 kRotTol and rounding)
 
-// FP32 screen: false only when the pair is certainly rejected in FP64.
-// Ordered cheapest-first: the energy band needs only q (E = c*|q|^2/(-q_z),
-// c = hc/4pi, tested by multiplication), which rejects most pairs before the
-// detector projection is computed.  Margins: the FP32 chain has relative
-// error ~1e-6 in |q|^2 and absolute ~2e-6*|q| in q_z, ~3e-6 in the unit
-// vectors; every test below leaves >= 30x that.
-__device__ __forceinline__ bool screen(const float T[9], const float4 hf, const BuildGeo &g) {
-  const float qx = fmaf(T[0], hf.x, fmaf(T[1], hf.y, T[2] * hf.z));
-  const float qy = fmaf(T[3], hf.x, fmaf(T[4], hf.y, T[5] * hf.z));
-  const float qz = fmaf(T[6], hf.x, fmaf(T[7], hf.y, T[8] * hf.z));
-  const float ql2 = fmaf(qx, qx, fmaf(qy, qy, qz * qz));
-  if (!(ql2 > 1e-30f) || !(ql2 < 1e30f)) return true;  // let FP64 decide
-  const float rq = rsqrtf(ql2);
-  const float ql = ql2 * rq;
-  const float nq = -qz;   // |q| sin(theta)
-  const float s = nq * rq;  // sin(theta)
-  if (fabsf(s) >= 1e-5f) {
-    const float cq = g.hc4pif * ql2;  // E * (-q_z)
-    if (s < 0.f) {
-      if (g.elof > 0.f) return false;  // E < 0 < Elo
-    } else {
-      if (g.ehif > 0.f && cq > g.ehif * fmaf(nq, 1e-4f, nq) + g.ehif * 1e-4f * ql) return false;
-      if (g.elof > 0.f && cq < g.elof * fmaf(nq, -1e-4f, nq) - g.elof * 1e-4f * ql) return false;
-    }
-  }
-  const float hx = qx * rq, hy = qy * rq, hz = qz * rq;
-  const float td = -2.f * hz;
-  const float k0 = td * hx, k1 = td * hy, k2 = fmaf(td, hz, 1.f);
-  const float z = fmaf(g.rtf[6], k0, fmaf(g.rtf[7], k1, g.rtf[8] * k2));
-  if (z < -1e-4f) return false;  // xyz[2] <= 0 for sure
-  if (z <= 1e-4f) return true;   // too close to call
-  const float iz = __fdividef(1.f, z);
-  const float x = fmaf(g.rtf[0], k0, fmaf(g.rtf[1], k1, g.rtf[2] * k2)) * iz;
-  const float y = fmaf(g.rtf[3], k0, fmaf(g.rtf[4], k1, g.rtf[5] * k2)) * iz;
-  // pixel = (x/z * p2 - p0) / px + (N-1)/2 ; accepted iff trunc in [0, N-1],
-  // i.e. pixel in (-1, N).  |error| <= 3e-6 (1+|x/z|)/z * p2/px (FP32 chain),
-  // the margin below is ~30x that plus 0.05 px.
-  const float pxv = fmaf(fmaf(x, g.p2f, -g.p0f), g.inv_pxxf, g.cxf);
-  const float tx = fmaf(g.tolx * (1.f + fabsf(x)), iz, 0.05f);
-  if (pxv < -1.f - tx || pxv > (float)g.W + tx) return false;
-  const float pyv = fmaf(fmaf(y, g.p2f, -g.p1f), g.inv_pyf, g.cyf);
-  const float ty = fmaf(g.toly * (1.f + fabsf(y)), iz, 0.05f);
-  if (pyv < -1.f - ty || pyv > (float)g.H + ty) return false;
-  return true;
-}
+// The units of a chunk: hkl (as floats) and the interval of |q_z| it can be seen
+// in, as two bf16 (the lower bound in the high half, rounded down; the upper one
+// rounded up); the relative error of its projection; the chunk positions of h
+// (taken when q_z < 0) and of -h (q_z > 0), 0xFFFF for none.
+struct BuildUnits {
+  float4 hkl_band[kHklChunk];
+  float eps[kHklChunk];
+  uint32_t pos[kHklChunk];
+};
 
 // FP64 evaluation in the reference's exact order (LaueMatchingCPU.c:605-636,
 // MatrixMultF LaueMatchingHeaders.h:361-369).  Returns acceptance and pixel.
@@ -119,27 +112,30 @@ __device__ __forceinline__ bool exact_spot(const double T[9], const int4 hk, con
 }
 
 template <bool kExactAll>
-__global__ void dbbuild_kernel(const double *__restrict__ om, uint64_t n,
-                               const int4 *__restrict__ hkl, int nh, BuildGeo g,
-                               uint16_t *__restrict__ out) {
+__global__ void __launch_bounds__(128) dbbuild_kernel(const double *__restrict__ om, uint64_t n,
+                                                      const int4 *__restrict__ hkl, int nh,
+                                                      const int4 *__restrict__ seen, int nseen,
+                                                      const BuildUnits *__restrict__ units,
+                                                      const uint32_t *__restrict__ unit_count,
+                                                      const __grid_constant__ BuildGeo g,
+                                                      uint16_t *__restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int TB = blockDim.x;
-  int4 *sh_hkl = reinterpret_cast<int4 *>(smem);
-  float4 *sh_hklf = reinterpret_cast<float4 *>(smem + kHklChunk * sizeof(int4));
-  uint32_t *sh_list = reinterpret_cast<uint32_t *>(smem + kHklChunk * 2 * sizeof(int4));
-  int *sh_cnt = reinterpret_cast<int *>(sh_list + (size_t)g.S * TB);
-  // per warp, the pairs that passed the screen and wait for FP64: lane << 16 | HKL
-  uint32_t *q = reinterpret_cast<uint32_t *>(sh_cnt + TB) + (threadIdx.x >> 5) * (2 * 32);
+  BuildUnits *su = reinterpret_cast<BuildUnits *>(smem);
+  uint32_t *sh_list = reinterpret_cast<uint32_t *>(smem + sizeof(BuildUnits));
+  uint32_t *sh_cnt = sh_list + (size_t)g.S * TB;
+  uint32_t *band = sh_cnt + TB;              // [kChunkWords][TB] units inside their band
+  uint32_t *keep = band + kChunkWords * TB;  // [kChunkWords][TB] HKLs for FP64
 
   const int t = threadIdx.x;
-  const int lane = t & 31;
-  const unsigned lt = (1u << lane) - 1u;
   const uint64_t base = (uint64_t)blockIdx.x * TB;
   const uint64_t oid = base + t;
   const bool valid = oid < n;
 
   double T[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  float Tf[9];
+  float U[9];           // detector rotation . T
+  float t0 = 0, t1 = 0, t2 = 0;  // T's last row
+  bool regular = true;
   if (valid) {
     double m[9];
 #pragma unroll
@@ -152,80 +148,112 @@ __global__ void dbbuild_kernel(const double *__restrict__ om, uint64_t n,
         T[r * 3 + c] = dadd(dadd(dmul(m[r * 3 + 0], g.recip[0 * 3 + c]),
                                  dmul(m[r * 3 + 1], g.recip[1 * 3 + c])),
                             dmul(m[r * 3 + 2], g.recip[2 * 3 + c]));
+    if (!kExactAll) {
+      // the band screen holds for rotations (NaN: not one)
 #pragma unroll
-    for (int i = 0; i < 9; i++) Tf[i] = (float)T[i];
+      for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = i; j < 3; j++) {
+          const double d = m[i] * m[j] + m[3 + i] * m[3 + j] + m[6 + i] * m[6 + j] - (i == j ? 1.0 : 0.0);
+          regular = regular && fabs(d) <= kRotTol;
+        }
+#pragma unroll
+      for (int r = 0; r < 3; r++)
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+          U[r * 3 + c] = (float)(g.rt[r * 3] * T[c] + g.rt[r * 3 + 1] * T[3 + c] + g.rt[r * 3 + 2] * T[6 + c]);
+      t0 = (float)T[6];
+      t1 = (float)T[7];
+      t2 = (float)T[8];
+    }
   }
   int cnt = 0;
   bool done = !valid || g.S <= 0;
-  // The FP64 evaluations of the first m queued pairs (m <= 32), one per lane
-  // with the owner's matrix, then their outcomes in queue order: each owner
-  // takes its own in HKL order (dedup, append, stop at S) exactly as it
-  // would have evaluating them one by one.
-  auto evaluate = [&](int m) {
-    const uint32_t ent = lane < m ? q[lane] : 0u;
-    const int o = lane < m ? (int)(ent >> 16) : lane;
-    double To[9];
-#pragma unroll
-    for (int j = 0; j < 9; j++) To[j] = __shfl_sync(0xffffffffu, T[j], o);
+  auto take = [&](const int4 h) {  // one HKL in FP64
     int ix = 0, iy = 0;
-    const bool ok = lane < m && exact_spot(To, sh_hkl[ent & 0xFFFFu], g, ix, iy);
+    if (!exact_spot(T, h, g, ix, iy)) return;
     const uint32_t key = (uint32_t)(ix & 0xFFFF) | ((uint32_t)(iy & 0xFFFF) << 16);
-    const unsigned okm = __ballot_sync(0xffffffffu, ok);
-    for (int e = 0; e < m; e++) {
-      const int oe = __shfl_sync(0xffffffffu, o, e);
-      const uint32_t ke = __shfl_sync(0xffffffffu, key, e);
-      if (lane == oe && ((okm >> e) & 1u) && !done) {
-        bool dup = false;
-        for (int s = 0; s < cnt; s++) dup |= (sh_list[(size_t)s * TB + t] == ke);
-        if (!dup) {
-          sh_list[(size_t)cnt * TB + t] = ke;
-          done = (++cnt == g.S);
-        }
-      }
-    }
-    __syncwarp();
+    bool dup = false;
+    for (int s = 0; s < cnt; s++) dup |= (sh_list[(size_t)s * TB + t] == key);
+    if (dup) return;
+    sh_list[(size_t)cnt * TB + t] = key;
+    done = ++cnt == g.S;
   };
-  for (int c0 = 0; c0 < nh; c0 += kHklChunk) {
-    const int cn = min(kHklChunk, nh - c0);
+  if (kExactAll || !regular) {
+    for (int i = 0; i < nh && !done; i++) take(__ldg(hkl + i));
+    done = true;
+  }
+  for (int c0 = 0, chunk = 0; !kExactAll && c0 < nseen; c0 += kHklChunk, chunk++) {
+    const int words = (min(kHklChunk, nseen - c0) + 31) / 32;
+    const int nu = (int)unit_count[chunk];  // a multiple of 32, the rest never passes
     __syncthreads();
-    for (int i = t; i < cn; i += TB) {
-      const int4 v = hkl[c0 + i];
-      sh_hkl[i] = v;
-      sh_hklf[i] = make_float4((float)v.x, (float)v.y, (float)v.z, 0.f);
+    const BuildUnits *src = units + chunk;
+    for (int i = t; i < nu; i += TB) {
+      su->hkl_band[i] = src->hkl_band[i];
+      su->eps[i] = src->eps[i];
+      su->pos[i] = src->pos[i];
     }
     __syncthreads();
-    // Warp-uniform loop over the chunk: every lane screens its orientation
-    // against HKL i in FP32; the pairs that pass join the warp's queue in
-    // HKL order, and every 32 of them are evaluated in FP64 on all lanes at
-    // once (a lane that has reached S spots queues nothing more; pairs it
-    // queued before its last spot are evaluated and dropped).
-    int qn = 0;
-    for (int i = 0; i < cn; i++) {
-      bool go = !done;
-      if (!kExactAll && go) go = screen(Tf, sh_hklf[i], g);
-      const unsigned bm = __ballot_sync(0xffffffffu, go);
-      if (bm) {
-        if (go) q[qn + __popc(bm & lt)] = ((uint32_t)lane << 16) | (uint32_t)i;
-        qn += __popc(bm);
-        if (qn >= 32) {
-          __syncwarp();
-          evaluate(32);
-          const int rest = qn - 32;  // < 32: move the tail to the front
-          const uint32_t v = lane < rest ? q[32 + lane] : 0u;
-          __syncwarp();
-          if (lane < rest) q[lane] = v;
-          __syncwarp();
-          qn = rest;
+    if (!done) {
+      for (int w = 0; w < words; w++) keep[w * TB + t] = 0u;
+      const int uw = nu / 32;
+      for (int w = 0; w < uw; w++) {
+        uint32_t bits = 0u;
+#pragma unroll
+        for (int b = 0; b < 32; b++) {
+          const float4 h = su->hkl_band[w * 32 + b];
+          const float q = fabsf(fmaf(t0, h.x, fmaf(t1, h.y, t2 * h.z)));
+          const float lo = __uint_as_float(__float_as_uint(h.w) & 0xFFFF0000u);
+          const float hi = __uint_as_float(__float_as_uint(h.w) << 16);
+          if (!(q < lo) && !(q > hi)) bits |= 1u << b;
         }
+        band[w * TB + t] = bits;
       }
-    }
-    if (qn) {  // the chunk's last pairs, before its HKLs leave shared memory
-      __syncwarp();
-      evaluate(qn);
+      // detector
+      int w = -1;
+      uint32_t bits = 0u;
+      for (;;) {
+        while (bits == 0u && ++w < uw) bits = band[w * TB + t];
+        if (w >= uw) break;
+        const int u = w * 32 + __ffs(bits) - 1;
+        bits &= bits - 1u;
+        const float4 h = su->hkl_band[u];
+        const float eps = su->eps[u];
+        const uint32_t pos = su->pos[u];
+        const float qz = fmaf(t0, h.x, fmaf(t1, h.y, t2 * h.z));
+        const float u0 = fmaf(U[0], h.x, fmaf(U[1], h.y, U[2] * h.z));
+        const float u1 = fmaf(U[3], h.x, fmaf(U[4], h.y, U[5] * h.z));
+        const float u2 = fmaf(U[6], h.x, fmaf(U[7], h.y, U[8] * h.z));
+        const float q2 = fmaf(u0, u0, fmaf(u1, u1, u2 * u2));
+        const float d = -2.f * qz;
+        const float x = fmaf(d, u0, g.rt2[0] * q2);
+        const float y = fmaf(d, u1, g.rt2[1] * q2);
+        const float z = fmaf(d, u2, g.rt2[2] * q2);
+        const float m = eps * q2;  // error of x, y and z
+        const bool off = z < -m || fmaf(g.ax, x, g.bx0 * z) < -m * g.tolx ||
+                         fmaf(g.ax, x, g.bx1 * z) > m * g.tolx ||
+                         fmaf(g.ay, y, g.by0 * z) < -m * g.toly ||
+                         fmaf(g.ay, y, g.by1 * z) > m * g.toly;
+        if (off) continue;
+        const bool either = !(qz * qz > m * eps);  // q_z may have either sign (or eps is NaN)
+        const uint32_t i = pos & 0xFFFFu, j = pos >> 16;
+        if ((qz < 0.f || either) && i != 0xFFFFu) keep[(i >> 5) * TB + t] |= 1u << (i & 31u);
+        if ((!(qz < 0.f) || either) && j != 0xFFFFu) keep[(j >> 5) * TB + t] |= 1u << (j & 31u);
+      }
+      // FP64 over the kept HKLs in file order
+      w = -1;
+      bits = 0u;
+      while (!done) {
+        while (bits == 0u && ++w < words) bits = keep[w * TB + t];
+        if (w >= words) break;
+        const int i = c0 + w * 32 + __ffs(bits) - 1;
+        bits &= bits - 1u;
+        take(__ldg(seen + i));
+      }
     }
     if (__syncthreads_and(done)) break;
   }
-  sh_cnt[t] = cnt;
+  sh_cnt[t] = (uint32_t)cnt;
   __syncthreads();
   // Coalesced store of this block's records: [count, x0, y0, ...] zero padded.
   if (base >= n) return;
@@ -233,19 +261,29 @@ __global__ void dbbuild_kernel(const double *__restrict__ om, uint64_t n,
   const uint32_t R = (uint32_t)g.R;
   const uint32_t total = nvalid * R;
   uint16_t *dst = out + base * R;
-  for (uint32_t w = t; w < total; w += TB) {
-    const uint32_t o = w / R, f = w - o * R;
-    uint16_t v = 0;
-    if (f == 0) {
-      v = (uint16_t)sh_cnt[o];
-    } else {
-      const uint32_t s = (f - 1) >> 1;
-      if ((int)s < sh_cnt[o]) {
-        const uint32_t key = sh_list[(size_t)s * TB + o];
-        v = (f & 1) ? (uint16_t)(key & 0xFFFF) : (uint16_t)(key >> 16);
-      }
+  auto field = [&](uint32_t o, uint32_t f) -> uint32_t {
+    if (f == 0) return sh_cnt[o];
+    const uint32_t s = (f - 1) >> 1;
+    if (s >= sh_cnt[o]) return 0u;
+    const uint32_t key = sh_list[(size_t)s * TB + o];
+    return (f & 1) ? key & 0xFFFFu : key >> 16;
+  };
+  // two fields per store: a block's records start on a 4-byte boundary (TB is even)
+  const uint32_t step_o = 2u * TB / R, step_f = 2u * TB - step_o * R;
+  uint32_t o = 2u * t / R, f = 2u * t - o * R;
+  for (uint32_t w = 2u * t; w < total; w += 2u * TB) {
+    const uint32_t lo = field(o, f);
+    const bool wrap = f + 1 == R;
+    if (w + 1 < total)
+      *reinterpret_cast<uint32_t *>(dst + w) = lo | field(wrap ? o + 1 : o, wrap ? 0u : f + 1) << 16;
+    else
+      dst[w] = (uint16_t)lo;
+    o += step_o;
+    f += step_f;
+    if (f >= R) {
+      f -= R;
+      o++;
     }
-    dst[w] = v;
   }
 }
 
@@ -324,7 +362,6 @@ static BuildGeo make_build_geo(const lmb_geometry &geo) {
   for (int i = 0; i < 9; i++) {
     g.recip[i] = geo.recip[i];
     g.rt[i] = geo.rot_t[i];
-    g.rtf[i] = (float)geo.rot_t[i];
   }
   g.p0 = geo.p[0];
   g.p1 = geo.p[1];
@@ -339,31 +376,150 @@ static BuildGeo make_build_geo(const lmb_geometry &geo) {
   g.H = geo.nr_px_y;
   g.S = geo.max_nr_spots;
   g.R = 1 + 2 * geo.max_nr_spots;
-  g.p0f = (float)g.p0;
-  g.p1f = (float)g.p1;
-  g.p2f = (float)g.p2;
-  g.inv_pxxf = (float)(1.0 / g.px_x);
-  g.inv_pyf = (float)(1.0 / g.px_y);
-  g.cxf = (float)g.cx;
-  g.cyf = (float)g.cy;
-  g.elof = (float)g.elo;
-  g.ehif = (float)g.ehi;
-  g.hc4pif = (float)(kHcKeVnm / kFourPi);
-  g.tolx = (float)(1e-4 * std::fabs(g.p2 / g.px_x));
-  g.toly = (float)(1e-4 * std::fabs(g.p2 / g.px_y));
+  for (int i = 0; i < 3; i++) g.rt2[i] = (float)g.rt[3 * i + 2];
+  // pixel * z = a * x + b * z must lie in (-z, N z)
+  const double ax = g.p2 / g.px_x, bx = g.cx - g.p0 / g.px_x;
+  const double ay = g.p2 / g.px_y, by = g.cy - g.p1 / g.px_y;
+  g.ax = (float)ax;
+  g.bx0 = (float)(bx + 1.0);
+  g.bx1 = (float)(bx - g.W);
+  g.ay = (float)ay;
+  g.by0 = (float)(by + 1.0);
+  g.by1 = (float)(by - g.H);
+  g.tolx = (float)(std::fabs(ax) + std::max(std::fabs(bx + 1.0), std::fabs(bx - g.W)));
+  g.toly = (float)(std::fabs(ay) + std::max(std::fabs(by + 1.0), std::fabs(by - g.H)));
   return g;
 }
 
-// The FP32 screen is only sound when every geometry value is finite and
-// within FP32 range; otherwise every pair takes the FP64 path.
+// The screens assume finite values in FP32 range, an orthonormal detector
+// rotation and a band of non-negative energies.
 static bool screen_sound(const lmb_geometry &geo) {
-  auto ok = [](double v) { return std::isfinite(v) && std::fabs(v) < 1e30; };
+  auto ok = [](double v) { return std::isfinite(v) && std::fabs(v) < 1e15; };
   for (int i = 0; i < 9; i++)
     if (!ok(geo.rot_t[i]) || !ok(geo.recip[i])) return false;
   for (int i = 0; i < 3; i++)
+    for (int j = i; j < 3; j++) {
+      double d = i == j ? -1.0 : 0.0;
+      for (int k = 0; k < 3; k++) d += geo.rot_t[3 * i + k] * geo.rot_t[3 * j + k];
+      if (!(std::fabs(d) < 1e-9)) return false;
+    }
+  for (int i = 0; i < 3; i++)
     if (!ok(geo.p[i])) return false;
-  return ok(geo.px_x) && ok(geo.px_y) && geo.px_x != 0 && geo.px_y != 0 && ok(geo.elo) &&
-         ok(geo.ehi) && std::fabs(geo.p[2] / geo.px_x) < 1e30 && std::fabs(geo.p[2] / geo.px_y) < 1e30;
+  if (!ok(geo.px_x) || !ok(geo.px_y) || geo.px_x == 0 || geo.px_y == 0) return false;
+  for (double v : {geo.p[2] / geo.px_x, geo.p[2] / geo.px_y, geo.p[0] / geo.px_x, geo.p[1] / geo.px_y})
+    if (!ok(v)) return false;
+  return ok(geo.elo) && ok(geo.ehi) && geo.elo >= 0.0 && geo.ehi > 0.0;
+}
+
+// sin(theta) of the directions that reach the detector (with a pixel to spare on
+// every side), from a grid of cells of the detector plane at z = 1: a cell's
+// directions lie within its half diagonal of its centre's (an angle is at most
+// the distance in that plane).
+static void detector_angles(const lmb_geometry &geo, double *smin, double *smax) {
+  *smin = 0.0;
+  *smax = 1.0;
+  if (geo.p[2] == 0.0) return;
+  const double xa = ((-1.0 - 0.5 * (geo.nr_px_x - 1)) * geo.px_x + geo.p[0]) / geo.p[2];
+  const double xb = ((geo.nr_px_x - 0.5 * (geo.nr_px_x - 1)) * geo.px_x + geo.p[0]) / geo.p[2];
+  const double ya = ((-1.0 - 0.5 * (geo.nr_px_y - 1)) * geo.px_y + geo.p[1]) / geo.p[2];
+  const double yb = ((geo.nr_px_y - 0.5 * (geo.nr_px_y - 1)) * geo.px_y + geo.p[1]) / geo.p[2];
+  const int kCells = 64;
+  const double dx = (xb - xa) / kCells, dy = (yb - ya) / kCells;
+  const double r = 0.5 * std::sqrt(dx * dx + dy * dy) * (1.0 + 1e-9) + 1e-9;
+  double lo = 4.0, hi = -4.0;  // 2 theta
+  for (int i = 0; i < kCells; i++)
+    for (int j = 0; j < kCells; j++) {
+      const double x = xa + (i + 0.5) * dx, y = ya + (j + 0.5) * dy;
+      const double k = (geo.rot_t[2] * x + geo.rot_t[5] * y + geo.rot_t[8]) / std::sqrt(x * x + y * y + 1.0);
+      const double a = std::acos(std::max(-1.0, std::min(1.0, k)));
+      lo = std::min(lo, a - r);
+      hi = std::max(hi, a + r);
+    }
+  const double pi = kFourPi / 4.0;
+  if (lo > 0.0 && lo < pi) *smin = std::sin(0.5 * lo) * (1.0 - 1e-6);
+  if (hi > 0.0 && hi < pi) *smax = std::min(1.0, std::sin(0.5 * hi) * (1.0 + 1e-6));
+}
+
+// A bf16 not above (down) or not below v >= 0, as its 16 bits.
+static uint32_t bf16_bound(double v, bool down) {
+  float f = (float)std::min(v, 3e38);
+  if (down && (double)f > v) f = std::nextafter(f, 0.f);
+  if (!down && (double)f < v) f = std::nextafter(f, std::numeric_limits<float>::infinity());
+  uint32_t b;
+  memcpy(&b, &f, 4);
+  return (down ? b : b + 0xFFFFu) >> 16;
+}
+
+// The HKLs that some rotation can put on the detector within the energy band, in
+// file order, and their units, chunk by chunk.  Errors: the FP32 q_z of a rotation
+// is within 8 x 2^-24 of sum |recip column| |h| (rounded inputs, one product, two
+// FMAs); eps bounds that of x, y and z against |q|^2, with a factor of 4 to spare.
+static void build_units(const lmb_geometry &geo, const int4 *hkl, int nh, std::vector<int4> *seen,
+                        std::vector<BuildUnits> *units, std::vector<uint32_t> *count) {
+  const double c = kHcKeVnm / kFourPi, ulp = std::ldexp(1.0, -24);
+  double col[3], smin, smax;
+  for (int j = 0; j < 3; j++)
+    col[j] = std::sqrt(geo.recip[j] * geo.recip[j] + geo.recip[3 + j] * geo.recip[3 + j] +
+                       geo.recip[6 + j] * geo.recip[6 + j]);
+  detector_angles(geo, &smin, &smax);
+  std::map<std::tuple<int, int, int>, std::vector<int>> open;  // units still without their -h
+  int nu = 0;
+  auto close_chunk = [&]() {
+    if (units->empty()) return;
+    BuildUnits &bu = units->back();
+    for (; nu % 32; nu++) {  // padding: an empty interval, no HKL
+      const uint32_t none = 0x7F800000u;  // +inf, 0
+      memcpy(&bu.hkl_band[nu].w, &none, 4);
+      bu.eps[nu] = 1.f;
+      bu.pos[nu] = 0xFFFFFFFFu;
+    }
+    count->push_back((uint32_t)nu);
+  };
+  for (int n = 0; n < nh; n++) {
+    const int4 h = hkl[n];
+    double q2 = 0.0;
+    for (int r = 0; r < 3; r++) {
+      const double q = geo.recip[3 * r] * h.x + geo.recip[3 * r + 1] * h.y + geo.recip[3 * r + 2] * h.z;
+      q2 += q * q;
+    }
+    const double sum = col[0] * std::fabs((double)h.x) + col[1] * std::fabs((double)h.y) +
+                       col[2] * std::fabs((double)h.z);
+    const double err = 8.0 * ulp * sum, q = std::sqrt(q2);
+    const bool plain = q2 > 1e-20 && q2 < 1e20 && sum < 1e15;  // else FP64 decides
+    double lo = 0.0, hi = 3e38;
+    if (plain) {
+      lo = std::max(0.0, std::max(c * q2 / geo.ehi, q * smin) * (1.0 - kBandTol) - err);
+      hi = std::min(geo.elo > 0 ? c * q2 / geo.elo : 3e38, q * smax) * (1.0 + kBandTol) + err;
+      if (lo > hi) continue;  // no rotation puts it on the detector
+    }
+    const int i = (int)(seen->size() % kHklChunk);
+    if (i == 0) {
+      close_chunk();
+      units->push_back(BuildUnits{});
+      open.clear();
+      nu = 0;
+    }
+    BuildUnits &bu = units->back();
+    seen->push_back(h);
+    auto it = open.find(std::make_tuple(-h.x, -h.y, -h.z));
+    const bool zero = h.x == 0 && h.y == 0 && h.z == 0;
+    if (!zero && it != open.end() && !it->second.empty()) {
+      uint32_t &pos = bu.pos[it->second.back()];
+      pos = (pos & 0xFFFFu) | ((uint32_t)i << 16);
+      it->second.pop_back();
+      continue;
+    }
+    // NaN eps: every comparison of the detector screen fails, so it rejects nothing
+    const uint32_t band = plain ? bf16_bound(lo, true) << 16 | bf16_bound(hi, false) : 0x00007F80u;
+    float w;
+    memcpy(&w, &band, 4);
+    bu.hkl_band[nu] = make_float4((float)h.x, (float)h.y, (float)h.z, w);
+    bu.eps[nu] = plain ? (float)(256.0 * ulp * sum / q + 4e-6) : std::numeric_limits<float>::quiet_NaN();
+    bu.pos[nu] = (uint32_t)i | 0xFFFF0000u;
+    open[std::make_tuple(h.x, h.y, h.z)].push_back(nu);
+    nu++;
+  }
+  close_chunk();
 }
 
 // Threads per block so that the [S][TB] pixel lists fit in shared memory.
@@ -373,33 +529,90 @@ static int build_block(int S) {
   return tb;
 }
 
-size_t dbbuild_smem_bytes(int S) {
+static size_t dbbuild_smem_bytes(int S) {
   const int tb = build_block(S);
-  // HKL chunk (int and float copies), pixel lists, counts, per-warp queues of 64
-  return kHklChunk * 2 * sizeof(int4) + (size_t)S * tb * 4 + (size_t)tb * 4 + (size_t)tb * 8;
+  // a chunk's units, pixel lists, counts, two bit maps
+  return sizeof(BuildUnits) + (size_t)tb * 4 * ((size_t)S + 1 + 2 * kChunkWords);
 }
 
-int dbbuild_launch(const double *d_om, uint64_t n, const int4 *d_hkl, int nh,
-                   const lmb_geometry &geo, uint16_t *d_out, cudaStream_t st, bool exact_all) {
-  if (n == 0) return LMB_OK;
+// The HKL list with its screens on the device, for the builds of one call.
+struct BuildTables {
+  int4 *hkl = nullptr, *seen = nullptr;
+  BuildUnits *units = nullptr;
+  uint32_t *count = nullptr;
+  BuildGeo g{};
+  int nh = 0, nseen = 0;
+  bool all = false;  // FP64 for every pair
+};
+
+int dbbuild_tables(const lmb_geometry &geo, const int32_t *hkls, int nh, bool exact_all,
+                   cudaStream_t st, BuildTables **out) {
   const int S = geo.max_nr_spots;
   LMB_REQUIRE(S >= 1 && (size_t)S * 32 * 4 <= 160 * 1024,
               "MaxNrLaueSpots=%d outside the supported range 1..1280", S);
-  const BuildGeo g = make_build_geo(geo);
-  const bool all = exact_all || !screen_sound(geo);
-  const int tb = build_block(S);
-  const size_t smem = dbbuild_smem_bytes(S);
+  BuildTables *t = new BuildTables();
+  t->g = make_build_geo(geo);
+  t->nh = nh;
+  t->all = exact_all || !screen_sound(geo);
+  std::vector<int4> h((size_t)std::max(nh, 1));
+  for (int i = 0; i < nh; i++) h[i] = make_int4(hkls[3 * i], hkls[3 * i + 1], hkls[3 * i + 2], 0);
+  std::vector<int4> seen;
+  std::vector<BuildUnits> units;
+  std::vector<uint32_t> count;
+  if (!t->all) build_units(geo, h.data(), nh, &seen, &units, &count);
+  t->nseen = (int)seen.size();
+  // one allocation and one copy: HKLs | seen HKLs | units | unit counts
+  std::vector<unsigned char> host;
+  auto part = [&](const void *src, size_t bytes) {  // 256-byte aligned parts
+    const size_t at = host.size();
+    host.resize(at + (bytes + 255) / 256 * 256);
+    std::copy_n(static_cast<const unsigned char *>(src), bytes, host.begin() + (ptrdiff_t)at);
+    return at;
+  };
+  const size_t oh = part(h.data(), h.size() * sizeof(int4));
+  const size_t os = part(seen.data(), seen.size() * sizeof(int4));
+  const size_t ou = part(units.data(), units.size() * sizeof(BuildUnits));
+  const size_t oc = part(count.data(), count.size() * sizeof(uint32_t));
+  unsigned char *d = nullptr;
+  cudaError_t ce = cudaMalloc(&d, host.size());
+  if (ce == cudaSuccess) ce = cudaMemcpyAsync(d, host.data(), host.size(), cudaMemcpyHostToDevice, st);
+  if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
+  const void *fn = t->all ? (const void *)dbbuild_kernel<true> : (const void *)dbbuild_kernel<false>;
+  if (ce == cudaSuccess)
+    ce = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)dbbuild_smem_bytes(S));
+  if (ce != cudaSuccess) {
+    cudaFree(d);
+    delete t;
+    return cuda_fail(ce, "DB build tables", __FILE__, __LINE__);
+  }
+  t->hkl = reinterpret_cast<int4 *>(d + oh);  // oh = 0: the allocation itself
+  t->seen = reinterpret_cast<int4 *>(d + os);
+  t->units = reinterpret_cast<BuildUnits *>(d + ou);
+  t->count = reinterpret_cast<uint32_t *>(d + oc);
+  *out = t;
+  return LMB_OK;
+}
+
+void dbbuild_tables_free(BuildTables *t) {
+  if (!t) return;
+  cudaFree(t->hkl);
+  delete t;
+}
+
+int dbbuild_launch(const double *d_om, uint64_t n, const BuildTables *t, uint16_t *d_out,
+                   cudaStream_t st) {
+  if (n == 0) return LMB_OK;
+  const int tb = build_block(t->g.S);
+  const size_t smem = dbbuild_smem_bytes(t->g.S);
   const uint64_t blocks = (n + tb - 1) / tb;
   LMB_REQUIRE(blocks < (1ull << 31), "too many orientations (%llu)", (unsigned long long)n);
-  if (all) {
-    LMB_CUDA(cudaFuncSetAttribute(dbbuild_kernel<true>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dbbuild_kernel<true><<<(unsigned)blocks, tb, smem, st>>>(d_om, n, d_hkl, nh, g, d_out);
-  } else {
-    LMB_CUDA(cudaFuncSetAttribute(dbbuild_kernel<false>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dbbuild_kernel<false><<<(unsigned)blocks, tb, smem, st>>>(d_om, n, d_hkl, nh, g, d_out);
-  }
+  if (t->all)
+    dbbuild_kernel<true><<<(unsigned)blocks, tb, smem, st>>>(d_om, n, t->hkl, t->nh, t->seen, t->nseen,
+                                                             t->units, t->count, t->g, d_out);
+  else
+    dbbuild_kernel<false><<<(unsigned)blocks, tb, smem, st>>>(d_om, n, t->hkl, t->nh, t->seen, t->nseen,
+                                                              t->units, t->count, t->g, d_out);
   LMB_CUDA(cudaGetLastError());
   return LMB_OK;
 }

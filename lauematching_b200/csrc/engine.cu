@@ -304,15 +304,6 @@ int alloc_db(lmb_engine *e, uint64_t n) {
   return LMB_OK;
 }
 
-int upload_hkls(const int32_t *hkls, int nh, int4 **d_out) {
-  std::vector<int4> h((size_t)std::max(nh, 1));
-  for (int i = 0; i < nh; i++) h[i] = make_int4(hkls[3 * i], hkls[3 * i + 1], hkls[3 * i + 2], 0);
-  LMB_CUDA(cudaMalloc(d_out, h.size() * sizeof(int4)));
-  LMB_CUDA(cudaMemcpy(*d_out, h.data(), (size_t)nh * sizeof(int4), cudaMemcpyHostToDevice));
-  return LMB_OK;
-}
-
-
 // Host scan of a frame: if its positive pixels, as (uint32 index, value)
 // pairs, take less than half the dense bytes, upload the pairs (through a
 // ring of pinned staging buffers) and scatter them on the load stream;
@@ -898,14 +889,14 @@ static int db_build_common(lmb_engine *e, const double *orients, uint64_t seed, 
   LMB_CUDA(cudaStreamSynchronize(e->st));
   rc = alloc_db(e, n);
   if (rc) return rc;
-  int4 *d_hkl = nullptr;
-  rc = upload_hkls(hkls, nh, &d_hkl);
+  BuildTables *tables = nullptr;
+  rc = dbbuild_tables(e->geo, hkls, nh, (flags & LMB_BUILD_EXACT_FP64) != 0, e->st, &tables);
   if (rc) return rc;
   const uint64_t kChunk = 4ull << 20;  // orientations per chunk (288 MB of matrices)
   double *d_om = nullptr;
   cudaError_t ce = cudaMalloc(&d_om, std::min(kChunk, std::max<uint64_t>(n, 1)) * 72);
   if (ce != cudaSuccess) {
-    cudaFree(d_hkl);
+    dbbuild_tables_free(tables);
     return cuda_fail(ce, "cudaMalloc(orientation chunk)", __FILE__, __LINE__);
   }
   for (uint64_t off = 0; off < n && rc == LMB_OK; off += kChunk) {
@@ -916,8 +907,7 @@ static int db_build_common(lmb_engine *e, const double *orients, uint64_t seed, 
       rc = upload_chunked(e, d_om, orients + off * 9, len * 72, e->st);
     }
     if (rc == LMB_OK)
-      rc = dbbuild_launch(d_om, len, d_hkl, nh, e->geo, e->d_db + off * e->R, e->st,
-                          (flags & LMB_BUILD_EXACT_FP64) != 0);
+      rc = dbbuild_launch(d_om, len, tables, e->d_db + off * e->R, e->st);
     if (rc == LMB_OK && synthetic && orients_out) {
       ce = cudaMemcpyAsync(orients_out + off * 9, d_om, len * 72, cudaMemcpyDeviceToHost, e->st);
       e->bytes_d2h += len * 72;
@@ -927,7 +917,7 @@ static int db_build_common(lmb_engine *e, const double *orients, uint64_t seed, 
     if (ce != cudaSuccess && rc == LMB_OK) rc = cuda_fail(ce, "DB build", __FILE__, __LINE__);
   }
   cudaFree(d_om);
-  cudaFree(d_hkl);
+  dbbuild_tables_free(tables);
   e->on_detector = rc == LMB_OK;
   return rc;
 }

@@ -95,8 +95,13 @@ struct OrderArgs {
   int slots[LMB_MAX_SLOTS];
 };
 
-int dbbuild_launch(const double *d_om, uint64_t n, const int4 *d_hkl, int nh,
-                   const lmb_geometry &geo, uint16_t *d_out, cudaStream_t st, bool exact_all);
+// The HKL list and its screens on the device, for the chunks of one build.
+struct BuildTables;
+int dbbuild_tables(const lmb_geometry &geo, const int32_t *hkls, int nh, bool exact_all,
+                   cudaStream_t st, BuildTables **out);
+void dbbuild_tables_free(BuildTables *t);
+int dbbuild_launch(const double *d_om, uint64_t n, const BuildTables *t, uint16_t *d_out,
+                   cudaStream_t st);
 int synth_orient_launch(uint64_t seed, uint64_t first, uint64_t n, double *d_out,
                         cudaStream_t st, uint32_t flags = 0);
 int quantize_launch(const void *d_img, int dtype, size_t npx, unsigned long long *d_max_bits,
