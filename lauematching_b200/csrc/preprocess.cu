@@ -3,8 +3,9 @@
 // scipy and OpenCV, with identical results:
 //
 //   background   exact square median (scipy.ndimage.median_filter, mirrored
-//                borders): pixels become ranks among the frame's distinct
-//                values; one warp per (column, row segment) slides its window
+//                borders).  Frames of whole numbers: tile by tile, window counts
+//                below a few thresholds around the tile's medians.  Others: pixels
+//                become ranks among the frame's distinct values; one warp per (column, row segment) slides its window
 //                down, keeping 8-bit-digit rank histograms level by level and
 //                refilling a deeper level only when the digit above it moves.
 //   threshold    order statistics (np.median, np.percentile) by radix
@@ -1408,6 +1409,183 @@ __global__ void __launch_bounds__(kMedWarps * 32, 4)
   }
 }
 
+// Median of a frame of whole numbers (0..65535), tile by tile.
+//
+// A background changes slowly: the medians of the 64 x 32 windows around a tile are
+// a handful of neighbouring values.  For one threshold t the number of values below
+// t in every window of the tile comes from two sliding sums over the tile and its
+// halo (in shared memory), and median >= t exactly when that number is at most
+// k = s * s / 2.  A block starts at the median of 256 of its values and moves t by
+// doubling steps, then by halves, until every pixel has count(m) <= k <
+// count(m + 1).  A tile that needs more than kMedTries thresholds (wild values)
+// is counted in *unresolved and the frame takes the rank path.  Bound by
+// instruction issue: about 3 instructions per value of tile and halo and threshold,
+// against 2 s shared-memory atomics per pixel on the rank path.  Measured on B200,
+// 2048^2 detector frame, s = 101: ranks and median 4.50 ms there, 0.26 ms here.
+constexpr int kMtX = 64, kMtY = 32, kMtThreads = 256;
+constexpr int kMedTries = 48;
+constexpr int kMedTileMaxS = 255;  // a column sum is a byte
+
+size_t median_tile_smem(int s) {
+  const size_t cols = kMtX + s - 1, rows = kMtY + s - 1;
+  // values | column sums | per warp the prefix sums of a row | the sample
+  return (rows * cols * 2 + 15) / 16 * 16 + (kMtY * cols + 15) / 16 * 16 +
+         (kMtThreads / 32) * (cols + 1) * 4 + kMtThreads * 4;
+}
+
+__global__ void __launch_bounds__(kMtThreads)
+    median_tile_kernel(const uint16_t *__restrict__ img, int ny, int nx, int s, double *__restrict__ out,
+                       uint16_t *__restrict__ out16, unsigned *__restrict__ unresolved) {
+  extern __shared__ __align__(16) double sm[];  // (declared as the blur's)
+  const int cols = kMtX + s - 1, rows = kMtY + s - 1;
+  uint16_t *val = reinterpret_cast<uint16_t *>(sm);
+  unsigned char *csum = reinterpret_cast<unsigned char *>(sm) + ((size_t)rows * cols * 2 + 15) / 16 * 16;
+  unsigned *pre_all = reinterpret_cast<unsigned *>(csum + ((size_t)kMtY * cols + 15) / 16 * 16);
+  unsigned *sample = pre_all + (kMtThreads / 32) * (cols + 1);
+  __shared__ unsigned key_s, guess_s;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  unsigned *pre = pre_all + warp * (cols + 1);
+  const int lo = s / 2;
+  const int x0 = blockIdx.x * kMtX, y0 = blockIdx.y * kMtY;
+  for (int r = warp; r < rows; r += kMtThreads / 32) {
+    const uint16_t *src = img + (size_t)mirror(y0 - lo + r, ny) * nx;
+    for (int c = lane; c < cols; c += 32) val[r * cols + c] = src[mirror(x0 - lo + c, nx)];
+  }
+  if (t == 0) guess_s = 0u;
+  __syncthreads();
+  // the median of 256 values spread over tile and halo
+  sample[t] = val[(int)((long long)(2 * t + 1) * rows * cols / (2 * kMtThreads))];
+  __syncthreads();
+  {
+    const unsigned mine = sample[t];
+    int below = 0;
+    for (int j = 0; j < kMtThreads; j++) below += sample[j] < mine ? 1 : 0;
+    // the largest value with at most half of the sample below it
+    if (below <= kMtThreads / 2) atomicMax(&guess_s, mine);
+  }
+  __syncthreads();
+  // this thread's pixels: columns lane and lane + 32 of rows warp, warp + 8, ...
+  constexpr int kRows = kMtY / (kMtThreads / 32), kOwn = 2 * kRows;
+  unsigned L[kOwn], H[kOwn];  // L <= median < H
+#pragma unroll
+  for (int i = 0; i < kOwn; i++) {
+    const int gx = x0 + lane + 32 * (i & 1), gy = y0 + warp + (i >> 1) * (kMtThreads / 32);
+    L[i] = 0u;
+    H[i] = gx < nx && gy < ny ? 65536u : 1u;  // outside the frame: nothing to find
+  }
+  const unsigned k = (unsigned)s * (unsigned)s / 2u;
+  const int per = (cols + 31) / 32;
+  unsigned thr = guess_s;
+  unsigned step_up = 1u, step_down = 1u;
+  bool found = false;
+  for (int round = 0; round < kMedTries; round++) {
+    if (thr > 0u) {
+      // values below thr: column sums of s rows, for every row of the tile
+      for (int c = t; c < cols; c += kMtThreads) {
+        const uint16_t *col = val + c;
+        unsigned n = 0;
+        for (int r = 0; r < s; r++) n += col[r * cols] < thr ? 1u : 0u;
+        csum[c] = (unsigned char)n;
+#pragma unroll 4
+        for (int r = 1; r < kMtY; r++) {
+          n += (col[(r + s - 1) * cols] < thr ? 1u : 0u) - (col[(r - 1) * cols] < thr ? 1u : 0u);
+          csum[r * cols + c] = (unsigned char)n;
+        }
+      }
+      if (t == 0) key_s = 0xffffffffu;
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < kRows; q++) {
+        const unsigned char *row = csum + (warp + q * (kMtThreads / 32)) * cols;
+        unsigned sum = 0;
+        for (int j = 0; j < per; j++) {
+          const int c = lane * per + j;
+          sum += c < cols ? row[c] : 0u;
+        }
+        unsigned run = sum;  // exclusive prefix sum over the lanes
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const unsigned y = __shfl_up_sync(0xffffffffu, run, o);
+          if (lane >= o) run += y;
+        }
+        run -= sum;
+        for (int j = 0; j < per; j++) {
+          const int c = lane * per + j;
+          if (c > cols) break;
+          pre[c] = run;
+          run += c < cols ? row[c] : 0u;
+        }
+        if (lane == 31 && 32 * per <= cols) pre[cols] = run;
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int x = lane + 32 * h;
+          const unsigned cnt = pre[x + s] - pre[x];
+          const int i = 2 * q + h;
+          if (cnt <= k)
+            L[i] = max(L[i], thr);
+          else
+            H[i] = min(H[i], thr);
+        }
+        __syncwarp();
+      }
+    } else {
+      if (t == 0) key_s = 0xffffffffu;
+      __syncthreads();
+    }
+    // the lowest interval still open: its ends say where to look next
+    unsigned key = 0xffffffffu;
+#pragma unroll
+    for (int i = 0; i < kOwn; i++)
+      if (H[i] > L[i] + 1u) key = min(key, (L[i] << 16) | (H[i] - 1u));
+    key = __reduce_min_sync(0xffffffffu, key);
+    if (lane == 0 && key != 0xffffffffu) atomicMin(&key_s, key);
+    __syncthreads();
+    const unsigned open = key_s;
+    __syncthreads();  // before the next round's reset
+    if (open == 0xffffffffu) {
+      found = true;
+      break;
+    }
+    const unsigned l = open >> 16, h = (open & 0xFFFFu) + 1u;
+    if (l == 0u && h == 65536u) {  // nothing known: only thr = 0 comes here
+      thr = 1u;
+    } else if (h == 65536u) {  // no upper end yet
+      thr = min(l + step_up, 65535u);
+      step_up *= 2u;
+    } else if (l == 0u && h > step_down) {  // no lower end yet
+      thr = h - step_down;
+      step_down *= 2u;
+    } else {
+      thr = (l + h) / 2u;
+    }
+  }
+  if (!found && t == 0) atomicAdd(unresolved, 1u);
+#pragma unroll
+  for (int i = 0; i < kOwn; i++) {
+    const int gx = x0 + lane + 32 * (i & 1), gy = y0 + warp + (i >> 1) * (kMtThreads / 32);
+    if (gx < nx && gy < ny) {
+      out[(size_t)gy * nx + gx] = (double)L[i];
+      out16[(size_t)gy * nx + gx] = (uint16_t)L[i];
+    }
+  }
+}
+
+// A frame as 16-bit whole numbers; *other is set when a value is not one.
+template <typename T>
+__global__ void whole_kernel(const T *__restrict__ in, uint16_t *__restrict__ out,
+                             unsigned *__restrict__ other, size_t n) {
+  bool bad = false;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x) {
+    const double v = to_f64(in[i]);
+    const bool ok = v >= 0.0 && v <= 65535.0 && v == trunc(v) && !signbit(v);
+    bad |= !ok;
+    out[i] = ok ? (uint16_t)v : (uint16_t)0;
+  }
+  if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(other, 1u);
+}
+
 }  // namespace
 
 // ---- handle ------------------------------------------------------------------------
@@ -1440,6 +1618,10 @@ struct lmb_pre {
   double *m_vals = nullptr, *m_img = nullptr;
   void *m_cub = nullptr;
   size_t m_cub_bytes = 0;
+  // medians of whole numbers: frame and result as uint16 (taken in turn), and what
+  // sends a frame to the rank path (not whole numbers, unresolved tiles)
+  uint16_t *m_v16[2] = {nullptr, nullptr};
+  unsigned *m_flag16 = nullptr;
   bool segmented = false;
   lmb_pre_counts last{};
   // stage events: frame upload, threshold, components, blur, download, median ranks, median
@@ -1471,7 +1653,8 @@ void free_pre(lmb_pre *p) {
                   p->c.fb, p->c.sw, p->c.swx, p->c.swy, p->c.label, p->c.keep, p->d_flags,
                   p->d_pos, p->d_compact, p->d_centres, p->d_w, p->d_stats, p->d_head, p->d_next,
                   p->d_state, p->d_cub, p->d_hist16, p->d_fg, p->d_nfg, p->d_fg_tmp, p->m_keys, p->m_keys2, p->m_idx, p->m_idx2, p->m_flag,
-                  p->m_incl, p->m_rank, p->m_nd, p->m_vals, p->m_img, p->m_cub};
+                  p->m_incl, p->m_rank, p->m_nd, p->m_vals, p->m_img, p->m_cub,
+                  p->m_v16[0], p->m_v16[1], p->m_flag16};
   for (void *b : bufs)
     if (b) cudaFree(b);
   if (p->h_state) cudaFreeHost(p->h_state);
@@ -1677,6 +1860,52 @@ int median_pass(lmb_pre *p, const double *d_in, double *d_out, int size) {
   return LMB_OK;
 }
 
+// All median passes of a frame of whole numbers; *done = false when it is none or a
+// tile was not resolved (the rank path then starts again from the frame).
+int median_whole(lmb_pre *p, int dtype, int size, int passes, bool *done) {
+  *done = false;
+  if (size > kMedTileMaxS) return LMB_OK;
+  cudaStream_t st = p->st;
+  const size_t smem = median_tile_smem(size);
+  if (!p->m_flag16) {
+    int rc;
+    if ((rc = alloc(&p->m_v16[0], p->npx)) || (rc = alloc(&p->m_v16[1], p->npx)) ||
+        (rc = alloc(&p->m_flag16, 1)))
+      return rc;
+  }
+  LMB_CUDA(cudaFuncSetAttribute(median_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)median_tile_smem(kMedTileMaxS)));
+  LMB_CUDA(cudaEventRecord(p->ev[EV_MED_PASS], st));
+  LMB_CUDA(cudaMemsetAsync(p->m_flag16, 0, sizeof(unsigned), st));
+  const unsigned g = (unsigned)grid_for(p->npx, p->num_sms);
+  const uint16_t *in = p->m_v16[0];
+  if (dtype == LMB_U16) {
+    in = static_cast<const uint16_t *>(p->d_raw);
+  } else {
+    const int rc = by_dtype(dtype, [&](auto tag) {
+      using T = std::remove_const_t<std::remove_pointer_t<decltype(tag)>>;
+      whole_kernel<T><<<g, kT, 0, st>>>(static_cast<const T *>(p->d_raw), p->m_v16[0], p->m_flag16,
+                                        p->npx);
+      return LMB_OK;
+    });
+    if (rc) return rc;
+  }
+  LMB_CUDA(cudaEventRecord(p->ev[EV_MED_RANK], st));
+  const dim3 tiles((p->nx + kMtX - 1) / kMtX, (p->ny + kMtY - 1) / kMtY);
+  for (int i = 0; i < passes; ++i) {
+    uint16_t *to = p->m_v16[(i + 1) & 1];
+    median_tile_kernel<<<tiles, kMtThreads, smem, st>>>(in, p->ny, p->nx, size, p->d_bg, to,
+                                                        p->m_flag16);
+    in = to;
+  }
+  LMB_CUDA(cudaGetLastError());
+  LMB_CUDA(cudaEventRecord(p->ev[EV_MED_K], st));
+  LMB_CUDA(cudaMemcpyAsync(&p->h_state->n_comp, p->m_flag16, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+  LMB_CUDA(cudaStreamSynchronize(st));
+  *done = p->h_state->n_comp == 0;
+  return LMB_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1798,15 +2027,17 @@ int lmb_pre_median(lmb_pre *p, const void *frame, int32_t dtype, int32_t size, i
   LMB_CUDA(cudaEventRecord(p->ev[EV_MED0], p->st));
   if ((rc = upload_frame(p, frame, dtype))) return rc;
   LMB_CUDA(cudaEventRecord(p->ev[EV_MED_UP], p->st));
-  if ((rc = ensure_median_scratch(p))) return rc;
+  bool done = false;
+  if (size > 1 && passes > 0 && (rc = median_whole(p, dtype, size, passes, &done))) return rc;
+  if (!done && (rc = ensure_median_scratch(p))) return rc;
   const unsigned g = (unsigned)grid_for(p->npx, p->num_sms);
-  rc = by_dtype(dtype, [&](auto tag) {
+  if (!done) rc = by_dtype(dtype, [&](auto tag) {
     using T = std::remove_const_t<std::remove_pointer_t<decltype(tag)>>;
     to_f64_kernel<T><<<g, kT, 0, p->st>>>(static_cast<const T *>(p->d_raw), p->d_bg, p->npx);
     return LMB_OK;
   });
   if (rc) return rc;
-  if (size > 1) {
+  if (size > 1 && !done) {
     for (int i = 0; i < passes; ++i) {
       LMB_CUDA(cudaMemcpyAsync(p->m_img, p->d_bg, p->npx * sizeof(double),
                                cudaMemcpyDeviceToDevice, p->st));
