@@ -22,6 +22,7 @@
 // (2 s of global time) and report through an error word.
 #include <climits>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "kernels.cuh"
@@ -51,14 +52,37 @@ static int ensure_smem(const void *fn, int bytes) {
 // ----------------------------------------------------------------------------
 // Quantisation: max of the positive pixels, then uint8 + occupancy bit.
 // ----------------------------------------------------------------------------
+// Four pixels per thread where the frame allows it (npx a multiple of 4, as every
+// slot's base then is): 16-byte loads of the frame.  Bound by the frame's read; the
+// occupancy words (8 bytes per pixel, 32 MB at 2048^2) are touched only where a
+// pixel becomes or ceases to be positive, since a slot's bit is set exactly while
+// its uint8 pixel is positive.  Measured on B200 (cold caches), 2048^2 float32 frame
+// with 0.1 % of its pixels positive: quantisation 18.5 -> 11.7 us.
 template <typename T>
+struct alignas(sizeof(T) * 4 > 16 ? 16 : sizeof(T) * 4) Four {
+  T v[4];
+};
+
+template <typename T, int V>
 __global__ void quant_max_kernel(const T *__restrict__ img, size_t npx,
                                  unsigned long long *__restrict__ max_bits) {
   double m = 0.0;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < npx;
+  const size_t n = npx / V;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
-    const double v = (double)img[i];
-    if (v > m) m = v;  // NaN never compares greater (LaueMatchingCPU.c:357-359)
+    T x[V];
+    if constexpr (V == 4) {
+      const Four<T> f = reinterpret_cast<const Four<T> *>(img)[i];
+#pragma unroll
+      for (int j = 0; j < 4; j++) x[j] = f.v[j];
+    } else {
+      x[0] = img[i];
+    }
+#pragma unroll
+    for (int j = 0; j < V; j++) {
+      const double v = (double)x[j];
+      if (v > m) m = v;  // NaN never compares greater (LaueMatchingCPU.c:357-359)
+    }
   }
   for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
   __shared__ double sm[32];
@@ -74,7 +98,7 @@ __global__ void quant_max_kernel(const T *__restrict__ img, size_t npx,
 
 // u8 = v>=255 ? 255 : v<1 ? 1 : (uint8)v  with v = pixel * (255/max), for
 // positive pixels; 0 otherwise (LaueMatchingCPU.c:367-375).
-template <typename T>
+template <typename T, int V>
 __global__ void quant_u8_kernel(const T *__restrict__ img, size_t npx,
                                 const unsigned long long *__restrict__ max_bits,
                                 uint8_t *__restrict__ u8, double *__restrict__ f64_keep,
@@ -83,19 +107,50 @@ __global__ void quant_u8_kernel(const T *__restrict__ img, size_t npx,
   const double mx = __longlong_as_double((long long)*max_bits);
   const double inv = (mx > 0) ? ddiv(255.0, mx) : 0.0;
   if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = (mx > 0) ? ddiv(mx, 255.0) : 1.0;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < npx;
+  const size_t n = npx / V;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
-    const double x = (double)img[i];
-    uint8_t q = 0;
-    if (x > 0) {
-      const double v = dmul(x, inv);
-      // (uint8_t)v of a double: x86 converts via a 32-bit cvttsd2si (NaN -> 0)
-      q = (v >= 255.0) ? 255 : (v < 1.0) ? 1 : (uint8_t)(x86_trunc_i32(v) & 0xFF);
+    T xs[V];
+    uint8_t old[V], now[V];
+    if constexpr (V == 4) {
+      const Four<T> f = reinterpret_cast<const Four<T> *>(img)[i];
+      const Four<uint8_t> o = reinterpret_cast<const Four<uint8_t> *>(u8)[i];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        xs[j] = f.v[j];
+        old[j] = o.v[j];
+      }
+    } else {
+      xs[0] = img[i];
+      old[0] = u8[i];
     }
-    u8[i] = q;
-    if (f64_keep) f64_keep[i] = x;
-    const unsigned long long w = occ[i];
-    occ[i] = q ? (w | bit) : (w & ~bit);
+    bool changed = false;
+#pragma unroll
+    for (int j = 0; j < V; j++) {
+      const double x = (double)xs[j];
+      uint8_t q = 0;
+      if (x > 0) {
+        const double v = dmul(x, inv);
+        // (uint8_t)v of a double: x86 converts via a 32-bit cvttsd2si (NaN -> 0)
+        q = (v >= 255.0) ? 255 : (v < 1.0) ? 1 : (uint8_t)(x86_trunc_i32(v) & 0xFF);
+      }
+      now[j] = q;
+      changed |= q != old[j];
+      if (f64_keep) f64_keep[i * V + j] = x;
+      if ((q != 0) != (old[j] != 0)) {
+        const unsigned long long w = occ[i * V + j];
+        occ[i * V + j] = q ? (w | bit) : (w & ~bit);
+      }
+    }
+    if (!changed) continue;
+    if constexpr (V == 4) {
+      Four<uint8_t> o;
+#pragma unroll
+      for (int j = 0; j < 4; j++) o.v[j] = now[j];
+      reinterpret_cast<Four<uint8_t> *>(u8)[i] = o;
+    } else {
+      u8[i] = now[0];
+    }
   }
 }
 
@@ -1466,28 +1521,39 @@ __global__ void __launch_bounds__(1024) order_kernel(OrderArgs a) {
 // ----------------------------------------------------------------------------
 // Launchers
 // ----------------------------------------------------------------------------
+template <typename T, int V>
+static void quantize_as(const T *img, size_t npx, unsigned long long *d_max_bits, bool max_ready,
+                        uint8_t *d_u8, double *d_f64_keep, unsigned long long *d_occ,
+                        unsigned long long bit, double *d_scale_slot, int num_sms, cudaStream_t st) {
+  const unsigned blocks =
+      (unsigned)std::max<size_t>(1, std::min<size_t>((npx / V + 255) / 256, (size_t)num_sms * 8));
+  if (!max_ready) quant_max_kernel<T, V><<<blocks, 256, 0, st>>>(img, npx, d_max_bits);
+  quant_u8_kernel<T, V><<<blocks, 256, 0, st>>>(img, npx, d_max_bits, d_u8, d_f64_keep, d_occ, bit,
+                                                d_scale_slot);
+}
+
 int quantize_launch(const void *d_img, int dtype, size_t npx, unsigned long long *d_max_bits,
-                    uint8_t *d_u8, double *d_f64_keep, unsigned long long *d_occ, int slot,
-                    double *d_scale_slot, int num_sms, cudaStream_t st) {
-  LMB_CUDA(cudaMemsetAsync(d_max_bits, 0, sizeof(unsigned long long), st));
-  const unsigned blocks = (unsigned)std::min<size_t>((npx + 255) / 256, (size_t)num_sms * 8);
+                    bool max_ready, uint8_t *d_u8, double *d_f64_keep, unsigned long long *d_occ,
+                    int slot, double *d_scale_slot, int num_sms, cudaStream_t st) {
+  if (!max_ready) LMB_CUDA(cudaMemsetAsync(d_max_bits, 0, sizeof(unsigned long long), st));
   const unsigned long long bit = 1ull << slot;
-  if (dtype == LMB_F64) {
-    const double *p = static_cast<const double *>(d_img);
-    quant_max_kernel<double><<<blocks, 256, 0, st>>>(p, npx, d_max_bits);
-    quant_u8_kernel<double><<<blocks, 256, 0, st>>>(p, npx, d_max_bits, d_u8, d_f64_keep, d_occ,
-                                                     bit, d_scale_slot);
-  } else if (dtype == LMB_F32) {
-    const float *p = static_cast<const float *>(d_img);
-    quant_max_kernel<float><<<blocks, 256, 0, st>>>(p, npx, d_max_bits);
-    quant_u8_kernel<float><<<blocks, 256, 0, st>>>(p, npx, d_max_bits, d_u8, d_f64_keep, d_occ,
-                                                    bit, d_scale_slot);
-  } else {
-    const uint8_t *p = static_cast<const uint8_t *>(d_img);
-    quant_max_kernel<uint8_t><<<blocks, 256, 0, st>>>(p, npx, d_max_bits);
-    quant_u8_kernel<uint8_t><<<blocks, 256, 0, st>>>(p, npx, d_max_bits, d_u8, d_f64_keep, d_occ,
-                                                      bit, d_scale_slot);
-  }
+  const bool four = npx % 4 == 0 && (reinterpret_cast<uintptr_t>(d_img) & 15) == 0 &&
+                    (reinterpret_cast<uintptr_t>(d_u8) & 3) == 0;
+  auto go = [&](auto *img) {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(img)>>;
+    if (four)
+      quantize_as<T, 4>(img, npx, d_max_bits, max_ready, d_u8, d_f64_keep, d_occ, bit, d_scale_slot,
+                        num_sms, st);
+    else
+      quantize_as<T, 1>(img, npx, d_max_bits, max_ready, d_u8, d_f64_keep, d_occ, bit, d_scale_slot,
+                        num_sms, st);
+  };
+  if (dtype == LMB_F64)
+    go(static_cast<const double *>(d_img));
+  else if (dtype == LMB_F32)
+    go(static_cast<const float *>(d_img));
+  else
+    go(static_cast<const uint8_t *>(d_img));
   LMB_CUDA(cudaGetLastError());
   return LMB_OK;
 }

@@ -1011,7 +1011,7 @@ int lmb_image_load(lmb_engine *e, int32_t slot, const void *pixels, int32_t dtyp
     LMB_CUDA(cudaMemcpyAsync(e->d_stage, pixels, e->npx * dtype_bytes(dtype),
                              cudaMemcpyHostToDevice, e->ld));
     e->bytes_h2d += e->npx * dtype_bytes(dtype);
-    rc = quantize_launch(e->d_stage, dtype, e->npx, e->d_max_bits,
+    rc = quantize_launch(e->d_stage, dtype, e->npx, e->d_max_bits, false,
                          e->d_u8 + (size_t)slot * e->npx,
                          keep_f64 ? e->d_f64 + (size_t)slot * e->npx : nullptr, e->d_occ, slot,
                          e->d_scale + slot, e->num_sms, e->ld);
@@ -1051,7 +1051,7 @@ int dense_load(lmb_engine *e, int slot, const void *pixels, int dtype) {
   const size_t bytes = e->npx * dtype_bytes(dtype);
   LMB_CUDA(cudaMemcpyAsync(e->d_stage, pixels, bytes, cudaMemcpyHostToDevice, e->ld));
   e->bytes_h2d += bytes;
-  const int rc = quantize_launch(e->d_stage, dtype, e->npx, e->d_max_bits,
+  const int rc = quantize_launch(e->d_stage, dtype, e->npx, e->d_max_bits, false,
                                  e->d_u8 + (size_t)slot * e->npx, nullptr, e->d_occ, slot,
                                  e->d_scale + slot, e->num_sms, e->ld);
   if (rc) return rc;
@@ -1568,11 +1568,12 @@ namespace lmb {
 
 // A frame already in this engine's device memory (written on another stream
 // that recorded `ready`) into a slot: the dense quantisation of
-// lmb_image_load without any host copy; `consumed` is recorded once the
-// frame has been read, so its producer may overwrite it.
+// lmb_image_load without any host copy; d_max_bits, unless null, already holds
+// the frame's maximum; `consumed` is recorded once frame and maximum have been
+// read, so their producer may overwrite them.
 int engine_load_device_frame(lmb_engine *e, int slot, const void *d_img, int dtype,
-                             int nr_px_y, int nr_px_x, cudaEvent_t ready, cudaEvent_t consumed,
-                             double *im_scale) {
+                             int nr_px_y, int nr_px_x, unsigned long long *d_max_bits,
+                             cudaEvent_t ready, cudaEvent_t consumed, double *im_scale) {
   int rc = check_engine(e);
   if (rc) return rc;
   LMB_REQUIRE(slot >= 0 && slot < LMB_MAX_SLOTS, "slot %d outside 0..%d", slot,
@@ -1583,8 +1584,8 @@ int engine_load_device_frame(lmb_engine *e, int slot, const void *d_img, int dty
               e->geo.nr_px_x);
   LMB_CUDA(cudaStreamWaitEvent(e->ld, e->ev_released[slot], 0));
   LMB_CUDA(cudaStreamWaitEvent(e->ld, ready, 0));
-  rc = quantize_launch(d_img, dtype, e->npx, e->d_max_bits, e->d_u8 + (size_t)slot * e->npx,
-                       nullptr, e->d_occ, slot, e->d_scale + slot, e->num_sms, e->ld);
+  rc = quantize_launch(d_img, dtype, e->npx, d_max_bits ? d_max_bits : e->d_max_bits,
+                       d_max_bits != nullptr, e->d_u8 + (size_t)slot * e->npx, nullptr, e->d_occ, slot, e->d_scale + slot, e->num_sms, e->ld);
   if (rc) return rc;
   LMB_CUDA(cudaEventRecord(consumed, e->ld));
   LMB_CUDA(cudaEventRecord(e->ev_loaded[slot], e->ld));

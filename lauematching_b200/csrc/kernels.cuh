@@ -104,12 +104,14 @@ int dbbuild_launch(const double *d_om, uint64_t n, const BuildTables *t, uint16_
                    cudaStream_t st);
 int synth_orient_launch(uint64_t seed, uint64_t first, uint64_t n, double *d_out,
                         cudaStream_t st, uint32_t flags = 0);
+// max_ready: *d_max_bits holds the bits of the frame's largest positive value (0
+// without one) already; else it is found first.
 int quantize_launch(const void *d_img, int dtype, size_t npx, unsigned long long *d_max_bits,
-                    uint8_t *d_u8, double *d_f64_keep, unsigned long long *d_occ, int slot,
-                    double *d_scale_slot, int num_sms, cudaStream_t st);
+                    bool max_ready, uint8_t *d_u8, double *d_f64_keep, unsigned long long *d_occ,
+                    int slot, double *d_scale_slot, int num_sms, cudaStream_t st);
 int engine_load_device_frame(lmb_engine *e, int slot, const void *d_img, int dtype,
-                             int nr_px_y, int nr_px_x, cudaEvent_t ready, cudaEvent_t consumed,
-                             double *im_scale);
+                             int nr_px_y, int nr_px_x, unsigned long long *d_max_bits,
+                             cudaEvent_t ready, cudaEvent_t consumed, double *im_scale);
 int engine_device(const lmb_engine *e);
 int sparse_load_launch(const uint32_t *d_idx, const void *d_val, int dtype, size_t nnz, double mx,
                        uint8_t *d_u8, unsigned long long *d_occ, int slot, double *d_scale_slot,

@@ -1163,10 +1163,16 @@ __global__ void __launch_bounds__(256)
 // a row (axis-1 pass) in registers, 4 + 2R inputs, each converted once.
 constexpr int kBlurFixedMaxR = 8;
 
+// A tile without a positive pixel in reach (most of a filtered frame) is all zero
+// (skip_zero: the weights are finite and not negative, so no term has a sign).
+// max_bits, unless null, takes the bits of the frame's largest positive value.
+// Measured on B200 (cold caches), 2048^2 frame of 50 spots, float32 result: 37.4 us
+// with every tile computed (FP64 issue), 25.3 us.
 template <int R, typename TOut>
 __global__ void __launch_bounds__(256)
     blur_tile_r_kernel(const uint16_t *__restrict__ in, const double *__restrict__ wts, int ny,
-                       int nx, TOut *__restrict__ out) {
+                       int nx, int skip_zero, unsigned long long *__restrict__ max_bits,
+                       TOut *__restrict__ out) {
   constexpr int W = kBlurTile + 2 * R;
   __shared__ double w[2 * R + 1];
   __shared__ double vert[kBlurTile * W];
@@ -1177,12 +1183,19 @@ __global__ void __launch_bounds__(256)
   // mirrored source columns of this lane (W <= 48 < 64)
   const int c0 = mirror(x0 - R + lane, nx);
   const int c1 = lane + 32 < W ? mirror(x0 - R + lane + 32, nx) : 0;
+  unsigned any = 0u;
   for (int row = warp; row < W; row += 8) {
     const uint16_t *src = in + (size_t)mirror(y0 - R + row, ny) * nx;
-    tile[row * W + lane] = src[c0];
-    if (lane + 32 < W) tile[row * W + lane + 32] = src[c1];
+    any |= tile[row * W + lane] = src[c0];
+    if (lane + 32 < W) any |= tile[row * W + lane + 32] = src[c1];
   }
-  __syncthreads();
+  if (!__syncthreads_or(any != 0u) && skip_zero) {
+    const int gx = x0 + lane;
+    for (int row = warp; row < kBlurTile; row += 8)
+      if (y0 + row < ny && gx < nx) out[(size_t)(y0 + row) * nx + gx] = (TOut)0;
+    return;
+  }
+  double most = 0.0;
   // axis 0: task = (group of 4 output rows, tile column)
   for (int task = t; task < 8 * W; task += 256) {
     const int rg = task / W, col = task - rg * W;
@@ -1214,24 +1227,30 @@ __global__ void __launch_bounds__(256)
       for (int j = R; j >= 1; --j)
         acc = lmb::dadd(acc, lmb::dmul(lmb::dadd(v[o + R - j], v[o + R + j]), w[R - j]));
       const int gx = x0 + cg + o;
-      if (gy < ny && gx < nx) out[(size_t)gy * nx + gx] = (TOut)acc;
+      if (gy < ny && gx < nx) {
+        out[(size_t)gy * nx + gx] = (TOut)acc;
+        if ((double)(TOut)acc > most) most = (double)(TOut)acc;
+      }
     }
+  }
+  if (max_bits) {  // non-negative doubles order like their bits
+    const unsigned long long b = warp_max_u64((unsigned long long)__double_as_longlong(most));
+    if (lane == 0 && b) atomicMax(max_bits, b);
   }
 }
 
 template <typename TOut>
 void blur_tile_r_launch(int r, dim3 grid, const uint16_t *in, const double *w, int ny, int nx,
-                        TOut *out, cudaStream_t st) {
+                        int skip_zero, unsigned long long *max_bits, TOut *out, cudaStream_t st) {
+#define LMB_BLUR_R(R)                                                                           \
+  case R:                                                                                       \
+    blur_tile_r_kernel<R, TOut><<<grid, 256, 0, st>>>(in, w, ny, nx, skip_zero, max_bits, out); \
+    break;
   switch (r) {
-    case 1: blur_tile_r_kernel<1, TOut><<<grid, 256, 0, st>>>(in, w, ny, nx, out); break;
-    case 2: blur_tile_r_kernel<2, TOut><<<grid, 256, 0, st>>>(in, w, ny, nx, out); break;
-    case 3: blur_tile_r_kernel<3, TOut><<<grid, 256, 0, st>>>(in, w, ny, nx, out); break;
-    case 4: blur_tile_r_kernel<4, TOut><<<grid, 256, 0, st>>>(in, w, ny, nx, out); break;
-    case 5: blur_tile_r_kernel<5, TOut><<<grid, 256, 0, st>>>(in, w, ny, nx, out); break;
-    case 6: blur_tile_r_kernel<6, TOut><<<grid, 256, 0, st>>>(in, w, ny, nx, out); break;
-    case 7: blur_tile_r_kernel<7, TOut><<<grid, 256, 0, st>>>(in, w, ny, nx, out); break;
-    default: blur_tile_r_kernel<8, TOut><<<grid, 256, 0, st>>>(in, w, ny, nx, out); break;
+    LMB_BLUR_R(1) LMB_BLUR_R(2) LMB_BLUR_R(3) LMB_BLUR_R(4)
+    LMB_BLUR_R(5) LMB_BLUR_R(6) LMB_BLUR_R(7) LMB_BLUR_R(8)
   }
+#undef LMB_BLUR_R
 }
 
 // ---- median ------------------------------------------------------------------------
@@ -1606,6 +1625,7 @@ struct lmb_pre {
   size_t fg_bytes = 0;
   bool labels_ready = false;  // label images of the last segment built
   double *d_centres = nullptr, *d_w = nullptr;
+  unsigned long long *d_max = nullptr;  // maximum of the blurred frame in d_out
   int *d_stats = nullptr, *d_head = nullptr, *d_next = nullptr;
   int gcx = 1, gcy = 1;
   PreState *d_state = nullptr, *h_state = nullptr;
@@ -1651,7 +1671,7 @@ void free_pre(lmb_pre *p) {
   void *bufs[] = {p->d_raw, p->d_bg, p->d_sub, p->d_tmp, p->d_out, p->d_t16, p->d_filt, p->d_par,
                   p->d_cid, p->d_lab, p->d_flab, p->c.area, p->c.x0, p->c.y0, p->c.x1, p->c.y1,
                   p->c.fb, p->c.sw, p->c.swx, p->c.swy, p->c.label, p->c.keep, p->d_flags,
-                  p->d_pos, p->d_compact, p->d_centres, p->d_w, p->d_stats, p->d_head, p->d_next,
+                  p->d_pos, p->d_compact, p->d_centres, p->d_w, p->d_max, p->d_stats, p->d_head, p->d_next,
                   p->d_state, p->d_cub, p->d_hist16, p->d_fg, p->d_nfg, p->d_fg_tmp, p->m_keys, p->m_keys2, p->m_idx, p->m_idx2, p->m_flag,
                   p->m_incl, p->m_rank, p->m_nd, p->m_vals, p->m_img, p->m_cub,
                   p->m_v16[0], p->m_v16[1], p->m_flag16};
@@ -1945,7 +1965,7 @@ int lmb_pre_create(int32_t device, int32_t nr_px_y, int32_t nr_px_x, lmb_pre **o
       (rc = alloc(&p->c.label, nb)) || (rc = alloc(&p->c.keep, nb)) ||
       (rc = alloc(&p->d_flags, nb)) || (rc = alloc(&p->d_pos, nb)) ||
       (rc = alloc(&p->d_compact, n)) || (rc = alloc(&p->d_centres, nb * 4)) ||
-      (rc = alloc(&p->d_w, 1024)) || (rc = alloc(&p->d_stats, nb * 5)) ||
+      (rc = alloc(&p->d_w, 1024)) || (rc = alloc(&p->d_max, 1)) || (rc = alloc(&p->d_stats, nb * 5)) ||
       (rc = alloc(&p->d_head, (size_t)p->gcx * p->gcy)) || (rc = alloc(&p->d_next, nb)) ||
       (rc = alloc(&p->d_state, 1)) || (rc = alloc(&p->d_hist16, 65536)) ||
       (rc = alloc(&p->d_fg, n)) || (rc = alloc(&p->d_nfg, 1)))
@@ -2174,8 +2194,11 @@ int lmb_pre_images(lmb_pre *p, uint16_t *thresholded, int32_t *labels, uint16_t 
 
 namespace {
 
-// Both blur passes of the last segment's filtered frame into p->d_out.
-int blur_launch(lmb_pre *p, const double *weights, int32_t radius, int32_t out_dtype) {
+// Both blur passes of the last segment's filtered frame into p->d_out; with
+// want_max and a radius whose kernel finds it, the frame's maximum into p->d_max
+// (*have_max).
+int blur_launch(lmb_pre *p, const double *weights, int32_t radius, int32_t out_dtype,
+                bool want_max = false, bool *have_max = nullptr) {
   LMB_REQUIRE(p->segmented, "no frame segmented yet");
   LMB_REQUIRE(weights, "null weights");
   LMB_REQUIRE(radius >= 0 && 2 * radius + 1 <= 1024, "blur radius %d outside 0..511", radius);
@@ -2190,12 +2213,18 @@ int blur_launch(lmb_pre *p, const double *weights, int32_t radius, int32_t out_d
   const unsigned g = (unsigned)grid_for(p->npx, p->num_sms);
   if (radius >= 1 && radius <= kBlurFixedMaxR) {
     const dim3 tg((p->nx + kBlurTile - 1) / kBlurTile, (p->ny + kBlurTile - 1) / kBlurTile);
+    int skip_zero = 1;
+    for (int j = 0; j <= 2 * radius; j++)
+      if (!(std::isfinite(weights[j]) && !std::signbit(weights[j]))) skip_zero = 0;
+    if (want_max) LMB_CUDA(cudaMemsetAsync(p->d_max, 0, sizeof(unsigned long long), p->st));
+    unsigned long long *mx = want_max ? p->d_max : nullptr;
     if (out_dtype == LMB_F64)
-      blur_tile_r_launch<double>(radius, tg, p->d_filt, p->d_w, p->ny, p->nx,
+      blur_tile_r_launch<double>(radius, tg, p->d_filt, p->d_w, p->ny, p->nx, skip_zero, mx,
                                  static_cast<double *>(p->d_out), p->st);
     else
-      blur_tile_r_launch<float>(radius, tg, p->d_filt, p->d_w, p->ny, p->nx,
+      blur_tile_r_launch<float>(radius, tg, p->d_filt, p->d_w, p->ny, p->nx, skip_zero, mx,
                                 static_cast<float *>(p->d_out), p->st);
+    if (have_max) *have_max = want_max;
   } else if (radius <= kBlurTileMaxR) {
     const dim3 tg((p->nx + kBlurTile - 1) / kBlurTile, (p->ny + kBlurTile - 1) / kBlurTile);
     const size_t tsm = blur_tile_smem(radius);
@@ -2244,10 +2273,12 @@ int lmb_pre_blur_to_slot(lmb_pre *p, const double *weights, int32_t radius, lmb_
   LMB_REQUIRE(e, "null engine");
   LMB_REQUIRE(engine_device(e) == p->device, "engine on device %d, preprocessing on device %d",
               engine_device(e), p->device);
-  if ((rc = blur_launch(p, weights, radius, frame_dtype))) return rc;
+  bool have_max = false;
+  if ((rc = blur_launch(p, weights, radius, frame_dtype, true, &have_max))) return rc;
   LMB_CUDA(cudaEventRecord(p->ev_out_ready, p->st));
-  rc = engine_load_device_frame(e, slot, p->d_out, frame_dtype, p->ny, p->nx, p->ev_out_ready,
-                                p->ev_out_free, im_scale);
+  rc = engine_load_device_frame(e, slot, p->d_out, frame_dtype, p->ny, p->nx,
+                                have_max ? p->d_max : nullptr, p->ev_out_ready, p->ev_out_free,
+                                im_scale);
   if (rc) return rc;
   p->out_in_use = true;
   LMB_CUDA(cudaStreamSynchronize(p->st));
