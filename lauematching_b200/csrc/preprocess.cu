@@ -5,21 +5,22 @@
 //   background   exact square median (scipy.ndimage.median_filter, mirrored
 //                borders).  Frames of whole numbers: tile by tile, window counts
 //                below a few thresholds around the tile's medians.  Others: pixels
-//                become ranks among the frame's distinct values; one warp per (column, row segment) slides its window
-//                down, keeping 8-bit-digit rank histograms level by level and
-//                refilling a deeper level only when the digit above it moves.
-//   threshold    order statistics (np.median, np.percentile) by radix
-//                selection over order-preserving 64-bit keys, on the device.
+//                become ranks among the frame's distinct values; one warp per
+//                (column, row segment) slides its window down, keeping 8-bit-digit
+//                rank histograms level by level and refilling a deeper level only
+//                when the digit above it moves.
+//   threshold    order statistics (np.median, np.percentile) from a histogram of
+//                whole-number values, else by radix selection over
+//                order-preserving 64-bit keys, on the device.
 //   components   union-find over 8-neighbours (atomicMin on the parent
 //                array); OpenCV numbers components by the raster order of
 //                the first 2x2 pixel block each touches, so labels come from
-//                a prefix sum over per-block flags.
+//                the ranks of their bits in a map of blocks.
 //   centres      integer moments per component (exact), one division each.
 //   blur width   closest pair of centres: cell grid, brute force when the
 //                pair is farther apart than a cell.
 //   blur         separable float64 passes in scipy's summation order.
 #include <cub/cub.cuh>
-#include <thrust/iterator/counting_iterator.h>
 
 #include <cmath>
 #include <cstring>
@@ -102,6 +103,9 @@ struct PreState {
   double med;
   double thresh;
   unsigned int blocks_done;  // blocks of the running selection pass that finished
+  unsigned int max_bin;      // largest value of the running value histogram
+  unsigned int n_fg;         // foreground pixels
+  unsigned int finish_done;  // blocks of the finishing kernel that are through
   unsigned int nonint;       // a candidate value was not an integer in [0, 65535]
   unsigned int value_path;   // the threshold came from the value histogram
   unsigned int n_comp;      // components
@@ -133,14 +137,10 @@ __global__ void subtract_kernel(const T *__restrict__ raw, const double *__restr
 
 // ---- order statistics ----------------------------------------------------------
 __global__ void sel_init_kernel(PreState *st, int mode, unsigned long long n,
-                                unsigned long long k0, int two, int new_frame) {
+                                unsigned long long k0, int two) {
   const int t = threadIdx.x;
   for (int i = t; i < 512; i += blockDim.x) (&st->hist[0][0])[i] = 0;
   if (t == 0) {
-    if (new_frame) {
-      st->nonint = 0;
-      st->value_path = 0;
-    }
     Select &s = st->sel;
     s.n = mode == SEL_ALL ? n : 0;
     s.k[0] = k0;
@@ -560,9 +560,14 @@ __global__ void __launch_bounds__(kHist16Threads, 1)
 // directly, and the median of |v - median| as the smallest distance d with
 // more than k values within d of the median.  Any other value (fraction,
 // negative zero, NaN, above 65535) leaves the work to the radix selection.
-__device__ __forceinline__ unsigned long long vh_count_le(const unsigned *P, int v) {
-  return v < 0 ? 0ull : (unsigned long long)__ldcg(P + v);
-}
+// Prefix sums P[0..top] of the histogram: values at most v.
+struct ValueCounts {
+  const unsigned *P;
+  int top;
+  __device__ __forceinline__ unsigned long long le(int v) const {
+    return v < 0 ? 0ull : (unsigned long long)P[min(v, top)];
+  }
+};
 
 // Smallest x in [lo, hi] with pred(x), pred monotone and true at hi; the
 // whole warp probes 32 points per round.
@@ -586,95 +591,85 @@ __device__ long long warp_search(long long lo, long long hi, Pred pred) {
 }
 
 // Smallest value v >= lo with more than r values in [lo, v].
-__device__ int vh_rank(const unsigned *P, int lo, unsigned long long r) {
-  const unsigned long long base = vh_count_le(P, lo - 1);
-  return (int)warp_search(lo, 65535, [&](long long v) {
-    return vh_count_le(P, (int)v) - base > r;
-  });
+__device__ int vh_rank(const ValueCounts &c, int lo, unsigned long long r) {
+  const unsigned long long base = c.le(lo - 1);
+  return (int)warp_search(lo, max(lo, c.top), [&](long long v) { return c.le((int)v) - base > r; });
 }
 
 // Values in [lo, 65535] within t/2 of med.
-__device__ unsigned long long vh_within(const unsigned *P, int lo, double med, long long t) {
+__device__ unsigned long long vh_within(const ValueCounts &c, int lo, double med, long long t) {
   const double h = 0.5 * (double)t;
   long long a = (long long)ceil(med - h), b = (long long)floor(med + h);
   if (a < lo) a = lo;
   if (b > 65535) b = 65535;
   if (b < a) return 0ull;
-  return vh_count_le(P, (int)b) - vh_count_le(P, (int)a - 1);
+  return c.le((int)b) - c.le((int)a - 1);
 }
 
 // Smallest distance (a multiple of 1/2) with more than r values within it.
-__device__ double vh_dist(const unsigned *P, int lo, double med, unsigned long long r) {
-  const long long t = warp_search(0, 2 * 65536, [&](long long x) {
-    return vh_within(P, lo, med, x) > r;
+__device__ double vh_dist(const ValueCounts &c, int lo, double med, unsigned long long r) {
+  const long long t = warp_search(0, 2 * ((long long)c.top + 1), [&](long long x) {
+    return vh_within(c, lo, med, x) > r;
   });
   return 0.5 * (double)t;
 }
 
-// Last block (1024 threads): prefix sums in place, then the threshold (warp 0).
-__device__ void vh_finish(PreState *st, unsigned *g16, int mode, unsigned long long k0, int two,
-                          double gamma) {
-  __shared__ unsigned long long warp_tot[32];
+constexpr int kVhLocal = 4096;
+constexpr int kVhThreads = 256;
+
+// Last block: prefix sums of bins [0, top] -- in shared memory (h, kVhLocal bins)
+// when they fit, in place otherwise --, the threshold (warp 0), and the global
+// histogram empty again.
+__device__ void vh_finish(PreState *st, unsigned *g16, unsigned *h, int top, int mode,
+                          unsigned long long k0, int two, double gamma) {
+  __shared__ unsigned warp_tot[kVhThreads / 32];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  const int nq = 65536 / 4 / blockDim.x;  // uint4 words of bins per thread
-  uint4 *src = reinterpret_cast<uint4 *>(g16) + (size_t)t * nq;
-  unsigned mine = 0;
-  for (int j0 = 0; j0 < nq; j0 += 16) {
-    uint4 q[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) q[j] = __ldcg(src + j0 + j);
-#pragma unroll
-    for (int j = 0; j < 16; ++j) mine += q[j].x + q[j].y + q[j].z + q[j].w;
+  const bool local = top < kVhLocal;
+  unsigned *P = local ? h : g16;
+  const int per = ((top + kVhThreads) / kVhThreads + 3) / 4 * 4;  // bins per thread
+  const int b0 = t * per, b1 = min(b0 + per, top + 1);
+  if (local) {
+    for (int b = t; b <= top; b += kVhThreads) h[b] = __ldcg(g16 + b);
+    __syncthreads();
   }
-  unsigned long long incl = mine;
+  unsigned mine = 0;  // counts fit 32 bits (frames < 2^31 pixels)
+  for (int b = b0; b < b1; ++b) mine += local ? h[b] : __ldcg(g16 + b);
+  unsigned incl = mine;
   for (int o = 1; o < 32; o <<= 1) {
-    const unsigned long long v = __shfl_up_sync(0xffffffffu, incl, o);
+    const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += v;
   }
   if (lane == 31) warp_tot[w] = incl;
   __syncthreads();
-  if (w == 0) {
-    const int nw = blockDim.x >> 5;
-    unsigned long long v = lane < nw ? warp_tot[lane] : 0ull, x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned long long u = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += u;
-    }
-    if (lane < nw) warp_tot[lane] = x - v;
+  unsigned run = incl - mine;
+  for (int j = 0; j < w; ++j) run += warp_tot[j];
+  for (int b = b0; b < b1; ++b) {
+    run += local ? h[b] : __ldcg(g16 + b);
+    P[b] = run;
   }
-  __syncthreads();
-  unsigned run = (unsigned)(warp_tot[w] + incl - mine);  // counts fit 32 bits (frames < 2^31 px)
-  for (int j = 0; j < nq; ++j) {
-    uint4 q = __ldcg(src + j);
-    q.x = (run += q.x);
-    q.y = (run += q.y);
-    q.z = (run += q.z);
-    q.w = (run += q.w);
-    src[j] = q;
-  }
-  __threadfence();
+  __threadfence_block();
   __syncthreads();
   if (w == 0) {
-    const unsigned *P = g16;
+    const ValueCounts c{P, top};
     double thresh;
     if (mode == SEL_ALL) {  // np.percentile over every pixel
-      const double a = (double)vh_rank(P, 0, k0);
-      const double b = two ? (double)vh_rank(P, 0, k0 + 1) : a;
+      const double a = (double)vh_rank(c, 0, k0);
+      const double b = two ? (double)vh_rank(c, 0, k0 + 1) : a;
       const double diff = lmb::dsub(b, a);
       thresh = lmb::dadd(a, lmb::dmul(diff, gamma));
       if (gamma >= 0.5) thresh = lmb::dsub(b, lmb::dmul(diff, lmb::dsub(1.0, gamma)));
     } else {  // the adaptive noise floor over the nonzero pixels
-      const unsigned long long n = vh_count_le(P, 65535) - vh_count_le(P, 0);
+      const unsigned long long n = c.le(65535) - c.le(0);
       if (n == 0) {
         thresh = 1.0;
       } else {
         const unsigned long long k = (n - 1) / 2;
         const bool even = (n % 2) == 0;
-        const double a = (double)vh_rank(P, 1, k);
+        const double a = (double)vh_rank(c, 1, k);
         const double med =
-            even ? lmb::ddiv(lmb::dadd(a, (double)vh_rank(P, 1, k + 1)), 2.0) : a;
-        const double m1 = vh_dist(P, 1, med, k);
-        const double md = even ? lmb::ddiv(lmb::dadd(m1, vh_dist(P, 1, med, k + 1)), 2.0) : m1;
+            even ? lmb::ddiv(lmb::dadd(a, (double)vh_rank(c, 1, k + 1)), 2.0) : a;
+        const double m1 = vh_dist(c, 1, med, k);
+        const double md = even ? lmb::ddiv(lmb::dadd(m1, vh_dist(c, 1, med, k + 1)), 2.0) : m1;
         const double mad = lmb::dmul(1.4826, md);
         const double thr = lmb::dadd(med, lmb::dmul(4.0, mad));
         thresh = (1.0 > thr) ? 1.0 : thr;
@@ -686,29 +681,35 @@ __device__ void vh_finish(PreState *st, unsigned *g16, int mode, unsigned long l
     }
   }
   __syncthreads();
-  for (int j = 0; j < nq; ++j) src[j] = make_uint4(0, 0, 0, 0);
+  for (int b = t; b <= top; b += kVhThreads) g16[b] = 0u;
 }
 
-// Subtraction fused with the value histogram (see above).  Each block counts
-// values below kVhLocal in shared memory (runs of equal values in registers)
-// and adds larger ones straight into the global 65536-bin histogram.
-constexpr int kVhLocal = 4096;
-constexpr int kVhThreads = 256;
-
+// Subtraction fused with the value histogram (see above); the differences are
+// kept as 16-bit values.  Each block counts values below kVhLocal in shared
+// memory (runs of equal values in registers) and adds larger ones straight into
+// the global 65536-bin histogram.  A frame with another value leaves the value
+// path: its threshold is infinite, so nothing follows from the 16-bit values, and
+// the host starts again with the radix selection.  *bg_other = 0: the background
+// is whole numbers too and read as bg16.  Measured on B200 (cold caches), 2048^2
+// uint16 frame: 70.7 us with the background and the differences as float64 and the
+// last block's search over all 65536 bins in global memory, 34.3 us.
 template <typename T>
 __global__ void __launch_bounds__(kVhThreads, 4)
     value_hist_kernel(const T *__restrict__ raw, const double *__restrict__ bg,
-                      double *__restrict__ sub, unsigned n, PreState *st, unsigned *g16, int mode,
+                      const uint16_t *__restrict__ bg16, const unsigned *__restrict__ bg_other,
+                      uint16_t *__restrict__ sub16, unsigned n, PreState *st, unsigned *g16, int mode,
                       unsigned long long k0, int two, double gamma) {
   __shared__ unsigned h[kVhLocal];
   __shared__ bool last;
-  __shared__ int nonint_s;
+  __shared__ unsigned max_s;
   for (int i = threadIdx.x; i < kVhLocal; i += blockDim.x) h[i] = 0;
-  if (threadIdx.x == 0) nonint_s = 0;
+  if (threadIdx.x == 0) max_s = 0;
   __syncthreads();
   DigitRun run;  // bins below kVhLocal
   bool nonint = false;
+  unsigned most = 0;
   constexpr int U = 8;
+  const bool whole_bg = *bg_other == 0u;
   const unsigned stride = gridDim.x * blockDim.x;
   const unsigned rounds = (n + stride * U - 1) / (stride * U);
   for (unsigned it = 0; it < rounds; ++it) {
@@ -720,9 +721,9 @@ __global__ void __launch_bounds__(kVhThreads, 4)
       in[u] = i < n;
       v[u] = 0.0;
       if (in[u]) {
-        const double d = lmb::dsub(to_f64(raw[i]), bg[i]);
+        const double d = lmb::dsub(to_f64(raw[i]), whole_bg ? (double)bg16[i] : bg[i]);
         v[u] = (d >= 0.0 || isnan(d)) ? d : 0.0;
-        sub[i] = v[u];
+        sub16[i] = (uint16_t)((unsigned)x86_trunc_i32(v[u]) & 0xFFFFu);
       }
     }
 #pragma unroll
@@ -731,6 +732,7 @@ __global__ void __launch_bounds__(kVhThreads, 4)
       const double x = v[u];
       if (x == trunc(x) && x <= 65535.0 && !signbit(x)) {
         const unsigned b = (unsigned)x;
+        most = max(most, b);
         if (b < (unsigned)kVhLocal) run.add(h, b);
         else atomicAdd(g16 + b, 1u);
       } else {
@@ -739,9 +741,10 @@ __global__ void __launch_bounds__(kVhThreads, 4)
     }
   }
   run.flush(h);
-  if (nonint) nonint_s = 1;
-  __syncthreads();
-  if (threadIdx.x == 0 && nonint_s) atomicOr(&st->nonint, 1u);
+  most = __reduce_max_sync(0xffffffffu, most);
+  if ((threadIdx.x & 31) == 0 && most) atomicMax(&max_s, most);
+  if (__syncthreads_or(nonint) && threadIdx.x == 0) atomicOr(&st->nonint, 1u);
+  if (threadIdx.x == 0) atomicMax(&st->max_bin, max_s);
   for (int b = threadIdx.x; b < kVhLocal; b += blockDim.x)
     if (h[b]) atomicAdd(g16 + b, h[b]);
   __threadfence();
@@ -750,13 +753,21 @@ __global__ void __launch_bounds__(kVhThreads, 4)
   __syncthreads();
   if (last) {
     __threadfence();
+    const int top = (int)__ldcg(&st->max_bin);
     if (__ldcg(&st->nonint) == 0) {
-      vh_finish(st, g16, mode, k0, two, gamma);
+      vh_finish(st, g16, h, top, mode, k0, two, gamma);
     } else {  // leave an empty histogram for the radix selection
-      for (int q = threadIdx.x; q < 65536 / 4; q += blockDim.x)
-        reinterpret_cast<uint4 *>(g16)[q] = make_uint4(0, 0, 0, 0);
+      for (int b = threadIdx.x; b <= top; b += kVhThreads) g16[b] = 0u;
+      if (threadIdx.x == 0) {
+        st->thresh = __longlong_as_double(0x7ff0000000000000ll);
+        st->value_path = 0;
+      }
     }
-    if (threadIdx.x == 0) st->blocks_done = 0;
+    if (threadIdx.x == 0) {
+      st->blocks_done = 0;
+      st->nonint = 0;
+      st->max_bin = 0;
+    }
   }
 }
 
@@ -799,36 +810,122 @@ __global__ void finish_percentile_kernel(PreState *st, double gamma) {
 __global__ void set_thresh_kernel(PreState *st, double t) { st->thresh = t; }
 
 __global__ void reset_counts_kernel(PreState *st) {
+  st->n_fg = 0;
   st->n_comp = 0;
+  st->finish_done = 0;
   st->best = 0x7ff0000000000000ull;  // +inf
 }
 
 // ---- threshold, uint16, components ---------------------------------------------
-// Threshold and uint16 cast (thresholds.py:29-32, preprocess.py:291), and
-// the union-find parents along row runs (see init_parents_kernel).
-__global__ void apply_kernel(const double *__restrict__ sub, const PreState *st,
-                             uint16_t *__restrict__ t16, int *__restrict__ par, int nx, size_t n) {
-  const double thr = st->thresh;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const double v = sub[i];
-    const uint16_t u = (v <= thr) ? (uint16_t)0 : u16_cast(v);
-    t16[i] = u;
-    bool left = false;
-    if (u && (i % nx) != 0) {
-      const double vl = sub[i - 1];
-      left = !(vl <= thr) && u16_cast(vl) != 0;
-    }
-    par[i] = u ? (left ? (int)i - 1 : (int)i) : -1;
-  }
+// Where a frame's thresholded uint16 pixels come from (thresholds.py:29-32,
+// preprocess.py:291): the subtracted frame in float64 or as whole numbers and the
+// threshold, or the thresholded frame itself.
+__device__ __forceinline__ uint16_t over(double v, double thr) {
+  return (v <= thr) ? (uint16_t)0 : u16_cast(v);
 }
+struct FromSub {
+  const double *sub;
+  static constexpr bool kStored = false;
+  __device__ __forceinline__ uint16_t at(size_t i, double thr) const { return over(sub[i], thr); }
+  __device__ __forceinline__ void four(size_t q, double thr, uint16_t (&u)[4]) const {
+    const double2 a = reinterpret_cast<const double2 *>(sub)[2 * q];
+    const double2 b = reinterpret_cast<const double2 *>(sub)[2 * q + 1];
+    u[0] = over(a.x, thr);
+    u[1] = over(a.y, thr);
+    u[2] = over(b.x, thr);
+    u[3] = over(b.y, thr);
+  }
+};
+struct FromSub16 {
+  const uint16_t *sub;
+  static constexpr bool kStored = false;
+  static __device__ __forceinline__ uint16_t pass(uint16_t v, double thr) {
+    return ((double)v <= thr) ? (uint16_t)0 : v;
+  }
+  __device__ __forceinline__ uint16_t at(size_t i, double thr) const { return pass(sub[i], thr); }
+  __device__ __forceinline__ void four(size_t q, double thr, uint16_t (&u)[4]) const {
+    const ushort4 a = reinterpret_cast<const ushort4 *>(sub)[q];
+    u[0] = pass(a.x, thr);
+    u[1] = pass(a.y, thr);
+    u[2] = pass(a.z, thr);
+    u[3] = pass(a.w, thr);
+  }
+};
+struct FromThresholded {
+  const uint16_t *t16;
+  static constexpr bool kStored = true;
+  __device__ __forceinline__ uint16_t at(size_t i, double) const { return t16[i]; }
+  __device__ __forceinline__ void four(size_t q, double, uint16_t (&u)[4]) const {
+    const ushort4 a = reinterpret_cast<const ushort4 *>(t16)[q];
+    u[0] = a.x;
+    u[1] = a.y;
+    u[2] = a.z;
+    u[3] = a.w;
+  }
+};
 
-// Parents start along row runs: a foreground pixel points at its left
-// neighbour when that one is foreground too.
-__global__ void init_parents_kernel(const uint16_t *t16, int *par, int nx, size_t n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x)
-    par[i] = t16[i] ? ((i % nx) != 0 && t16[i - 1] ? (int)i - 1 : (int)i) : -1;
+// One pass over the frame: the thresholded pixels, the filtered frame cleared, and
+// of the foreground pixels (in any order: components are numbered by their first
+// block, sums are exact) the list and the union-find parents along row runs: a
+// foreground pixel points at its left neighbour when that one is foreground too.
+// Also clears the cell grid and the tile flags of the later kernels.  V pixels per
+// thread at a time (V = 4 needs n a multiple of 4).
+template <int V, typename Src>
+__global__ void foreground_kernel(const Src src, PreState *st, uint16_t *__restrict__ t16,
+                                  uint16_t *__restrict__ filt, int *__restrict__ par,
+                                  unsigned *__restrict__ fg, int nx, size_t n, int *__restrict__ head,
+                                  int cells, uint8_t *__restrict__ tiles, int ntiles) {
+  const double thr = st->thresh;
+  const int lane = threadIdx.x & 31;
+  const size_t first = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  for (size_t i = first; i < (size_t)cells; i += stride) head[i] = -1;
+  for (size_t i = first; i < (size_t)ntiles; i += stride) tiles[i] = 0;
+  const size_t nv = n / V, rounds = (nv + stride - 1) / stride;
+  for (size_t it = 0; it < rounds; ++it) {  // whole warps
+    const size_t q = it * stride + first, i0 = q * V;
+    uint16_t u[V];
+    unsigned bits = 0;
+#pragma unroll
+    for (int j = 0; j < V; ++j) u[j] = 0;
+    if (q < nv) {
+      if constexpr (V == 4)
+        src.four(q, thr, u);
+      else
+        u[0] = src.at(q, thr);
+    }
+#pragma unroll
+    for (int j = 0; j < V; ++j) bits |= u[j] ? 1u << j : 0u;
+    if (q < nv) {
+      if constexpr (V == 4) {
+        if (!Src::kStored)
+          reinterpret_cast<ushort4 *>(t16)[q] = make_ushort4(u[0], u[1], u[2], u[3]);
+        reinterpret_cast<ushort4 *>(filt)[q] = make_ushort4(0, 0, 0, 0);
+      } else {
+        if (!Src::kStored) t16[q] = u[0];
+        filt[q] = 0;
+      }
+    }
+    if (!__any_sync(0xffffffffu, bits != 0u)) continue;
+    const int cnt = __popc(bits);
+    int x = cnt;  // the warp's places in the list
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    unsigned base = 0;
+    if (lane == 31) base = atomicAdd(&st->n_fg, (unsigned)x);
+    base = __shfl_sync(0xffffffffu, base, 31) + (unsigned)(x - cnt);
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      if (!u[j]) continue;
+      const size_t i = i0 + j;
+      fg[base++] = (unsigned)i;
+      const bool left = i % nx != 0 && (j > 0 ? u[j > 0 ? j - 1 : 0] != 0 : src.at(i - 1, thr) != 0);
+      par[i] = left ? (int)i - 1 : (int)i;
+    }
+  }
 }
 
 __device__ __forceinline__ int uf_find(int *L, int x) {
@@ -864,8 +961,8 @@ __device__ void uf_union(int *L, int a, int b) {
 // x = s; the upper one when x = s and the upper-left is background; the
 // upper-right one when the upper one is background.
 __global__ void merge_kernel(const uint16_t *t16, int *L, int nx, const unsigned *fg,
-                             const unsigned *n_fg) {
-  const unsigned nf = *n_fg;
+                             const PreState *st) {
+  const unsigned nf = st->n_fg;
   for (unsigned f = blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += gridDim.x * blockDim.x) {
     const unsigned i = fg[f];
     const int y = (int)(i / nx), x = (int)(i % nx);
@@ -890,9 +987,8 @@ struct Comps {
 
 // Every foreground pixel points straight at its root; each root takes the
 // next component id.
-__global__ void compress_kernel(int *L, int *cid, PreState *st, Comps c, const unsigned *fg,
-                                const unsigned *n_fg) {
-  const unsigned nf = *n_fg;
+__global__ void compress_kernel(int *L, int *cid, PreState *st, Comps c, const unsigned *fg) {
+  const unsigned nf = st->n_fg;
   for (unsigned f = blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += gridDim.x * blockDim.x) {
     const unsigned i = fg[f];
     const int r = uf_find(L, (int)i);
@@ -913,8 +1009,8 @@ __global__ void compress_kernel(int *L, int *cid, PreState *st, Comps c, const u
 }
 
 __global__ void moments_kernel(const int *L, const int *cid, const uint16_t *t16, Comps c, int nx,
-                               const unsigned *fg, const unsigned *n_fg) {
-  const unsigned nf = *n_fg;
+                               const unsigned *fg, const PreState *st) {
+  const unsigned nf = st->n_fg;
   const unsigned bw = (unsigned)(nx + 1) / 2;
   for (unsigned f = blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += gridDim.x * blockDim.x) {
     const unsigned i = fg[f];
@@ -934,25 +1030,80 @@ __global__ void moments_kernel(const int *L, const int *cid, const uint16_t *t16
   }
 }
 
-// Flag each component's first block: low word counts components, high word
-// kept ones; a prefix sum over blocks then numbers them in OpenCV's order.
-__global__ void flags_kernel(const PreState *st, Comps c, int min_area,
-                             unsigned long long *flags, size_t cap) {
-  const size_t nc = st->n_comp;
-  for (size_t id = blockIdx.x * (size_t)blockDim.x + threadIdx.x; id < nc && id < cap;
-       id += (size_t)gridDim.x * blockDim.x) {
-    const bool keep = c.area[id] >= min_area;
-    flags[c.fb[id]] = 1ull | (keep ? (1ull << 32) : 0ull);
-  }
-}
-
-__global__ void label_kernel(PreState *st, Comps c, int min_area, const unsigned long long *pos,
-                             size_t nblocks, double *centres, int *stats) {
+// OpenCV numbers components by their first 2x2 block in raster order: a bit per
+// block that is some component's first (and in a second map, some kept one's), the
+// bits before each of 1024 segments of a map, and a component's number is the
+// bits before its own.
+__global__ void flags_kernel(const PreState *st, Comps c, int min_area, unsigned *bits,
+                             unsigned *keep_bits) {
   const size_t nc = st->n_comp;
   for (size_t id = blockIdx.x * (size_t)blockDim.x + threadIdx.x; id < nc;
        id += (size_t)gridDim.x * blockDim.x) {
-    const unsigned long long p = pos[c.fb[id]];
-    const int label = (int)(p & 0xffffffffull);
+    const unsigned fb = c.fb[id], bit = 1u << (fb & 31u);
+    atomicOr(bits + (fb >> 5), bit);
+    if (c.area[id] >= min_area) atomicOr(keep_bits + (fb >> 5), bit);
+  }
+}
+
+constexpr int kSegs = 1024;
+// Blocks 0 and 1: the two maps.  seg[s] = bits before segment s of len words;
+// totals into the state.
+__global__ void __launch_bounds__(kSegs) rank_bits_kernel(PreState *st, const unsigned *bits,
+                                                          const unsigned *keep_bits, unsigned nwords,
+                                                          unsigned len, unsigned *seg,
+                                                          unsigned *keep_seg) {
+  __shared__ unsigned warp_tot[kSegs / 32];
+  const unsigned *b = blockIdx.x ? keep_bits : bits;
+  unsigned *out = blockIdx.x ? keep_seg : seg;
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const unsigned w0 = min((unsigned)t * len, nwords), w1 = min(w0 + len, nwords);
+  unsigned mine = 0;
+  unsigned k = w0;
+  for (; k + 4 <= w1; k += 4) {  // len and the map's start are multiples of 4 words
+    const uint4 v = *reinterpret_cast<const uint4 *>(b + k);
+    mine += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
+  }
+  for (; k < w1; ++k) mine += __popc(b[k]);
+  unsigned incl = mine;
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) warp_tot[w] = incl;
+  __syncthreads();
+  unsigned before = incl - mine, total = 0;
+  for (int j = 0; j < kSegs / 32; ++j) {
+    if (j < w) before += warp_tot[j];
+    total += warp_tot[j];
+  }
+  out[t] = before;
+  if (t == 0) {
+    if (blockIdx.x)
+      st->n_keep = total;
+    else
+      st->n_labels = total + 1u;
+  }
+}
+
+__device__ __forceinline__ unsigned bits_before(const unsigned *bits, const unsigned *seg, unsigned len,
+                                                unsigned fb) {
+  const unsigned w = fb >> 5, s = w / len;
+  unsigned n = seg[s];
+  for (unsigned k = s * len; k < w; ++k) n += __popc(bits[k]);
+  return n + __popc(bits[w] & ((1u << (fb & 31u)) - 1u));
+}
+
+// Labels, boxes and centres; a kept component's centre joins its cell of the
+// closest-pair grid.
+__global__ void label_kernel(const PreState *st, Comps c, int min_area, const unsigned *bits,
+                             const unsigned *keep_bits, const unsigned *seg, const unsigned *keep_seg,
+                             unsigned len, double *centres, int *stats, int *head, int *next, int gcx,
+                             int gcy) {
+  const size_t nc = st->n_comp;
+  for (size_t id = blockIdx.x * (size_t)blockDim.x + threadIdx.x; id < nc;
+       id += (size_t)gridDim.x * blockDim.x) {
+    const unsigned fb = c.fb[id];
+    const int label = (int)bits_before(bits, seg, len, fb) + 1;
     const bool keep = c.area[id] >= min_area;
     c.label[id] = label;
     const int x0 = c.x0[id], y0 = c.y0[id];
@@ -963,7 +1114,7 @@ __global__ void label_kernel(PreState *st, Comps c, int min_area, const unsigned
     sr[3] = c.y1[id] - y0 + 1;
     sr[4] = c.area[id];
     if (keep) {
-      const int k = (int)(p >> 32) - 1;
+      const int k = (int)bits_before(keep_bits, keep_seg, len, fb);
       c.keep[id] = k;
       const unsigned long long sw = c.sw[id];
       const double rx = (double)(c.swx[id] - (unsigned long long)x0 * sw);
@@ -973,25 +1124,12 @@ __global__ void label_kernel(PreState *st, Comps c, int min_area, const unsigned
       cr[1] = lmb::dadd(lmb::ddiv(rx, (double)sw), (double)x0);
       cr[2] = lmb::dadd(lmb::ddiv(ry, (double)sw), (double)y0);
       cr[3] = (double)c.area[id];
+      const int cx = min(max((int)(cr[1] / kCell), 0), gcx - 1);
+      const int cy = min(max((int)(cr[2] / kCell), 0), gcy - 1);
+      next[k] = atomicExch(head + cy * gcx + cx, k);
     } else {
       c.keep[id] = -1;
     }
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    const unsigned long long t = nblocks ? pos[nblocks - 1] : 0;
-    st->n_labels = (unsigned)(t & 0xffffffffull) + 1u;
-    st->n_keep = (unsigned)(t >> 32);
-  }
-}
-
-// The filtered frame (kept components' pixels) over a zeroed frame.
-__global__ void filt_kernel(const int *__restrict__ L, const int *__restrict__ cid,
-                            const uint16_t *__restrict__ t16, Comps c, uint16_t *__restrict__ filt,
-                            const unsigned *fg, const unsigned *n_fg) {
-  const unsigned nf = *n_fg;
-  for (unsigned f = blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += gridDim.x * blockDim.x) {
-    const unsigned i = fg[f];
-    if (c.keep[cid[L[i]]] >= 0) filt[i] = t16[i];
   }
 }
 
@@ -999,8 +1137,8 @@ __global__ void filt_kernel(const int *__restrict__ L, const int *__restrict__ c
 // when a caller asks for them).
 __global__ void labels_kernel(const int *__restrict__ L, const int *__restrict__ cid, Comps c,
                               int *__restrict__ labels, int *__restrict__ flabels,
-                              const unsigned *fg, const unsigned *n_fg) {
-  const unsigned nf = *n_fg;
+                              const unsigned *fg, const PreState *st) {
+  const unsigned nf = st->n_fg;
   for (unsigned f = blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += gridDim.x * blockDim.x) {
     const unsigned i = fg[f];
     const int id = cid[L[i]];
@@ -1009,12 +1147,6 @@ __global__ void labels_kernel(const int *__restrict__ L, const int *__restrict__
     if (c.keep[id] >= 0) flabels[i] = lab;
   }
 }
-
-// Foreground test of the list selection.
-struct IsForeground {
-  const uint16_t *t16;
-  __device__ __forceinline__ bool operator()(const unsigned &i) const { return t16[i] != 0; }
-};
 
 // ---- closest pair of centres (blur width) ---------------------------------------
 __device__ __forceinline__ double pair_d2(const double *a, const double *b) {
@@ -1029,21 +1161,49 @@ __device__ __forceinline__ void warp_min_to(unsigned long long *dst, double v) {
     atomicMin(dst, (unsigned long long)__double_as_longlong(v));
 }
 
-__global__ void cell_insert_kernel(const PreState *st, const double *centres, int *head, int *next,
-                                   int gcx, int gcy) {
-  const unsigned n = st->n_keep;
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int cx = min(max((int)(centres[(size_t)i * 4 + 1] / kCell), 0), gcx - 1);
-    const int cy = min(max((int)(centres[(size_t)i * 4 + 2] / kCell), 0), gcy - 1);
-    next[i] = atomicExch(head + cy * gcx + cx, (int)i);
-  }
+// Every pair of kept centres (blocks share them; one block: nblocks = 1).
+__device__ void brute_pairs(PreState *st, const double *centres, unsigned n, unsigned block,
+                            unsigned nblocks) {
+  double best = __longlong_as_double(0x7ff0000000000000ll);
+  for (unsigned i = block * blockDim.x + threadIdx.x; i < n; i += nblocks * blockDim.x)
+    for (unsigned j = i + 1; j < n; ++j)
+      best = fmin(best, pair_d2(centres + (size_t)i * 4, centres + (size_t)j * 4));
+  warp_min_to(&st->best, best);
 }
 
-__global__ void cell_pairs_kernel(PreState *st, const double *centres, const int *head,
-                                  const int *next, int gcx, int gcy) {
-  const unsigned n = st->n_keep;
+constexpr int kBlurTile = 32;  // side of a blur tile
+// Centres whose pairs one block may take.  Three of them at most lie in one cell
+// when every two are more than a cell's side apart.
+constexpr unsigned kBruteLast = 16384;
+
+// After the labels: the filtered frame (kept components' pixels over a cleared
+// frame) with the blur tiles it touches, the closest pair of centres within
+// neighbouring cells, and the first-block maps empty again.  Pairs in cells that
+// are not neighbours lie more than a cell apart, so the grid's answer is exact when
+// it is within a cell; otherwise every pair counts: the last block takes them when
+// there are at most kBruteLast centres, else brute_pairs_kernel follows.
+__global__ void finish_kernel(PreState *st, Comps c, const int *__restrict__ L,
+                              const int *__restrict__ cid, const uint16_t *__restrict__ t16,
+                              uint16_t *__restrict__ filt, const unsigned *fg, int nx,
+                              uint8_t *__restrict__ tiles, int tiles_x, unsigned *bits,
+                              unsigned *keep_bits, const double *centres, const int *head,
+                              const int *next, int gcx, int gcy) {
+  __shared__ bool last;
+  const unsigned first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  const unsigned nf = st->n_fg, nc = st->n_comp, n = st->n_keep;
+  for (unsigned f = first; f < nf; f += stride) {
+    const unsigned i = fg[f];
+    if (c.keep[cid[L[i]]] < 0) continue;
+    filt[i] = t16[i];
+    tiles[(i / nx / kBlurTile) * tiles_x + i % nx / kBlurTile] = 1;
+  }
+  for (unsigned id = first; id < nc; id += stride) {
+    const unsigned w = c.fb[id] >> 5;
+    bits[w] = 0u;
+    keep_bits[w] = 0u;
+  }
   double best = __longlong_as_double(0x7ff0000000000000ll);
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (unsigned i = first; i < n; i += stride) {
     const double *a = centres + (size_t)i * 4;
     const int cx = min(max((int)(a[1] / kCell), 0), gcx - 1);
     const int cy = min(max((int)(a[2] / kCell), 0), gcy - 1);
@@ -1053,19 +1213,22 @@ __global__ void cell_pairs_kernel(PreState *st, const double *centres, const int
           if ((unsigned)j > i) best = fmin(best, pair_d2(a, centres + (size_t)j * 4));
   }
   warp_min_to(&st->best, best);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&st->finish_done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last || n > kBruteLast) return;
+  __threadfence();
+  if (__longlong_as_double((long long)__ldcg(&st->best)) > (double)kCell * (double)kCell)
+    brute_pairs(st, centres, n, 0, 1);
 }
 
-// Pairs in cells that are not neighbours lie more than a cell apart, so the
-// grid's answer is exact when it is within a cell; otherwise every pair.
 __global__ void brute_pairs_kernel(PreState *st, const double *centres) {
-  const double cell2 = (double)kCell * (double)kCell;
-  if (__longlong_as_double((long long)st->best) <= cell2) return;
   const unsigned n = st->n_keep;
-  double best = __longlong_as_double(0x7ff0000000000000ll);
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    for (unsigned j = i + 1; j < n; ++j)
-      best = fmin(best, pair_d2(centres + (size_t)i * 4, centres + (size_t)j * 4));
-  warp_min_to(&st->best, best);
+  if (n <= kBruteLast ||
+      __longlong_as_double((long long)st->best) <= (double)kCell * (double)kCell)
+    return;
+  brute_pairs(st, centres, n, blockIdx.x, gridDim.x);
 }
 
 // ---- Gaussian blur ---------------------------------------------------------------
@@ -1113,7 +1276,6 @@ __global__ void blur_cols_kernel(const double *in, const double *wts, int r, int
 // in shared memory, the axis-0 pass over the tile's rows and halo columns,
 // then the axis-1 pass; the same operations in the same order as the two
 // separate passes, without the float64 intermediate in global memory.
-constexpr int kBlurTile = 32;
 constexpr int kBlurTileMaxR = 32;
 
 size_t blur_tile_smem(int r) {
@@ -1163,15 +1325,22 @@ __global__ void __launch_bounds__(256)
 // a row (axis-1 pass) in registers, 4 + 2R inputs, each converted once.
 constexpr int kBlurFixedMaxR = 8;
 
-// A tile without a positive pixel in reach (most of a filtered frame) is all zero
-// (skip_zero: the weights are finite and not negative, so no term has a sign).
+// tiles, unless null: the 32 x 32 tiles that hold a positive pixel.  A tile with
+// none there nor in its eight neighbours (most of a filtered frame; a reach of R <=
+// 8 pixels, mirrored or not, stays among them) is all zero: tiles is given when the
+// weights are finite and not negative, so that no term has a sign.
 // max_bits, unless null, takes the bits of the frame's largest positive value.
 // Measured on B200 (cold caches), 2048^2 frame of 50 spots, float32 result: 37.4 us
-// with every tile computed (FP64 issue), 25.3 us.
+// with every tile computed (FP64 issue), 25.3 us with empty tiles found by loading
+// them, 14.2 us by the flags.
+struct BlurWeights {
+  double w[2 * kBlurFixedMaxR + 1];
+};
+
 template <int R, typename TOut>
 __global__ void __launch_bounds__(256)
-    blur_tile_r_kernel(const uint16_t *__restrict__ in, const double *__restrict__ wts, int ny,
-                       int nx, int skip_zero, unsigned long long *__restrict__ max_bits,
+    blur_tile_r_kernel(const uint16_t *__restrict__ in, const BlurWeights wts, int ny, int nx,
+                       const uint8_t *__restrict__ tiles, unsigned long long *__restrict__ max_bits,
                        TOut *__restrict__ out) {
   constexpr int W = kBlurTile + 2 * R;
   __shared__ double w[2 * R + 1];
@@ -1179,22 +1348,36 @@ __global__ void __launch_bounds__(256)
   __shared__ uint16_t tile[W * W];
   const int x0 = blockIdx.x * kBlurTile, y0 = blockIdx.y * kBlurTile;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  if (t <= 2 * R) w[t] = wts[t];
+  if (tiles) {
+    const int tx = (int)blockIdx.x + t % 3 - 1, ty = (int)blockIdx.y + t / 3 - 1;
+    const bool any = t < 9 && tx >= 0 && tx < (int)gridDim.x && ty >= 0 && ty < (int)gridDim.y &&
+                     tiles[ty * (int)gridDim.x + tx];
+    if (!__syncthreads_or(any)) {
+      if (x0 + kBlurTile <= nx && nx % 4 == 0) {  // 16-byte stores
+        constexpr int kPer = 16 / sizeof(TOut), kRow = kBlurTile / kPer;
+        for (int i = t; i < kBlurTile * kRow; i += 256) {
+          const int gy = y0 + i / kRow;
+          if (gy < ny)
+            *reinterpret_cast<uint4 *>(out + (size_t)gy * nx + x0 + i % kRow * kPer) =
+                make_uint4(0u, 0u, 0u, 0u);
+        }
+      } else {
+        for (int row = warp; row < kBlurTile; row += 8)
+          if (y0 + row < ny && x0 + lane < nx) out[(size_t)(y0 + row) * nx + x0 + lane] = (TOut)0;
+      }
+      return;
+    }
+  }
+  if (t <= 2 * R) w[t] = wts.w[t];
   // mirrored source columns of this lane (W <= 48 < 64)
   const int c0 = mirror(x0 - R + lane, nx);
   const int c1 = lane + 32 < W ? mirror(x0 - R + lane + 32, nx) : 0;
-  unsigned any = 0u;
   for (int row = warp; row < W; row += 8) {
     const uint16_t *src = in + (size_t)mirror(y0 - R + row, ny) * nx;
-    any |= tile[row * W + lane] = src[c0];
-    if (lane + 32 < W) any |= tile[row * W + lane + 32] = src[c1];
+    tile[row * W + lane] = src[c0];
+    if (lane + 32 < W) tile[row * W + lane + 32] = src[c1];
   }
-  if (!__syncthreads_or(any != 0u) && skip_zero) {
-    const int gx = x0 + lane;
-    for (int row = warp; row < kBlurTile; row += 8)
-      if (y0 + row < ny && gx < nx) out[(size_t)(y0 + row) * nx + gx] = (TOut)0;
-    return;
-  }
+  __syncthreads();
   double most = 0.0;
   // axis 0: task = (group of 4 output rows, tile column)
   for (int task = t; task < 8 * W; task += 256) {
@@ -1240,11 +1423,12 @@ __global__ void __launch_bounds__(256)
 }
 
 template <typename TOut>
-void blur_tile_r_launch(int r, dim3 grid, const uint16_t *in, const double *w, int ny, int nx,
-                        int skip_zero, unsigned long long *max_bits, TOut *out, cudaStream_t st) {
-#define LMB_BLUR_R(R)                                                                           \
-  case R:                                                                                       \
-    blur_tile_r_kernel<R, TOut><<<grid, 256, 0, st>>>(in, w, ny, nx, skip_zero, max_bits, out); \
+void blur_tile_r_launch(int r, dim3 grid, const uint16_t *in, const BlurWeights &w, int ny, int nx,
+                        const uint8_t *tiles, unsigned long long *max_bits, TOut *out,
+                        cudaStream_t st) {
+#define LMB_BLUR_R(R)                                                                       \
+  case R:                                                                                   \
+    blur_tile_r_kernel<R, TOut><<<grid, 256, 0, st>>>(in, w, ny, nx, tiles, max_bits, out); \
     break;
   switch (r) {
     LMB_BLUR_R(1) LMB_BLUR_R(2) LMB_BLUR_R(3) LMB_BLUR_R(4)
@@ -1618,19 +1802,21 @@ struct lmb_pre {
   uint16_t *d_t16 = nullptr, *d_filt = nullptr;
   int *d_par = nullptr, *d_cid = nullptr, *d_lab = nullptr, *d_flab = nullptr;
   Comps c{};
-  unsigned long long *d_flags = nullptr, *d_pos = nullptr, *d_compact = nullptr;
+  unsigned long long *d_compact = nullptr;
+  unsigned *d_bits = nullptr;  // first-block maps (all, kept) and their segments' counts
+  unsigned nwords = 0, seg_len = 4;
+  uint16_t *d_sub16 = nullptr, *d_bg16 = nullptr;  // whole-number differences, background
+  unsigned *d_bg_other = nullptr;                  // the background is no whole numbers
+  uint8_t *d_tiles = nullptr;                      // blur tiles with a positive pixel
+  int tiles_x = 1, tiles_y = 1;
   unsigned *d_hist16 = nullptr;  // 65536-bin histogram of the first selection pass
-  unsigned *d_fg = nullptr, *d_nfg = nullptr;  // foreground pixel list and its length
-  void *d_fg_tmp = nullptr;
-  size_t fg_bytes = 0;
+  unsigned *d_fg = nullptr;  // foreground pixel list
   bool labels_ready = false;  // label images of the last segment built
   double *d_centres = nullptr, *d_w = nullptr;
   unsigned long long *d_max = nullptr;  // maximum of the blurred frame in d_out
   int *d_stats = nullptr, *d_head = nullptr, *d_next = nullptr;
   int gcx = 1, gcy = 1;
   PreState *d_state = nullptr, *h_state = nullptr;
-  void *d_cub = nullptr;
-  size_t cub_bytes = 0;
   // median scratch, allocated on first use
   unsigned long long *m_keys = nullptr, *m_keys2 = nullptr;
   unsigned *m_idx = nullptr, *m_idx2 = nullptr, *m_flag = nullptr, *m_incl = nullptr,
@@ -1670,9 +1856,9 @@ void free_pre(lmb_pre *p) {
   if (p->st) cudaStreamSynchronize(p->st);
   void *bufs[] = {p->d_raw, p->d_bg, p->d_sub, p->d_tmp, p->d_out, p->d_t16, p->d_filt, p->d_par,
                   p->d_cid, p->d_lab, p->d_flab, p->c.area, p->c.x0, p->c.y0, p->c.x1, p->c.y1,
-                  p->c.fb, p->c.sw, p->c.swx, p->c.swy, p->c.label, p->c.keep, p->d_flags,
-                  p->d_pos, p->d_compact, p->d_centres, p->d_w, p->d_max, p->d_stats, p->d_head, p->d_next,
-                  p->d_state, p->d_cub, p->d_hist16, p->d_fg, p->d_nfg, p->d_fg_tmp, p->m_keys, p->m_keys2, p->m_idx, p->m_idx2, p->m_flag,
+                  p->c.fb, p->c.sw, p->c.swx, p->c.swy, p->c.label, p->c.keep, p->d_bits,
+                  p->d_sub16, p->d_bg16, p->d_bg_other, p->d_tiles, p->d_compact, p->d_centres, p->d_w, p->d_max, p->d_stats, p->d_head, p->d_next,
+                  p->d_state, p->d_hist16, p->d_fg, p->m_keys, p->m_keys2, p->m_idx, p->m_idx2, p->m_flag,
                   p->m_incl, p->m_rank, p->m_nd, p->m_vals, p->m_img, p->m_cub,
                   p->m_v16[0], p->m_v16[1], p->m_flag16};
   for (void *b : bufs)
@@ -1736,27 +1922,38 @@ int run_select(lmb_pre *p, int mode, bool first_pass) {
   return LMB_OK;
 }
 
-// Subtraction fused with the value histogram; *done when every candidate was
-// an integer in [0, 65535] and the threshold is set (else the frame's
-// subtraction is in place for the radix selection).
-int value_select(lmb_pre *p, int dtype, int mode, unsigned long long k0, int two, double gamma,
-                 bool *done) {
+// Subtraction fused with the value histogram.  Where every candidate is a whole
+// number in [0, 65535] the threshold is set and the state's value_path with it.
+int value_select(lmb_pre *p, int dtype, int mode, unsigned long long k0, int two, double gamma) {
   int rc = by_dtype(dtype, [&](auto tag) {
     using T = std::remove_const_t<std::remove_pointer_t<decltype(tag)>>;
     value_hist_kernel<T><<<(unsigned)(p->num_sms * 4), kVhThreads, 0, p->st>>>(
-        static_cast<const T *>(p->d_raw), p->d_bg, p->d_sub, (unsigned)p->npx, p->d_state,
-        p->d_hist16, mode, k0, two, gamma);
+        static_cast<const T *>(p->d_raw), p->d_bg, p->d_bg16, p->d_bg_other, p->d_sub16,
+        (unsigned)p->npx, p->d_state, p->d_hist16, mode, k0, two, gamma);
     return LMB_OK;
   });
   if (rc) return rc;
   LMB_CUDA(cudaGetLastError());
-  LMB_CUDA(cudaMemcpyAsync(&p->h_state->value_path, &p->d_state->value_path, sizeof(unsigned),
-                           cudaMemcpyDeviceToHost, p->st));
-  LMB_CUDA(cudaStreamSynchronize(p->st));
-  *done = p->h_state->value_path != 0;
   return LMB_OK;
 }
 
+int subtract(lmb_pre *p, int dtype) {
+  return by_dtype(dtype, [&](auto tag) {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(tag)>>;
+    subtract_kernel<T><<<(unsigned)grid_for(p->npx, p->num_sms), kT, 0, p->st>>>(
+        static_cast<const T *>(p->d_raw), p->d_bg, p->d_sub, p->npx);
+    return LMB_OK;
+  });
+}
+
+// The background as 16-bit whole numbers, where it is.
+int background_changed(lmb_pre *p) {
+  LMB_CUDA(cudaMemsetAsync(p->d_bg_other, 0, sizeof(unsigned), p->st));
+  whole_kernel<double><<<(unsigned)grid_for(p->npx, p->num_sms), kT, 0, p->st>>>(
+      p->d_bg, p->d_bg16, p->d_bg_other, p->npx);
+  LMB_CUDA(cudaGetLastError());
+  return LMB_OK;
+}
 
 // np.percentile's order statistics and weight for n values (linear method).
 void percentile_plan(size_t n, double pct, unsigned long long *k0, int *two, double *gamma) {
@@ -1778,36 +1975,41 @@ void percentile_plan(size_t n, double pct, unsigned long long *k0, int *two, dou
   *gamma = vi - prev;
 }
 
-// Components, centres and closest pair from d_t16 / d_par.
-int segment_tail(lmb_pre *p, int min_area, lmb_pre_counts *counts, bool parents_ready) {
-  const unsigned g = (unsigned)grid_for(p->npx, p->num_sms);
+// Thresholded pixels, components, centres, filtered frame and closest pair; then
+// the state on the host.
+template <typename Src>
+int segment_tail(lmb_pre *p, const Src &src, int min_area, lmb_pre_counts *counts) {
   cudaStream_t st = p->st;
-  if (!parents_ready) init_parents_kernel<<<g, kT, 0, st>>>(p->d_t16, p->d_par, p->nx, p->npx);
-  // the foreground pixels, in raster order; the component kernels run over them
-  size_t sb = p->fg_bytes;
-  LMB_CUDA(cub::DeviceSelect::If(p->d_fg_tmp, sb, thrust::counting_iterator<unsigned>(0u),
-                                 p->d_fg, p->d_nfg, (int)p->npx, IsForeground{p->d_t16}, st));
-  merge_kernel<<<g, kT, 0, st>>>(p->d_t16, p->d_par, p->nx, p->d_fg, p->d_nfg);
+  // kernels over the foreground list: its length is on the device
+  const unsigned g = (unsigned)p->num_sms * 4;
   reset_counts_kernel<<<1, 1, 0, st>>>(p->d_state);
-  compress_kernel<<<g, kT, 0, st>>>(p->d_par, p->d_cid, p->d_state, p->c, p->d_fg, p->d_nfg);
-  moments_kernel<<<g, kT, 0, st>>>(p->d_par, p->d_cid, p->d_t16, p->c, p->nx, p->d_fg, p->d_nfg);
-  LMB_CUDA(cudaMemsetAsync(p->d_flags, 0, p->nblocks * sizeof(unsigned long long), st));
-  const unsigned gc = (unsigned)grid_for(p->nblocks, p->num_sms);
-  flags_kernel<<<gc, kT, 0, st>>>(p->d_state, p->c, min_area, p->d_flags, p->nblocks);
-  size_t tb = p->cub_bytes;
-  LMB_CUDA(cub::DeviceScan::InclusiveSum(p->d_cub, tb, p->d_flags, p->d_pos, (int)p->nblocks, st));
-  label_kernel<<<gc, kT, 0, st>>>(p->d_state, p->c, min_area, p->d_pos, p->nblocks,
-                                  p->d_centres, p->d_stats);
-  LMB_CUDA(cudaMemsetAsync(p->d_filt, 0, p->npx * sizeof(uint16_t), st));
-  filt_kernel<<<g, kT, 0, st>>>(p->d_par, p->d_cid, p->d_t16, p->c, p->d_filt, p->d_fg, p->d_nfg);
+  const int cells = p->gcx * p->gcy, ntiles = p->tiles_x * p->tiles_y;
+  if (p->npx % 4 == 0)
+    foreground_kernel<4, Src><<<(unsigned)grid_for(p->npx / 4, p->num_sms), kT, 0, st>>>(
+        src, p->d_state, p->d_t16, p->d_filt, p->d_par, p->d_fg, p->nx, p->npx, p->d_head, cells,
+        p->d_tiles, ntiles);
+  else
+    foreground_kernel<1, Src><<<(unsigned)grid_for(p->npx, p->num_sms), kT, 0, st>>>(
+        src, p->d_state, p->d_t16, p->d_filt, p->d_par, p->d_fg, p->nx, p->npx, p->d_head, cells,
+        p->d_tiles, ntiles);
+  LMB_CUDA(cudaEventRecord(p->ev[EV_SEG_THR], st));
+  merge_kernel<<<g, kT, 0, st>>>(p->d_t16, p->d_par, p->nx, p->d_fg, p->d_state);
+  compress_kernel<<<g, kT, 0, st>>>(p->d_par, p->d_cid, p->d_state, p->c, p->d_fg);
+  moments_kernel<<<g, kT, 0, st>>>(p->d_par, p->d_cid, p->d_t16, p->c, p->nx, p->d_fg, p->d_state);
+  unsigned *bits = p->d_bits, *keep_bits = bits + p->nwords;
+  unsigned *seg = keep_bits + p->nwords, *keep_seg = seg + kSegs;
+  flags_kernel<<<g, kT, 0, st>>>(p->d_state, p->c, min_area, bits, keep_bits);
+  rank_bits_kernel<<<2, kSegs, 0, st>>>(p->d_state, bits, keep_bits, p->nwords, p->seg_len, seg,
+                                        keep_seg);
+  label_kernel<<<g, kT, 0, st>>>(p->d_state, p->c, min_area, bits, keep_bits, seg, keep_seg,
+                                 p->seg_len, p->d_centres, p->d_stats, p->d_head, p->d_next, p->gcx,
+                                 p->gcy);
+  finish_kernel<<<(unsigned)p->num_sms * 2, kT, 0, st>>>(
+      p->d_state, p->c, p->d_par, p->d_cid, p->d_t16, p->d_filt, p->d_fg, p->nx, p->d_tiles,
+      p->tiles_x, bits, keep_bits, p->d_centres, p->d_head, p->d_next, p->gcx, p->gcy);
+  if (3 * (size_t)cells > kBruteLast)  // else the last block has taken them
+    brute_pairs_kernel<<<p->num_sms * 2, kT, 0, st>>>(p->d_state, p->d_centres);
   p->labels_ready = false;
-  // closest pair of kept centres
-  LMB_CUDA(cudaMemsetAsync(p->d_head, 0xff, (size_t)p->gcx * p->gcy * sizeof(int), st));
-  cell_insert_kernel<<<gc, kT, 0, st>>>(p->d_state, p->d_centres, p->d_head, p->d_next, p->gcx,
-                                        p->gcy);
-  cell_pairs_kernel<<<gc, kT, 0, st>>>(p->d_state, p->d_centres, p->d_head, p->d_next, p->gcx,
-                                       p->gcy);
-  brute_pairs_kernel<<<p->num_sms * 2, kT, 0, st>>>(p->d_state, p->d_centres);
   LMB_CUDA(cudaGetLastError());
   LMB_CUDA(cudaEventRecord(p->ev[EV_SEG_CC], st));
   PreState *hs = p->h_state;
@@ -1945,6 +2147,11 @@ int lmb_pre_create(int32_t device, int32_t nr_px_y, int32_t nr_px_x, lmb_pre **o
   p->nblocks = (size_t)((nr_px_y + 1) / 2) * ((nr_px_x + 1) / 2);
   p->gcx = (nr_px_x + kCell - 1) / kCell;
   p->gcy = (nr_px_y + kCell - 1) / kCell;
+  p->tiles_x = (nr_px_x + kBlurTile - 1) / kBlurTile;
+  p->tiles_y = (nr_px_y + kBlurTile - 1) / kBlurTile;
+  // a map's words, and its segments' lengths, in multiples of 4
+  p->nwords = (unsigned)((p->nblocks + 127) / 128 * 4);
+  p->seg_len = std::max(4u, ((p->nwords + kSegs - 1) / kSegs + 3) / 4 * 4);
   cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, device);
   int rc = LMB_OK;
   auto fail = [&](int r) {
@@ -1963,21 +2170,15 @@ int lmb_pre_create(int32_t device, int32_t nr_px_y, int32_t nr_px_x, lmb_pre **o
       (rc = alloc(&p->c.y1, nb)) || (rc = alloc(&p->c.fb, nb)) || (rc = alloc(&p->c.sw, nb)) ||
       (rc = alloc(&p->c.swx, nb)) || (rc = alloc(&p->c.swy, nb)) ||
       (rc = alloc(&p->c.label, nb)) || (rc = alloc(&p->c.keep, nb)) ||
-      (rc = alloc(&p->d_flags, nb)) || (rc = alloc(&p->d_pos, nb)) ||
+      (rc = alloc(&p->d_bits, 2 * (size_t)p->nwords + 2 * kSegs)) || (rc = alloc(&p->d_sub16, n)) ||
+      (rc = alloc(&p->d_bg16, n)) || (rc = alloc(&p->d_bg_other, 1)) ||
+      (rc = alloc(&p->d_tiles, (size_t)p->tiles_x * p->tiles_y)) ||
       (rc = alloc(&p->d_compact, n)) || (rc = alloc(&p->d_centres, nb * 4)) ||
       (rc = alloc(&p->d_w, 1024)) || (rc = alloc(&p->d_max, 1)) || (rc = alloc(&p->d_stats, nb * 5)) ||
       (rc = alloc(&p->d_head, (size_t)p->gcx * p->gcy)) || (rc = alloc(&p->d_next, nb)) ||
       (rc = alloc(&p->d_state, 1)) || (rc = alloc(&p->d_hist16, 65536)) ||
-      (rc = alloc(&p->d_fg, n)) || (rc = alloc(&p->d_nfg, 1)))
+      (rc = alloc(&p->d_fg, n)))
     return fail(rc);
-  {
-    size_t fb = 0;
-    if (cub::DeviceSelect::If(nullptr, fb, thrust::counting_iterator<unsigned>(0u), p->d_fg,
-                              p->d_nfg, (int)n, IsForeground{p->d_t16}) != cudaSuccess ||
-        cudaMalloc(&p->d_fg_tmp, std::max<size_t>(fb, 1)) != cudaSuccess)
-      return fail(cuda_fail(cudaGetLastError(), "foreground list set-up", __FILE__, __LINE__));
-    p->fg_bytes = fb;
-  }
   if (cudaMemset(p->d_hist16, 0, 65536 * sizeof(unsigned)) != cudaSuccess)
     return fail(cuda_fail(cudaGetLastError(), "cudaMemset", __FILE__, __LINE__));
   {
@@ -1998,14 +2199,11 @@ int lmb_pre_create(int32_t device, int32_t nr_px_y, int32_t nr_px_x, lmb_pre **o
   memset(p->h_state, 0, sizeof(PreState));
   p->h_state->best = 0x7ff0000000000000ull;
   if (cudaMemset(p->d_bg, 0, n * sizeof(double)) != cudaSuccess ||
+      cudaMemset(p->d_bg16, 0, n * sizeof(uint16_t)) != cudaSuccess ||
+      cudaMemset(p->d_bg_other, 0, sizeof(unsigned)) != cudaSuccess ||
+      cudaMemset(p->d_bits, 0, 2 * (size_t)p->nwords * sizeof(unsigned)) != cudaSuccess ||
       cudaMemset(p->d_state, 0, sizeof(PreState)) != cudaSuccess)
     return fail(cuda_fail(cudaGetLastError(), "cudaMemset", __FILE__, __LINE__));
-  size_t tb = 0;
-  if (cub::DeviceScan::InclusiveSum(nullptr, tb, p->d_flags, p->d_pos, (int)nb) != cudaSuccess)
-    return fail(cuda_fail(cudaGetLastError(), "scan sizing", __FILE__, __LINE__));
-  p->cub_bytes = tb;
-  if (cudaMalloc(&p->d_cub, std::max<size_t>(tb, 1)) != cudaSuccess)
-    return fail(cuda_fail(cudaErrorMemoryAllocation, "cudaMalloc", __FILE__, __LINE__));
   *out = p;
   return LMB_OK;
 }
@@ -2024,6 +2222,7 @@ int lmb_pre_set_background(lmb_pre *p, const double *background) {
                              p->st));
   else
     LMB_CUDA(cudaMemsetAsync(p->d_bg, 0, p->npx * sizeof(double), p->st));
+  if ((rc = background_changed(p))) return rc;
   LMB_CUDA(cudaStreamSynchronize(p->st));
   return LMB_OK;
 }
@@ -2064,6 +2263,7 @@ int lmb_pre_median(lmb_pre *p, const void *frame, int32_t dtype, int32_t size, i
       if ((rc = median_pass(p, p->m_img, p->d_bg, size))) return rc;
     }
   }
+  if ((rc = background_changed(p))) return rc;
   if (out)
     LMB_CUDA(cudaMemcpyAsync(out, p->d_bg, p->npx * sizeof(double), cudaMemcpyDeviceToHost, p->st));
   LMB_CUDA(cudaStreamSynchronize(p->st));
@@ -2081,49 +2281,43 @@ int lmb_pre_segment(lmb_pre *p, const void *frame, int32_t dtype, const lmb_pre_
   LMB_CUDA(cudaEventRecord(p->ev[EV_SEG0], p->st));
   if ((rc = upload_frame(p, frame, dtype))) return rc;
   LMB_CUDA(cudaEventRecord(p->ev[EV_SEG_UP], p->st));
-  const unsigned g = (unsigned)grid_for(p->npx, p->num_sms);
   if (prm->override_thresh > 0 || prm->threshold_method == LMB_THR_FIXED) {
-    rc = by_dtype(dtype, [&](auto tag) {
-      using T = std::remove_const_t<std::remove_pointer_t<decltype(tag)>>;
-      subtract_kernel<T><<<g, kT, 0, p->st>>>(static_cast<const T *>(p->d_raw), p->d_bg,
-                                              p->d_sub, p->npx);
-      return LMB_OK;
-    });
-    if (rc) return rc;
+    if ((rc = subtract(p, dtype))) return rc;
     set_thresh_kernel<<<1, 1, 0, p->st>>>(
         p->d_state, prm->override_thresh > 0 ? prm->override_thresh : prm->threshold_value);
-  } else if (prm->threshold_method == LMB_THR_PERCENTILE) {
-    unsigned long long k0;
-    int two;
-    double gamma;
-    LMB_REQUIRE(prm->threshold_percentile >= 0.0 && prm->threshold_percentile <= 100.0,
-                "Percentiles must be in the range [0, 100]");
-    percentile_plan(p->npx, prm->threshold_percentile, &k0, &two, &gamma);
-    sel_init_kernel<<<1, kT, 0, p->st>>>(p->d_state, SEL_ALL, p->npx, k0, two, 1);
-    bool done = false;
-    if ((rc = value_select(p, dtype, SEL_ALL, k0, two, gamma, &done))) return rc;
-    if (!done) {
-      if ((rc = run_select(p, SEL_ALL, true))) return rc;
-      finish_percentile_kernel<<<1, 1, 0, p->st>>>(p->d_state, gamma);
-    }
+    rc = segment_tail(p, FromSub{p->d_sub}, prm->min_area, counts);
   } else {
-    LMB_REQUIRE(prm->threshold_method == LMB_THR_ADAPTIVE, "threshold method %d",
+    const bool pct = prm->threshold_method == LMB_THR_PERCENTILE;
+    LMB_REQUIRE(pct || prm->threshold_method == LMB_THR_ADAPTIVE, "threshold method %d",
                 prm->threshold_method);
-    sel_init_kernel<<<1, kT, 0, p->st>>>(p->d_state, SEL_NZ, p->npx, 0, 0, 1);
-    bool done = false;
-    if ((rc = value_select(p, dtype, SEL_NZ, 0, 0, 0.0, &done))) return rc;
-    if (!done) {
-      if ((rc = run_select(p, SEL_NZ, true))) return rc;
-      finish_median_kernel<<<1, 1, 0, p->st>>>(p->d_state);
-      sel_init_kernel<<<1, kT, 0, p->st>>>(p->d_state, SEL_ABSDEV, p->npx, 0, 0, 0);
-      if ((rc = run_select(p, SEL_ABSDEV, true))) return rc;
-      finish_adaptive_kernel<<<1, 1, 0, p->st>>>(p->d_state);
+    unsigned long long k0 = 0;
+    int two = 0;
+    double gamma = 0.0;
+    if (pct) {
+      LMB_REQUIRE(prm->threshold_percentile >= 0.0 && prm->threshold_percentile <= 100.0,
+                  "Percentiles must be in the range [0, 100]");
+      percentile_plan(p->npx, prm->threshold_percentile, &k0, &two, &gamma);
+    }
+    // whole-number frames: everything in one go, the state read once at its end
+    if ((rc = value_select(p, dtype, pct ? SEL_ALL : SEL_NZ, k0, two, gamma))) return rc;
+    rc = segment_tail(p, FromSub16{p->d_sub16}, prm->min_area, counts);
+    if (rc == LMB_OK && !p->h_state->value_path) {  // another frame: nothing was segmented
+      if ((rc = subtract(p, dtype))) return rc;
+      if (pct) {
+        sel_init_kernel<<<1, kT, 0, p->st>>>(p->d_state, SEL_ALL, p->npx, k0, two);
+        if ((rc = run_select(p, SEL_ALL, true))) return rc;
+        finish_percentile_kernel<<<1, 1, 0, p->st>>>(p->d_state, gamma);
+      } else {
+        sel_init_kernel<<<1, kT, 0, p->st>>>(p->d_state, SEL_NZ, p->npx, 0, 0);
+        if ((rc = run_select(p, SEL_NZ, true))) return rc;
+        finish_median_kernel<<<1, 1, 0, p->st>>>(p->d_state);
+        sel_init_kernel<<<1, kT, 0, p->st>>>(p->d_state, SEL_ABSDEV, p->npx, 0, 0);
+        if ((rc = run_select(p, SEL_ABSDEV, true))) return rc;
+        finish_adaptive_kernel<<<1, 1, 0, p->st>>>(p->d_state);
+      }
+      rc = segment_tail(p, FromSub{p->d_sub}, prm->min_area, counts);
     }
   }
-  apply_kernel<<<g, kT, 0, p->st>>>(p->d_sub, p->d_state, p->d_t16, p->d_par, p->nx, p->npx);
-  LMB_CUDA(cudaGetLastError());
-  LMB_CUDA(cudaEventRecord(p->ev[EV_SEG_THR], p->st));
-  rc = segment_tail(p, prm->min_area, counts, true);
   if (rc) return rc;
   return stage_times(p, EV_SEG0, EV_SEG_UP, 0) || stage_times(p, EV_SEG_UP, EV_SEG_THR, 1) ||
          stage_times(p, EV_SEG_THR, EV_SEG_CC, 2);
@@ -2138,7 +2332,7 @@ int lmb_pre_segment_thresholded(lmb_pre *p, const uint16_t *thresholded, int32_t
                            cudaMemcpyHostToDevice, p->st));
   set_thresh_kernel<<<1, 1, 0, p->st>>>(p->d_state, 0.0);
   LMB_CUDA(cudaGetLastError());
-  return segment_tail(p, min_area, counts, false);
+  return segment_tail(p, FromThresholded{p->d_t16}, min_area, counts);
 }
 
 int lmb_pre_centres(lmb_pre *p, double *centres, int32_t cap) {
@@ -2175,7 +2369,7 @@ int lmb_pre_images(lmb_pre *p, uint16_t *thresholded, int32_t *labels, uint16_t 
     LMB_CUDA(cudaMemsetAsync(p->d_lab, 0, n * sizeof(int), p->st));
     LMB_CUDA(cudaMemsetAsync(p->d_flab, 0, n * sizeof(int), p->st));
     labels_kernel<<<(unsigned)grid_for(n, p->num_sms), kT, 0, p->st>>>(
-        p->d_par, p->d_cid, p->c, p->d_lab, p->d_flab, p->d_fg, p->d_nfg);
+        p->d_par, p->d_cid, p->c, p->d_lab, p->d_flab, p->d_fg, p->d_state);
     LMB_CUDA(cudaGetLastError());
     p->labels_ready = true;
   }
@@ -2208,21 +2402,27 @@ int blur_launch(lmb_pre *p, const double *weights, int32_t radius, int32_t out_d
     p->out_in_use = false;
   }
   LMB_CUDA(cudaEventRecord(p->ev[EV_BLUR0], p->st));
-  LMB_CUDA(cudaMemcpyAsync(p->d_w, weights, (size_t)(2 * radius + 1) * sizeof(double),
-                           cudaMemcpyHostToDevice, p->st));
+  const bool fixed = radius >= 1 && radius <= kBlurFixedMaxR;
+  if (!fixed)
+    LMB_CUDA(cudaMemcpyAsync(p->d_w, weights, (size_t)(2 * radius + 1) * sizeof(double),
+                             cudaMemcpyHostToDevice, p->st));
   const unsigned g = (unsigned)grid_for(p->npx, p->num_sms);
-  if (radius >= 1 && radius <= kBlurFixedMaxR) {
-    const dim3 tg((p->nx + kBlurTile - 1) / kBlurTile, (p->ny + kBlurTile - 1) / kBlurTile);
-    int skip_zero = 1;
-    for (int j = 0; j <= 2 * radius; j++)
-      if (!(std::isfinite(weights[j]) && !std::signbit(weights[j]))) skip_zero = 0;
+  if (fixed) {
+    const dim3 tg((unsigned)p->tiles_x, (unsigned)p->tiles_y);
+    bool skip_zero = p->nx >= 2 * kBlurTile && p->ny >= 2 * kBlurTile;
+    BlurWeights bw{};
+    for (int j = 0; j <= 2 * radius; j++) {
+      bw.w[j] = weights[j];
+      if (!(std::isfinite(weights[j]) && !std::signbit(weights[j]))) skip_zero = false;
+    }
+    const uint8_t *tiles = skip_zero ? p->d_tiles : nullptr;
     if (want_max) LMB_CUDA(cudaMemsetAsync(p->d_max, 0, sizeof(unsigned long long), p->st));
     unsigned long long *mx = want_max ? p->d_max : nullptr;
     if (out_dtype == LMB_F64)
-      blur_tile_r_launch<double>(radius, tg, p->d_filt, p->d_w, p->ny, p->nx, skip_zero, mx,
+      blur_tile_r_launch<double>(radius, tg, p->d_filt, bw, p->ny, p->nx, tiles, mx,
                                  static_cast<double *>(p->d_out), p->st);
     else
-      blur_tile_r_launch<float>(radius, tg, p->d_filt, p->d_w, p->ny, p->nx, skip_zero, mx,
+      blur_tile_r_launch<float>(radius, tg, p->d_filt, bw, p->ny, p->nx, tiles, mx,
                                 static_cast<float *>(p->d_out), p->st);
     if (have_max) *have_max = want_max;
   } else if (radius <= kBlurTileMaxR) {
