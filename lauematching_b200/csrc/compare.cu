@@ -1498,8 +1498,20 @@ __device__ void bitonic_tiled(unsigned long long *g, uint32_t P, unsigned long l
   }
 }
 
-__global__ void __launch_bounds__(1024) order_kernel(OrderArgs a) {
+// One block per slot of the pass.  Short lists and the pass's status words also
+// go to page-locked host memory from here, so that a caller who waits for the pass
+// has its results without another copy (a gather kernel, a copy and its
+// synchronisation; 20-25 us of a small pass, measured on B200).
+__global__ void __launch_bounds__(1024) order_kernel(const __grid_constant__ OrderArgs a) {
   extern __shared__ __align__(16) unsigned long long sk[];  // kSmemSortMax keys
+  if (blockIdx.x == 0) {
+    const unsigned r = *a.seq % a.ring;
+    for (uint32_t w = threadIdx.x; w < a.words; w += blockDim.x)
+      a.host_status[r * a.words + w] = a.status[w];
+    __syncthreads();
+    if (threadIdx.x == 0) *a.seq += 1u;
+  }
+  if ((int)blockIdx.x >= a.nslots) return;  // a pass without slots
   const int k = a.slots[blockIdx.x];
   const uint32_t n = min(a.surv_cnt[k], a.cap);
   if (n == 0) return;
@@ -1514,8 +1526,15 @@ __global__ void __launch_bounds__(1024) order_kernel(OrderArgs a) {
     bitonic(keys, P);
   else
     bitonic_tiled(keys, P, sk);
-  lmb_survivor *dst = a.out + (size_t)k * a.cap;
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[keys[i] & 0xFFFFFFull];
+  // 16-byte halves of the 32-byte survivors
+  const uint4 *from = reinterpret_cast<const uint4 *>(src);
+  uint4 *dst = reinterpret_cast<uint4 *>(a.out + (size_t)k * a.cap);
+  uint4 *host = n <= a.host_cap ? reinterpret_cast<uint4 *>(a.host_list + (size_t)k * a.host_cap) : nullptr;
+  for (uint32_t w = threadIdx.x; w < 2 * n; w += blockDim.x) {
+    const uint4 v = from[2 * (keys[w >> 1] & 0xFFFFFFull) + (w & 1u)];
+    dst[w] = v;
+    if (host) host[w] = v;
+  }
 }
 
 // ----------------------------------------------------------------------------
@@ -1775,12 +1794,11 @@ int gather_launch(const GatherArgs &g, cudaStream_t st) {
   return LMB_OK;
 }
 
-int order_launch(const OrderArgs &a, int nslots, cudaStream_t st) {
-  if (nslots == 0) return LMB_OK;
+int order_launch(const OrderArgs &a, cudaStream_t st) {
   const int smem = (int)(kSmemSortMax * sizeof(unsigned long long));
   const int rc = ensure_smem((const void *)order_kernel, smem);
   if (rc) return rc;
-  order_kernel<<<nslots, 1024, smem, st>>>(a);
+  order_kernel<<<std::max(a.nslots, 1), 1024, smem, st>>>(a);
   LMB_CUDA(cudaGetLastError());
   return LMB_OK;
 }

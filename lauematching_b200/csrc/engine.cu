@@ -37,6 +37,9 @@ using namespace lmb;
 // results are read from the entry of the last pass that included it.
 static constexpr int kStatusWords = 2 * LMB_MAX_SLOTS + 1;
 static constexpr int kStatusRing = 4;
+static constexpr int kEventRing = 64;  // events of passes and loads
+// Survivor lists up to this long are written to host memory by the pass itself.
+static constexpr uint32_t kHostList = 4096;
 
 static constexpr int kSparseRing = 4;  // pinned staging buffers for sparse frames
 
@@ -113,7 +116,8 @@ struct lmb_engine {
   unsigned long long *d_scratch = nullptr;
   unsigned int *d_status = nullptr;
   unsigned int *h_status = nullptr;  // pinned, kStatusRing x kStatusWords
-  cudaEvent_t ev_done[kStatusRing] = {};  // a pass and its status copy finished
+  unsigned int *d_seq = nullptr;          // passes ordered so far (the order kernel's count)
+  lmb_survivor *h_list = nullptr;         // pinned: [64][kHostList], short lists of each slot
   uint64_t pass_seq = 0;                  // passes enqueued so far
   int slot_ring[LMB_MAX_SLOTS] = {};      // status entry of each slot's last pass
   uint64_t done_mask = 0;                 // slots that have been in a pass
@@ -121,10 +125,15 @@ struct lmb_engine {
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
   // image uploads run on their own stream so they overlap a running pass:
   // a pass waits for its slots' uploads, an upload waits until the last pass
-  // that read its slot has finished.
+  // that read its slot has finished.  One event per pass and one per load call,
+  // from rings: an event used again has a later point of the same stream, so a
+  // wait for its old meaning still holds.
   cudaStream_t ld = nullptr;
-  cudaEvent_t ev_loaded[LMB_MAX_SLOTS] = {};
-  cudaEvent_t ev_released[LMB_MAX_SLOTS] = {};
+  cudaEvent_t ev_pass[kEventRing] = {}, ev_load[kEventRing] = {};
+  uint64_t load_seq = 0;
+  int slot_pass[LMB_MAX_SLOTS] = {};  // ev_pass of the slot's last pass (done_mask)
+  int slot_load[LMB_MAX_SLOTS] = {};  // ev_load of the slot's last load
+  uint64_t fresh_mask = 0;            // slots loaded since a pass waited for them
   // automatic variant with the compact pass's tuned shape (2 stages, 3 consumer
   // warps, 8 blocks per SM)
   CompareTuning tuning{3, 0, 2, 3, 1, 8, 0, 0, 0, 0, 0};
@@ -176,6 +185,31 @@ void free_grouped(lmb_engine *e) {
   e->gl_bytes = 0;
 }
 
+// Slots about to be written on the load stream: after the last passes that read
+// them.
+int wait_released(lmb_engine *e, uint64_t slots) {
+  uint64_t waited = 0;  // events of the ring
+  for (int k = 0; k < LMB_MAX_SLOTS; k++) {
+    if (!((slots & e->done_mask) >> k & 1)) continue;
+    const int v = e->slot_pass[k];
+    if (waited >> v & 1) continue;
+    waited |= 1ull << v;
+    LMB_CUDA(cudaStreamWaitEvent(e->ld, e->ev_pass[v], 0));
+  }
+  return LMB_OK;
+}
+
+// Slots written on the load stream up to here.
+int mark_loaded(lmb_engine *e, uint64_t slots) {
+  const int v = (int)(e->load_seq++ % kEventRing);
+  LMB_CUDA(cudaEventRecord(e->ev_load[v], e->ld));
+  for (int k = 0; k < LMB_MAX_SLOTS; k++)
+    if (slots >> k & 1) e->slot_load[k] = v;
+  e->fresh_mask |= slots;
+  e->loaded_mask |= slots;
+  return LMB_OK;
+}
+
 int check_engine(lmb_engine *e) {
   if (!e) {
     set_error("null engine");
@@ -205,8 +239,8 @@ void free_engine(lmb_engine *e) {
   cudaFree(e->d_scratch);
   cudaFree(e->d_status);
   cudaFreeHost(e->h_status);
-  for (auto &v : e->ev_done)
-    if (v) cudaEventDestroy(v);
+  cudaFreeHost(e->h_list);
+  cudaFree(e->d_seq);
   if (e->dl) {
     cudaStreamSynchronize(e->dl);
     cudaStreamDestroy(e->dl);
@@ -227,9 +261,9 @@ void free_engine(lmb_engine *e) {
   cudaFree(e->d_gather);
   for (auto &v : e->ev)
     if (v) cudaEventDestroy(v);
-  for (int k = 0; k < LMB_MAX_SLOTS; k++) {
-    if (e->ev_loaded[k]) cudaEventDestroy(e->ev_loaded[k]);
-    if (e->ev_released[k]) cudaEventDestroy(e->ev_released[k]);
+  for (int k = 0; k < kEventRing; k++) {
+    if (e->ev_pass[k]) cudaEventDestroy(e->ev_pass[k]);
+    if (e->ev_load[k]) cudaEventDestroy(e->ev_load[k]);
   }
   if (e->st) cudaStreamDestroy(e->st);
   if (e->ld) cudaStreamDestroy(e->ld);
@@ -756,10 +790,16 @@ int enqueue_pass(lmb_engine *e, const PassKey &k, bool capturing) {
   o.cap = e->cap;
   o.scratch = e->d_scratch;
   o.cap2 = e->cap2;
-  int ns = 0;
+  o.host_list = e->h_list;
+  o.host_cap = std::min(kHostList, e->cap);
+  o.host_status = e->h_status;
+  o.status = e->d_status;
+  o.words = kStatusWords;
+  o.ring = kStatusRing;
+  o.seq = e->d_seq;
   for (int i = 0; i < LMB_MAX_SLOTS; i++)
-    if (k.mask >> i & 1) o.slots[ns++] = i;
-  const int rc = order_launch(o, ns, e->st);
+    if (k.mask >> i & 1) o.slots[o.nslots++] = i;
+  const int rc = order_launch(o, e->st);
   if (rc) return rc;
   LMB_CUDA(cudaEventRecordWithFlags(e->ev[2], e->st, evf));
   return LMB_OK;
@@ -829,11 +869,10 @@ int lmb_engine_create(int32_t device, const lmb_geometry *geo, uint64_t survivor
   TRY(cudaStreamCreateWithFlags(&e->st, cudaStreamNonBlocking));
   TRY(cudaStreamCreateWithFlags(&e->ld, cudaStreamNonBlocking));
   TRY(cudaStreamCreateWithFlags(&e->dl, cudaStreamNonBlocking));
-  for (auto &v : e->ev_done) TRY(cudaEventCreateWithFlags(&v, cudaEventDisableTiming));
   for (auto &v : e->ev) TRY(cudaEventCreate(&v));
-  for (int k = 0; k < LMB_MAX_SLOTS; k++) {
-    TRY(cudaEventCreateWithFlags(&e->ev_loaded[k], cudaEventDisableTiming));
-    TRY(cudaEventCreateWithFlags(&e->ev_released[k], cudaEventDisableTiming));
+  for (int k = 0; k < kEventRing; k++) {
+    TRY(cudaEventCreateWithFlags(&e->ev_pass[k], cudaEventDisableTiming));
+    TRY(cudaEventCreateWithFlags(&e->ev_load[k], cudaEventDisableTiming));
   }
   TRY(cudaMalloc(&e->d_u8, e->npx * LMB_MAX_SLOTS));
   TRY(cudaMemset(e->d_u8, 0, e->npx * LMB_MAX_SLOTS));
@@ -855,6 +894,10 @@ int lmb_engine_create(int32_t device, const lmb_geometry *geo, uint64_t survivor
   TRY(cudaHostAlloc(&e->h_status, kStatusRing * kStatusWords * sizeof(unsigned int),
                     cudaHostAllocDefault));
   memset(e->h_status, 0, kStatusRing * kStatusWords * sizeof(unsigned int));
+  TRY(cudaHostAlloc(&e->h_list, (size_t)LMB_MAX_SLOTS * kHostList * sizeof(lmb_survivor),
+                    cudaHostAllocDefault));
+  TRY(cudaMalloc(&e->d_seq, sizeof(unsigned int)));
+  TRY(cudaMemset(e->d_seq, 0, sizeof(unsigned int)));
 #undef TRY
   *out = e;
   return LMB_OK;
@@ -997,7 +1040,7 @@ int lmb_image_load(lmb_engine *e, int32_t slot, const void *pixels, int32_t dtyp
   LMB_REQUIRE(dtype == LMB_F64 || dtype == LMB_F32 || dtype == 2, "unknown dtype %d", dtype);
   if (keep_f64 && !e->d_f64)
     LMB_CUDA(cudaMalloc(&e->d_f64, e->npx * sizeof(double) * LMB_MAX_SLOTS));
-  LMB_CUDA(cudaStreamWaitEvent(e->ld, e->ev_released[slot], 0));
+  if ((rc = wait_released(e, 1ull << slot))) return rc;
   // A sparse frame (the usual thresholded Laue image) crosses the host link
   // as (index, value) pairs of its positive pixels; a dense one as is.
   bool sparse = false;
@@ -1017,8 +1060,7 @@ int lmb_image_load(lmb_engine *e, int32_t slot, const void *pixels, int32_t dtyp
                          e->d_scale + slot, e->num_sms, e->ld);
     if (rc) return rc;
   }
-  LMB_CUDA(cudaEventRecord(e->ev_loaded[slot], e->ld));
-  e->loaded_mask |= 1ull << slot;
+  if ((rc = mark_loaded(e, 1ull << slot))) return rc;
   if (keep_f64)
     e->f64_mask |= 1ull << slot;
   else
@@ -1047,16 +1089,16 @@ namespace {
 // One frame the dense way (copy of the whole frame, max + quantise kernels)
 // on the load stream, without a host scan.
 int dense_load(lmb_engine *e, int slot, const void *pixels, int dtype) {
-  LMB_CUDA(cudaStreamWaitEvent(e->ld, e->ev_released[slot], 0));
+  int rc = wait_released(e, 1ull << slot);
+  if (rc) return rc;
   const size_t bytes = e->npx * dtype_bytes(dtype);
   LMB_CUDA(cudaMemcpyAsync(e->d_stage, pixels, bytes, cudaMemcpyHostToDevice, e->ld));
   e->bytes_h2d += bytes;
-  const int rc = quantize_launch(e->d_stage, dtype, e->npx, e->d_max_bits, false,
-                                 e->d_u8 + (size_t)slot * e->npx, nullptr, e->d_occ, slot,
-                                 e->d_scale + slot, e->num_sms, e->ld);
+  rc = quantize_launch(e->d_stage, dtype, e->npx, e->d_max_bits, false,
+                       e->d_u8 + (size_t)slot * e->npx, nullptr, e->d_occ, slot, e->d_scale + slot,
+                       e->num_sms, e->ld);
   if (rc) return rc;
-  LMB_CUDA(cudaEventRecord(e->ev_loaded[slot], e->ld));
-  e->loaded_mask |= 1ull << slot;
+  if ((rc = mark_loaded(e, 1ull << slot))) return rc;
   e->f64_mask &= ~(1ull << slot);
   return LMB_OK;
 }
@@ -1167,8 +1209,9 @@ int load_batch_sparse(lmb_engine *e, const int32_t *slots, const void *const *fr
       memcpy(pidx + toff[t], sidx + (size_t)t * capf, c * 4);
       memcpy(pval + toff[t], sval + (size_t)t * capf, c * vb);
     }
-    for (int i = 0; i < ns; i++)
-      LMB_CUDA(cudaStreamWaitEvent(e->ld, e->ev_released[desc[i].slot], 0));
+    uint64_t written = 0;
+    for (int i = 0; i < ns; i++) written |= 1ull << desc[i].slot;
+    if (const int rc = wait_released(e, written)) return rc;
     LMB_CUDA(cudaMemcpyAsync(e->d_batch, h, bytes, cudaMemcpyHostToDevice, e->ld));
     LMB_CUDA(cudaEventRecord(e->bt_ev[r], e->ld));
     e->bytes_h2d += bytes;
@@ -1179,12 +1222,8 @@ int load_batch_sparse(lmb_engine *e, const int32_t *slots, const void *const *fr
         e->d_scale, npx, e->num_sms, e->ld);
     if (rc) return rc;
     e->sparse_loads += ns;
-    for (int i = 0; i < ns; i++) {
-      const int s = desc[i].slot;
-      LMB_CUDA(cudaEventRecord(e->ev_loaded[s], e->ld));
-      e->loaded_mask |= 1ull << s;
-      e->f64_mask &= ~(1ull << s);
-    }
+    if (const int rc = mark_loaded(e, written)) return rc;
+    e->f64_mask &= ~written;
   }
   for (int f : dense) {
     const int rc = lmb_image_load(e, slots[f], frames[f], dtype, 0, nullptr);
@@ -1308,8 +1347,13 @@ int lmb_match(lmb_engine *e, uint64_t slot_mask, int32_t min_nr_spots, double mi
       tun = CompareTuning{1, 0, 0, 0, 0, 0, tun.full_gather, tun.test_consumer_wait_us, 0, 0, 0};
   }
   e->last_variant = tun.variant;
-  for (int k = 0; k < LMB_MAX_SLOTS; k++)
-    if (slot_mask >> k & 1) LMB_CUDA(cudaStreamWaitEvent(e->st, e->ev_loaded[k], 0));
+  uint64_t waited = 0;
+  for (int k = 0; k < LMB_MAX_SLOTS; k++) {
+    if (!((slot_mask & e->fresh_mask) >> k & 1) || (waited >> e->slot_load[k] & 1)) continue;
+    waited |= 1ull << e->slot_load[k];
+    LMB_CUDA(cudaStreamWaitEvent(e->st, e->ev_load[e->slot_load[k]], 0));
+  }
+  e->fresh_mask &= ~slot_mask;
   // The pass (status reset, compare, ordering, status copy-back) replays from
   // a CUDA graph once a configuration has been seen before; the first pass of
   // a configuration runs eagerly (it also sets the kernels' attributes).
@@ -1351,16 +1395,15 @@ int lmb_match(lmb_engine *e, uint64_t slot_mask, int32_t min_nr_spots, double mi
     rc = enqueue_pass(e, key, false);
     if (rc) return rc;
   }
-  for (int k = 0; k < LMB_MAX_SLOTS; k++)
-    if (slot_mask >> k & 1) LMB_CUDA(cudaEventRecord(e->ev_released[k], e->st));
-  // the pass's status words into the next ring entry
-  const int r = (int)(e->pass_seq % kStatusRing);
-  LMB_CUDA(cudaMemcpyAsync(e->h_status + (size_t)r * kStatusWords, e->d_status,
-                           kStatusWords * sizeof(unsigned int), cudaMemcpyDeviceToHost, e->st));
-  LMB_CUDA(cudaEventRecord(e->ev_done[r], e->st));
+  // the pass's ordering kernel has written its status words into the next ring entry
+  const int r = (int)(e->pass_seq % kStatusRing), v = (int)(e->pass_seq % kEventRing);
+  LMB_CUDA(cudaEventRecord(e->ev_pass[v], e->st));
   e->bytes_d2h += kStatusWords * sizeof(unsigned int);
   for (int k = 0; k < LMB_MAX_SLOTS; k++)
-    if (slot_mask >> k & 1) e->slot_ring[k] = r;
+    if (slot_mask >> k & 1) {
+      e->slot_ring[k] = r;
+      e->slot_pass[k] = v;
+    }
   e->done_mask |= slot_mask;
   e->pass_seq++;
   return LMB_OK;
@@ -1370,12 +1413,15 @@ int lmb_match(lmb_engine *e, uint64_t slot_mask, int32_t min_nr_spots, double mi
 
 namespace {
 
-// Wait for the last pass that included `slot`; its status words.
-int slot_status(lmb_engine *e, int slot, const unsigned int **st) {
+// Wait for the last pass that included `slot`; its status words.  waited: the
+// events of the ring that the caller has waited for already.
+int slot_status(lmb_engine *e, int slot, const unsigned int **st, uint64_t *waited) {
   LMB_REQUIRE(slot >= 0 && slot < LMB_MAX_SLOTS && (e->done_mask >> slot & 1),
               "slot %d has not been part of a pass", slot);
   const int r = e->slot_ring[slot];
-  LMB_CUDA(cudaEventSynchronize(e->ev_done[r]));
+  const int v = e->slot_pass[slot];
+  if (!(*waited >> v & 1)) LMB_CUDA(cudaEventSynchronize(e->ev_pass[v]));
+  *waited |= 1ull << v;
   *st = e->h_status + (size_t)r * kStatusWords;
   const int derr = (int)(*st)[2 * LMB_MAX_SLOTS];
   if (derr == DEV_BAD_QUEUE) {
@@ -1389,6 +1435,12 @@ int slot_status(lmb_engine *e, int slot, const unsigned int **st) {
   return LMB_OK;
 }
 
+// A slot's list in host memory, when its pass wrote it there.
+uint64_t host_list_cap(const lmb_engine *e) { return std::min(kHostList, e->cap); }
+const lmb_survivor *host_list(const lmb_engine *e, int slot) {
+  return e->h_list + (size_t)slot * host_list_cap(e);
+}
+
 }  // namespace
 
 extern "C" {
@@ -1398,7 +1450,8 @@ int lmb_results(lmb_engine *e, int32_t slot, lmb_survivor *out, uint64_t out_cap
   int rc = check_engine(e);
   if (rc) return rc;
   const unsigned int *sw = nullptr;
-  rc = slot_status(e, slot, &sw);
+  uint64_t waited = 0;
+  rc = slot_status(e, slot, &sw, &waited);
   if (rc) return rc;
   const uint64_t cnt = sw[slot];
   if (n_survivors) *n_survivors = cnt;
@@ -1414,7 +1467,9 @@ int lmb_results(lmb_engine *e, int32_t slot, lmb_survivor *out, uint64_t out_cap
               (unsigned long long)cnt, (unsigned long long)out_capacity);
     return LMB_ERR_OVERFLOW;
   }
-  if (cnt)
+  if (cnt && cnt <= host_list_cap(e))
+    memcpy(out, host_list(e, slot), cnt * sizeof(lmb_survivor));
+  else if (cnt)
     LMB_CUDA(cudaMemcpy(out, e->d_sorted + (size_t)slot * e->cap, cnt * sizeof(lmb_survivor),
                         cudaMemcpyDeviceToHost));
   e->bytes_d2h += cnt * sizeof(lmb_survivor);
@@ -1426,12 +1481,12 @@ int lmb_results_batch(lmb_engine *e, const int32_t *slots, int32_t nslots, lmb_s
   int rc = check_engine(e);
   if (rc) return rc;
   LMB_REQUIRE(nslots >= 0 && (slots || nslots == 0) && counts, "bad slot list");
-  uint64_t total = 0;
+  uint64_t total = 0, waited = 0;
   bool over = false;
   for (int i = 0; i < nslots; i++) {
     const int k = slots[i];
     const unsigned int *sw = nullptr;
-    rc = slot_status(e, k, &sw);
+    rc = slot_status(e, k, &sw, &waited);
     if (rc) return rc;
     counts[i] = sw[k];
     if (n_pass) n_pass[i] = sw[LMB_MAX_SLOTS + k];
@@ -1446,6 +1501,17 @@ int lmb_results_batch(lmb_engine *e, const int32_t *slots, int32_t nslots, lmb_s
     set_error("%llu survivors exceed the output capacity %llu", (unsigned long long)total,
               (unsigned long long)out_capacity);
     return LMB_ERR_OVERFLOW;
+  }
+  bool short_lists = true;
+  for (int i = 0; i < nslots; i++) short_lists &= counts[i] <= host_list_cap(e);
+  if (short_lists) {  // in host memory already
+    uint64_t at = 0;
+    for (int i = 0; i < nslots; i++) {
+      if (counts[i]) memcpy(out + at, host_list(e, slots[i]), counts[i] * sizeof(lmb_survivor));
+      at += counts[i];
+    }
+    e->bytes_d2h += total * sizeof(lmb_survivor);
+    return LMB_OK;
   }
   // the survivor lists are final (their passes' events have completed): pack
   // them back to back on the device and copy once, on the download stream so
@@ -1582,14 +1648,13 @@ int engine_load_device_frame(lmb_engine *e, int slot, const void *d_img, int dty
   LMB_REQUIRE(nr_px_y == e->geo.nr_px_y && nr_px_x == e->geo.nr_px_x,
               "frame of %d x %d pixels, detector of %d x %d", nr_px_y, nr_px_x, e->geo.nr_px_y,
               e->geo.nr_px_x);
-  LMB_CUDA(cudaStreamWaitEvent(e->ld, e->ev_released[slot], 0));
+  if ((rc = wait_released(e, 1ull << slot))) return rc;
   LMB_CUDA(cudaStreamWaitEvent(e->ld, ready, 0));
   rc = quantize_launch(d_img, dtype, e->npx, d_max_bits ? d_max_bits : e->d_max_bits,
                        d_max_bits != nullptr, e->d_u8 + (size_t)slot * e->npx, nullptr, e->d_occ, slot, e->d_scale + slot, e->num_sms, e->ld);
   if (rc) return rc;
   LMB_CUDA(cudaEventRecord(consumed, e->ld));
-  LMB_CUDA(cudaEventRecord(e->ev_loaded[slot], e->ld));
-  e->loaded_mask |= 1ull << slot;
+  if ((rc = mark_loaded(e, 1ull << slot))) return rc;
   e->f64_mask &= ~(1ull << slot);
   if (im_scale) {
     LMB_CUDA(cudaMemcpyAsync(im_scale, e->d_scale + slot, sizeof(double), cudaMemcpyDeviceToHost,

@@ -92,6 +92,15 @@ struct OrderArgs {
   uint32_t cap;
   unsigned long long *scratch;  // [64][cap2] keys for lists above the shared-memory size
   uint32_t cap2;                // power of two >= cap
+  // page-locked host memory that the kernel writes itself: slot k's list when it
+  // has at most host_cap entries, and the pass's status words
+  lmb_survivor *host_list;  // [64][host_cap]
+  uint32_t host_cap;
+  unsigned int *host_status;    // [ring][words], entry *seq % ring
+  const unsigned int *status;   // [words]
+  uint32_t words, ring;
+  unsigned int *seq;            // passes ordered so far
+  int nslots;
   int slots[LMB_MAX_SLOTS];
 };
 
@@ -137,7 +146,7 @@ int batch_sparse_load_launch(const SparseFrameDesc *d_desc, int nframes, uint32_
                              unsigned long long *d_occ, double *d_scale, size_t npx, int num_sms,
                              cudaStream_t st);
 int compare_launch(CmpArgs a, const CompareTuning &req, int num_sms, cudaStream_t st);
-int order_launch(const OrderArgs &a, int nslots, cudaStream_t st);
+int order_launch(const OrderArgs &a, cudaStream_t st);
 
 // Survivor lists of several slots packed back to back (slot i's list at
 // off[i]) for one device-to-host copy.
