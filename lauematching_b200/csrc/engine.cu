@@ -9,6 +9,7 @@
 #include <omp.h>
 
 #include "kernels.cuh"
+#include "staging.h"
 
 namespace lmb {
 
@@ -65,6 +66,27 @@ struct PassGraph {
   cudaGraphExec_t exec;
 };
 
+// Device memory kept from one use to the next of about the same size.
+struct DeviceBuffer {
+  void *p = nullptr;
+  size_t cap = 0;
+  cudaError_t need(size_t bytes) {
+    if (p && cap >= bytes && (cap / 2 <= bytes || cap <= (1u << 20))) return cudaSuccess;
+    free();
+    const cudaError_t e = cudaMalloc(&p, std::max<size_t>(bytes, 1));
+    if (e == cudaSuccess)
+      cap = bytes;
+    else
+      p = nullptr;
+    return e;
+  }
+  void free() {
+    cudaFree(p);
+    p = nullptr;
+    cap = 0;
+  }
+};
+
 struct lmb_engine {
   int device = 0;
   int num_sms = 148;
@@ -74,7 +96,9 @@ struct lmb_engine {
   cudaStream_t st = nullptr;
   // resident DB
   uint16_t *d_db = nullptr;
+  size_t db_cap = 0;
   uint64_t n = 0;
+  DeviceBuffer om;  // orientation matrices of a build's chunks
   // compact layout derived from it for compare variant 2 (built on first use)
   unsigned char *d_cl = nullptr;
   uint64_t cl_tiles = 0;
@@ -85,6 +109,7 @@ struct lmb_engine {
   int cl_qs = 0;  // largest on-detector spot count of a record (sizes the pass's queues)
   // records grouped by falling on-detector spot count (built on first use)
   uint32_t *d_perm = nullptr;
+  DeviceBuffer b_perm, b_codes, b_cand, b_aux;  // memory of d_perm, d_codes, d_cand, the grouping
   int gl_state = 0;  // 0 not built, 1 built, -1 this DB cannot use it
   unsigned long long gl_hist[256] = {};  // records per on-detector spot count
   int gl_qs = 0;                         // largest on-detector spot count
@@ -146,8 +171,7 @@ struct lmb_engine {
   cudaEvent_t sp_ev[kSparseRing] = {};
   int sp_next = 0;
   uint64_t sparse_loads = 0;
-  void *h_stage[2] = {nullptr, nullptr};   // pinned upload staging (lazy)
-  cudaEvent_t ev_stage[2] = {nullptr, nullptr};
+  Staging staging;
   uint64_t bytes_h2d = 0, bytes_d2h = 0;   // host<->device bytes moved so far
   // batched sparse uploads: per-task scan output (pageable), a two-deep ring
   // of pinned packed staging buffers, the device copy of the packed batch
@@ -166,23 +190,29 @@ struct lmb_engine {
 
 namespace {
 
-void free_grouped(lmb_engine *e) {
-  cudaFree(e->d_perm);
-  cudaFree(e->d_codes);
-  cudaFree(e->d_gl_tab);
-  cudaFree(e->d_group_mask);
-  cudaFree(e->d_cand);
-  cudaFree(e->d_cand_cnt);
+// The grouped records no longer describe the DB; their memory serves the next one.
+void drop_grouped(lmb_engine *e) {
   e->d_perm = nullptr;
   e->d_codes = nullptr;
-  e->d_gl_tab = nullptr;
-  e->d_group_mask = nullptr;
   e->d_cand = nullptr;
-  e->d_cand_cnt = nullptr;
   e->gl_tab.clear();
   e->gl_state = 0;
   e->gl_qs = 0;
   e->gl_bytes = 0;
+}
+
+void free_grouped(lmb_engine *e) {
+  drop_grouped(e);
+  e->b_perm.free();
+  e->b_codes.free();
+  e->b_cand.free();
+  e->b_aux.free();
+  cudaFree(e->d_gl_tab);
+  cudaFree(e->d_group_mask);
+  cudaFree(e->d_cand_cnt);
+  e->d_gl_tab = nullptr;
+  e->d_group_mask = nullptr;
+  e->d_cand_cnt = nullptr;
 }
 
 // Slots about to be written on the load stream: after the last passes that read
@@ -227,6 +257,7 @@ void free_engine(lmb_engine *e) {
   cudaFree(e->d_db);
   cudaFree(e->d_cl);
   free_grouped(e);
+  e->om.free();
   cudaFree(e->d_u8);
   cudaFree(e->d_f64);
   cudaFree(e->d_occ);
@@ -252,8 +283,6 @@ void free_engine(lmb_engine *e) {
     if (e->sp_ev[i]) cudaEventDestroy(e->sp_ev[i]);
   }
   for (int i = 0; i < 2; i++) {
-    if (e->h_stage[i]) cudaFreeHost(e->h_stage[i]);
-    if (e->ev_stage[i]) cudaEventDestroy(e->ev_stage[i]);
     if (e->bt_host[i]) cudaFreeHost(e->bt_host[i]);
     if (e->bt_ev[i]) cudaEventDestroy(e->bt_ev[i]);
   }
@@ -274,53 +303,12 @@ size_t dtype_bytes(int dtype) {
   return dtype == LMB_F64 ? 8 : dtype == LMB_F32 ? 4 : 1;
 }
 
-// Host->device copy of a large pageable buffer (a memory-mapped cache or
-// orientation file) through the engine's two pinned 64 MiB staging chunks:
-// the host copy into chunk b (split over OpenMP threads) overlaps the DMA of
-// chunk b^1.
-int upload_chunked(lmb_engine *e, void *dst, const void *src, size_t bytes, cudaStream_t st) {
-  const size_t kChunk = 64ull << 20;
-  e->bytes_h2d += bytes;
-  if (bytes <= (4ull << 20)) {
-    LMB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
-    LMB_CUDA(cudaStreamSynchronize(st));
-    return LMB_OK;
-  }
-  for (int i = 0; i < 2; i++) {
-    if (!e->h_stage[i]) LMB_CUDA(cudaHostAlloc(&e->h_stage[i], kChunk, cudaHostAllocDefault));
-    if (!e->ev_stage[i]) LMB_CUDA(cudaEventCreateWithFlags(&e->ev_stage[i], cudaEventDisableTiming));
-  }
-  size_t off = 0;
-  int b = 0;
-  while (off < bytes) {
-    const size_t len = std::min(kChunk, bytes - off);
-    LMB_CUDA(cudaEventSynchronize(e->ev_stage[b]));  // chunk b free again
-    char *dstp = static_cast<char *>(e->h_stage[b]);
-    const char *srcp = static_cast<const char *>(src) + off;
-    const size_t piece = 4ull << 20;
-    const long np = (long)((len + piece - 1) / piece);
-#pragma omp parallel for schedule(static) num_threads(8)
-    for (long i = 0; i < np; i++) {
-      const size_t o = (size_t)i * piece;
-      memcpy(dstp + o, srcp + o, std::min(piece, len - o));
-    }
-    LMB_CUDA(cudaMemcpyAsync(static_cast<char *>(dst) + off, dstp, len, cudaMemcpyHostToDevice, st));
-    LMB_CUDA(cudaEventRecord(e->ev_stage[b], st));
-    off += len;
-    b ^= 1;
-  }
-  LMB_CUDA(cudaStreamSynchronize(st));
-  return LMB_OK;
-}
-
 int alloc_db(lmb_engine *e, uint64_t n) {
   LMB_REQUIRE(n < (1ull << 40), "at most 2^40 orientations are supported (got %llu)",
               (unsigned long long)n);
   for (auto &g : e->graphs)  // captured passes name the old DB
     if (g.exec) cudaGraphExecDestroy(g.exec);
   e->graphs.clear();
-  cudaFree(e->d_db);
-  e->d_db = nullptr;
   e->n = 0;
   cudaFree(e->d_cl);
   e->d_cl = nullptr;
@@ -328,12 +316,20 @@ int alloc_db(lmb_engine *e, uint64_t n) {
   e->cl_state = 0;
   e->cl_bytes = 0;
   e->cl_qs = 0;
-  free_grouped(e);
+  drop_grouped(e);
   e->on_detector = false;
   const size_t bytes = (size_t)n * e->R * 2;
   const size_t alloc = ((bytes + 255) / 256) * 256 + 256;
-  LMB_CUDA(cudaMalloc(&e->d_db, alloc));
-  LMB_CUDA(cudaMemsetAsync(e->d_db, 0, alloc, e->st));
+  // a DB of about the same size takes the old one's memory
+  if (!(e->d_db && e->db_cap >= alloc && e->db_cap / 2 <= alloc)) {
+    cudaFree(e->d_db);
+    e->d_db = nullptr;
+    e->db_cap = 0;
+    LMB_CUDA(cudaMalloc(&e->d_db, alloc));
+    e->db_cap = alloc;
+  }
+  // the caller writes every record; the padding behind them is zero
+  LMB_CUDA(cudaMemsetAsync(reinterpret_cast<char *>(e->d_db) + bytes, 0, alloc - bytes, e->st));
   e->n = n;
   return LMB_OK;
 }
@@ -591,16 +587,17 @@ int build_grouped(lmb_engine *e) {
   if (e->S > 255 || e->n == 0 || e->n >= (1ull << 32)) return LMB_OK;
   const uint64_t n = e->n, nt = glist_tiles(n);
   const size_t hist_bytes = 256 * sizeof(unsigned long long);
-  unsigned char *d_aux = nullptr;  // histogram, per-tile counts, counts
-  cudaError_t ce = cudaMalloc(&d_aux, hist_bytes + nt * 256 * sizeof(uint32_t) + n);
-  if (ce == cudaSuccess) ce = cudaMalloc(&e->d_perm, n * sizeof(uint32_t));
+  // histogram, per-tile counts, counts
+  cudaError_t ce = e->b_aux.need(hist_bytes + nt * 256 * sizeof(uint32_t) + n);
+  if (ce == cudaSuccess) ce = e->b_perm.need(n * sizeof(uint32_t));
   if (ce != cudaSuccess) {
     cudaGetLastError();
-    cudaFree(d_aux);
-    e->d_perm = nullptr;
+    e->b_aux.free();
     return ce == cudaErrorMemoryAllocation ? LMB_OK
                                            : cuda_fail(ce, "grouped records", __FILE__, __LINE__);
   }
+  unsigned char *d_aux = static_cast<unsigned char *>(e->b_aux.p);
+  e->d_perm = static_cast<uint32_t *>(e->b_perm.p);
   unsigned long long *d_hist = reinterpret_cast<unsigned long long *>(d_aux);
   uint32_t *d_bh = reinterpret_cast<uint32_t *>(d_aux + hist_bytes);
   uint8_t *d_cnt = d_aux + hist_bytes + nt * 256 * sizeof(uint32_t);
@@ -612,9 +609,8 @@ int build_grouped(lmb_engine *e) {
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->st);
     if (ce != cudaSuccess) rc = cuda_fail(ce, "grouped records", __FILE__, __LINE__);
   }
-  cudaFree(d_aux);
+  if (e->b_aux.cap > (16u << 20)) e->b_aux.free();
   if (rc) {
-    cudaFree(e->d_perm);
     e->d_perm = nullptr;
     return rc;
   }
@@ -650,29 +646,25 @@ int ensure_filter(lmb_engine *e, bool *ok) {
   const uint32_t grid = (uint32_t)e->num_sms;
   // the filter addresses codes and candidates with 32 bits
   if (code >= (1ull << 32) || grid * filter_region(chunk, grid) >= (1ull << 32)) return LMB_OK;
-  cudaError_t ce = cudaMalloc(&e->d_cand, grid * filter_region(chunk, grid) * sizeof(uint32_t));
-  if (ce == cudaSuccess) ce = cudaMalloc(&e->d_codes, code * sizeof(uint2));
-  if (ce == cudaSuccess) ce = cudaMalloc(&e->d_cand_cnt, grid * sizeof(uint32_t));
-  if (ce == cudaSuccess) ce = cudaMalloc(&e->d_group_mask, 65536 * sizeof(uint16_t));
-  if (ce == cudaSuccess) ce = cudaMalloc(&e->d_gl_tab, e->gl_tab.size() * sizeof(GroupBucket));
+  cudaError_t ce = e->b_cand.need(grid * filter_region(chunk, grid) * sizeof(uint32_t));
+  if (ce == cudaSuccess) ce = e->b_codes.need(code * sizeof(uint2));
+  if (ce == cudaSuccess && !e->d_cand_cnt) ce = cudaMalloc(&e->d_cand_cnt, grid * sizeof(uint32_t));
+  if (ce == cudaSuccess && !e->d_group_mask)
+    ce = cudaMalloc(&e->d_group_mask, 65536 * sizeof(uint16_t));
+  if (ce == cudaSuccess && !e->d_gl_tab) ce = cudaMalloc(&e->d_gl_tab, 256 * sizeof(GroupBucket));
   if (ce == cudaSuccess)
     ce = cudaMemcpyAsync(e->d_gl_tab, e->gl_tab.data(), e->gl_tab.size() * sizeof(GroupBucket),
                          cudaMemcpyHostToDevice, e->st);
+  e->d_cand = static_cast<uint32_t *>(e->b_cand.p);
+  e->d_codes = static_cast<uint2 *>(e->b_codes.p);
   int rc = LMB_OK;
   for (size_t i = 0; i < e->gl_tab.size() && ce == cudaSuccess && rc == LMB_OK; i++)
     rc = glist_code_launch(e->d_db, e->R, e->S, e->geo.nr_px_x, e->geo.nr_px_y, e->d_perm,
                            e->gl_tab[i], e->cells, e->d_codes, e->st);
   if (ce == cudaSuccess && rc == LMB_OK) ce = cudaStreamSynchronize(e->st);
   if (ce != cudaSuccess || rc) {
-    cudaFree(e->d_cand);
-    cudaFree(e->d_codes);
-    cudaFree(e->d_cand_cnt);
-    cudaFree(e->d_group_mask);
-    cudaFree(e->d_gl_tab);
-    e->d_cand = e->d_cand_cnt = nullptr;
+    e->d_cand = nullptr;
     e->d_codes = nullptr;
-    e->d_group_mask = nullptr;
-    e->d_gl_tab = nullptr;
     if (rc) return rc;
     if (ce != cudaErrorMemoryAllocation) return cuda_fail(ce, "cell codes", __FILE__, __LINE__);
     cudaGetLastError();
@@ -918,8 +910,11 @@ int lmb_db_upload(lmb_engine *e, const uint16_t *records, uint64_t n) {
   LMB_CUDA(cudaStreamSynchronize(e->st));
   rc = alloc_db(e, n);
   if (rc) return rc;
+  rc = e->staging.upload(e->d_db, records, (size_t)n * e->R * 2, e->st);
+  if (rc) return rc;
+  e->bytes_h2d += (size_t)n * e->R * 2;
   LMB_CUDA(cudaStreamSynchronize(e->st));
-  return upload_chunked(e, e->d_db, records, (size_t)n * e->R * 2, e->st);
+  return LMB_OK;
 }
 
 static int db_build_common(lmb_engine *e, const double *orients, uint64_t seed, bool synthetic,
@@ -935,32 +930,47 @@ static int db_build_common(lmb_engine *e, const double *orients, uint64_t seed, 
   BuildTables *tables = nullptr;
   rc = dbbuild_tables(e->geo, hkls, nh, (flags & LMB_BUILD_EXACT_FP64) != 0, e->st, &tables);
   if (rc) return rc;
-  const uint64_t kChunk = 4ull << 20;  // orientations per chunk (288 MB of matrices)
-  double *d_om = nullptr;
-  cudaError_t ce = cudaMalloc(&d_om, std::min(kChunk, std::max<uint64_t>(n, 1)) * 72);
-  if (ce != cudaSuccess) {
-    dbbuild_tables_free(tables);
-    return cuda_fail(ce, "cudaMalloc(orientation chunk)", __FILE__, __LINE__);
+  // Chunks of matrices in two halves of a buffer kept with the engine: while one is
+  // simulated (st), the next comes from the host (ld).  Synthetic ones are made on
+  // st, in one chunk of both halves at a time.
+  const uint64_t kChunk = 256ull << 10;  // 18 MiB of matrices
+  const uint64_t step = synthetic ? 2 * kChunk : kChunk;
+  cudaEvent_t up[2] = {}, used[2] = {};
+  cudaError_t ce = e->om.need((size_t)std::min(2 * kChunk, std::max<uint64_t>(n, 1)) * 72);
+  for (int b = 0; b < 2 && ce == cudaSuccess && !synthetic; b++) {
+    ce = cudaEventCreateWithFlags(&up[b], cudaEventDisableTiming);
+    if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&used[b], cudaEventDisableTiming);
   }
-  for (uint64_t off = 0; off < n && rc == LMB_OK; off += kChunk) {
-    const uint64_t len = std::min(kChunk, n - off);
+  int b = 0;
+  for (uint64_t off = 0; off < n && rc == LMB_OK && ce == cudaSuccess; off += step, b ^= 1) {
+    const uint64_t len = std::min(step, n - off);
+    double *d_om = static_cast<double *>(e->om.p) + (synthetic || b == 0 ? 0 : kChunk * 9);
     if (synthetic) {
       rc = synth_orient_launch(seed, off, len, d_om, e->st, flags);
     } else {
-      rc = upload_chunked(e, d_om, orients + off * 9, len * 72, e->st);
+      ce = cudaStreamWaitEvent(e->ld, used[b], 0);
+      if (ce == cudaSuccess) rc = e->staging.upload(d_om, orients + off * 9, len * 72, e->ld);
+      e->bytes_h2d += len * 72;
+      if (ce == cudaSuccess) ce = cudaEventRecord(up[b], e->ld);
+      if (ce == cudaSuccess) ce = cudaStreamWaitEvent(e->st, up[b], 0);
     }
-    if (rc == LMB_OK)
+    if (rc == LMB_OK && ce == cudaSuccess)
       rc = dbbuild_launch(d_om, len, tables, e->d_db + off * e->R, e->st);
-    if (rc == LMB_OK && synthetic && orients_out) {
+    if (rc == LMB_OK && ce == cudaSuccess && !synthetic) ce = cudaEventRecord(used[b], e->st);
+    if (rc == LMB_OK && ce == cudaSuccess && synthetic && orients_out) {
       ce = cudaMemcpyAsync(orients_out + off * 9, d_om, len * 72, cudaMemcpyDeviceToHost, e->st);
       e->bytes_d2h += len * 72;
-      if (ce != cudaSuccess) rc = cuda_fail(ce, "orientation download", __FILE__, __LINE__);
     }
-    ce = cudaStreamSynchronize(e->st);
-    if (ce != cudaSuccess && rc == LMB_OK) rc = cuda_fail(ce, "DB build", __FILE__, __LINE__);
   }
-  cudaFree(d_om);
+  const cudaError_t se = cudaStreamSynchronize(e->ld), te = cudaStreamSynchronize(e->st);
+  if (ce == cudaSuccess) ce = se != cudaSuccess ? se : te;
+  if (ce != cudaSuccess && rc == LMB_OK) rc = cuda_fail(ce, "DB build", __FILE__, __LINE__);
+  for (int i = 0; i < 2; i++) {
+    if (up[i]) cudaEventDestroy(up[i]);
+    if (used[i]) cudaEventDestroy(used[i]);
+  }
   dbbuild_tables_free(tables);
+  if (rc) cudaMemset(e->d_db, 0, (size_t)n * e->R * 2);  // no half-built records
   e->on_detector = rc == LMB_OK;
   return rc;
 }
@@ -1051,8 +1061,7 @@ int lmb_image_load(lmb_engine *e, int32_t slot, const void *pixels, int32_t dtyp
     if (rc) return rc;
   }
   if (!sparse) {
-    LMB_CUDA(cudaMemcpyAsync(e->d_stage, pixels, e->npx * dtype_bytes(dtype),
-                             cudaMemcpyHostToDevice, e->ld));
+    if ((rc = e->staging.upload(e->d_stage, pixels, e->npx * dtype_bytes(dtype), e->ld))) return rc;
     e->bytes_h2d += e->npx * dtype_bytes(dtype);
     rc = quantize_launch(e->d_stage, dtype, e->npx, e->d_max_bits, false,
                          e->d_u8 + (size_t)slot * e->npx,

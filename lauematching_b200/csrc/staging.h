@@ -1,0 +1,31 @@
+// Copies between ordinary (pageable) host memory and the device through a small
+// ring of page-locked buffers: host threads copy one piece while the copy engine
+// moves the others.  cudaMemcpy alone does both on one thread, and touches the
+// pages of a fresh destination from it too.  Measured on B200 (16 host cores):
+// see Staging::upload and Staging::download.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stddef.h>
+
+namespace lmb {
+
+class Staging {
+ public:
+  ~Staging();
+  // dst (device) <- src (host), enqueued on st; on return src may be reused unless
+  // it is page-locked (as with cudaMemcpyAsync).
+  int upload(void *dst, const void *src, size_t bytes, cudaStream_t st);
+  // dst (host) <- src (device), complete on return.
+  int download(void *dst, const void *src, size_t bytes, cudaStream_t st);
+
+ private:
+  static constexpr int kPieces = 4;
+  static constexpr size_t kPiece = 8ull << 20;
+  int ready();
+  void *buf_[kPieces] = {};
+  cudaEvent_t ev_[kPieces] = {};
+  int next_ = 0;
+};
+
+}  // namespace lmb
