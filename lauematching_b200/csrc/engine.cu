@@ -1027,8 +1027,8 @@ int lmb_db_download(lmb_engine *e, uint64_t first, uint64_t count, uint16_t *out
   LMB_REQUIRE(first <= e->n && count <= e->n - first, "record range outside the DB");
   LMB_REQUIRE(out || count == 0, "null output");
   LMB_CUDA(cudaStreamSynchronize(e->st));
-  LMB_CUDA(cudaMemcpy(out, e->d_db + first * e->R, (size_t)count * e->R * 2,
-                      cudaMemcpyDeviceToHost));
+  rc = e->staging.download(out, e->d_db + first * e->R, (size_t)count * e->R * 2, e->dl);
+  if (rc) return rc;
   e->bytes_d2h += (size_t)count * e->R * 2;
   return LMB_OK;
 }

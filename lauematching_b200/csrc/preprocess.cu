@@ -29,6 +29,7 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "staging.h"
 
 using namespace lmb;
 
@@ -1817,6 +1818,7 @@ struct lmb_pre {
   int *d_stats = nullptr, *d_head = nullptr, *d_next = nullptr;
   int gcx = 1, gcy = 1;
   PreState *d_state = nullptr, *h_state = nullptr;
+  Staging staging;  // results into ordinary memory
   // median scratch, allocated on first use
   unsigned long long *m_keys = nullptr, *m_keys2 = nullptr;
   unsigned *m_idx = nullptr, *m_idx2 = nullptr, *m_flag = nullptr, *m_incl = nullptr,
@@ -2231,9 +2233,7 @@ int lmb_pre_get_background(lmb_pre *p, double *out) {
   int rc = check_pre(p);
   if (rc) return rc;
   LMB_REQUIRE(out, "null output");
-  LMB_CUDA(cudaMemcpyAsync(out, p->d_bg, p->npx * sizeof(double), cudaMemcpyDeviceToHost, p->st));
-  LMB_CUDA(cudaStreamSynchronize(p->st));
-  return LMB_OK;
+  return p->staging.download(out, p->d_bg, p->npx * sizeof(double), p->st);
 }
 
 int lmb_pre_median(lmb_pre *p, const void *frame, int32_t dtype, int32_t size, int32_t passes,
@@ -2264,8 +2264,7 @@ int lmb_pre_median(lmb_pre *p, const void *frame, int32_t dtype, int32_t size, i
     }
   }
   if ((rc = background_changed(p))) return rc;
-  if (out)
-    LMB_CUDA(cudaMemcpyAsync(out, p->d_bg, p->npx * sizeof(double), cudaMemcpyDeviceToHost, p->st));
+  if (out && (rc = p->staging.download(out, p->d_bg, p->npx * sizeof(double), p->st))) return rc;
   LMB_CUDA(cudaStreamSynchronize(p->st));
   if (size > 1 && passes > 0)
     return stage_times(p, EV_MED0, EV_MED_UP, 5) || stage_times(p, EV_MED_PASS, EV_MED_RANK, 6) ||
@@ -2373,14 +2372,14 @@ int lmb_pre_images(lmb_pre *p, uint16_t *thresholded, int32_t *labels, uint16_t 
     LMB_CUDA(cudaGetLastError());
     p->labels_ready = true;
   }
-  if (thresholded)
-    LMB_CUDA(cudaMemcpyAsync(thresholded, p->d_t16, n * 2, cudaMemcpyDeviceToHost, p->st));
-  if (labels) LMB_CUDA(cudaMemcpyAsync(labels, p->d_lab, n * 4, cudaMemcpyDeviceToHost, p->st));
-  if (filt_img)
-    LMB_CUDA(cudaMemcpyAsync(filt_img, p->d_filt, n * 2, cudaMemcpyDeviceToHost, p->st));
-  if (filt_labels)
-    LMB_CUDA(cudaMemcpyAsync(filt_labels, p->d_flab, n * 4, cudaMemcpyDeviceToHost, p->st));
-  LMB_CUDA(cudaStreamSynchronize(p->st));
+  const struct {
+    void *to;
+    const void *from;
+    size_t bytes;
+  } frames[] = {{thresholded, p->d_t16, n * 2}, {labels, p->d_lab, n * 4}, {filt_img, p->d_filt, n * 2},
+                {filt_labels, p->d_flab, n * 4}};
+  for (const auto &f : frames)
+    if (f.to && (rc = p->staging.download(f.to, f.from, f.bytes, p->st))) return rc;
   return LMB_OK;
 }
 
@@ -2459,8 +2458,8 @@ int lmb_pre_blur(lmb_pre *p, const double *weights, int32_t radius, void *out, i
   if (rc) return rc;
   LMB_REQUIRE(out, "null output");
   if ((rc = blur_launch(p, weights, radius, out_dtype))) return rc;
-  LMB_CUDA(cudaMemcpyAsync(out, p->d_out, p->npx * (out_dtype == LMB_F64 ? 8 : 4),
-                           cudaMemcpyDeviceToHost, p->st));
+  rc = p->staging.download(out, p->d_out, p->npx * (out_dtype == LMB_F64 ? 8 : 4), p->st);
+  if (rc) return rc;
   LMB_CUDA(cudaEventRecord(p->ev[EV_BLUR_DL], p->st));
   LMB_CUDA(cudaStreamSynchronize(p->st));
   return stage_times(p, EV_BLUR0, EV_BLUR_K, 3) || stage_times(p, EV_BLUR_K, EV_BLUR_DL, 4);

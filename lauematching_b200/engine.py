@@ -297,10 +297,11 @@ class Engine:
                 continue
             check(rc)
             break
+        if total < cap // 2:
+            out = out[:total].copy()  # the lists below keep it alive
         res, off = {}, 0
-        for i, s in enumerate(sl.tolist()):
-            c = int(counts[i])
-            res[s] = (out[off:off + c].copy(), int(npass[i]))
+        for s, c, k in zip(sl.tolist(), counts.tolist(), npass.tolist()):
+            res[s] = (out[off:off + c], k)  # disjoint parts of this call's own array
             off += c
         return res
 

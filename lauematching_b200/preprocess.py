@@ -398,8 +398,11 @@ def _run(h: DevicePreprocessor, raw_image, cfg, override_thresh, return_intermed
 
 def _prepare_background(h: DevicePreprocessor, raw_image, cfg, background):
     if background is None:
-        bg = load_background(cfg.get("background_file", ""), cfg["nr_px_x"], cfg["nr_px_y"])
-        if np.count_nonzero(bg) == 0:
+        path = cfg.get("background_file", "")
+        # without a file load_background gives zeros: nothing to make or to count
+        bg = load_background(path, cfg["nr_px_x"], cfg["nr_px_y"]) \
+            if path and os.path.exists(path) else None
+        if bg is None or np.count_nonzero(bg) == 0:
             if cfg["filter_radius"] <= 0 or cfg["median_passes"] <= 0:
                 h.set_background(None, token=("zeros",))
             else:
