@@ -1222,6 +1222,12 @@ __device__ __forceinline__ uint2 ld_stream8(const uint2 *p) {
   return v;
 }
 
+__device__ __forceinline__ uint32_t ld_stream4(const uint32_t *p) {
+  uint32_t v;
+  asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
 __device__ __forceinline__ unsigned majority(unsigned x, unsigned y, unsigned z) {
   return (x & y) | (x & z) | (y & z);
 }
@@ -1240,21 +1246,23 @@ struct SlicedCount {
     for (int b = 0; b < NB; b++) z[b] = (from >> b) & 1u ? 0xFFFFu : 0u;
     z[NB] = 0u;
   }
-  // full adder at weight 2^b
-  __device__ __forceinline__ unsigned add(int b, unsigned p, unsigned q) {
-    const unsigned c = majority(z[b], p, q);
-    z[b] ^= p ^ q;
-    return c;
-  }
-  // a carry of weight 2^b and up
-  __device__ __forceinline__ void ripple(int b, unsigned c) {
+  // N words of weight 2^B: pairs through full adders, their carries one level up
+  template <int B, int N>
+  __device__ __forceinline__ void add(const unsigned (&w)[N]) {
+    if constexpr (B <= NB) {
+      constexpr int M = (N + 1) / 2;
+      unsigned c[M];
 #pragma unroll
-    for (int k = 0; k <= NB; k++)
-      if (k >= b) {
-        const unsigned t = z[k] & c;
-        z[k] ^= c;
-        c = t;
+      for (int j = 0; j < N / 2; j++) {
+        c[j] = majority(z[B], w[2 * j], w[2 * j + 1]);
+        z[B] ^= w[2 * j] ^ w[2 * j + 1];
       }
+      if constexpr (N & 1) {
+        c[M - 1] = z[B] & w[N - 1];
+        z[B] ^= w[N - 1];
+      }
+      add<B + 1, M>(c);
+    }
   }
   __device__ __forceinline__ bool reached() const {
     unsigned c = 0u;
@@ -1265,100 +1273,130 @@ struct SlicedCount {
 };
 
 constexpr int kFilterWarps = 32;
-constexpr int kAhead = 8;  // groups of four spots held in registers (32 spots)
 
-// Persistent: one block per SM, its warps take every grid-th chunk of 32 records,
-// with two chunks' codes in registers: one being counted, the next on its way.
+// The mask words of a unit's two spots side by side.
+__device__ __forceinline__ unsigned look_up(const uint16_t *cm, uint32_t unit) {
+  return __byte_perm(cm[unit & 0xFFFFu], cm[unit >> 16], 0x5410);
+}
+
+// A chunk's candidates into the block's region.
+__device__ __forceinline__ void keep_candidates(const FilterArgs &f, uint32_t *found, uint32_t out,
+                                                uint32_t chunk, bool keep) {
+  const int lane = threadIdx.x & 31;
+  const unsigned km = __ballot_sync(0xffffffffu, keep);
+  if (!km) return;
+  uint32_t base = 0;
+  if (lane == 0) base = atomicAdd(found, (uint32_t)__popc(km));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (keep) f.cand[out + base + __popc(km & ((1u << lane) - 1u))] = chunk * 32u + (uint32_t)lane;
+}
+
+// The chunks of one run, U units each: everything about a chunk is known at compile
+// time.  A chunk's codes are loaded while the one before is counted, each register
+// as soon as its codes have been looked up (a second set of registers would spill).
+template <int NB, int U>
+__device__ __forceinline__ void filter_run(const FilterArgs &f, const GroupRun &r, const uint16_t *cm,
+                                           uint32_t *found, uint32_t out, uint32_t ch, uint32_t step) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t end = r.chunk_end;
+  if (ch >= end) return;
+  const uint32_t *src = f.codes + r.code0 + (uint64_t)(ch - r.chunk0) * (U * 32);
+  const uint64_t stride = (uint64_t)step * (U * 32);
+  uint2 pair[U / 2 > 0 ? U / 2 : 1];
+  uint32_t last = 0;
+#pragma unroll
+  for (int p = 0; p < U / 2; p++)
+    pair[p] = ld_stream8(reinterpret_cast<const uint2 *>(src + p * 64) + lane);
+  if constexpr (U & 1) last = ld_stream4(src + (U - 1) * 32 + lane);
+  for (;;) {
+    src += stride;
+    const bool more = end - ch > step;
+    SlicedCount<NB> sc;
+    sc.start(f.need);
+#pragma unroll
+    for (int p0 = 0; p0 + 2 <= U / 2; p0 += 2) {
+      const uint2 x = pair[p0], y = pair[p0 + 1];
+      if (more) {
+        pair[p0] = ld_stream8(reinterpret_cast<const uint2 *>(src + p0 * 64) + lane);
+        pair[p0 + 1] = ld_stream8(reinterpret_cast<const uint2 *>(src + p0 * 64 + 64) + lane);
+      }
+      const unsigned w[4] = {look_up(cm, x.x), look_up(cm, x.y), look_up(cm, y.x), look_up(cm, y.y)};
+      sc.template add<0, 4>(w);
+    }
+    if constexpr (U % 4 != 0) {
+      constexpr int N = U % 4;
+      unsigned w[N];
+      if constexpr (N >= 2) {
+        const uint2 x = pair[U / 2 - 1];
+        if (more) pair[U / 2 - 1] = ld_stream8(reinterpret_cast<const uint2 *>(src + (U / 2 - 1) * 64) + lane);
+        w[0] = look_up(cm, x.x);
+        w[1] = look_up(cm, x.y);
+      }
+      if constexpr (U & 1) {
+        const uint32_t x = last;
+        if (more) last = ld_stream4(src + (U - 1) * 32 + lane);
+        w[N - 1] = look_up(cm, x);
+      }
+      sc.template add<0, N>(w);
+    }
+    keep_candidates(f, found, out, ch, sc.reached());
+    if (!more) break;
+    ch += step;
+  }
+}
+
+// Persistent: one block per SM, its warps take every grid-th chunk of the list, run
+// after run.  What bounds it is the look-ups (2.9 shared-memory wavefronts each) and,
+// close behind, the stream of codes.  Measured on B200, compare stage at 1e8 records:
+// see the commit of the layout it reads; filter kernel alone, tilted detector with
+// 64 slots (3.1 GB of codes): 775 us with one loop over chunks of any size, 640 us
+// with a loop per size; hexagonal with 32 slots (0.27 GB): 126 us, 72 us.
 template <int NB>
 __global__ void __launch_bounds__(32 * kFilterWarps, 1)
     group_filter_kernel(const __grid_constant__ FilterArgs f) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ uint32_t found;
-  const uint32_t mask_bytes = filter_mask_bytes(f.cells.n);
   const uint16_t *cm = reinterpret_cast<const uint16_t *>(smem);
-  const GroupBucket *tab = reinterpret_cast<const GroupBucket *>(smem + mask_bytes);
   {
     const uint4 *src = reinterpret_cast<const uint4 *>(f.mask);  // padded to 16 bytes
     uint4 *dst = reinterpret_cast<uint4 *>(smem);
-    for (uint32_t i = threadIdx.x; i < mask_bytes / 16; i += blockDim.x) dst[i] = src[i];
-    const uint4 *ts = reinterpret_cast<const uint4 *>(f.tab);
-    uint4 *td = reinterpret_cast<uint4 *>(smem + mask_bytes);
-    for (uint32_t i = threadIdx.x; i < (uint32_t)f.nb * 2u; i += blockDim.x) td[i] = ts[i];
+    for (uint32_t i = threadIdx.x; i < filter_mask_bytes(f.cells.n) / 16; i += blockDim.x) dst[i] = src[i];
     if (threadIdx.x == 0) found = 0u;
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31;
   const uint32_t step = gridDim.x * kFilterWarps;
+  const uint32_t me = blockIdx.x * kFilterWarps + (threadIdx.x >> 5);
   const uint32_t out = blockIdx.x * (uint32_t)filter_region(f.nchunks, gridDim.x);
-  // the next chunk to load, its bucket and where its codes and records are
-  uint32_t ch = blockIdx.x * kFilterWarps + (threadIdx.x >> 5), chunk_end = 0, next_pos = 0;
-  int bi = -1, next_groups = 0;
-  uint32_t next = 0;  // 8-byte words of codes fit 32 bits (ensure_filter)
-  struct Chunk {
-    uint2 v[kAhead];
-    uint32_t src, pos;
-    int groups;  // 0: no more chunks
-  };
-  auto fetch = [&](Chunk &c) {
-    c.groups = 0;
-    if (ch >= f.nchunks) return;
-    if (ch >= chunk_end) {
-      do bi++;
-      while (ch >= tab[bi].chunk_end);
-      const GroupBucket b = tab[bi];
-      chunk_end = b.chunk_end;
-      next_groups = (int)(b.c + 3) / 4;
-      next = (uint32_t)b.code0 + (ch - b.chunk0) * (uint32_t)next_groups * 32u + (uint32_t)lane;
-      next_pos = b.pos0 + (ch - b.chunk0) * 32u + (uint32_t)lane;
+  for (int i = 0; i < f.nruns; i++) {
+    const GroupRun &r = f.runs[i];
+    // this warp's first chunk of the run: chunks go round the grid's warps
+    const uint32_t past = r.chunk0 % step;
+    const uint32_t ch = r.chunk0 + (me >= past ? me - past : me + step - past);
+#define LMB_RUN(U)                                             \
+  case U:                                                      \
+    filter_run<NB, U>(f, r, cm, &found, out, ch, step);        \
+    break;
+    switch (r.units) {
+      LMB_RUN(1) LMB_RUN(2) LMB_RUN(3) LMB_RUN(4) LMB_RUN(5) LMB_RUN(6) LMB_RUN(7) LMB_RUN(8)
+      LMB_RUN(9) LMB_RUN(10) LMB_RUN(11) LMB_RUN(12) LMB_RUN(13) LMB_RUN(14) LMB_RUN(15) LMB_RUN(16)
+      default:
+        if constexpr (NB > 5) {  // more than 32 spots: a unit at a time
+          const int lane = threadIdx.x & 31;
+          for (uint32_t c = ch; c < r.chunk_end; c += step) {
+            const uint32_t *src = f.codes + r.code0 + (uint64_t)(c - r.chunk0) * r.units * 32;
+            SlicedCount<NB> sc;
+            sc.start(f.need);
+            for (uint32_t u = 0; u < r.units; u++) {
+              const uint32_t at = u + 1 < r.units || u % 2 ? u / 2 * 64 + 2 * (uint32_t)lane + u % 2
+                                                           : u * 32 + (uint32_t)lane;
+              const unsigned w[1] = {look_up(cm, ld_stream4(src + at))};
+              sc.template add<0, 1>(w);
+            }
+            keep_candidates(f, &found, out, c, sc.reached());
+          }
+        }
     }
-    c.groups = next_groups;
-    c.src = next;
-    c.pos = next_pos;
-#pragma unroll
-    for (int g = 0; g < kAhead; g++)
-      if (g < next_groups) c.v[g] = ld_stream8(f.codes + next + g * 32);
-    ch += step;
-    next += step * (uint32_t)next_groups * 32u;
-    next_pos += step * 32u;
-  };
-  auto count = [&](const Chunk &c) {
-    SlicedCount<NB> sc;
-    sc.start(f.need);
-    auto four = [&](uint2 u) {
-      const unsigned p = __byte_perm(cm[u.x & 0xFFFFu], cm[u.x >> 16], 0x5410);
-      const unsigned q = __byte_perm(cm[u.y & 0xFFFFu], cm[u.y >> 16], 0x5410);
-      return sc.add(0, p, q);
-    };
-#pragma unroll
-    for (int g = 0; g < kAhead; g += 4) {
-      if (g >= c.groups) break;
-      const unsigned c0 = four(c.v[g]);
-      const unsigned c1 = g + 1 < c.groups ? four(c.v[g + 1]) : 0u;
-      const unsigned c2 = g + 2 < c.groups ? four(c.v[g + 2]) : 0u;
-      const unsigned c3 = g + 3 < c.groups ? four(c.v[g + 3]) : 0u;
-      const unsigned d0 = sc.add(1, c0, c1), d1 = sc.add(1, c2, c3);
-      sc.ripple(3, sc.add(2, d0, d1));
-    }
-    if (NB > 5)
-      for (int g = kAhead; g < c.groups; g++) sc.ripple(1, four(ld_stream8(f.codes + c.src + g * 32)));
-    const bool keep = sc.reached();  // never for a lane past the last record: no spots
-    const unsigned km = __ballot_sync(0xffffffffu, keep);
-    if (km) {
-      uint32_t base = 0;
-      if (lane == 0) base = atomicAdd(&found, (uint32_t)__popc(km));
-      base = __shfl_sync(0xffffffffu, base, 0);
-      if (keep) f.cand[out + base + __popc(km & ((1u << lane) - 1u))] = c.pos;
-    }
-  };
-  Chunk a, b;
-  fetch(a);
-  for (;;) {
-    fetch(b);
-    if (!a.groups) break;
-    count(a);
-    fetch(a);
-    if (!b.groups) break;
-    count(b);
+#undef LMB_RUN
   }
   __syncthreads();
   if (threadIdx.x == 0) f.cand_cnt[blockIdx.x] = found;
@@ -1374,16 +1412,17 @@ static int launch_filter(const FilterArgs &f, size_t smem, cudaStream_t st) {
 }
 
 int filter_launch(const FilterArgs &f, cudaStream_t st) {
-  LMB_REQUIRE(f.cells.n >= 1 && f.cells.n <= 65535 && f.need >= 1 && f.grid >= 1 && f.nb >= 1,
+  LMB_REQUIRE(f.cells.n >= 1 && f.cells.n <= 65535 && f.need >= 1 && f.grid >= 1 && f.nruns >= 1 &&
+                  f.nruns <= kMostRuns,
               "group filter: malformed arguments");
   groupmask_kernel<<<(f.cells.n * 4 + 255) / 256, 256, 0, st>>>(f);
   LMB_CUDA(cudaGetLastError());
-  const size_t smem = filter_mask_bytes(f.cells.n) + (size_t)f.nb * sizeof(GroupBucket);
+  const size_t smem = filter_mask_bytes(f.cells.n);
   return f.most_spots <= 32 ? launch_filter<5>(f, smem, st) : launch_filter<8>(f, smem, st);
 }
 
 // ----------------------------------------------------------------------------
-// Listed pass: the records perm[0, nlist), those with at least MinNrSpots
+// Listed pass: the records at perm[0, nlist), those with at least MinNrSpots
 // on-detector spots, or the filter's candidates, 32 per warp.  Each lane copies
 // its record's on-detector pixels into the warp's shared-memory rows (odd stride:
 // conflict-free), then the warp runs the per-record logic of the other variants
@@ -1401,8 +1440,10 @@ __global__ void __launch_bounds__(256) listed_kernel(const __grid_constant__ Cmp
   const uint64_t n = a.cand ? a.cand_cnt[blockIdx.y] : a.nlist;
   const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); g < n; g += step) {
-    const bool v = g + lane < n;
-    const uint64_t oid = v ? a.perm[cand ? cand[g + lane] : g + lane] : 0;
+    const bool in = g + lane < n;
+    const uint32_t id = in ? a.perm[cand ? cand[g + lane] : g + lane] : kNoRecord;
+    const bool v = id != kNoRecord;  // a place without a record
+    const uint64_t oid = v ? id : 0;
     int c = 0;
     if (v) {
       const uint16_t *rec = a.db + oid * (uint64_t)a.R;

@@ -115,11 +115,14 @@ struct lmb_engine {
   int gl_qs = 0;                         // largest on-detector spot count
   bool on_detector = false;  // every stored spot is on the detector (a DB built here)
   // variant 5 (built on first use): cell codes of the grouped records, their
-  // buckets by falling count (host and device), the mask of a pass, the filter's
+  // buckets by falling count, the mask of a pass, the filter's
   // candidates (a region per block) and their counts
-  std::vector<GroupBucket> gl_tab;
-  uint2 *d_codes = nullptr;
-  GroupBucket *d_gl_tab = nullptr;
+  struct Bucket {  // the records of one count: a run's chunks and its count
+    GroupRun run;
+    int c;
+  };
+  std::vector<Bucket> gl_tab;
+  uint32_t *d_codes = nullptr;
   uint16_t *d_group_mask = nullptr;
   uint32_t *d_cand = nullptr, *d_cand_cnt = nullptr;
   GroupCells cells{};
@@ -207,10 +210,8 @@ void free_grouped(lmb_engine *e) {
   e->b_codes.free();
   e->b_cand.free();
   e->b_aux.free();
-  cudaFree(e->d_gl_tab);
   cudaFree(e->d_group_mask);
   cudaFree(e->d_cand_cnt);
-  e->d_gl_tab = nullptr;
   e->d_group_mask = nullptr;
   e->d_cand_cnt = nullptr;
 }
@@ -457,10 +458,11 @@ double gathered_per_record(const lmb_engine *e, const unsigned long long *hist, 
   for (int c = m; c < 256; c++) g += (double)c * (double)hist[c];
   return e->n ? g / (double)e->n : 0.0;
 }
-// Records with at least min_spots on-detector spots: the first of d_perm.
-uint64_t listed_records(const lmb_engine *e, int min_spots) {
+// Places of the records with at least min_spots on-detector spots: the first of
+// d_perm.
+uint64_t listed_places(const lmb_engine *e, int min_spots) {
   uint64_t k = 0;
-  for (int c = std::max(0, min_spots); c < 256; c++) k += e->gl_hist[c];
+  for (int c = std::max(0, min_spots); c < 256; c++) k += (e->gl_hist[c] + 31) / 32 * 32;
   return k;
 }
 
@@ -584,12 +586,12 @@ int build_compact(lmb_engine *e, int min_spots) {
 // memory for 4 bytes per record) keeps the other layouts.
 int build_grouped(lmb_engine *e) {
   e->gl_state = -1;
-  if (e->S > 255 || e->n == 0 || e->n >= (1ull << 32)) return LMB_OK;
+  if (e->S > 255 || e->n == 0 || e->n >= kGlMost) return LMB_OK;
   const uint64_t n = e->n, nt = glist_tiles(n);
   const size_t hist_bytes = 256 * sizeof(unsigned long long);
   // histogram, per-tile counts, counts
   cudaError_t ce = e->b_aux.need(hist_bytes + nt * 256 * sizeof(uint32_t) + n);
-  if (ce == cudaSuccess) ce = e->b_perm.need(n * sizeof(uint32_t));
+  if (ce == cudaSuccess) ce = e->b_perm.need(glist_places(n) * sizeof(uint32_t));
   if (ce != cudaSuccess) {
     cudaGetLastError();
     e->b_aux.free();
@@ -632,35 +634,33 @@ int ensure_filter(lmb_engine *e, bool *ok) {
   if (*ok) return LMB_OK;
   e->cells = group_cells(e->geo.nr_px_x, e->geo.nr_px_y);
   e->gl_tab.clear();
-  uint32_t chunk = 0, pos = 0;
+  uint32_t chunk = 0;
   uint64_t code = 0;
   for (int c = e->gl_qs; c >= 1; c--) {
-    const uint32_t nrec = (uint32_t)e->gl_hist[c], nch = (nrec + 31) / 32;
-    if (!nrec) continue;
-    e->gl_tab.push_back(GroupBucket{chunk + nch, chunk, pos, nrec, code, (uint32_t)c, 0});
+    const uint32_t nch = (uint32_t)((e->gl_hist[c] + 31) / 32), units = (uint32_t)(c + 1) / 2;
+    if (!nch) continue;
+    e->gl_tab.push_back({GroupRun{chunk, chunk + nch, units, 0, code}, c});
     chunk += nch;
-    pos += nrec;
-    code += (uint64_t)nch * ((c + 3) / 4) * 32;
+    code += (uint64_t)nch * units * 32;
   }
   if (e->gl_tab.empty()) return LMB_OK;  // no record has a spot
   const uint32_t grid = (uint32_t)e->num_sms;
-  // the filter addresses codes and candidates with 32 bits
-  if (code >= (1ull << 32) || grid * filter_region(chunk, grid) >= (1ull << 32)) return LMB_OK;
+  // the filter addresses candidates with 32 bits
+  if (grid * filter_region(chunk, grid) >= (1ull << 32)) return LMB_OK;
   cudaError_t ce = e->b_cand.need(grid * filter_region(chunk, grid) * sizeof(uint32_t));
-  if (ce == cudaSuccess) ce = e->b_codes.need(code * sizeof(uint2));
+  if (ce == cudaSuccess) ce = e->b_codes.need(code * sizeof(uint32_t));
   if (ce == cudaSuccess && !e->d_cand_cnt) ce = cudaMalloc(&e->d_cand_cnt, grid * sizeof(uint32_t));
   if (ce == cudaSuccess && !e->d_group_mask)
     ce = cudaMalloc(&e->d_group_mask, 65536 * sizeof(uint16_t));
-  if (ce == cudaSuccess && !e->d_gl_tab) ce = cudaMalloc(&e->d_gl_tab, 256 * sizeof(GroupBucket));
-  if (ce == cudaSuccess)
-    ce = cudaMemcpyAsync(e->d_gl_tab, e->gl_tab.data(), e->gl_tab.size() * sizeof(GroupBucket),
-                         cudaMemcpyHostToDevice, e->st);
   e->d_cand = static_cast<uint32_t *>(e->b_cand.p);
-  e->d_codes = static_cast<uint2 *>(e->b_codes.p);
+  e->d_codes = static_cast<uint32_t *>(e->b_codes.p);
   int rc = LMB_OK;
-  for (size_t i = 0; i < e->gl_tab.size() && ce == cudaSuccess && rc == LMB_OK; i++)
-    rc = glist_code_launch(e->d_db, e->R, e->S, e->geo.nr_px_x, e->geo.nr_px_y, e->d_perm,
-                           e->gl_tab[i], e->cells, e->d_codes, e->st);
+  for (const auto &t : e->gl_tab) {
+    if (ce != cudaSuccess || rc) break;
+    rc = glist_code_launch(e->d_db, e->R, e->S, e->geo.nr_px_x, e->geo.nr_px_y,
+                           e->d_perm + 32ull * t.run.chunk0, t.c, t.run.chunk_end - t.run.chunk0,
+                           e->cells, e->d_codes + t.run.code0, e->st);
+  }
   if (ce == cudaSuccess && rc == LMB_OK) ce = cudaStreamSynchronize(e->st);
   if (ce != cudaSuccess || rc) {
     e->d_cand = nullptr;
@@ -670,7 +670,7 @@ int ensure_filter(lmb_engine *e, bool *ok) {
     cudaGetLastError();
     return LMB_OK;
   }
-  e->gl_bytes += code * sizeof(uint2);
+  e->gl_bytes += code * sizeof(uint32_t);
   *ok = true;
   return LMB_OK;
 }
@@ -691,12 +691,14 @@ int enqueue_filter(lmb_engine *e, const PassKey &k, CmpArgs *a) {
       r++;
     }
   f.codes = e->d_codes;
-  f.tab = e->d_gl_tab;
-  for (const GroupBucket &b : e->gl_tab)
-    if ((int)b.c >= k.min_spots) {
-      f.nb++;
-      f.nchunks = b.chunk_end;
-    }
+  for (const auto &t : e->gl_tab) {  // counts of equal units join: their chunks and codes do
+    if (t.c < k.min_spots) break;
+    if (f.nruns && f.runs[f.nruns - 1].units == t.run.units)
+      f.runs[f.nruns - 1].chunk_end = t.run.chunk_end;
+    else
+      f.runs[f.nruns++] = t.run;
+    f.nchunks = t.run.chunk_end;
+  }
   f.need = (uint32_t)k.min_spots;
   f.most_spots = e->gl_qs;
   f.cand = e->d_cand;
@@ -764,7 +766,7 @@ int enqueue_pass(lmb_engine *e, const PassKey &k, bool capturing) {
     if (k.listed) {  // nothing can pass when no record has that many spots
       a.qS = e->gl_qs;
       a.perm = e->d_perm;
-      a.nlist = k.min_spots <= e->gl_qs ? listed_records(e, a.full_gather ? 0 : k.min_spots) : 0;
+      a.nlist = k.min_spots <= e->gl_qs ? listed_places(e, a.full_gather ? 0 : k.min_spots) : 0;
       if (k.filter && a.nlist) {
         const int rc = enqueue_filter(e, k, &a);
         if (rc) return rc;

@@ -4,10 +4,11 @@
 // (LaueMatchingCPU.c:671-683), so a pass needs the records of the large counts
 // alone.  `perm` lists the record numbers by falling count (within one count in
 // tiles of kGlTile records, ascending in each), so the records with at least m
-// spots are its first entries whatever m is: 4 bytes per record, made once per
-// DB by a counting sort on the device.  Measured on B200 at 1e8 records of 122
-// bytes, with the host's packing of the tiled compact layout (clist.cu) for
-// comparison: see build_grouped in engine.cu.
+// spots are its first entries whatever m is.  Each count starts at a multiple of 32
+// (places without a record hold kNoRecord): a chunk of 32 places has one count.
+// 4 bytes per record, made once per DB by a counting sort on the device: 6 to 7 ms
+// to the end of the first pass at 1e8 records of 122 bytes on B200, where packing
+// the tiled compact layout (clist.cu) on the host took 42 to 490 ms.
 #include "kernels.cuh"
 
 namespace lmb {
@@ -65,7 +66,7 @@ __global__ void __launch_bounds__(1024) glist_scan_kernel(uint32_t *__restrict__
   if (hist[blockIdx.x] == 0) return;
   if (threadIdx.x == 0) {
     unsigned long long base = 0;
-    for (int c = 255; c > (int)blockIdx.x; c--) base += hist[c];
+    for (int c = 255; c > (int)blockIdx.x; c--) base += (hist[c] + 31) / 32 * 32;
     carry = (uint32_t)base;
   }
   __syncthreads();
@@ -121,11 +122,12 @@ __global__ void __launch_bounds__(256) glist_scatter_kernel(const uint8_t *__res
   }
 }
 
-// Cell codes of the records of one count (c >= 1), perm[0, nrec): a spot's cell
-// of cw x ch pixels, 16 bits each.  32 records make a chunk; a lane's codes are
-// stored four at a time, [chunk][ceil(c / 4)][lane][4], so that a warp reads a
-// group of four spots of its 32 records with one 8-byte load per lane.  Codes
-// past the last spot or record are `none`, the code of a cell that is never marked.
+// Cell codes of the records of one count (c >= 1), perm[0, 32 chunks): a spot's
+// cell of cw x ch pixels, 16 bits each, two to a unit.  A chunk's codes are ceil(c /
+// 2) units per lane: pairs of them as [pair][lane][2], so that a warp reads four
+// spots of its 32 records with one 8-byte load per lane, and an odd last one as
+// [lane].  Codes past the last spot, and of places without a record, are `none`, the
+// code of a cell that is never marked.
 //
 // The order of a record's codes is free, and the filter's lanes look up their
 // k-th codes together: for records of up to 32 spots the k-th codes of a chunk are
@@ -135,30 +137,35 @@ __global__ void __launch_bounds__(256) glist_scatter_kernel(const uint8_t *__res
 __global__ void __launch_bounds__(256) glist_code_kernel(const uint16_t *__restrict__ db, int R, int S,
                                                          int W, int H,
                                                          const uint32_t *__restrict__ perm,
-                                                         uint32_t nrec, int c, int cw, int ch,
+                                                         uint32_t chunks, int c, int cw, int ch,
                                                          int cells_x, uint32_t none,
-                                                         uint2 *__restrict__ codes) {
+                                                         uint32_t *__restrict__ codes) {
   constexpr int kMost = 32;  // spots of a record whose codes are ordered
   __shared__ uint16_t held[8][kMost][33];
   const uint32_t chunk = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (chunk >= (nrec + 31) / 32) return;  // whole warps
-  const int groups = (c + 3) / 4;
-  uint2 *out = codes + (uint64_t)chunk * groups * 32 + lane;
-  const uint32_t at = chunk * 32 + lane;
-  const uint16_t *rec = db + (at < nrec ? (uint64_t)perm[at] * R : 0);
-  const int stored = at < nrec ? min((int)rec[0], S) : 0;
+  if (chunk >= chunks) return;  // whole warps
+  const int units = (c + 1) / 2;
+  uint32_t *out = codes + (uint64_t)chunk * units * 32;
+  const uint32_t id = perm[chunk * 32 + lane];
+  const uint16_t *rec = db + (id != kNoRecord ? (uint64_t)id * R : 0);
+  const int stored = id != kNoRecord ? min((int)rec[0], S) : 0;
   uint32_t four[4] = {none, none, none, none};
-  int k = 0, g = 0;
+  int k = 0;
+  auto flush = [&](int first) {  // the unit `first` and the next
+    if (first + 1 < units)
+      *reinterpret_cast<uint2 *>(out + first * 32 + 2 * lane) =
+          make_uint2(four[0] | four[1] << 16, four[2] | four[3] << 16);
+    else
+      out[first * 32 + lane] = four[0] | four[1] << 16;
+#pragma unroll
+    for (int j = 0; j < 4; j++) four[j] = none;
+  };
   auto put = [&](uint32_t q) {
 #pragma unroll
     for (int j = 0; j < 4; j++)
       if ((k & 3) == j) four[j] = q;
-    if ((++k & 3) == 0) {
-      out[(uint64_t)g++ * 32] = make_uint2(four[0] | four[1] << 16, four[2] | four[3] << 16);
-#pragma unroll
-      for (int j = 0; j < 4; j++) four[j] = none;
-    }
+    if ((++k & 3) == 0) flush(k / 2 - 2);
   };
   uint16_t(*mine)[33] = held[threadIdx.x >> 5];
   int n = 0;
@@ -207,27 +214,21 @@ __global__ void __launch_bounds__(256) glist_code_kernel(const uint16_t *__restr
       }
     }
   }
-  for (; g < groups; g++) {
-    out[(uint64_t)g * 32] = make_uint2(four[0] | four[1] << 16, four[2] | four[3] << 16);
-#pragma unroll
-    for (int j = 0; j < 4; j++) four[j] = none;
-  }
+  for (int u = k / 4 * 2; u < units; u += 2) flush(u);
 }
 
-int glist_code_launch(const uint16_t *d_db, int R, int S, int W, int H, const uint32_t *d_perm,
-                      const GroupBucket &b, const GroupCells &cells, uint2 *d_codes, cudaStream_t st) {
-  if (b.nrec == 0) return LMB_OK;
-  const uint32_t chunks = (b.nrec + 31) / 32;
-  glist_code_kernel<<<(chunks + 7) / 8, 256, 0, st>>>(d_db, R, S, W, H, d_perm + b.pos0, b.nrec,
-                                                      (int)b.c, cells.cw, cells.ch, cells.nx,
-                                                      cells.n, d_codes + b.code0);
+int glist_code_launch(const uint16_t *d_db, int R, int S, int W, int H, const uint32_t *d_perm, int c,
+                      uint32_t chunks, const GroupCells &cells, uint32_t *d_codes, cudaStream_t st) {
+  if (chunks == 0) return LMB_OK;
+  glist_code_kernel<<<(chunks + 7) / 8, 256, 0, st>>>(d_db, R, S, W, H, d_perm, chunks, c, cells.cw,
+                                                      cells.ch, cells.nx, cells.n, d_codes);
   LMB_CUDA(cudaGetLastError());
   return LMB_OK;
 }
 
 int glist_count_launch(const uint16_t *d_db, uint64_t n, int R, int S, int W, int H, bool on_detector,
                        uint8_t *d_cnt, uint32_t *d_bh, unsigned long long *d_hist, cudaStream_t st) {
-  LMB_REQUIRE(S <= 255 && n > 0 && n < (1ull << 32), "records cannot be grouped by count");
+  LMB_REQUIRE(S <= 255 && n > 0 && n < kGlMost, "records cannot be grouped by count");
   const uint32_t nt = glist_tiles(n);
   glist_count_kernel<<<nt, 256, 0, st>>>(d_db, n, R, S, W, H, on_detector ? 1 : 0, nt, d_cnt, d_bh);
   glist_total_kernel<<<256, 256, 0, st>>>(d_bh, nt, d_hist);
@@ -239,6 +240,7 @@ int glist_count_launch(const uint16_t *d_db, uint64_t n, int R, int S, int W, in
 int glist_scatter_launch(const uint8_t *d_cnt, uint64_t n, const uint32_t *d_bh, uint32_t *d_perm,
                          cudaStream_t st) {
   const uint32_t nt = glist_tiles(n);
+  LMB_CUDA(cudaMemsetAsync(d_perm, 0xff, glist_places(n) * sizeof(uint32_t), st));
   glist_scatter_kernel<<<nt, 256, 0, st>>>(d_cnt, n, nt, d_bh, d_perm);
   LMB_CUDA(cudaGetLastError());
   return LMB_OK;

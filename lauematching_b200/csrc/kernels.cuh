@@ -239,6 +239,10 @@ constexpr uint32_t kGlTile = 4096;  // records per tile of the counting sort
 __host__ __device__ __forceinline__ uint32_t glist_tiles(uint64_t n) {
   return (uint32_t)((n + kGlTile - 1) / kGlTile);
 }
+constexpr uint64_t kGlMost = (1ull << 32) - (1ull << 14);  // records that can be grouped: below this
+constexpr uint32_t kNoRecord = 0xFFFFFFFFu;
+// Places of the list: every count's records from a multiple of 32 on.
+__host__ __device__ __forceinline__ uint64_t glist_places(uint64_t n) { return n + 32ull * 256; }
 int glist_count_launch(const uint16_t *d_db, uint64_t n, int R, int S, int W, int H, bool on_detector,
                        uint8_t *d_cnt, uint32_t *d_bh, unsigned long long *d_hist, cudaStream_t st);
 int glist_scatter_launch(const uint8_t *d_cnt, uint64_t n, const uint32_t *d_bh, uint32_t *d_perm,
@@ -251,18 +255,17 @@ struct GroupCells {
   int cw, ch, nx, ny;
   uint32_t n;
 };
-// The records of one spot count: perm[pos0, pos0 + nrec), chunks [chunk0,
-// chunk_end) of 32 of them, their codes from code0 on.  Ordered by falling count.
-struct GroupBucket {
-  uint32_t chunk_end, chunk0, pos0, nrec;
+// Chunks of records whose codes take the same number of units (two spots each): [chunk0,
+// chunk_end) of the list, their codes from code0 (32-bit words) on.
+struct GroupRun {
+  uint32_t chunk0, chunk_end, units, pad;
   uint64_t code0;
-  uint32_t c, pad;
 };
-static_assert(sizeof(GroupBucket) == 32, "bucket layout");
+constexpr int kMostRuns = 128;  // 255 spots
 constexpr int kMaskGroups = 16;  // image groups of a mask word
 GroupCells group_cells(int W, int H);
-int glist_code_launch(const uint16_t *d_db, int R, int S, int W, int H, const uint32_t *d_perm,
-                      const GroupBucket &b, const GroupCells &cells, uint2 *d_codes, cudaStream_t st);
+int glist_code_launch(const uint16_t *d_db, int R, int S, int W, int H, const uint32_t *d_perm, int c,
+                      uint32_t chunks, const GroupCells &cells, uint32_t *d_codes, cudaStream_t st);
 
 // The filter over the grouped records (compare.cu).
 struct FilterArgs {
@@ -271,15 +274,15 @@ struct FilterArgs {
   GroupCells cells;
   uint16_t *mask;  // one 16-bit word per cell: bit g = a pixel of it is positive in a slot of group g
   unsigned long long group[kMaskGroups];  // slots of each group
-  const uint2 *codes;
-  const GroupBucket *tab;
-  int nb;            // buckets of the records that can pass
+  const uint32_t *codes;
+  int nruns;         // of the records that can pass
   uint32_t nchunks;  // their chunks
   uint32_t need;     // MinNrSpots (>= 1)
   int most_spots;    // largest count
   uint32_t *cand;    // per block a region of positions in perm
   uint32_t *cand_cnt;
   uint32_t grid;     // blocks
+  GroupRun runs[kMostRuns];
 };
 // Positions a filter block can keep: its 32 warps' chunks of 32 records.
 __host__ __device__ __forceinline__ uint64_t filter_region(uint32_t nchunks, uint32_t grid) {
