@@ -1292,8 +1292,8 @@ __device__ __forceinline__ void keep_candidates(const FilterArgs &f, uint32_t *f
 }
 
 // The chunks of one run, U units each: everything about a chunk is known at compile
-// time.  A chunk's codes are loaded while the one before is counted, each register
-// as soon as its codes have been looked up (a second set of registers would spill).
+// time.  Codes are loaded one or two chunks ahead, each register again as soon as its
+// codes have been looked up (a set of registers more per chunk would spill).
 template <int NB, int U>
 __device__ __forceinline__ void filter_run(const FilterArgs &f, const GroupRun &r, const uint16_t *cm,
                                            uint32_t *found, uint32_t out, uint32_t ch, uint32_t step) {
@@ -1302,55 +1302,73 @@ __device__ __forceinline__ void filter_run(const FilterArgs &f, const GroupRun &
   if (ch >= end) return;
   const uint32_t *src = f.codes + r.code0 + (uint64_t)(ch - r.chunk0) * (U * 32);
   const uint64_t stride = (uint64_t)step * (U * 32);
-  uint2 pair[U / 2 > 0 ? U / 2 : 1];
-  uint32_t last = 0;
+  // Chunks on their way.  Small ones are counted in less than a load's latency: two
+  // ahead (hexagonal, 32 slots: compare stage 0.109 -> 0.092 ms); four for up to 4
+  // units and two for up to 8 spilled and lost (0.119; tilted 0.668 -> 0.795).
+  constexpr int D = U <= 4 ? 2 : 1;
+  constexpr int P = U / 2 > 0 ? U / 2 : 1;
+  uint2 pair[D][P];
+  uint32_t last[D];
+  auto fetch_pair = [&](int d, int p) {
+    pair[d][p] = ld_stream8(reinterpret_cast<const uint2 *>(src + p * 64) + lane);
+  };
+  auto fetch_last = [&](int d) { last[d] = ld_stream4(src + (U - 1) * 32 + lane); };
 #pragma unroll
-  for (int p = 0; p < U / 2; p++)
-    pair[p] = ld_stream8(reinterpret_cast<const uint2 *>(src + p * 64) + lane);
-  if constexpr (U & 1) last = ld_stream4(src + (U - 1) * 32 + lane);
-  for (;;) {
+  for (int d = 0; d < D; d++) {  // end - ch > d * step, without overflow
+    if ((end - 1 - ch) / step >= (uint32_t)d) {
+#pragma unroll
+      for (int p = 0; p < U / 2; p++) fetch_pair(d, p);
+      if constexpr (U & 1) fetch_last(d);
+    }
     src += stride;
-    const bool more = end - ch > step;
-    SlicedCount<NB> sc;
-    sc.start(f.need);
+  }
+  uint32_t left = (end - 1 - ch) / step + 1;  // chunks of this warp
+  for (;;) {
 #pragma unroll
-    for (int p0 = 0; p0 + 2 <= U / 2; p0 += 2) {
-      const uint2 x = pair[p0], y = pair[p0 + 1];
-      if (more) {
-        pair[p0] = ld_stream8(reinterpret_cast<const uint2 *>(src + p0 * 64) + lane);
-        pair[p0 + 1] = ld_stream8(reinterpret_cast<const uint2 *>(src + p0 * 64 + 64) + lane);
+    for (int d = 0; d < D; d++) {
+      const bool more = left > (uint32_t)D;
+      SlicedCount<NB> sc;
+      sc.start(f.need);
+#pragma unroll
+      for (int p0 = 0; p0 + 2 <= U / 2; p0 += 2) {
+        const uint2 x = pair[d][p0], y = pair[d][p0 + 1];
+        if (more) {
+          fetch_pair(d, p0);
+          fetch_pair(d, p0 + 1);
+        }
+        const unsigned w[4] = {look_up(cm, x.x), look_up(cm, x.y), look_up(cm, y.x),
+                               look_up(cm, y.y)};
+        sc.template add<0, 4>(w);
       }
-      const unsigned w[4] = {look_up(cm, x.x), look_up(cm, x.y), look_up(cm, y.x), look_up(cm, y.y)};
-      sc.template add<0, 4>(w);
+      if constexpr (U % 4 != 0) {
+        constexpr int N = U % 4;
+        unsigned w[N];
+        if constexpr (N >= 2) {
+          const uint2 x = pair[d][P - 1];
+          if (more) fetch_pair(d, P - 1);
+          w[0] = look_up(cm, x.x);
+          w[1] = look_up(cm, x.y);
+        }
+        if constexpr (U & 1) {
+          const uint32_t x = last[d];
+          if (more) fetch_last(d);
+          w[N - 1] = look_up(cm, x);
+        }
+        sc.template add<0, N>(w);
+      }
+      keep_candidates(f, found, out, ch, sc.reached());
+      if (--left == 0) return;
+      ch += step;
+      src += stride;
     }
-    if constexpr (U % 4 != 0) {
-      constexpr int N = U % 4;
-      unsigned w[N];
-      if constexpr (N >= 2) {
-        const uint2 x = pair[U / 2 - 1];
-        if (more) pair[U / 2 - 1] = ld_stream8(reinterpret_cast<const uint2 *>(src + (U / 2 - 1) * 64) + lane);
-        w[0] = look_up(cm, x.x);
-        w[1] = look_up(cm, x.y);
-      }
-      if constexpr (U & 1) {
-        const uint32_t x = last;
-        if (more) last = ld_stream4(src + (U - 1) * 32 + lane);
-        w[N - 1] = look_up(cm, x);
-      }
-      sc.template add<0, N>(w);
-    }
-    keep_candidates(f, found, out, ch, sc.reached());
-    if (!more) break;
-    ch += step;
   }
 }
 
 // Persistent: one block per SM, its warps take every grid-th chunk of the list, run
-// after run.  What bounds it is the look-ups (2.9 shared-memory wavefronts each) and,
-// close behind, the stream of codes.  Measured on B200, compare stage at 1e8 records:
-// see the commit of the layout it reads; filter kernel alone, tilted detector with
-// 64 slots (3.1 GB of codes): 775 us with one loop over chunks of any size, 640 us
-// with a loop per size; hexagonal with 32 slots (0.27 GB): 126 us, 72 us.
+// after run.  Bound by the look-ups (2.9 shared-memory wavefronts each) and, close
+// behind, the stream of codes.  Measured on B200 at 1e8 records, this kernel alone:
+// tilted detector, 64 slots (3.1 GB of codes) 775 us with one loop over chunks of any
+// size, 562 us with a loop per size.
 template <int NB>
 __global__ void __launch_bounds__(32 * kFilterWarps, 1)
     group_filter_kernel(const __grid_constant__ FilterArgs f) {
