@@ -1839,6 +1839,7 @@ struct lmb_pre {
   // engine's quantisation has read it
   cudaEvent_t ev_out_ready = nullptr, ev_out_free = nullptr;
   bool out_in_use = false;
+  bool blur_untimed = false;  // the last blur's events have not been read
 };
 
 namespace {
@@ -1856,6 +1857,7 @@ void free_pre(lmb_pre *p) {
   if (!p) return;
   cudaSetDevice(p->device);
   if (p->st) cudaStreamSynchronize(p->st);
+  if (p->out_in_use) cudaEventSynchronize(p->ev_out_free);  // an engine may still read d_out
   void *bufs[] = {p->d_raw, p->d_bg, p->d_sub, p->d_tmp, p->d_out, p->d_t16, p->d_filt, p->d_par,
                   p->d_cid, p->d_lab, p->d_flab, p->c.area, p->c.x0, p->c.y0, p->c.x1, p->c.y1,
                   p->c.fb, p->c.sw, p->c.swx, p->c.swy, p->c.label, p->c.keep, p->d_bits,
@@ -2462,6 +2464,7 @@ int lmb_pre_blur(lmb_pre *p, const double *weights, int32_t radius, void *out, i
   if (rc) return rc;
   LMB_CUDA(cudaEventRecord(p->ev[EV_BLUR_DL], p->st));
   LMB_CUDA(cudaStreamSynchronize(p->st));
+  p->blur_untimed = false;
   return stage_times(p, EV_BLUR0, EV_BLUR_K, 3) || stage_times(p, EV_BLUR_K, EV_BLUR_DL, 4);
 }
 
@@ -2480,12 +2483,23 @@ int lmb_pre_blur_to_slot(lmb_pre *p, const double *weights, int32_t radius, lmb_
                                 im_scale);
   if (rc) return rc;
   p->out_in_use = true;
-  LMB_CUDA(cudaStreamSynchronize(p->st));
-  return stage_times(p, EV_BLUR0, EV_BLUR_K, 3);
+  // The blur need not be waited for: the engine's stream waits for it, and what comes
+  // next on this one follows it.  Small radii take their weights with the launch; for
+  // others the caller's array must have been read.
+  if (radius < 1 || radius > kBlurFixedMaxR) LMB_CUDA(cudaStreamSynchronize(p->st));
+  p->blur_untimed = true;
+  return LMB_OK;
 }
 
 int lmb_pre_timings(lmb_pre *p, float *ms, int32_t n) {
   LMB_REQUIRE(p && ms, "null argument");
+  if (p->blur_untimed) {
+    LMB_CUDA(cudaSetDevice(p->device));
+    LMB_CUDA(cudaEventSynchronize(p->ev[EV_BLUR_K]));
+    const int rc = stage_times(p, EV_BLUR0, EV_BLUR_K, 3);
+    if (rc) return rc;
+    p->blur_untimed = false;
+  }
   for (int i = 0; i < n && i < LMB_PRE_STAGES; ++i) ms[i] = p->ms[i];
   return LMB_OK;
 }

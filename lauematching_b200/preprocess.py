@@ -171,10 +171,11 @@ class DevicePreprocessor:
         return out
 
     def blur_to_slot(self, weights: np.ndarray, radius: int, engine, slot: int,
-                     frame_dtype=np.float32) -> float:
+                     frame_dtype=np.float32, want_scale: bool = True) -> Optional[float]:
         """The blurred frame straight into an engine slot on this device,
         quantised as if ``frame_dtype`` copies of it had been loaded from the
-        host; returns the slot's imScale."""
+        host; returns the slot's imScale (without ``want_scale`` None, and the
+        call does not wait for the device)."""
         w = np.ascontiguousarray(weights, dtype=np.float64)
         if w.shape != (2 * radius + 1,):
             raise ValueError("weights must have 2*radius+1 entries")
@@ -183,8 +184,8 @@ class DevicePreprocessor:
         check(lib().lmb_pre_blur_to_slot(self._h, w.ctypes.data, int(radius), engine._h,
                                          int(slot),
                                          _lib.LMB_F64 if dt == np.float64 else _lib.LMB_F32,
-                                         C.byref(sc)))
-        return sc.value
+                                         C.byref(sc) if want_scale else None))
+        return sc.value if want_scale else None
 
     def blur(self, weights: np.ndarray, radius: int, dtype=np.float64,
              out: Optional[np.ndarray] = None) -> np.ndarray:
@@ -489,7 +490,7 @@ class Preprocessor:
         sigma = _sigma_from(int(cnt.n_centres), cnt.min_dist2, cfg["px_x"], cfg["distance"],
                             cfg["orientation_spacing"])
         w, r = gaussian_weights(sigma)
-        self._h.blur_to_slot(w, r, engine, slot, frame_dtype)
+        self._h.blur_to_slot(w, r, engine, slot, frame_dtype, want_scale=False)
         return self._h.centres(int(cnt.n_centres)) if want_centres else int(cnt.n_centres)
 
     def close(self):
@@ -529,7 +530,7 @@ class PreprocessPool:
                                 cfg["orientation_spacing"])
             wts, r = gaussian_weights(sigma)
             with self._engine_lock:
-                pre._h.blur_to_slot(wts, r, engine, slot, frame_dtype)
+                pre._h.blur_to_slot(wts, r, engine, slot, frame_dtype, want_scale=False)
             if host_copy:  # the blurred frame as the matcher read it, for the post-stage
                 return int(cnt.n_centres), pre._h.blur(wts, r, frame_dtype)
             return int(cnt.n_centres)
