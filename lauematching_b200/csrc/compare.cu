@@ -1623,22 +1623,22 @@ __device__ void bitonic_tiled(unsigned long long *g, uint32_t P, unsigned long l
   }
 }
 
-// One block per slot of the pass.  Short lists and the pass's status words also
-// go to page-locked host memory from here, so that a caller who waits for the pass
+// One block per slot of the pass.  Short lists and the slot's counters also go to page-locked host memory from here, so that a caller who waits for the pass
 // has its results without another copy (a gather kernel, a copy and its
 // synchronisation; 20-25 us of a small pass, measured on B200).
 __global__ void __launch_bounds__(1024) order_kernel(const __grid_constant__ OrderArgs a) {
   extern __shared__ __align__(16) unsigned long long sk[];  // kSmemSortMax keys
-  if (blockIdx.x == 0) {
-    const unsigned r = *a.seq % a.ring;
-    for (uint32_t w = threadIdx.x; w < a.words; w += blockDim.x)
-      a.host_status[r * a.words + w] = a.status[w];
-    __syncthreads();
-    if (threadIdx.x == 0) *a.seq += 1u;
-  }
+  if (blockIdx.x == 0 && threadIdx.x == 0)
+    a.host_status[2 * LMB_MAX_SLOTS] = a.status[2 * LMB_MAX_SLOTS];
   if ((int)blockIdx.x >= a.nslots) return;  // a pass without slots
   const int k = a.slots[blockIdx.x];
-  const uint32_t n = min(a.surv_cnt[k], a.cap);
+  const uint32_t found = a.status[k], n = min(found, a.cap);
+  __syncthreads();  // every thread has the count
+  if (threadIdx.x == 0) {
+    a.host_status[k] = found;
+    a.host_status[LMB_MAX_SLOTS + k] = a.status[LMB_MAX_SLOTS + k];
+    a.status[k] = a.status[LMB_MAX_SLOTS + k] = 0u;  // for the slot's next pass
+  }
   if (n == 0) return;
   uint32_t P = 1;
   while (P < n) P <<= 1;
@@ -1879,23 +1879,6 @@ int listed_launch(CmpArgs a, int num_sms, cudaStream_t st) {
   if (B <= 3) return launch_listed<3>(a, grid, threads, smem, st);
   if (B <= 5) return launch_listed<5>(a, grid, threads, smem, st);
   return launch_listed<8>(a, grid, threads, smem, st);
-}
-
-// Zero the survivor and pass counters of the pass's slots only: the counters
-// of other slots keep the results of their own last pass, so a pass can be
-// queued before the previous one has been collected.
-__global__ void status_reset_kernel(unsigned int *__restrict__ status, unsigned long long mask) {
-  const int k = threadIdx.x;
-  if (k < LMB_MAX_SLOTS && ((mask >> k) & 1ull)) {
-    status[k] = 0u;
-    status[LMB_MAX_SLOTS + k] = 0u;
-  }
-}
-
-int status_reset_launch(unsigned int *d_status, uint64_t mask, cudaStream_t st) {
-  status_reset_kernel<<<1, LMB_MAX_SLOTS, 0, st>>>(d_status, (unsigned long long)mask);
-  LMB_CUDA(cudaGetLastError());
-  return LMB_OK;
 }
 
 // blockIdx.y = position in the slot list; 16-byte words of the 32-byte survivors.

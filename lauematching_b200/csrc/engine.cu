@@ -31,13 +31,11 @@ int cuda_fail(cudaError_t e, const char *what, const char *file, int line) {
 
 using namespace lmb;
 
-// Status words copied back after every pass: [0,64) survivor counts,
-// [64,128) pass counts, [128] device error word (sticky).  A pass resets only
-// its own slots' counters and copies all words into the next entry of a
-// small pinned ring, so several passes can be in flight and each slot's
-// results are read from the entry of the last pass that included it.
+// Status words: [0,64) survivor counts, [64,128) pass counts, [128] device error word
+// (sticky).  A pass's ordering kernel moves its slots' counters to host memory and
+// clears them on the device, so a slot's words there are those of its last pass
+// whatever other passes are in flight.
 static constexpr int kStatusWords = 2 * LMB_MAX_SLOTS + 1;
-static constexpr int kStatusRing = 4;
 static constexpr int kEventRing = 64;  // events of passes and loads
 // Survivor lists up to this long are written to host memory by the pass itself.
 static constexpr uint32_t kHostList = 4096;
@@ -143,11 +141,9 @@ struct lmb_engine {
   lmb_survivor *d_surv = nullptr, *d_sorted = nullptr;
   unsigned long long *d_scratch = nullptr;
   unsigned int *d_status = nullptr;
-  unsigned int *h_status = nullptr;  // pinned, kStatusRing x kStatusWords
-  unsigned int *d_seq = nullptr;          // passes ordered so far (the order kernel's count)
+  unsigned int *h_status = nullptr;  // pinned, kStatusWords
   lmb_survivor *h_list = nullptr;         // pinned: [64][kHostList], short lists of each slot
   uint64_t pass_seq = 0;                  // passes enqueued so far
-  int slot_ring[LMB_MAX_SLOTS] = {};      // status entry of each slot's last pass
   uint64_t done_mask = 0;                 // slots that have been in a pass
   cudaStream_t dl = nullptr;              // survivor downloads
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
@@ -272,7 +268,6 @@ void free_engine(lmb_engine *e) {
   cudaFree(e->d_status);
   cudaFreeHost(e->h_status);
   cudaFreeHost(e->h_list);
-  cudaFree(e->d_seq);
   if (e->dl) {
     cudaStreamSynchronize(e->dl);
     cudaStreamDestroy(e->dl);
@@ -474,7 +469,6 @@ uint64_t listed_places(const lmb_engine *e, int min_spots) {
 // at the same warp count, 3.70 ms with 12 KiB tiles and three warps per stage).
 constexpr uint64_t kCellTileBytes = 8192;
 
-// One pass: status reset, compare, ordering, status copy-back, on e->st.
 // Derive the compact layout of the resident DB (see clist.cu): spots per
 // 32-record chunk on the device; on the host, the tile size (about 64 chunks
 // of the DB's average size, 4-24 KiB, at least the largest chunk) and a
@@ -718,10 +712,6 @@ int enqueue_pass(lmb_engine *e, const PassKey &k, bool capturing) {
   // timing events recorded inside a captured graph must be external to be
   // observable (and timed) after each replay
   const unsigned evf = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
-  {
-    const int rc = status_reset_launch(e->d_status, k.mask, e->st);
-    if (rc) return rc;
-  }
   LMB_CUDA(cudaEventRecordWithFlags(e->ev[0], e->st, evf));
   CmpArgs a{};
   a.db = e->d_db;
@@ -780,7 +770,6 @@ int enqueue_pass(lmb_engine *e, const PassKey &k, bool capturing) {
   OrderArgs o{};
   o.surv = e->d_surv;
   o.out = e->d_sorted;
-  o.surv_cnt = e->d_status;
   o.cap = e->cap;
   o.scratch = e->d_scratch;
   o.cap2 = e->cap2;
@@ -788,9 +777,6 @@ int enqueue_pass(lmb_engine *e, const PassKey &k, bool capturing) {
   o.host_cap = std::min(kHostList, e->cap);
   o.host_status = e->h_status;
   o.status = e->d_status;
-  o.words = kStatusWords;
-  o.ring = kStatusRing;
-  o.seq = e->d_seq;
   for (int i = 0; i < LMB_MAX_SLOTS; i++)
     if (k.mask >> i & 1) o.slots[o.nslots++] = i;
   const int rc = order_launch(o, e->st);
@@ -885,13 +871,11 @@ int lmb_engine_create(int32_t device, const lmb_geometry *geo, uint64_t survivor
   TRY(cudaMalloc(&e->d_scratch, (size_t)LMB_MAX_SLOTS * e->cap2 * sizeof(unsigned long long)));
   TRY(cudaMalloc(&e->d_status, kStatusWords * sizeof(unsigned int)));
   TRY(cudaMemset(e->d_status, 0, kStatusWords * sizeof(unsigned int)));
-  TRY(cudaHostAlloc(&e->h_status, kStatusRing * kStatusWords * sizeof(unsigned int),
+  TRY(cudaHostAlloc(&e->h_status, kStatusWords * sizeof(unsigned int),
                     cudaHostAllocDefault));
-  memset(e->h_status, 0, kStatusRing * kStatusWords * sizeof(unsigned int));
+  memset(e->h_status, 0, kStatusWords * sizeof(unsigned int));
   TRY(cudaHostAlloc(&e->h_list, (size_t)LMB_MAX_SLOTS * kHostList * sizeof(lmb_survivor),
                     cudaHostAllocDefault));
-  TRY(cudaMalloc(&e->d_seq, sizeof(unsigned int)));
-  TRY(cudaMemset(e->d_seq, 0, sizeof(unsigned int)));
 #undef TRY
   *out = e;
   return LMB_OK;
@@ -1365,7 +1349,7 @@ int lmb_match(lmb_engine *e, uint64_t slot_mask, int32_t min_nr_spots, double mi
     LMB_CUDA(cudaStreamWaitEvent(e->st, e->ev_load[e->slot_load[k]], 0));
   }
   e->fresh_mask &= ~slot_mask;
-  // The pass (status reset, compare, ordering, status copy-back) replays from
+  // The pass (status reset, compare, ordering, ) replays from
   // a CUDA graph once a configuration has been seen before; the first pass of
   // a configuration runs eagerly (it also sets the kernels' attributes).
   PassKey key;
@@ -1406,15 +1390,11 @@ int lmb_match(lmb_engine *e, uint64_t slot_mask, int32_t min_nr_spots, double mi
     rc = enqueue_pass(e, key, false);
     if (rc) return rc;
   }
-  // the pass's ordering kernel has written its status words into the next ring entry
-  const int r = (int)(e->pass_seq % kStatusRing), v = (int)(e->pass_seq % kEventRing);
+  const int v = (int)(e->pass_seq % kEventRing);
   LMB_CUDA(cudaEventRecord(e->ev_pass[v], e->st));
   e->bytes_d2h += kStatusWords * sizeof(unsigned int);
   for (int k = 0; k < LMB_MAX_SLOTS; k++)
-    if (slot_mask >> k & 1) {
-      e->slot_ring[k] = r;
-      e->slot_pass[k] = v;
-    }
+    if (slot_mask >> k & 1) e->slot_pass[k] = v;
   e->done_mask |= slot_mask;
   e->pass_seq++;
   return LMB_OK;
@@ -1429,11 +1409,10 @@ namespace {
 int slot_status(lmb_engine *e, int slot, const unsigned int **st, uint64_t *waited) {
   LMB_REQUIRE(slot >= 0 && slot < LMB_MAX_SLOTS && (e->done_mask >> slot & 1),
               "slot %d has not been part of a pass", slot);
-  const int r = e->slot_ring[slot];
   const int v = e->slot_pass[slot];
   if (!(*waited >> v & 1)) LMB_CUDA(cudaEventSynchronize(e->ev_pass[v]));
   *waited |= 1ull << v;
-  *st = e->h_status + (size_t)r * kStatusWords;
+  *st = e->h_status;
   const int derr = (int)(*st)[2 * LMB_MAX_SLOTS];
   if (derr == DEV_BAD_QUEUE) {
     set_error("compare pass: a compact-layout record longer than the pass's queue entries");

@@ -88,18 +88,15 @@ CompareTuning compare_config(int R, const CompareTuning &req);
 struct OrderArgs {
   const lmb_survivor *surv;
   lmb_survivor *out;
-  const unsigned int *surv_cnt;
   uint32_t cap;
   unsigned long long *scratch;  // [64][cap2] keys for lists above the shared-memory size
   uint32_t cap2;                // power of two >= cap
   // page-locked host memory that the kernel writes itself: slot k's list when it
-  // has at most host_cap entries, and the pass's status words
-  lmb_survivor *host_list;  // [64][host_cap]
+  // has at most host_cap entries, its counters and the error word
+  lmb_survivor *host_list;     // [64][host_cap]
   uint32_t host_cap;
-  unsigned int *host_status;    // [ring][words], entry *seq % ring
-  const unsigned int *status;   // [words]
-  uint32_t words, ring;
-  unsigned int *seq;            // passes ordered so far
+  unsigned int *host_status;   // [64] survivors, [64] passing, error word
+  unsigned int *status;        // the same on the device; the pass's counters end at 0
   int nslots;
   int slots[LMB_MAX_SLOTS];
 };
@@ -178,7 +175,6 @@ struct MergeArgs {
   double max_angle, rad2deg;
   double mid, window;  // float rounding boundary at max_angle, and the band left to the host
 };
-int status_reset_launch(unsigned int *d_status, uint64_t mask, cudaStream_t st);
 
 // Compact DB layout (clist.cu): on-detector spots per 32-record chunk, then
 // the fixed-size tiles from the host's packing of chunks into tiles.  Byte
