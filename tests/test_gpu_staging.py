@@ -1,0 +1,45 @@
+"""Copies through the page-locked pieces and the build's chunks at their edges (GPU)."""
+import numpy as np
+import pytest
+
+from lauematching_b200 import params as P
+from lauematching_b200 import synth
+from lauematching_b200.engine import PinnedBuffer
+from test_gpu_parity import engine_for
+
+pytestmark = pytest.mark.gpu
+
+
+# 1 + 2 S uint16 = 64 bytes a record; 2 MiB go directly, pieces are 8 MiB, four in the ring
+@pytest.mark.parametrize("mib,extra", [(2, 0), (2, 1), (8, -1), (8, 0), (8, 1), (32, 0), (32, 1), (45, 7)])
+def test_records_go_up_and_down_unchanged(mib, extra):
+    p = P.parse_params_text(synth.params_text(nr_px=(64, 64), max_nr_spots=15))
+    rng = np.random.default_rng(mib)
+    n = (mib << 20) // 62 + extra
+    rec = rng.integers(0, 65536, (n, 31), dtype=np.uint16)
+    pin = PinnedBuffer(rec.shape, np.uint16)
+    pin.array[...] = rec
+    with engine_for(p) as e:
+        e.upload_db(rec)
+        assert np.array_equal(e.download_db(), rec)
+        assert np.array_equal(e.download_db(5, n - 11), rec[5:n - 6])
+        e.upload_db(pin.array[:n - 3])  # page-locked, into the same memory
+        assert np.array_equal(e.download_db(), rec[:n - 3])
+    pin.free()
+
+
+@pytest.mark.parametrize("n", [1, 127, 32768, 98305, 200_000, (256 << 10) * 2 + 1])
+def test_chunked_build_equals_its_parts(n):
+    """A build over several chunks gives each orientation the record that a build of
+    a short list around it gives; the synthetic build of the same matrices too."""
+    p = P.parse_params_text(synth.params_text(max_nr_spots=10))
+    hk = synth.hkls_cubic(4)
+    with engine_for(p) as e:
+        om = e.build_db_synthetic(seed=5, n=n, hkls=hk, return_orients=True)
+        synthetic = e.download_db()
+        e.build_db(om, hk)
+        got = e.download_db()
+        assert np.array_equal(got, synthetic)
+        for at in {0, n // 3, n // 2, max(0, n - 300)}:
+            e.build_db(om[at:at + 300], hk)
+            assert np.array_equal(e.download_db(), got[at:at + 300])
