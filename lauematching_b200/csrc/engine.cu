@@ -127,7 +127,8 @@ struct lmb_engine {
   uint64_t gl_bytes = 0;  // perm and codes
   // image slots
   uint8_t *d_u8 = nullptr;
-  double *d_f64 = nullptr;  // allocated on first keep_f64 load
+  double *d_f64 = nullptr;  // float64 copies of slots [0, f64_slots): made by keep_f64 loads
+  int f64_slots = 0;
   unsigned long long *d_occ = nullptr;
   uint32_t *d_cellmask = nullptr;  // compare variant 4: the pass's cell mask
   uint32_t cm_bytes = 0;
@@ -210,6 +211,36 @@ void free_grouped(lmb_engine *e) {
   cudaFree(e->d_cand_cnt);
   e->d_group_mask = nullptr;
   e->d_cand_cnt = nullptr;
+}
+
+void drop_graphs(lmb_engine *e) {
+  for (auto &g : e->graphs)
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+  e->graphs.clear();
+}
+
+// Room for the float64 copy of `slot`: the command line keeps one frame (33 MB at
+// 2048^2), all 64 slots take 2.1 GB.
+int ensure_f64(lmb_engine *e, int slot) {
+  if (slot < e->f64_slots) return LMB_OK;
+  const int want = std::min(LMB_MAX_SLOTS, std::max(slot + 1, 2 * e->f64_slots));
+  double *d = nullptr;
+  LMB_CUDA(cudaMalloc(&d, e->npx * sizeof(double) * want));
+  cudaError_t ce = cudaStreamSynchronize(e->ld);  // loads and passes on the old copies
+  if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->st);
+  if (ce == cudaSuccess && e->f64_slots)
+    ce = cudaMemcpyAsync(d, e->d_f64, e->npx * sizeof(double) * e->f64_slots,
+                         cudaMemcpyDeviceToDevice, e->ld);
+  if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->ld);
+  if (ce != cudaSuccess) {
+    cudaFree(d);
+    return cuda_fail(ce, "float64 frames", __FILE__, __LINE__);
+  }
+  drop_graphs(e);  // captured passes name the old copies
+  cudaFree(e->d_f64);
+  e->d_f64 = d;
+  e->f64_slots = want;
+  return LMB_OK;
 }
 
 // Slots about to be written on the load stream: after the last passes that read
@@ -302,9 +333,7 @@ size_t dtype_bytes(int dtype) {
 int alloc_db(lmb_engine *e, uint64_t n) {
   LMB_REQUIRE(n < (1ull << 40), "at most 2^40 orientations are supported (got %llu)",
               (unsigned long long)n);
-  for (auto &g : e->graphs)  // captured passes name the old DB
-    if (g.exec) cudaGraphExecDestroy(g.exec);
-  e->graphs.clear();
+  drop_graphs(e);  // captured passes name the old DB
   e->n = 0;
   cudaFree(e->d_cl);
   e->d_cl = nullptr;
@@ -1037,8 +1066,7 @@ int lmb_image_load(lmb_engine *e, int32_t slot, const void *pixels, int32_t dtyp
               LMB_MAX_SLOTS - 1);
   LMB_REQUIRE(pixels, "null pixels");
   LMB_REQUIRE(dtype == LMB_F64 || dtype == LMB_F32 || dtype == 2, "unknown dtype %d", dtype);
-  if (keep_f64 && !e->d_f64)
-    LMB_CUDA(cudaMalloc(&e->d_f64, e->npx * sizeof(double) * LMB_MAX_SLOTS));
+  if (keep_f64 && (rc = ensure_f64(e, slot))) return rc;
   if ((rc = wait_released(e, 1ull << slot))) return rc;
   // A sparse frame (the usual thresholded Laue image) crosses the host link
   // as (index, value) pairs of its positive pixels; a dense one as is.

@@ -43,3 +43,35 @@ def test_chunked_build_equals_its_parts(n):
         for at in {0, n // 3, n // 2, max(0, n - 300)}:
             e.build_db(om[at:at + 300], hk)
             assert np.array_equal(e.download_db(), got[at:at + 300])
+
+
+def test_float64_copies_survive_the_growth_of_their_room():
+    """keep_f64 loads into slots that make the room grow: each slot's float64 pass
+    gives what it gave alone."""
+    rng = np.random.default_rng(2)
+    p = P.parse_params_text(synth.params_text(nr_px=(300, 200), max_nr_spots=7, min_nr_spots=2))
+    rec = np.zeros((5000, 15), np.uint16)
+    rec[:, 0] = 7
+    rec[:, 1::2] = rng.integers(0, 300, (5000, 7))
+    rec[:, 2::2] = rng.integers(0, 200, (5000, 7))
+    slots = [0, 3, 1, 40, 63]
+    imgs = {s: np.where(rng.random(60000) < 0.2, rng.random(60000) * 50, 0.0) for s in slots}
+
+    def one(e, s):
+        e.match([s], 2, 3.0, value_mode=1)
+        return e.results(s)
+
+    alone = {}
+    for s in slots:
+        with engine_for(p) as e:
+            e.upload_db(rec)
+            e.load_image(s, imgs[s], keep_f64=True)
+            alone[s] = one(e, s)
+    with engine_for(p) as e:
+        e.upload_db(rec)
+        for i, s in enumerate(slots):
+            e.load_image(s, imgs[s], keep_f64=True)
+            for t in slots[:i + 1]:  # eager, then from a graph, then over new room
+                for _ in range(2):
+                    got, n_pass = one(e, t)
+                    assert n_pass == alone[t][1] and np.array_equal(got, alone[t][0])
