@@ -75,3 +75,36 @@ def test_float64_copies_survive_the_growth_of_their_room():
                 for _ in range(2):
                     got, n_pass = one(e, t)
                     assert n_pass == alone[t][1] and np.array_equal(got, alone[t][0])
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.float32, np.float64])
+def test_pairs_read_in_place_and_pairs_copied_give_the_dense_slots(dtype):
+    """Pairs of one frame are read from page-locked memory up to 128 KiB and copied
+    beyond: both sides of that line, more frames in a row than staging buffers."""
+    rng = np.random.default_rng(11)
+    nx, ny = 800, 700
+    p = P.parse_params_text(synth.params_text(nr_px=(nx, ny), max_nr_spots=7, min_nr_spots=1))
+    rec = np.zeros((4000, 15), np.uint16)
+    rec[:, 0] = 7
+    rec[:, 1::2] = rng.integers(0, nx, (4000, 7))
+    rec[:, 2::2] = rng.integers(0, ny, (4000, 7))
+    size = np.dtype(dtype).itemsize
+    bytes_of = lambda n: -(-4 * n // 16) * 16 + n * size
+    last = max(n for n in range(1, 40000) if bytes_of(n) <= 128 << 10)
+    frames = []
+    for n in (1, last, last + 1, last - 1, last + 2000, 100, last):
+        f = np.zeros(nx * ny, dtype)
+        f[rng.choice(nx * ny, n, replace=False)] = rng.integers(1, 256, n)
+        frames.append(f)
+    slots = list(range(len(frames)))
+    got = {}
+    for sparse in (True, False):
+        with engine_for(p) as e:
+            e.upload_db(rec)
+            e.set_sparse_uploads(sparse)
+            for s in slots:
+                e.load_image(s, frames[s])
+            e.match(slots, 1, 0.0)
+            got[sparse] = [e.results(s) for s in slots]
+    for a, b in zip(got[True], got[False]):
+        assert a[1] == b[1] and np.array_equal(a[0], b[0])
