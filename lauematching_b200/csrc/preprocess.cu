@@ -478,9 +478,11 @@ __device__ void sel_pick16(PreState *st, unsigned *g16, int mode) {
     if (s.n == 0) s.valid = 0;
   }
   __syncthreads();
+  const unsigned long long kk[2] = {s.k[0], s.k[1]};
+  __syncthreads();  // the owner of a rank's bin replaces the rank below
   if (s.valid) {
     for (int L = 0; L < (s.two ? 2 : 1); ++L) {
-      const unsigned long long k = s.k[L];
+      const unsigned long long k = kk[L];
       if (k >= excl && k < excl + mine) {
         unsigned long long r = k - excl;
         int jj = 63;
