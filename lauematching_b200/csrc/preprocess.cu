@@ -687,15 +687,80 @@ __device__ void vh_finish(PreState *st, unsigned *g16, unsigned *h, int top, int
   for (int b = t; b <= top; b += kVhThreads) g16[b] = 0u;
 }
 
+// Eight neighbouring pixels of an 8- or 16-bit frame as 16-bit pairs.
+__device__ __forceinline__ uint4 load_eight(const uint16_t *raw, unsigned q) {
+  return reinterpret_cast<const uint4 *>(raw)[q];
+}
+__device__ __forceinline__ uint4 load_eight(const uint8_t *raw, unsigned q) {
+  const uint2 b = reinterpret_cast<const uint2 *>(raw)[q];
+  return make_uint4(__byte_perm(b.x, 0, 0x4140), __byte_perm(b.x, 0, 0x4342),
+                    __byte_perm(b.y, 0, 0x4140), __byte_perm(b.y, 0, 0x4342));
+}
+
+// A frame and a background of 8- or 16-bit whole numbers: differences (not below
+// zero) eight pixels at a time in integers, zeros counted in a register.
+template <typename T>
+__device__ __forceinline__ void value_hist_whole(const T *__restrict__ raw, const uint16_t *__restrict__ bg16,
+                                                 uint16_t *__restrict__ sub16, unsigned n, unsigned *g16,
+                                                 int mode, unsigned *h, DigitRun &run, unsigned &most) {
+  unsigned zeros = 0;
+  auto count = [&](unsigned b) {
+    if (b == 0) {
+      ++zeros;
+      return;
+    }
+    most = max(most, b);
+    if (b < (unsigned)kVhLocal) run.add(h, b);
+    else atomicAdd(g16 + b, 1u);
+  };
+  const unsigned groups = n / 8, stride = gridDim.x * blockDim.x;
+  const unsigned first = blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr int U = 2;
+  for (unsigned q0 = first; q0 < groups; q0 += U * stride) {
+    uint4 a[U], b[U];
+    bool in[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const unsigned q = q0 + u * stride;
+      in[u] = u == 0 || q < groups;
+      if (in[u]) {
+        a[u] = load_eight(raw, q);
+        b[u] = reinterpret_cast<const uint4 *>(bg16)[q];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (!in[u]) continue;
+      const uint4 d = make_uint4(__vsubus2(a[u].x, b[u].x), __vsubus2(a[u].y, b[u].y),
+                                 __vsubus2(a[u].z, b[u].z), __vsubus2(a[u].w, b[u].w));
+      reinterpret_cast<uint4 *>(sub16)[q0 + u * stride] = d;
+      for (unsigned w : {d.x, d.y, d.z, d.w}) {
+        count(w & 0xFFFFu);
+        count(w >> 16);
+      }
+    }
+  }
+  for (unsigned i = groups * 8 + first; i < n; i += stride) {  // up to seven pixels
+    const unsigned r = raw[i], g = bg16[i], d = r > g ? r - g : 0u;
+    sub16[i] = (uint16_t)d;
+    count(d);
+  }
+  zeros = __reduce_add_sync(0xffffffffu, zeros);
+  if (mode == SEL_ALL && (threadIdx.x & 31) == 0 && zeros) atomicAdd(h, zeros);
+}
+
 // Subtraction fused with the value histogram (see above); the differences are
 // kept as 16-bit values.  Each block counts values below kVhLocal in shared
 // memory (runs of equal values in registers) and adds larger ones straight into
 // the global 65536-bin histogram.  A frame with another value leaves the value
 // path: its threshold is infinite, so nothing follows from the 16-bit values, and
 // the host starts again with the radix selection.  *bg_other = 0: the background
-// is whole numbers too and read as bg16.  Measured on B200 (cold caches), 2048^2
+// is whole numbers too and read as bg16; with 8- and 16-bit frames all of it is
+// integers then.  Measured on B200 (cold caches), 2048^2
 // uint16 frame: 70.7 us with the background and the differences as float64 and the
-// last block's search over all 65536 bins in global memory, 34.3 us.
+// last block's search over all 65536 bins in global memory, 34.3 us with one pixel
+// at a time in float64; in integers the whole threshold stage takes 36-43 us
+// instead of 49-50 (a frame into its slot 333 -> 322 us).
 template <typename T>
 __global__ void __launch_bounds__(kVhThreads, 4)
     value_hist_kernel(const T *__restrict__ raw, const double *__restrict__ bg,
@@ -711,10 +776,16 @@ __global__ void __launch_bounds__(kVhThreads, 4)
   DigitRun run;  // bins below kVhLocal
   bool nonint = false;
   unsigned most = 0;
-  constexpr int U = 8;
   const bool whole_bg = *bg_other == 0u;
+  bool counted = false;
+  if constexpr (std::is_same_v<T, uint16_t> || std::is_same_v<T, uint8_t>)
+    if (whole_bg) {
+      value_hist_whole(raw, bg16, sub16, n, g16, mode, h, run, most);
+      counted = true;
+    }
+  constexpr int U = 8;
   const unsigned stride = gridDim.x * blockDim.x;
-  const unsigned rounds = (n + stride * U - 1) / (stride * U);
+  const unsigned rounds = counted ? 0u : (n + stride * U - 1) / (stride * U);
   for (unsigned it = 0; it < rounds; ++it) {
     double v[U];
     bool in[U];
