@@ -21,8 +21,10 @@
 //             together (they differ in the sign of q_z, which says which of the two
 //             has a positive energy; both reflect the same way).
 //   detector  of those: z > 0 and the pixel inside the frame as linear
-//             inequalities in the unnormalised direction, without a division or a
-//             square root.
+//             inequalities in the direction, without a division or a square root.
+//             The list holds unit vectors, so a coordinate is one dot product and
+//             one FMA (about 25 operations; |q|^2 and scaled margins per unit took
+//             40).
 //
 // The HKLs that can be seen are taken in chunks of file order.  Each thread owns one orientation
 // and keeps a bit per unit (a pair h, -h of the chunk, or a single HKL) that
@@ -33,7 +35,11 @@
 // other two by the lane with the most bits of its warp.  Measured on B200 at 1e8
 // synthetic orientations (whole build, one warp-wide FP32 test of energy and
 // detector per HKL before): fcc beam-normal 644 -> 39 ms, tilted 34-ID-E detector
-// 890 -> 234 ms, hexagonal beam-normal 3250 -> 66 ms.  A build flag
+// 890 -> 234 ms, hexagonal beam-normal 3250 -> 66 ms; with unit vectors and
+// chunks of 384 HKLs instead of 512 (six blocks per SM fit instead of five), 3e7
+// orientations: tilted 60.8 -> 52.6 ms (of them FP64 20, detector test 27 before and
+// about 20 now), hexagonal 13.5 -> 12.1, fcc 8.9 -> 8.0.  Chunks of 256: tilted 59.7
+// where 384 gave 57.9, the lanes' numbers of bits being less equal.  A build flag
 // (exact_all), an orientation that is no rotation, and geometry outside the
 // screens' assumptions take FP64 for every HKL.
 //
@@ -57,22 +63,23 @@ struct BuildGeo {
   double recip[9], rt[9];
   double p0, p1, p2, px_x, px_y, cx, cy, elo, ehi;
   int W, H, S, R;
-  // detector screen: pixel * z = a * x + b * z, and its margins
-  float rt2[3];
-  float ax, bx0, bx1, ay, by0, by1, tolx, toly;
+  // detector screen, direction d = (x, y, z) of a unit reflection vector q as
+  // d = (-2 q_z) u + rt2, u = detector rotation . q: X = a x / tol = q_z (su u_x) + c and
+  // the frame's edges as X + b0 z > 0, X + b1 z < 0 (b / tol), the same for y; z itself
+  float sux, suy, cx2, cy2, cz2, bx0, bx1, by0, by1;
 };
 
 static constexpr double kHcKeVnm = 1.2398419739;              // LaueMatchingHeaders.h:41
 static constexpr double kFourPi = 4.0 * 3.14159265358979323846;  // 4 * M_PI as C folds it
-static constexpr int kHklChunk = 512;                // HKLs per chunk
+static constexpr int kHklChunk = 384;                // HKLs per chunk
 static constexpr int kChunkWords = kHklChunk / 32;
 static constexpr double kRotTol = 1e-4;  // a rotation: |OM^T OM - 1| below this
-static constexpr double kBandTol = 4e-4;  // relative margin of the energy band (3 kRotTol and rounding)
+static constexpr double kBandTol = 4e-4;  // relative margin of |q| and |q|^2 (3 kRotTol and rounding)
 
-// The units of a chunk: hkl (as floats) and the interval of |q_z| it can be seen
-// in, as two bf16 (the lower bound in the high half, rounded down; the upper one
-// rounded up); the relative error of its projection; the chunk positions of h
-// (taken when q_z < 0) and of -h (q_z > 0), 0xFFFF for none.
+// The units of a chunk: hkl / |q| (as floats) and the interval of |q_z| / |q| it can
+// be seen in, as two bf16 (the lower bound in the high half, rounded down; the upper
+// one rounded up); the error of its unit direction; the chunk positions of h (taken
+// when q_z < 0) and of -h (q_z > 0), 0xFFFF for none.
 struct BuildUnits {
   float4 hkl_band[kHklChunk];
   float eps[kHklChunk];
@@ -112,7 +119,7 @@ __device__ __forceinline__ bool exact_spot(const double T[9], const int4 hk, con
 }
 
 template <bool kExactAll>
-__global__ void __launch_bounds__(128) dbbuild_kernel(const double *__restrict__ om, uint64_t n,
+__global__ void __launch_bounds__(128, 6) dbbuild_kernel(const double *__restrict__ om, uint64_t n,
                                                       const int4 *__restrict__ hkl, int nh,
                                                       const int4 *__restrict__ seen, int nseen,
                                                       const BuildUnits *__restrict__ units,
@@ -133,7 +140,7 @@ __global__ void __launch_bounds__(128) dbbuild_kernel(const double *__restrict__
   const bool valid = oid < n;
 
   double T[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  float U[9];           // detector rotation . T
+  float U[9];           // detector rotation . T, rows scaled (BuildGeo)
   float t0 = 0, t1 = 0, t2 = 0;  // T's last row
   bool regular = true;
   if (valid) {
@@ -161,7 +168,8 @@ __global__ void __launch_bounds__(128) dbbuild_kernel(const double *__restrict__
       for (int r = 0; r < 3; r++)
 #pragma unroll
         for (int c = 0; c < 3; c++)
-          U[r * 3 + c] = (float)(g.rt[r * 3] * T[c] + g.rt[r * 3 + 1] * T[3 + c] + g.rt[r * 3 + 2] * T[6 + c]);
+          U[r * 3 + c] = (float)(g.rt[r * 3] * T[c] + g.rt[r * 3 + 1] * T[3 + c] + g.rt[r * 3 + 2] * T[6 + c]) *
+                         (r == 0 ? g.sux : r == 1 ? g.suy : -2.f);
       t0 = (float)T[6];
       t1 = (float)T[7];
       t2 = (float)T[8];
@@ -218,24 +226,17 @@ __global__ void __launch_bounds__(128) dbbuild_kernel(const double *__restrict__
         const int u = w * 32 + __ffs(bits) - 1;
         bits &= bits - 1u;
         const float4 h = su->hkl_band[u];
-        const float eps = su->eps[u];
+        const float m = su->eps[u];  // error of the unit direction
         const uint32_t pos = su->pos[u];
         const float qz = fmaf(t0, h.x, fmaf(t1, h.y, t2 * h.z));
         const float u0 = fmaf(U[0], h.x, fmaf(U[1], h.y, U[2] * h.z));
         const float u1 = fmaf(U[3], h.x, fmaf(U[4], h.y, U[5] * h.z));
         const float u2 = fmaf(U[6], h.x, fmaf(U[7], h.y, U[8] * h.z));
-        const float q2 = fmaf(u0, u0, fmaf(u1, u1, u2 * u2));
-        const float d = -2.f * qz;
-        const float x = fmaf(d, u0, g.rt2[0] * q2);
-        const float y = fmaf(d, u1, g.rt2[1] * q2);
-        const float z = fmaf(d, u2, g.rt2[2] * q2);
-        const float m = eps * q2;  // error of x, y and z
-        const bool off = z < -m || fmaf(g.ax, x, g.bx0 * z) < -m * g.tolx ||
-                         fmaf(g.ax, x, g.bx1 * z) > m * g.tolx ||
-                         fmaf(g.ay, y, g.by0 * z) < -m * g.toly ||
-                         fmaf(g.ay, y, g.by1 * z) > m * g.toly;
+        const float x = fmaf(qz, u0, g.cx2), y = fmaf(qz, u1, g.cy2), z = fmaf(qz, u2, g.cz2);
+        const bool off = z < -m || fmaf(g.bx0, z, x) < -m || fmaf(g.bx1, z, x) > m ||
+                         fmaf(g.by0, z, y) < -m || fmaf(g.by1, z, y) > m;
         if (off) continue;
-        const bool either = !(qz * qz > m * eps);  // q_z may have either sign (or eps is NaN)
+        const bool either = !(fabsf(qz) > m);  // q_z may have either sign (or m is NaN)
         const uint32_t i = pos & 0xFFFFu, j = pos >> 16;
         if ((qz < 0.f || either) && i != 0xFFFFu) keep[(i >> 5) * TB + t] |= 1u << (i & 31u);
         if ((!(qz < 0.f) || either) && j != 0xFFFFu) keep[(j >> 5) * TB + t] |= 1u << (j & 31u);
@@ -376,18 +377,21 @@ static BuildGeo make_build_geo(const lmb_geometry &geo) {
   g.H = geo.nr_px_y;
   g.S = geo.max_nr_spots;
   g.R = 1 + 2 * geo.max_nr_spots;
-  for (int i = 0; i < 3; i++) g.rt2[i] = (float)g.rt[3 * i + 2];
-  // pixel * z = a * x + b * z must lie in (-z, N z)
+  // pixel * z = a * x + b * z must lie in (-z, N z); an error m of x and z is one of
+  // tol * m in that
   const double ax = g.p2 / g.px_x, bx = g.cx - g.p0 / g.px_x;
   const double ay = g.p2 / g.px_y, by = g.cy - g.p1 / g.px_y;
-  g.ax = (float)ax;
-  g.bx0 = (float)(bx + 1.0);
-  g.bx1 = (float)(bx - g.W);
-  g.ay = (float)ay;
-  g.by0 = (float)(by + 1.0);
-  g.by1 = (float)(by - g.H);
-  g.tolx = (float)(std::fabs(ax) + std::max(std::fabs(bx + 1.0), std::fabs(bx - g.W)));
-  g.toly = (float)(std::fabs(ay) + std::max(std::fabs(by + 1.0), std::fabs(by - g.H)));
+  const double tolx = std::fabs(ax) + std::max(std::fabs(bx + 1.0), std::fabs(bx - g.W));
+  const double toly = std::fabs(ay) + std::max(std::fabs(by + 1.0), std::fabs(by - g.H));
+  g.sux = (float)(-2.0 * ax / tolx);
+  g.suy = (float)(-2.0 * ay / toly);
+  g.cx2 = (float)(ax / tolx * g.rt[2]);
+  g.cy2 = (float)(ay / toly * g.rt[5]);
+  g.cz2 = (float)g.rt[8];
+  g.bx0 = (float)((bx + 1.0) / tolx);
+  g.bx1 = (float)((bx - g.W) / tolx);
+  g.by0 = (float)((by + 1.0) / toly);
+  g.by1 = (float)((by - g.H) / toly);
   return g;
 }
 
@@ -452,8 +456,10 @@ static uint32_t bf16_bound(double v, bool down) {
 
 // The HKLs that some rotation can put on the detector within the energy band, in
 // file order, and their units, chunk by chunk.  Errors: the FP32 q_z of a rotation
-// is within 8 x 2^-24 of sum |recip column| |h| (rounded inputs, one product, two
-// FMAs); eps bounds that of x, y and z against |q|^2, with a factor of 4 to spare.
+// is within 10 x 2^-24 of sum |recip column| |h| (rounded inputs, one product, two
+// FMAs); eps bounds that of x, y and z for the unit vector (4 such products and a few
+// roundings, with a factor of 4 to spare) and its length, which is 1 within kBandTol
+// (|q| is taken from the list, the matrix is a rotation within kRotTol).
 static void build_units(const lmb_geometry &geo, const int4 *hkl, int nh, std::vector<int4> *seen,
                         std::vector<BuildUnits> *units, std::vector<uint32_t> *count) {
   const double c = kHcKeVnm / kFourPi, ulp = std::ldexp(1.0, -24);
@@ -484,7 +490,7 @@ static void build_units(const lmb_geometry &geo, const int4 *hkl, int nh, std::v
     }
     const double sum = col[0] * std::fabs((double)h.x) + col[1] * std::fabs((double)h.y) +
                        col[2] * std::fabs((double)h.z);
-    const double err = 8.0 * ulp * sum, q = std::sqrt(q2);
+    const double err = 10.0 * ulp * sum, q = std::sqrt(q2);
     const bool plain = q2 > 1e-20 && q2 < 1e20 && sum < 1e15;  // else FP64 decides
     double lo = 0.0, hi = 3e38;
     if (plain) {
@@ -510,11 +516,13 @@ static void build_units(const lmb_geometry &geo, const int4 *hkl, int nh, std::v
       continue;
     }
     // NaN eps: every comparison of the detector screen fails, so it rejects nothing
-    const uint32_t band = plain ? bf16_bound(lo, true) << 16 | bf16_bound(hi, false) : 0x00007F80u;
+    const double len = plain ? q : 1.0;
+    const uint32_t band =
+        plain ? bf16_bound(lo / len, true) << 16 | bf16_bound(hi / len, false) : 0x00007F80u;
     float w;
     memcpy(&w, &band, 4);
-    bu.hkl_band[nu] = make_float4((float)h.x, (float)h.y, (float)h.z, w);
-    bu.eps[nu] = plain ? (float)(256.0 * ulp * sum / q + 4e-6) : std::numeric_limits<float>::quiet_NaN();
+    bu.hkl_band[nu] = make_float4((float)(h.x / len), (float)(h.y / len), (float)(h.z / len), w);
+    bu.eps[nu] = plain ? (float)(256.0 * ulp * sum / q + 4e-6 + kBandTol) : std::numeric_limits<float>::quiet_NaN();
     bu.pos[nu] = (uint32_t)i | 0xFFFF0000u;
     open[std::make_tuple(h.x, h.y, h.z)].push_back(nu);
     nu++;
