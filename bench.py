@@ -101,7 +101,9 @@ class ClockSampler:
             bits[name] = v
         get_reasons = getattr(nv, "nvmlDeviceGetCurrentClocksEventReasons", None) or \
             nv.nvmlDeviceGetCurrentClocksThrottleReasons
-        while not self._stop.is_set():
+        last = False
+        while not last:
+            last = self._stop.is_set()  # one sample at the end of a region shorter than a call
             try:
                 self.sm.append(float(nv.nvmlDeviceGetClockInfo(h, nv.NVML_CLOCK_SM)))
                 r = get_reasons(h)
@@ -581,10 +583,9 @@ def tilted_leg(args, dev, K=64, n=None):
         auto = runs["auto"]
         t = auto["compare_ms"] * 1e-3
         ref_bytes = n * REC_BYTES_PER_ORIENT + K * p.nr_px_x * p.nr_px_y
-        # the filter reads the cell codes (2 B per spot, padded to four) of the
-        # records that can pass and the occupancy words (the mask's source); the
-        # layout's other part, 4 B per record, is read for candidates only
-        streamed = (lay["bytes"] - 4 * n + p.nr_px_x * p.nr_px_y * 8) \
+        # the filter reads the cell codes (2 B per spot) of the records that can pass
+        # and the occupancy words (the mask's source)
+        streamed = (round(2 * out["gathers"]["spots_per_record"] * n) + p.nr_px_x * p.nr_px_y * 8) \
             if auto["variant"] == 5 else ref_bytes
         out["roofline"] = {"bound": "hbm", "peak": peak, "peak_source": peak_src, "unit": "GB/s",
                            "reference_layout_bytes": ref_bytes,
@@ -1370,6 +1371,7 @@ def run_ours(args, rank, world):
     full_gather = {"value": round(K * fg_n / (fg_total * 1e-3), 2), "unit": UNIT,
                    "compare_ms": round(statistics.mean(fg_cmp), 4),
                    "same_survivor_counts": fg_surv == surv}
+    e.set_tuning(**shape_main)  # the legs below run the pass as it is by default
 
     merge = merge_timing(p.space_group, p.max_angle, dev) if rank == 0 else None
     refine = refine_timing(dev, cpu=not args.no_cpu_baseline) if rank == 0 else None

@@ -101,37 +101,45 @@ int lmb_engine_destroy(lmb_engine *e);
 void *lmb_engine_stream(lmb_engine *e);
 
 /* Launch shape of the compare pass: fields = {variant (0 block-barrier ring,
- * 1 warp-specialised, 2 warp-specialised over the compact layout, 3 automatic
- * -- the default: variant 2 while the records that can pass hold at most ~3
- * spots per DB record on average, variant 4 beyond, variant 1 when the
- * compact layout cannot be built --, 4 the compact layout filtered by the
- * cell mask of the pass's frames), tile_sub (32-orientation sub-tiles per
- * tile), stages, consumer warps, blocks per SM, grid multiplier,
- * full_gather, test_consumer_wait_us, cell_consumers, cell_stages,
- * cell_queue}; 0 = default.  cell_consumers, cell_stages and cell_queue (1:
- * the records that can still pass are queued and counted 32 at a time; 0:
- * counted chunk by chunk) shape variant 4 when the automatic variant picks it
- * (the autotuner's dense-DB entry); a pinned variant 4 takes cell_queue from
- * this field too.  full_gather = 1
+ * 1 warp-specialised, both over the reference records; 2 warp-specialised over
+ * the tiled compact layout; 3 automatic, the default; 4 the compact layout
+ * filtered by the cell mask of the pass's frames; 5 the records grouped by spot
+ * count, filtered by the cells of the frames' groups, the rest counted),
+ * tile_sub (32-orientation sub-tiles per tile), stages, consumer warps, blocks
+ * per SM, grid multiplier, full_gather, test_consumer_wait_us, cell_consumers,
+ * cell_stages, cell_queue}; 0 = default.  The automatic variant runs over the
+ * grouped records too: it counts those that can pass one by one while they are
+ * few and filters them first when they are many; without grouped records
+ * (MaxNrLaueSpots > 255, 2^32 - 2^14 records or more, no memory for 4 bytes per
+ * record) and for MinNrSpots < 1 or full_gather it takes variant 2 while the
+ * records that can pass hold at most 3 spots per DB record, variant 1 beyond.
+ * Variants 3 and 5 have no shape to choose over the grouped records;
+ * cell_consumers and cell_stages are accepted and kept, a pinned variant 4 takes
+ * cell_queue (1: the records that can still pass are queued and counted 32 at a
+ * time; 0: counted chunk by chunk) from the last field.  full_gather = 1
  * gathers every spot even of records with fewer spots than MinNrSpots (which
  * cannot pass; by default they are skipped; results are identical either
  * way), for measuring the full gather cost.  test_consumer_wait_us (tests
- * only, compact-layout variants) makes the pass's consumer warps wait that
+ * only, variants 2 and 4) makes the pass's consumer warps wait that
  * long on a barrier nothing arrives at, so the pass gives up and its results
  * report LMB_ERR_TIMEOUT; the engine's device error word is sticky, so that
  * engine reports the timeout from then on.  Written by the autotuner; get
  * returns the shape actually used for this DB.  No reference counterpart
  * (the reference launches <<<ceil(n/1024),1024>>>, LaueMatchingGPU.cu:739-743). */
 int lmb_engine_set_tuning(lmb_engine *e, const int32_t *fields, int32_t n_fields);
-/* get: fields 0-6 as set, 7: the variant the latest pass ran, 8: the test
- * wait, 9-11: the cell-mask pass's shape for the automatic variant. */
+/* get: fields 0-6 as set, 7: the variant the latest pass ran (of the automatic
+ * one over grouped records: 2 while the records that can pass hold at most 3
+ * spots per DB record, 5 beyond), 8: the test wait, 9-11: cell_consumers,
+ * cell_stages, cell_queue. */
 int lmb_engine_get_tuning(lmb_engine *e, int32_t *fields, int32_t n_fields);
 
-/* The compact device layout variant 2 streams: derived from the resident
- * records on the first variant-2 pass (1 byte per record + 4 bytes per
- * on-detector spot, in record order; the reference records stay resident).
- * compact = 1 built, 0 not yet, -1 this DB keeps the reference layout
- * (MaxNrLaueSpots > 255 or tiles too large).  No reference counterpart. */
+/* The device layouts derived from the resident records (which stay): the records
+ * grouped by spot count (4 bytes per record, and once a pass filters them 2 bytes
+ * per on-detector spot) and the tiled compact layout of variants 2 and 4 (1 byte
+ * per record + 4 bytes per on-detector spot).  compact = 1 one of them is built, 0
+ * not yet, -1 this DB keeps the reference layout (MaxNrLaueSpots > 255 or tiles too
+ * large).  compact_bytes: both; tiles, tile_bytes: of the tiled one (0 without).
+ * No reference counterpart. */
 int lmb_engine_layout_info(lmb_engine *e, int32_t *compact, uint64_t *compact_bytes,
                            int32_t *tiles, int32_t *tile_bytes);
 

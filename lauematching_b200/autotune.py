@@ -5,9 +5,10 @@ layout), tile size, ring depth, consumer warps and grid size on the device for
 a DB of the given record size and batch width, checks that every shape
 returns the same survivors, and writes the fastest shape per (record words,
 batch bucket) to ``tuning.json`` next to this file.  With ``--dense`` it
-sweeps the cell-mask pass (variant 4) on a DB of many spots per record and
-writes the ``_dense`` entries, the shape the automatic variant uses when it
-picks that pass.  Engines load the table at creation.
+compares the grouped records' filter (variant 5) with the cell-mask pass
+(variant 4) on a DB of many spots per record and writes the ``_dense`` entries.
+Engines load the table before their first pass; the automatic variant over
+grouped records has no shape to choose, pinned variants take theirs from it.
 
     python -m lauematching_b200.autotune --n-orient 100000000 --batches 1,64 --write
     python -m lauematching_b200.autotune --dense --n-orient 100000000 --batches 64 --write
@@ -45,8 +46,7 @@ def load_table() -> dict:
 
 def lookup(R: int, k: int, dense: bool = False) -> dict | None:
     """Best shape for records of R uint16 words and a pass of k images; with
-    ``dense``, the cell-mask pass's shape (variant 4), which the automatic
-    variant runs when the records that can pass hold many spots."""
+    ``dense``, that of a DB of many spots per record."""
     t = load_table().get("entries", {})
     suffix = f"_K{batch_bucket(k)}" + ("_dense" if dense else "")
     key = f"R{R}{suffix}"

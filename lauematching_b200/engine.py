@@ -109,8 +109,8 @@ class Engine:
     def set_tuning(self, test_consumer_wait_us: int = 0, cell_consumers: int = 0,
                    cell_stages: int = 0, cell_queue: int = 0, **kw) -> None:
         """Pin the compare pass's launch shape (TUNING_FIELDS; variant 3 =
-        automatic when not given; cell_consumers / cell_stages shape the
-        cell-mask pass when the automatic variant picks it).
+        automatic when not given; it and variant 5 run over the records grouped
+        by spot count and have no shape to choose).
         test_consumer_wait_us is for tests only: the pass gives up after that
         wait and reports a timeout."""
         check(lib().lmb_engine_set_tuning(
@@ -135,7 +135,7 @@ class Engine:
         check(lib().lmb_engine_set_dense_share(self._h, float(share)))
 
     def layout_info(self) -> dict:
-        """State of the compact device layout (compare variant 2)."""
+        """State of the device layouts derived from the records."""
         st, nb = C.c_int32(0), C.c_uint64(0)
         tr, tb = C.c_int32(0), C.c_int32(0)
         check(lib().lmb_engine_layout_info(self._h, C.byref(st), C.byref(nb), C.byref(tr),
