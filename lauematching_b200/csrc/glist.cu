@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(256) glist_scatter_kernel(const uint8_t *__res
 // chosen to spread over the shared-memory banks (two cells per 4-byte word).  A lane
 // offers the banks of the spots it has left, three rounds hand every bank to at most
 // two lanes that ask for it, and the lanes that got none take any spot.  (At most one
-// lane per bank leaves more lanes without: 2.9 wavefronts a look-up instead of 2.4,
+// lane per bank leaves more lanes without: 2.9 wavefronts a look-up instead of 2.3,
 // 3.7 unordered.)
 __global__ void __launch_bounds__(256) glist_code_kernel(const uint16_t *__restrict__ db, int R, int S,
                                                          int W, int H,
