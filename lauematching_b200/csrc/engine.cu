@@ -357,9 +357,9 @@ int alloc_db(lmb_engine *e, uint64_t n) {
     LMB_CUDA(cudaMalloc(&e->d_db, alloc));
     e->db_cap = alloc;
   }
-  // the caller writes every record; the padding behind them is zero
+  // the padding behind the records is zero; the caller writes every record, and sets n
+  // once they are there: a build or an upload that fails leaves an empty DB
   LMB_CUDA(cudaMemsetAsync(reinterpret_cast<char *>(e->d_db) + bytes, 0, alloc - bytes, e->st));
-  e->n = n;
   return LMB_OK;
 }
 
@@ -938,6 +938,7 @@ int lmb_db_upload(lmb_engine *e, const uint16_t *records, uint64_t n) {
   if (rc) return rc;
   e->bytes_h2d += (size_t)n * e->R * 2;
   LMB_CUDA(cudaStreamSynchronize(e->st));
+  e->n = n;
   return LMB_OK;
 }
 
@@ -997,9 +998,10 @@ static int db_build_common(lmb_engine *e, const double *orients, uint64_t seed, 
     if (used[i]) cudaEventDestroy(used[i]);
   }
   dbbuild_tables_free(tables);
-  if (rc) cudaMemset(e->d_db, 0, (size_t)n * e->R * 2);  // no half-built records
-  e->on_detector = rc == LMB_OK;
-  return rc;
+  if (rc) return rc;
+  e->n = n;
+  e->on_detector = true;
+  return LMB_OK;
 }
 
 int lmb_db_build(lmb_engine *e, const double *orients, uint64_t n, const int32_t *hkls,

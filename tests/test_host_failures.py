@@ -1,0 +1,112 @@
+"""What the library does when a call of the CUDA runtime fails (CPU).
+
+The library's objects are linked against a runtime on the host (fake_cudart.cu) in
+which allocations, copies and launches fail on request; no GPU takes part."""
+import concurrent.futures
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from lauematching_b200 import _lib, build
+from lauematching_b200 import params as P
+from lauematching_b200 import synth
+from lauematching_b200.engine import Engine
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+MIB = 1 << 20
+
+
+def _run(cmd):
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.fixture(scope="module")
+def fake_path(tmp_path_factory):
+    tmp = str(tmp_path_factory.mktemp("fake"))
+    objdir = os.path.join(build.HERE, "_build")
+    headers = [os.path.join(build.CSRC, f) for f in os.listdir(build.CSRC) if f.endswith(("h",))]
+    newest = max(os.path.getmtime(h) for h in headers)
+    inc = ["-I", os.path.join(build.ROOT, "include")]
+    objs, jobs = [], []
+    for src in build.sources():
+        obj = os.path.join(objdir, os.path.basename(src) + ".o")
+        if not os.path.exists(obj) or os.path.getmtime(obj) < max(newest, os.path.getmtime(src)):
+            obj = os.path.join(tmp, os.path.basename(src) + ".o")
+            jobs.append([build.nvcc(), *build.NVCC_FLAGS, *inc, "-dc", "-c", src, "-o", obj])
+        objs.append(obj)
+    fake = os.path.join(tmp, "fake_cudart.o")
+    jobs.append([build.nvcc(), *build.NVCC_FLAGS, *inc, "-c", os.path.join(HERE, "fake_cudart.cu"),
+                 "-o", fake])
+    with concurrent.futures.ThreadPoolExecutor(8) as ex:
+        list(ex.map(_run, jobs))
+    link = os.path.join(tmp, "dlink.o")
+    _run([build.nvcc(), *build.NVCC_FLAGS[:2], "-dlink", "-Xcompiler", "-fPIC", *objs, "-o", link])
+    so = os.path.join(tmp, "libfake.so")
+    _run(["g++", "-shared", "-Wl,-Bsymbolic", "-o", so, *objs, link, fake, "-lgomp"])
+    return so
+
+
+@pytest.fixture
+def fake(fake_path, monkeypatch):
+    monkeypatch.setattr(_lib, "_lib", None)
+    monkeypatch.setattr(_lib, "LIB_PATH", fake_path)
+    f = C.CDLL(fake_path)
+    f.fake_limits.argtypes = [C.c_size_t, C.c_size_t]
+    f.fake_counts.argtypes = [C.c_int, C.c_ulonglong]
+    for name in ("fake_device_used", "fake_host_used"):
+        getattr(f, name).restype = C.c_size_t
+    f.fake_fail_copies.argtypes = [C.c_long]
+    for name in ("fake_device_mallocs", "fake_launched"):
+        getattr(f, name).restype = C.c_long
+    f.fake_reset()
+    yield f
+    f.fake_reset()
+
+
+def _engine(max_nr_spots=15, **kw):
+    return Engine(P.parse_params_text(synth.params_text(nr_px=(64, 64), max_nr_spots=max_nr_spots, **kw)))
+
+
+def _db_size(e):
+    n, s = C.c_uint64(0), C.c_int32(0)
+    _lib.check(_lib.lib().lmb_db_info(e._h, C.byref(n), C.byref(s)))
+    return n.value
+
+
+def _records(n, S=15):
+    return np.random.default_rng(n).integers(0, 60, (n, 1 + 2 * S), dtype=np.uint16)
+
+
+def test_failed_upload_leaves_no_records(fake):
+    with _engine() as e:
+        e.upload_db(_records(100_000))
+        assert _db_size(e) == 100_000
+        fake.fake_fail_copies(MIB)
+        with pytest.raises(_lib.LmbError):
+            e.upload_db(_records(90_000))
+        assert _db_size(e) == 0
+        fake.fake_fail_copies(0)
+        rec = _records(80_000)
+        e.upload_db(rec)
+        assert _db_size(e) == 80_000 and np.array_equal(e.download_db(), rec)
+
+
+@pytest.mark.parametrize("what", ["spots", "copy", "kernel"])
+def test_failed_build_leaves_no_records(fake, what):
+    """More spots per record than a build takes, a failing copy, a failing launch."""
+    om, hk = synth.shoemake_orientations(50_000, 1), synth.hkls_cubic(4)
+    with _engine(1281 if what == "spots" else 15) as e:
+        if what != "spots":
+            e.build_db(om[:30_000], hk)
+            assert _db_size(e) == 30_000
+        else:
+            e.upload_db(_records(1000, 1281))
+        fake.fake_fail_copies(MIB if what == "copy" else 0)
+        fake.fake_fail_kernel(b"dbbuild_kernel" if what == "kernel" else b"")
+        with pytest.raises(_lib.LmbError):
+            e.build_db(om, hk)
+        assert _db_size(e) == 0
