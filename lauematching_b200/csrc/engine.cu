@@ -1391,9 +1391,9 @@ int lmb_match(lmb_engine *e, uint64_t slot_mask, int32_t min_nr_spots, double mi
     LMB_CUDA(cudaStreamWaitEvent(e->st, e->ev_load[e->slot_load[k]], 0));
   }
   e->fresh_mask &= ~slot_mask;
-  // The pass (status reset, compare, ordering, ) replays from
-  // a CUDA graph once a configuration has been seen before; the first pass of
-  // a configuration runs eagerly (it also sets the kernels' attributes).
+  // The pass (compare, ordering) replays from a CUDA graph once a configuration
+  // has been seen before; the first pass of a configuration runs eagerly (it also
+  // sets the kernels' attributes).
   PassKey key;
   key.mask = slot_mask;
   key.min_spots = min_nr_spots;
@@ -1430,7 +1430,10 @@ int lmb_match(lmb_engine *e, uint64_t slot_mask, int32_t min_nr_spots, double mi
       e->graphs.push_back(PassGraph{key, nullptr});
     }
     rc = enqueue_pass(e, key, false);
-    if (rc) return rc;
+    if (rc) {  // what has run of it must not count in the slots' next pass
+      cudaMemsetAsync(e->d_status, 0, 2 * LMB_MAX_SLOTS * sizeof(unsigned int), e->st);
+      return rc;
+    }
   }
   const int v = (int)(e->pass_seq % kEventRing);
   LMB_CUDA(cudaEventRecord(e->ev_pass[v], e->st));

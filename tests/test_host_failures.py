@@ -110,3 +110,20 @@ def test_failed_build_leaves_no_records(fake, what):
         with pytest.raises(_lib.LmbError):
             e.build_db(om, hk)
         assert _db_size(e) == 0
+
+
+def test_failed_pass_leaves_no_counts(fake):
+    """A pass whose ordering cannot be launched: what its counting kernel found is not
+    added to by the next pass."""
+    fake.fake_counts(9, 1000)
+    with _engine(min_nr_spots=5) as e:
+        e.upload_db(_records(1000))
+        e.load_image(0, np.ones(64 * 64))
+        fake.fake_survivors(3)
+        fake.fake_fail_kernel(b"order_kernel")
+        with pytest.raises(_lib.LmbError):
+            e.match([0], 5, 1.0)
+        fake.fake_fail_kernel(b"")
+        e.match([0], 5, 1.0)
+        assert fake.fake_launched(b"listed_kernel") == 2
+        assert len(e.results(0)[0]) == 3
