@@ -223,6 +223,13 @@ void drop_graphs(lmb_engine *e) {
   e->graphs.clear();
 }
 
+// Device memory that only speeds up a later use: what a failing allocation may have.
+void give_back(lmb_engine *e) {
+  free_grouped(e);
+  e->om.free();
+  cudaGetLastError();
+}
+
 // Room for the float64 copy of `slot`: the command line keeps one frame (33 MB at
 // 2048^2), all 64 slots take 2.1 GB.
 int ensure_f64(lmb_engine *e, int slot) {
@@ -354,7 +361,15 @@ int alloc_db(lmb_engine *e, uint64_t n) {
     cudaFree(e->d_db);
     e->d_db = nullptr;
     e->db_cap = 0;
-    LMB_CUDA(cudaMalloc(&e->d_db, alloc));
+    cudaError_t ce = cudaMalloc(&e->d_db, alloc);
+    if (ce == cudaErrorMemoryAllocation) {  // the old DB's list and codes are in its way
+      give_back(e);
+      ce = cudaMalloc(&e->d_db, alloc);
+    }
+    if (ce != cudaSuccess) {
+      e->d_db = nullptr;
+      return cuda_fail(ce, "cudaMalloc(DB)", __FILE__, __LINE__);
+    }
     e->db_cap = alloc;
   }
   // the padding behind the records is zero; the caller writes every record, and sets n
@@ -622,11 +637,21 @@ int build_grouped(lmb_engine *e) {
   const uint64_t n = e->n, nt = glist_tiles(n);
   const size_t hist_bytes = 256 * sizeof(unsigned long long);
   // histogram, per-tile counts, counts
-  cudaError_t ce = e->b_aux.need(hist_bytes + nt * 256 * sizeof(uint32_t) + n);
-  if (ce == cudaSuccess) ce = e->b_perm.need(glist_places(n) * sizeof(uint32_t));
+  const size_t aux_bytes = hist_bytes + nt * 256 * sizeof(uint32_t) + n;
+  const size_t perm_bytes = glist_places(n) * sizeof(uint32_t);
+  auto need = [&] {
+    const cudaError_t ce = e->b_aux.need(aux_bytes);
+    return ce == cudaSuccess ? e->b_perm.need(perm_bytes) : ce;
+  };
+  cudaError_t ce = need();
+  if (ce == cudaErrorMemoryAllocation) {  // an earlier DB's codes may hold it
+    give_back(e);
+    e->gl_state = -1;
+    ce = need();
+  }
   if (ce != cudaSuccess) {
-    cudaGetLastError();
-    e->b_aux.free();
+    give_back(e);
+    e->gl_state = -1;
     return ce == cudaErrorMemoryAllocation ? LMB_OK
                                            : cuda_fail(ce, "grouped records", __FILE__, __LINE__);
   }
@@ -964,7 +989,12 @@ static int db_build_common(lmb_engine *e, const double *orients, uint64_t seed, 
       std::min<uint64_t>(256ull << 10, std::max<uint64_t>(32ull << 10, (n / 3 + 127) / 128 * 128 + 128));
   const uint64_t step = synthetic ? 2 * kChunk : kChunk;
   cudaEvent_t up[2] = {}, used[2] = {};
-  cudaError_t ce = e->om.need((size_t)std::min(2 * kChunk, std::max<uint64_t>(n, 1)) * 72);
+  const size_t om_bytes = (size_t)std::min(2 * kChunk, std::max<uint64_t>(n, 1)) * 72;
+  cudaError_t ce = e->om.need(om_bytes);
+  if (ce == cudaErrorMemoryAllocation) {
+    give_back(e);
+    ce = e->om.need(om_bytes);
+  }
   for (int b = 0; b < 2 && ce == cudaSuccess && !synthetic; b++) {
     ce = cudaEventCreateWithFlags(&up[b], cudaEventDisableTiming);
     if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&used[b], cudaEventDisableTiming);

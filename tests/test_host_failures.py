@@ -127,3 +127,39 @@ def test_failed_pass_leaves_no_counts(fake):
         e.match([0], 5, 1.0)
         assert fake.fake_launched(b"listed_kernel") == 2
         assert len(e.results(0)[0]) == 3
+
+
+def _filtered(fake, e, n):
+    """A DB of n records of 15 spots each and a filtered pass over it."""
+    fake.fake_reset()
+    fake.fake_counts(15, n)
+    e.upload_db(_records(n))
+    e.load_image(0, np.ones(64 * 64))
+    e.match([0], 5, 1.0)
+    assert fake.fake_launched(b"group_filter_kernel") == 1
+
+
+@pytest.mark.parametrize("how", ["upload", "build", "first pass"])
+def test_memory_kept_for_the_next_db_is_given_back_when_it_does_not_fit(fake, how):
+    """List, codes and candidates of the old DB (some 40 of its 62 bytes a record) are
+    no reason for a new one not to fit, nor for a build's matrices or a new list."""
+    n = 1_000_000
+    with _engine(min_nr_spots=5) as e:
+        base = fake.fake_device_used()
+        _filtered(fake, e, n if how != "first pass" else n // 3)
+        if how == "upload":
+            rec = _records(n * 6 // 5)
+            fake.fake_limits(base + rec.nbytes + MIB, 1 << 40)
+            e.upload_db(rec)
+            assert _db_size(e) == len(rec) and np.array_equal(e.download_db(), rec)
+        elif how == "build":
+            fake.fake_limits(fake.fake_device_used() + 10 * MIB, 1 << 40)
+            e.build_db(synth.shoemake_orientations(n - 5, 1), synth.hkls_cubic(2))
+            assert _db_size(e) == n - 5
+        else:  # the list of a longer DB, the old one's codes in its way
+            e.upload_db(_records(n))
+            fake.fake_limits(fake.fake_device_used() + MIB, 1 << 40)
+            fake.fake_counts(15, 0)
+            fake.fake_counts(1, n)
+            e.match([0], 5, 1.0)
+            assert e.layout_info()["compact"] == 1 and e.layout_info()["tiles"] == 0
