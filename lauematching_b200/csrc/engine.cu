@@ -531,6 +531,11 @@ constexpr uint64_t kCellTileBytes = 8192;
 int build_compact(lmb_engine *e, int min_spots) {
   e->cl_state = -1;
   if (e->S > 255 || e->n == 0) return LMB_OK;  // counts are uint8
+  if (e->gl_state != 1) {  // what an earlier DB left is of no use to this pass
+    const int state = e->gl_state;
+    give_back(e);
+    e->gl_state = state;
+  }
   const uint64_t n = e->n, nch = (n + 31) / 32;
   uint32_t *d_aux = nullptr;  // chunk spots, then 4 arrays of the packing; count histogram
   LMB_CUDA(cudaMalloc(&d_aux, nch * 4 * 4 + 256 * sizeof(unsigned long long)));

@@ -139,10 +139,11 @@ def _filtered(fake, e, n):
     assert fake.fake_launched(b"group_filter_kernel") == 1
 
 
-@pytest.mark.parametrize("how", ["upload", "build", "first pass"])
+@pytest.mark.parametrize("how", ["upload", "build", "first pass", "tiled layout"])
 def test_memory_kept_for_the_next_db_is_given_back_when_it_does_not_fit(fake, how):
     """List, codes and candidates of the old DB (some 40 of its 62 bytes a record) are
-    no reason for a new one not to fit, nor for a build's matrices or a new list."""
+    no reason for a new one not to fit, nor for a build's matrices, a new list or a
+    tiled layout."""
     n = 1_000_000
     with _engine(min_nr_spots=5) as e:
         base = fake.fake_device_used()
@@ -156,6 +157,12 @@ def test_memory_kept_for_the_next_db_is_given_back_when_it_does_not_fit(fake, ho
             fake.fake_limits(fake.fake_device_used() + 10 * MIB, 1 << 40)
             e.build_db(synth.shoemake_orientations(n - 5, 1), synth.hkls_cubic(2))
             assert _db_size(e) == n - 5
+        elif how == "tiled layout":  # chunk counts: 16 bytes per 32 records
+            e.upload_db(_records(n))
+            fake.fake_limits(fake.fake_device_used(), 1 << 40)
+            e.set_tuning(variant=2)
+            e.match([0], 5, 1.0)
+            assert e.get_tuning()["last_variant"] == 2
         else:  # the list of a longer DB, the old one's codes in its way
             e.upload_db(_records(n))
             fake.fake_limits(fake.fake_device_used() + MIB, 1 << 40)
