@@ -124,6 +124,7 @@ struct lmb_engine {
     int c;
   };
   std::vector<Bucket> gl_tab;
+  int gl_filter = 0;  // 0 not tried, 1 built, -1 this DB goes without
   uint32_t *d_codes = nullptr;
   uint16_t *d_group_mask = nullptr;
   uint32_t *d_cand = nullptr, *d_cand_cnt = nullptr;
@@ -200,6 +201,7 @@ void drop_grouped(lmb_engine *e) {
   e->d_codes = nullptr;
   e->d_cand = nullptr;
   e->gl_tab.clear();
+  e->gl_filter = 0;
   e->gl_state = 0;
   e->gl_qs = 0;
   e->gl_bytes = 0;
@@ -690,10 +692,12 @@ int build_grouped(lmb_engine *e) {
 }
 
 // What variant 5 needs besides the grouped records: buckets, cell codes, mask
-// and room for every record as a candidate (4 bytes each).  false: no memory.
+// and room for every record as a candidate (4 bytes each).  false: no memory (tried
+// once for each DB).
 int ensure_filter(lmb_engine *e, bool *ok) {
-  *ok = e->d_codes != nullptr;
-  if (*ok) return LMB_OK;
+  *ok = e->gl_filter == 1;
+  if (e->gl_filter != 0) return LMB_OK;
+  e->gl_filter = -1;
   e->cells = group_cells(e->geo.nr_px_x, e->geo.nr_px_y);
   e->gl_tab.clear();
   uint32_t chunk = 0;
@@ -727,12 +731,15 @@ int ensure_filter(lmb_engine *e, bool *ok) {
   if (ce != cudaSuccess || rc) {
     e->d_cand = nullptr;
     e->d_codes = nullptr;
+    e->b_cand.free();
+    e->b_codes.free();
     if (rc) return rc;
     if (ce != cudaErrorMemoryAllocation) return cuda_fail(ce, "cell codes", __FILE__, __LINE__);
     cudaGetLastError();
     return LMB_OK;
   }
   e->gl_bytes += code * sizeof(uint32_t);
+  e->gl_filter = 1;
   *ok = true;
   return LMB_OK;
 }

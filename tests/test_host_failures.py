@@ -170,3 +170,26 @@ def test_memory_kept_for_the_next_db_is_given_back_when_it_does_not_fit(fake, ho
             fake.fake_counts(1, n)
             e.match([0], 5, 1.0)
             assert e.layout_info()["compact"] == 1 and e.layout_info()["tiles"] == 0
+
+
+def test_filter_without_memory_is_tried_once(fake):
+    """No room for the codes: the passes run over the list, without asking again and
+    without holding the candidates' memory; the next DB is tried anew."""
+    n = 1_000_000
+    with _engine(min_nr_spots=5) as e:
+        fake.fake_counts(15, n)
+        e.upload_db(_records(n))
+        e.load_image(0, np.ones(64 * 64))
+        before = fake.fake_device_used()
+        fake.fake_limits(before + 12 * MIB, 1 << 40)
+        e.match([0], 5, 1.0)
+        used, tried = fake.fake_device_used(), fake.fake_device_mallocs()
+        for ms in (5, 5, 5, 6):
+            e.match([0], ms, 1.0)
+        assert fake.fake_device_mallocs() == tried and fake.fake_launched(b"group_filter") == 0
+        assert fake.fake_launched(b"listed_kernel") >= 3
+        fake.fake_limits(fake.fake_device_used() + 100 * MIB, 1 << 40)
+        e.upload_db(_records(n))
+        e.match([0], 5, 1.0)
+        assert fake.fake_launched(b"group_filter_kernel") == 1
+        assert used - before < 6 * MIB  # list and counts 5.3 MB, candidates 4.2 MB
