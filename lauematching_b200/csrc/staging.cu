@@ -42,21 +42,30 @@ Staging::~Staging() {
   }
 }
 
-int Staging::ready() {
+bool Staging::ready() {
   for (int i = 0; i < kPieces; i++) {
-    if (!buf_[i]) LMB_CUDA(cudaHostAlloc(&buf_[i], kPiece, cudaHostAllocDefault));
-    if (!ev_[i]) LMB_CUDA(cudaEventCreateWithFlags(&ev_[i], cudaEventDisableTiming));
+    cudaError_t e = cudaSuccess;
+    if (!buf_[i]) {
+      e = cudaHostAlloc(&buf_[i], kPiece, cudaHostAllocDefault);
+      if (e != cudaSuccess) buf_[i] = nullptr;
+    }
+    if (e == cudaSuccess && !ev_[i]) {
+      e = cudaEventCreateWithFlags(&ev_[i], cudaEventDisableTiming);
+      if (e != cudaSuccess) ev_[i] = nullptr;
+    }
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
   }
-  return LMB_OK;
+  return true;
 }
 
 int Staging::upload(void *dst, const void *src, size_t bytes, cudaStream_t st) {
-  if (bytes <= kDirect || page_locked(src)) {
+  if (bytes <= kDirect || page_locked(src) || !ready()) {
     LMB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
     return LMB_OK;
   }
-  int rc = ready();
-  if (rc) return rc;
   for (size_t at = 0; at < bytes; at += kPiece) {
     const size_t len = std::min(kPiece, bytes - at);
     const int b = next_;
@@ -70,13 +79,12 @@ int Staging::upload(void *dst, const void *src, size_t bytes, cudaStream_t st) {
 }
 
 int Staging::download(void *dst, const void *src, size_t bytes, cudaStream_t st) {
-  if (bytes <= kDirect || page_locked(dst)) {
+  if (bytes <= kDirect || page_locked(dst) || !ready()) {
     LMB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
     LMB_CUDA(cudaStreamSynchronize(st));
     return LMB_OK;
   }
-  int rc = ready();
-  if (rc) return rc;
+  int rc = LMB_OK;
   const size_t n = (bytes + kPiece - 1) / kPiece;
   auto piece = [&](size_t i) { return std::min(kPiece, bytes - i * kPiece); };
   auto fetch = [&](size_t i) -> int {

@@ -22,7 +22,7 @@ class Staging {
  private:
   static constexpr int kPieces = 4;
   static constexpr size_t kPiece = 8ull << 20;
-  int ready();
+  bool ready();  // false: no page-locked memory to be had, the copy goes directly
   void *buf_[kPieces] = {};
   cudaEvent_t ev_[kPieces] = {};
   int next_ = 0;

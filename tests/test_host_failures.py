@@ -14,6 +14,7 @@ from lauematching_b200 import _lib, build
 from lauematching_b200 import params as P
 from lauematching_b200 import synth
 from lauematching_b200.engine import Engine
+from lauematching_b200.preprocess import DevicePreprocessor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 MIB = 1 << 20
@@ -193,3 +194,22 @@ def test_filter_without_memory_is_tried_once(fake):
         e.match([0], 5, 1.0)
         assert fake.fake_launched(b"group_filter_kernel") == 1
         assert used - before < 6 * MIB  # list and counts 5.3 MB, candidates 4.2 MB
+
+
+@pytest.mark.parametrize("pieces", [0, 1, 3])
+def test_large_copies_go_directly_without_page_locked_pieces(fake, pieces):
+    """Room for none, one or three of the four 8 MiB pieces: records, a background and
+    a preprocessed frame move all the same."""
+    with _engine() as e:
+        fake.fake_limits(1 << 50, fake.fake_host_used() + pieces * 8 * MIB)
+        rec = _records(700_000)
+        e.upload_db(rec)
+        assert np.array_equal(e.download_db(), rec)
+    fake.fake_reset()
+    ny, nx = 1100, 1001
+    h = DevicePreprocessor(ny, nx)
+    fake.fake_limits(1 << 50, fake.fake_host_used() + pieces * 8 * MIB)
+    bg = np.random.default_rng(1).random((ny, nx))
+    h.set_background(bg)
+    assert np.array_equal(h.background(), bg)
+    h.close()
