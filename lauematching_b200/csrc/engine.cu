@@ -149,6 +149,7 @@ struct lmb_engine {
   unsigned int *d_status = nullptr;
   unsigned int *h_status = nullptr;  // pinned, kStatusWords
   lmb_survivor *h_list = nullptr;         // pinned: [64][kHostList], short lists of each slot
+  bool lists_tried = false;
   uint64_t pass_seq = 0;                  // passes enqueued so far
   uint64_t done_mask = 0;                 // slots that have been in a pass
   cudaStream_t dl = nullptr;              // survivor downloads
@@ -255,6 +256,19 @@ int ensure_f64(lmb_engine *e, int slot) {
   e->f64_slots = want;
   return LMB_OK;
 }
+
+// Room for the passes' short lists (8 MiB), made for the first pass: an engine that
+// only builds records needs none.  Without it every list is fetched from the device.
+void ensure_lists(lmb_engine *e) {
+  if (e->lists_tried) return;
+  e->lists_tried = true;
+  if (cudaHostAlloc(&e->h_list, (size_t)LMB_MAX_SLOTS * kHostList * sizeof(lmb_survivor),
+                    cudaHostAllocDefault) == cudaSuccess)
+    return;
+  e->h_list = nullptr;
+  cudaGetLastError();
+}
+uint32_t host_list_cap(const lmb_engine *e) { return e->h_list ? std::min(kHostList, e->cap) : 0u; }
 
 // Slots about to be written on the load stream: after the last passes that read
 // them.
@@ -849,7 +863,7 @@ int enqueue_pass(lmb_engine *e, const PassKey &k, bool capturing) {
   o.scratch = e->d_scratch;
   o.cap2 = e->cap2;
   o.host_list = e->h_list;
-  o.host_cap = std::min(kHostList, e->cap);
+  o.host_cap = host_list_cap(e);
   o.host_status = e->h_status;
   o.status = e->d_status;
   for (int i = 0; i < LMB_MAX_SLOTS; i++)
@@ -949,8 +963,6 @@ int lmb_engine_create(int32_t device, const lmb_geometry *geo, uint64_t survivor
   TRY(cudaHostAlloc(&e->h_status, kStatusWords * sizeof(unsigned int),
                     cudaHostAllocDefault));
   memset(e->h_status, 0, kStatusWords * sizeof(unsigned int));
-  TRY(cudaHostAlloc(&e->h_list, (size_t)LMB_MAX_SLOTS * kHostList * sizeof(lmb_survivor),
-                    cudaHostAllocDefault));
 #undef TRY
   *out = e;
   return LMB_OK;
@@ -1426,6 +1438,7 @@ int lmb_match(lmb_engine *e, uint64_t slot_mask, int32_t min_nr_spots, double mi
       tun = CompareTuning{1, 0, 0, 0, 0, 0, tun.full_gather, tun.test_consumer_wait_us, 0, 0, 0};
   }
   e->last_variant = tun.variant;
+  ensure_lists(e);
   uint64_t waited = 0;
   for (int k = 0; k < LMB_MAX_SLOTS; k++) {
     if (!((slot_mask & e->fresh_mask) >> k & 1) || (waited >> e->slot_load[k] & 1)) continue;
@@ -1513,7 +1526,6 @@ int slot_status(lmb_engine *e, int slot, const unsigned int **st, uint64_t *wait
 }
 
 // A slot's list in host memory, when its pass wrote it there.
-uint64_t host_list_cap(const lmb_engine *e) { return std::min(kHostList, e->cap); }
 const lmb_survivor *host_list(const lmb_engine *e, int slot) {
   return e->h_list + (size_t)slot * host_list_cap(e);
 }

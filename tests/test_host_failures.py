@@ -213,3 +213,23 @@ def test_large_copies_go_directly_without_page_locked_pieces(fake, pieces):
     h.set_background(bg)
     assert np.array_equal(h.background(), bg)
     h.close()
+
+
+@pytest.mark.parametrize("room", [True, False])
+def test_room_for_short_lists_comes_with_the_first_pass(fake, room):
+    """An engine that only builds locks no 8 MiB of host memory; without them a list
+    is fetched from the device."""
+    fake.fake_counts(9, 1000)
+    host = fake.fake_host_used()
+    with _engine(min_nr_spots=5) as e:
+        e.build_db(synth.shoemake_orientations(1000, 1), synth.hkls_cubic(2))
+        e.download_db()
+        assert fake.fake_host_used() - host < MIB
+        e.load_image(0, np.ones(64 * 64))
+        fake.fake_survivors(3)
+        if not room:
+            fake.fake_limits(1 << 50, fake.fake_host_used())
+        for _ in range(2):
+            e.match([0], 5, 1.0)
+            assert len(e.results(0)[0]) == 3 and len(e.results_batch([0])[0][0]) == 3
+            fake.fake_limits(1 << 50, 1 << 50)
