@@ -750,21 +750,19 @@ __device__ __forceinline__ void value_hist_whole(const T *__restrict__ raw, cons
 }
 
 // Subtraction fused with the value histogram (see above); the differences are
-// kept as 16-bit values.  Each block counts values below kVhLocal in shared
-// memory (runs of equal values in registers) and adds larger ones straight into
-// the global 65536-bin histogram.  A frame with another value leaves the value
-// path: its threshold is infinite, so nothing follows from the 16-bit values, and
-// the host starts again with the radix selection.  *bg_other = 0: the background
-// is whole numbers too and read as bg16; with 8- and 16-bit frames all of it is
-// integers then.  Measured on B200 (cold caches), 2048^2
-// uint16 frame: 70.7 us with the background and the differences as float64 and the
-// last block's search over all 65536 bins in global memory, 34.3 us with one pixel
-// at a time in float64; in integers the whole threshold stage takes 36-43 us
-// instead of 49-50 (a frame into its slot 333 -> 322 us).
+// kept as 16-bit values.  The background is whole numbers (bg16).  Each block counts
+// values below kVhLocal in shared memory (runs of equal values in registers) and
+// adds larger ones straight into the global 65536-bin histogram.  8- and 16-bit
+// frames have whole differences, all of it is integers; a float frame with another
+// value leaves the value path, and the host takes the radix selection.  Measured on
+// B200 (cold caches), 2048^2 uint16 frame: 70.7 us with the background and the
+// differences as float64 and the last block's search over all 65536 bins in global
+// memory, 34.3 us with one pixel at a time in float64; in integers the whole
+// threshold stage takes 36-43 us instead of 49-50 (a frame into its slot 333 -> 322
+// us).
 template <typename T>
 __global__ void __launch_bounds__(kVhThreads, 4)
-    value_hist_kernel(const T *__restrict__ raw, const double *__restrict__ bg,
-                      const uint16_t *__restrict__ bg16, const unsigned *__restrict__ bg_other,
+    value_hist_kernel(const T *__restrict__ raw, const uint16_t *__restrict__ bg16,
                       uint16_t *__restrict__ sub16, unsigned n, PreState *st, unsigned *g16, int mode,
                       unsigned long long k0, int two, double gamma) {
   __shared__ unsigned h[kVhLocal];
@@ -776,41 +774,38 @@ __global__ void __launch_bounds__(kVhThreads, 4)
   DigitRun run;  // bins below kVhLocal
   bool nonint = false;
   unsigned most = 0;
-  const bool whole_bg = *bg_other == 0u;
-  bool counted = false;
-  if constexpr (std::is_same_v<T, uint16_t> || std::is_same_v<T, uint8_t>)
-    if (whole_bg) {
-      value_hist_whole(raw, bg16, sub16, n, g16, mode, h, run, most);
-      counted = true;
-    }
-  constexpr int U = 8;
-  const unsigned stride = gridDim.x * blockDim.x;
-  const unsigned rounds = counted ? 0u : (n + stride * U - 1) / (stride * U);
-  for (unsigned it = 0; it < rounds; ++it) {
-    double v[U];
-    bool in[U];
+  if constexpr (std::is_same_v<T, uint16_t> || std::is_same_v<T, uint8_t>) {
+    value_hist_whole(raw, bg16, sub16, n, g16, mode, h, run, most);
+  } else {
+    constexpr int U = 8;
+    const unsigned stride = gridDim.x * blockDim.x;
+    const unsigned rounds = (n + stride * U - 1) / (stride * U);
+    for (unsigned it = 0; it < rounds; ++it) {
+      double v[U];
+      bool in[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const unsigned i = (it * U + u) * stride + blockIdx.x * blockDim.x + threadIdx.x;
-      in[u] = i < n;
-      v[u] = 0.0;
-      if (in[u]) {
-        const double d = lmb::dsub(to_f64(raw[i]), whole_bg ? (double)bg16[i] : bg[i]);
-        v[u] = (d >= 0.0 || isnan(d)) ? d : 0.0;
-        sub16[i] = (uint16_t)((unsigned)x86_trunc_i32(v[u]) & 0xFFFFu);
+      for (int u = 0; u < U; ++u) {
+        const unsigned i = (it * U + u) * stride + blockIdx.x * blockDim.x + threadIdx.x;
+        in[u] = i < n;
+        v[u] = 0.0;
+        if (in[u]) {
+          const double d = lmb::dsub(to_f64(raw[i]), (double)bg16[i]);
+          v[u] = (d >= 0.0 || isnan(d)) ? d : 0.0;
+          sub16[i] = (uint16_t)((unsigned)x86_trunc_i32(v[u]) & 0xFFFFu);
+        }
       }
-    }
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (!in[u] || !(mode == SEL_ALL || v[u] > 0.0)) continue;
-      const double x = v[u];
-      if (x == trunc(x) && x <= 65535.0 && !signbit(x)) {
-        const unsigned b = (unsigned)x;
-        most = max(most, b);
-        if (b < (unsigned)kVhLocal) run.add(h, b);
-        else atomicAdd(g16 + b, 1u);
-      } else {
-        nonint = true;  // also NaN: every comparison with it is false
+      for (int u = 0; u < U; ++u) {
+        if (!in[u] || !(mode == SEL_ALL || v[u] > 0.0)) continue;
+        const double x = v[u];
+        if (x == trunc(x) && x <= 65535.0 && !signbit(x)) {
+          const unsigned b = (unsigned)x;
+          most = max(most, b);
+          if (b < (unsigned)kVhLocal) run.add(h, b);
+          else atomicAdd(g16 + b, 1u);
+        } else {
+          nonint = true;  // also NaN: every comparison with it is false
+        }
       }
     }
   }
@@ -832,10 +827,7 @@ __global__ void __launch_bounds__(kVhThreads, 4)
       vh_finish(st, g16, h, top, mode, k0, two, gamma);
     } else {  // leave an empty histogram for the radix selection
       for (int b = threadIdx.x; b <= top; b += kVhThreads) g16[b] = 0u;
-      if (threadIdx.x == 0) {
-        st->thresh = __longlong_as_double(0x7ff0000000000000ll);
-        st->value_path = 0;
-      }
+      if (threadIdx.x == 0) st->value_path = 0;
     }
     if (threadIdx.x == 0) {
       st->blocks_done = 0;
@@ -1880,7 +1872,8 @@ struct lmb_pre {
   unsigned *d_bits = nullptr;  // first-block maps (all, kept) and their segments' counts
   unsigned nwords = 0, seg_len = 4;
   uint16_t *d_sub16 = nullptr, *d_bg16 = nullptr;  // whole-number differences, background
-  unsigned *d_bg_other = nullptr;                  // the background is no whole numbers
+  unsigned *d_bg_other = nullptr;                  // the background is no whole numbers,
+  unsigned bg_other = 0;                           // on the host
   uint8_t *d_tiles = nullptr;                      // blur tiles with a positive pixel
   int tiles_x = 1, tiles_y = 1;
   unsigned *d_hist16 = nullptr;  // 65536-bin histogram of the first selection pass
@@ -1999,18 +1992,29 @@ int run_select(lmb_pre *p, int mode, bool first_pass) {
   return LMB_OK;
 }
 
-// Subtraction fused with the value histogram.  Where every candidate is a whole
-// number in [0, 65535] the threshold is set and the state's value_path with it.
-int value_select(lmb_pre *p, int dtype, int mode, unsigned long long k0, int two, double gamma) {
+// Subtraction fused with the value histogram, over a background of whole numbers.
+// *whole: every candidate is a whole number in [0, 65535] and the threshold is set.
+// 8- and 16-bit frames always are; of a float frame the host asks the device.  Not
+// asking, and segmenting again when it was none, gave a fractional frame all the
+// component kernels twice (2048^2 float32 call on B200: 1.23 ms, asking 1.19; a whole
+// frame pays 0.95 -> 0.97).
+int value_select(lmb_pre *p, int dtype, int mode, unsigned long long k0, int two, double gamma,
+                 bool *whole) {
   int rc = by_dtype(dtype, [&](auto tag) {
     using T = std::remove_const_t<std::remove_pointer_t<decltype(tag)>>;
     value_hist_kernel<T><<<(unsigned)(p->num_sms * 4), kVhThreads, 0, p->st>>>(
-        static_cast<const T *>(p->d_raw), p->d_bg, p->d_bg16, p->d_bg_other, p->d_sub16,
-        (unsigned)p->npx, p->d_state, p->d_hist16, mode, k0, two, gamma);
+        static_cast<const T *>(p->d_raw), p->d_bg16, p->d_sub16, (unsigned)p->npx, p->d_state,
+        p->d_hist16, mode, k0, two, gamma);
     return LMB_OK;
   });
   if (rc) return rc;
   LMB_CUDA(cudaGetLastError());
+  *whole = dtype == LMB_U8 || dtype == LMB_U16;
+  if (*whole) return LMB_OK;
+  LMB_CUDA(cudaMemcpyAsync(&p->h_state->value_path, &p->d_state->value_path, sizeof(unsigned),
+                           cudaMemcpyDeviceToHost, p->st));
+  LMB_CUDA(cudaStreamSynchronize(p->st));
+  *whole = p->h_state->value_path != 0;
   return LMB_OK;
 }
 
@@ -2023,12 +2027,15 @@ int subtract(lmb_pre *p, int dtype) {
   });
 }
 
-// The background as 16-bit whole numbers, where it is.
+// The background as 16-bit whole numbers, where it is; h_state->nonint says whether
+// once the stream has been waited for.
 int background_changed(lmb_pre *p) {
   LMB_CUDA(cudaMemsetAsync(p->d_bg_other, 0, sizeof(unsigned), p->st));
   whole_kernel<double><<<(unsigned)grid_for(p->npx, p->num_sms), kT, 0, p->st>>>(
       p->d_bg, p->d_bg16, p->d_bg_other, p->npx);
   LMB_CUDA(cudaGetLastError());
+  LMB_CUDA(cudaMemcpyAsync(&p->h_state->nonint, p->d_bg_other, sizeof(unsigned), cudaMemcpyDeviceToHost,
+                           p->st));
   return LMB_OK;
 }
 
@@ -2294,6 +2301,7 @@ int lmb_pre_destroy(lmb_pre *p) {
 int lmb_pre_set_background(lmb_pre *p, const double *background) {
   int rc = check_pre(p);
   if (rc) return rc;
+  p->bg_other = 1;  // until it has been looked at
   if (background)
     LMB_CUDA(cudaMemcpyAsync(p->d_bg, background, p->npx * sizeof(double), cudaMemcpyHostToDevice,
                              p->st));
@@ -2301,6 +2309,7 @@ int lmb_pre_set_background(lmb_pre *p, const double *background) {
     LMB_CUDA(cudaMemsetAsync(p->d_bg, 0, p->npx * sizeof(double), p->st));
   if ((rc = background_changed(p))) return rc;
   LMB_CUDA(cudaStreamSynchronize(p->st));
+  p->bg_other = p->h_state->nonint;
   return LMB_OK;
 }
 
@@ -2318,6 +2327,7 @@ int lmb_pre_median(lmb_pre *p, const void *frame, int32_t dtype, int32_t size, i
   LMB_REQUIRE(size >= 1, "median size %d", size);
   LMB_REQUIRE(!(p->ny > 1 && size >= 8 * p->ny) && !(p->nx > 1 && size >= 8 * p->nx),
               "median size %d reaches 8x the %d x %d frame", size, p->ny, p->nx);
+  p->bg_other = 1;  // until it has been looked at
   LMB_CUDA(cudaEventRecord(p->ev[EV_MED0], p->st));
   if ((rc = upload_frame(p, frame, dtype))) return rc;
   LMB_CUDA(cudaEventRecord(p->ev[EV_MED_UP], p->st));
@@ -2341,6 +2351,7 @@ int lmb_pre_median(lmb_pre *p, const void *frame, int32_t dtype, int32_t size, i
   if ((rc = background_changed(p))) return rc;
   if (out && (rc = p->staging.download(out, p->d_bg, p->npx * sizeof(double), p->st))) return rc;
   LMB_CUDA(cudaStreamSynchronize(p->st));
+  p->bg_other = p->h_state->nonint;
   if (size > 1 && passes > 0)
     return stage_times(p, EV_MED0, EV_MED_UP, 5) || stage_times(p, EV_MED_PASS, EV_MED_RANK, 6) ||
            stage_times(p, EV_MED_RANK, EV_MED_K, 7);
@@ -2372,10 +2383,12 @@ int lmb_pre_segment(lmb_pre *p, const void *frame, int32_t dtype, const lmb_pre_
                   "Percentiles must be in the range [0, 100]");
       percentile_plan(p->npx, prm->threshold_percentile, &k0, &two, &gamma);
     }
-    // whole-number frames: everything in one go, the state read once at its end
-    if ((rc = value_select(p, dtype, pct ? SEL_ALL : SEL_NZ, k0, two, gamma))) return rc;
-    rc = segment_tail(p, FromSub16{p->d_sub16}, prm->min_area, counts);
-    if (rc == LMB_OK && !p->h_state->value_path) {  // another frame: nothing was segmented
+    bool whole = false;  // a fractional background leaves hardly a whole difference
+    if (!p->bg_other && (rc = value_select(p, dtype, pct ? SEL_ALL : SEL_NZ, k0, two, gamma, &whole)))
+      return rc;
+    if (whole) {
+      rc = segment_tail(p, FromSub16{p->d_sub16}, prm->min_area, counts);
+    } else {
       if ((rc = subtract(p, dtype))) return rc;
       if (pct) {
         sel_init_kernel<<<1, kT, 0, p->st>>>(p->d_state, SEL_ALL, p->npx, k0, two);

@@ -30,7 +30,7 @@ std::map<std::string, long> launched;
 std::string fail_kernel;
 long fail_copies_of = 0;  // copies of at least this many bytes fail (0: none)
 unsigned long long hist[256];
-unsigned survivors = 0;
+unsigned survivors = 0, fractional = 0;
 cudaError_t last = cudaSuccess;
 
 cudaError_t result(cudaError_t e) {
@@ -80,6 +80,8 @@ void act(const std::string &name, void **args) {
     memcpy(*static_cast<unsigned long long **>(args[2]), hist, sizeof(hist));
   } else if (name.find("listed_kernel") != std::string::npos) {  // survivors in slot 0
     static_cast<lmb::CmpArgs *>(args[0])->surv_cnt[0] += survivors;
+  } else if (name.find("whole_kernel") != std::string::npos) {
+    **static_cast<unsigned **>(args[2]) |= fractional;
   } else if (name.find("order_kernel") != std::string::npos && name.find("noalloc") == std::string::npos) {
     const lmb::OrderArgs &a = *static_cast<lmb::OrderArgs *>(args[0]);
     for (int i = 0; i < a.nslots; i++) {
@@ -110,7 +112,7 @@ void fake_reset() {
   fail_kernel.clear();
   fail_copies_of = 0;
   memset(hist, 0, sizeof(hist));
-  survivors = 0;
+  survivors = fractional = 0;
   last = cudaSuccess;
 }
 void fake_limits(size_t device, size_t host) {
@@ -124,6 +126,7 @@ void fake_fail_kernel(const char *part) { fail_kernel = part; }
 void fake_fail_copies(long bytes) { fail_copies_of = bytes; }
 void fake_counts(int count, unsigned long long records) { hist[count] = records; }
 void fake_survivors(unsigned n) { survivors = n; }
+void fake_fractional(unsigned yes) { fractional = yes; }  // frames and backgrounds as 16-bit numbers
 long fake_launched(const char *part) {
   long n = 0;
   for (const auto &k : launched)

@@ -233,3 +233,23 @@ def test_room_for_short_lists_comes_with_the_first_pass(fake, room):
             e.match([0], 5, 1.0)
             assert len(e.results(0)[0]) == 3 and len(e.results_batch([0])[0][0]) == 3
             fake.fake_limits(1 << 50, 1 << 50)
+
+
+@pytest.mark.parametrize("method", ["adaptive", "percentile"])
+@pytest.mark.parametrize("dtype,fractional_bg", [(np.uint16, 0), (np.uint16, 1), (np.uint8, 1),
+                                                 (np.float32, 0), (np.float64, 1)])
+def test_components_are_found_once(fake, method, dtype, fractional_bg):
+    """A frame whose differences are no whole numbers goes to the radix selection
+    before its components are looked for, and over a fractional background without
+    a value histogram."""
+    h = DevicePreprocessor(100, 80)
+    fake.fake_fractional(fractional_bg)
+    h.set_background(np.full((100, 80), 0.5 * fractional_bg))
+    fake.fake_fractional(0)
+    h.segment(np.ones((100, 80), dtype), method=method)
+    assert fake.fake_launched(b"label_kernel") == 1
+    assert fake.fake_launched(b"foreground_kernel") == 1
+    assert fake.fake_launched(b"value_hist_kernel") == 1 - fractional_bg
+    radix = fractional_bg or dtype is np.float32  # the fake leaves the value path unset
+    assert (fake.fake_launched(b"sel_hist_kernel") > 0) == bool(radix)
+    h.close()
