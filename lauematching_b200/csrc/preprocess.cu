@@ -1686,13 +1686,22 @@ __global__ void __launch_bounds__(kMedWarps * 32, 4)
 // halo (in shared memory), and median >= t exactly when that number is at most
 // k = s * s / 2.  A block starts at the median of 256 of its values and moves t by
 // doubling steps, then by halves, until every pixel has count(m) <= k <
-// count(m + 1).  A tile that needs more than kMedTries thresholds (wild values)
-// is counted in *unresolved and the frame takes the rank path.  Bound by
-// instruction issue: about 3 instructions per value of tile and halo and threshold,
-// against 2 s shared-memory atomics per pixel on the rank path.  Measured on B200,
-// 2048^2 detector frame, s = 101: ranks and median 4.50 ms there, 0.26 ms here.
+// count(m + 1): about one threshold for each value among the tile's medians, and a
+// few more.  How many there are shows early: the range of the counts in the tile,
+// divided by what a step of one adds to them.  A tile with more than kMedMost by the
+// thresholds kMedLook and 0 (four times as many by 3 and 0), or one that kMedTries
+// have not resolved, is counted in *unresolved and the frame takes the rank path; other
+// blocks see that when they start and every eight thresholds.  A block's threshold
+// takes 5 to 15 us, mostly latency.  Measured on B200, 2048^2 frames, ranks and median:
+// a detector frame, s = 101, 2.75 ms on the rank path, 0.19 ms here; frames that end on
+// the rank path (a steep background, s = 101; noise of standard deviation 1000, s = 31;
+// random words, s = 31, three passes), whole call: 5.89, 2.96, 15.2 ms there alone,
+// 7.34, 4.05, 18.4 with all 48 thresholds of every tile first, 6.02, 3.06, 15.4 as it
+// is.
 constexpr int kMtX = 64, kMtY = 32, kMtThreads = 256;
 constexpr int kMedTries = 48;
+constexpr int kMedLook = 5;   // the last threshold that the estimate is made from
+constexpr int kMedMost = 40;  // as many values take some 48 thresholds (1.2 each and a few)
 constexpr int kMedTileMaxS = 255;  // a column sum is a byte
 
 size_t median_tile_smem(int s) {
@@ -1702,7 +1711,8 @@ size_t median_tile_smem(int s) {
          (kMtThreads / 32) * (cols + 1) * 4 + kMtThreads * 4;
 }
 
-__global__ void __launch_bounds__(kMtThreads)
+// 48 registers: five blocks an SM where the window leaves room for them.
+__global__ void __launch_bounds__(kMtThreads, 5)
     median_tile_kernel(const uint16_t *__restrict__ img, int ny, int nx, int s, double *__restrict__ out,
                        uint16_t *__restrict__ out16, unsigned *__restrict__ unresolved) {
   extern __shared__ __align__(16) double sm[];  // (declared as the blur's)
@@ -1712,7 +1722,9 @@ __global__ void __launch_bounds__(kMtThreads)
   unsigned *pre_all = reinterpret_cast<unsigned *>(csum + ((size_t)kMtY * cols + 15) / 16 * 16);
   unsigned *sample = pre_all + (kMtThreads / 32) * (cols + 1);
   __shared__ unsigned key_s, guess_s;
+  __shared__ unsigned least_s, most_s, sum_s;  // of the tile's counts below a threshold
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  unsigned lost = t == 0 ? __ldcg(unresolved) : 0u;
   unsigned *pre = pre_all + warp * (cols + 1);
   const int lo = s / 2;
   const int x0 = blockIdx.x * kMtX, y0 = blockIdx.y * kMtY;
@@ -1721,7 +1733,7 @@ __global__ void __launch_bounds__(kMtThreads)
     for (int c = lane; c < cols; c += 32) val[r * cols + c] = src[mirror(x0 - lo + c, nx)];
   }
   if (t == 0) guess_s = 0u;
-  __syncthreads();
+  if (__syncthreads_or(lost != 0u)) return;
   // the median of 256 values spread over tile and halo
   sample[t] = val[(int)((long long)(2 * t + 1) * rows * cols / (2 * kMtThreads))];
   __syncthreads();
@@ -1746,8 +1758,13 @@ __global__ void __launch_bounds__(kMtThreads)
   const int per = (cols + 31) / 32;
   unsigned thr = guess_s;
   unsigned step_up = 1u, step_down = 1u;
+  unsigned thr0 = 0, sum0 = 0;  // the first threshold and its counts
+  float medians = 1e30f;        // estimate of the values among the tile's medians
   bool found = false;
   for (int round = 0; round < kMedTries; round++) {
+    const bool poll = (round & 7) == 7, look = round == 0 || round == 3 || round == kMedLook;
+    if (poll && t == 0) lost = __ldcg(unresolved);
+    unsigned least = 0xffffffffu, largest = 0u, sum_all = 0u;
     if (thr > 0u) {
       // values below thr: column sums of s rows, for every row of the tile
       for (int c = t; c < cols; c += kMtThreads) {
@@ -1761,7 +1778,10 @@ __global__ void __launch_bounds__(kMtThreads)
           csum[r * cols + c] = (unsigned char)n;
         }
       }
-      if (t == 0) key_s = 0xffffffffu;
+      if (t == 0) {
+        key_s = least_s = 0xffffffffu;
+        most_s = sum_s = 0u;
+      }
       __syncthreads();
 #pragma unroll
       for (int q = 0; q < kRows; q++) {
@@ -1791,6 +1811,9 @@ __global__ void __launch_bounds__(kMtThreads)
           const int x = lane + 32 * h;
           const unsigned cnt = pre[x + s] - pre[x];
           const int i = 2 * q + h;
+          least = min(least, cnt);
+          largest = max(largest, cnt);
+          sum_all += cnt;
           if (cnt <= k)
             L[i] = max(L[i], thr);
           else
@@ -1799,7 +1822,10 @@ __global__ void __launch_bounds__(kMtThreads)
         __syncwarp();
       }
     } else {
-      if (t == 0) key_s = 0xffffffffu;
+      if (t == 0) {
+        key_s = least_s = 0xffffffffu;
+        most_s = sum_s = 0u;
+      }
       __syncthreads();
     }
     // the lowest interval still open: its ends say where to look next
@@ -1809,12 +1835,37 @@ __global__ void __launch_bounds__(kMtThreads)
       if (H[i] > L[i] + 1u) key = min(key, (L[i] << 16) | (H[i] - 1u));
     key = __reduce_min_sync(0xffffffffu, key);
     if (lane == 0 && key != 0xffffffffu) atomicMin(&key_s, key);
-    __syncthreads();
-    const unsigned open = key_s;
+    if (look && thr > 0u) {  // uniform in the block
+      least = __reduce_min_sync(0xffffffffu, least);
+      largest = __reduce_max_sync(0xffffffffu, largest);
+      sum_all = __reduce_add_sync(0xffffffffu, sum_all);
+      if (lane == 0) {
+        atomicMin(&least_s, least);
+        atomicMax(&most_s, largest);
+        atomicAdd(&sum_s, sum_all);
+      }
+    }
+    const bool leave = poll ? __syncthreads_or(lost != 0u) : (__syncthreads(), false);
+    const unsigned open = key_s, range = most_s - least_s, sum = sum_s;
     __syncthreads();  // before the next round's reset
     if (open == 0xffffffffu) {
       found = true;
       break;
+    }
+    if (leave) return;
+    if (look && thr > 0u) {
+      if (thr0 == 0u) {
+        thr0 = thr;
+        sum0 = sum;
+      } else if (sum != sum0) {
+        // values among the medians: the range over what a unit of threshold adds.  The
+        // least of the estimates: frames whose values have gaps look wilder the further
+        // the threshold moves without meeting one.
+        const float units = thr > thr0 ? (float)(thr - thr0) : (float)(thr0 - thr);
+        const float added = (sum > sum0 ? (float)(sum - sum0) : (float)(sum0 - sum)) / (kMtX * kMtY);
+        medians = fminf(medians, (float)range * units / added);
+      }
+      if (medians < 1e30f && medians > (float)(round == kMedLook ? kMedMost : 4 * kMedMost)) break;
     }
     const unsigned l = open >> 16, h = (open & 0xFFFFu) + 1u;
     if (l == 0u && h == 65536u) {  // nothing known: only thr = 0 comes here

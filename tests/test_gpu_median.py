@@ -53,3 +53,28 @@ def test_a_detector_frame_matches_scipy_on_a_strip():
     h.close()
     cut = f[:, 900:1100]
     assert np.array_equal(got[:, 950:1050], ndimage.median_filter(cut, 101)[:, 50:150])
+
+
+@pytest.mark.parametrize("size,passes", [(5, 1), (9, 2)])
+def test_frames_given_up_part_of_the_way_match_scipy(size, passes):
+    """More tiles than run at once, of which the first, the last or all are beyond the
+    tiles' thresholds, and values with gaps above and below the first threshold."""
+    ny, nx = 1250, 1500
+    rng = np.random.default_rng(size)
+    smooth = rng.poisson(30, (ny, nx))
+    first, last, second = smooth.copy(), smooth.copy(), smooth.copy()
+    first[:40, :70] = rng.integers(0, 65536, (40, 70))
+    last[-40:, -70:] = rng.integers(0, 65536, (40, 70))
+    second[600:640, ::2] = 50000  # half of the values, then none
+    frames = {"first": first, "last": last, "second": second, "gaps": 16 * smooth,
+              "noise": rng.normal(20000, 1000, (ny, nx)).astype(int),
+              "below": np.where(rng.random((ny, nx)) < 0.5, 3, 60000),
+              "ramp": smooth + 8 * np.arange(nx)}
+    h = PP.DevicePreprocessor(ny, nx)
+    for name, f in frames.items():
+        want = f.astype(np.uint16)
+        for _ in range(passes):
+            want = ndimage.median_filter(want, size)
+        got = h.median(f.astype(np.uint16), size, passes)
+        assert np.array_equal(got, want.astype(np.float64)), name
+    h.close()
