@@ -39,9 +39,13 @@
 // chunks of 384 HKLs instead of 512 (six blocks per SM fit instead of five), 3e7
 // orientations: tilted 60.8 -> 52.6 ms (of them FP64 20, detector test 27 before and
 // about 20 now), hexagonal 13.5 -> 12.1, fcc 8.9 -> 8.0.  Chunks of 256: tilted 59.7
-// where 384 gave 57.9, the lanes' numbers of bits being less equal.  A build flag
-// (exact_all), an orientation that is no rotation, and geometry outside the
-// screens' assumptions take FP64 for every HKL.
+// where 384 gave 57.9, the lanes' numbers of bits being less equal.
+//
+// A matrix that is no rotation (rounded to a few digits, scaled, strained) has
+// another |q| than the list says: its HKLs are all screened one by one, with |q|
+// taken from the matrix.  2e5 matrices of 3 digits, B200, normal / tilted: 1.6 / 2.0
+// ms, 4.6 / 5.0 with FP64 for every HKL.  A build flag (exact_all) and geometry
+// outside the screens' assumptions take FP64 for every HKL.
 //
 // Layout.  Blocks of TB orientations; accepted pixels live in shared memory as
 // [spot][thread] so the de-duplication scan is bank-conflict free; the block's
@@ -67,6 +71,7 @@ struct BuildGeo {
   // d = (-2 q_z) u + rt2, u = detector rotation . q: X = a x / tol = q_z (su u_x) + c and
   // the frame's edges as X + b0 z > 0, X + b1 z < 0 (b / tol), the same for y; z itself
   float sux, suy, cx2, cy2, cz2, bx0, bx1, by0, by1;
+  float hc, elof, ehif;  // hc / 4 pi and the energies, for matrices that are no rotations
 };
 
 static constexpr double kHcKeVnm = 1.2398419739;              // LaueMatchingHeaders.h:41
@@ -118,9 +123,13 @@ __device__ __forceinline__ bool exact_spot(const double T[9], const int4 hk, con
   return true;
 }
 
+constexpr float kUnitErr = 256.f / 16777216.f;  // BuildUnits::eps: this times sum |column| |h| / |q|
+constexpr float kUnitErr0 = 4e-6f;              // ... and this
+
 template <bool kExactAll>
 __global__ void __launch_bounds__(128, 6) dbbuild_kernel(const double *__restrict__ om, uint64_t n,
-                                                      const int4 *__restrict__ hkl, int nh,
+                                                      const int4 *__restrict__ hkl,
+                                                      const float4 *__restrict__ hklf, int nh,
                                                       const int4 *__restrict__ seen, int nseen,
                                                       const BuildUnits *__restrict__ units,
                                                       const uint32_t *__restrict__ unit_count,
@@ -187,8 +196,70 @@ __global__ void __launch_bounds__(128, 6) dbbuild_kernel(const double *__restric
     sh_list[(size_t)cnt * TB + t] = key;
     done = ++cnt == g.S;
   };
-  if (kExactAll || !regular) {
+  // The detector screen of a unit reflection vector (q_z, and u scaled as in BuildGeo)
+  // with error m; nothing is off when m is NaN.
+  auto off_detector = [&](float qz, float u0, float u1, float u2, float m) {
+    const float x = fmaf(qz, u0, g.cx2), y = fmaf(qz, u1, g.cy2), z = fmaf(qz, u2, g.cz2);
+    return z < -m || fmaf(g.bx0, z, x) < -m || fmaf(g.bx1, z, x) > m || fmaf(g.by0, z, y) < -m ||
+           fmaf(g.by1, z, y) > m;
+  };
+  if (kExactAll) {
     for (int i = 0; i < nh && !done; i++) take(__ldg(hkl + i));
+    done = true;
+  } else if (!regular) {
+    // No rotation: the whole list, a chunk's worth of bits at a time, with |q| from the
+    // matrix.  Not a number anywhere: nothing is rejected.
+    float col[3];
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+      col[j] = 1.00001f * (float)sqrt(T[j] * T[j] + T[3 + j] * T[3 + j] + T[6 + j] * T[6 + j]);
+    const float a0 = (float)T[0], a1 = (float)T[1], a2 = (float)T[2];
+    const float b0 = (float)T[3], b1 = (float)T[4], b2 = (float)T[5];
+    float qz, rq, m;  // of an HKL: q_z and 1 / |q|, error of the unit vector
+    auto reflect = [&](const float4 h) {
+      qz = fmaf(t0, h.x, fmaf(t1, h.y, t2 * h.z));
+      const float qx = fmaf(a0, h.x, fmaf(a1, h.y, a2 * h.z)), qy = fmaf(b0, h.x, fmaf(b1, h.y, b2 * h.z));
+      const float ql2 = fmaf(qx, qx, fmaf(qy, qy, qz * qz));
+      rq = ql2 > 1e-20f && ql2 < 1e20f ? rsqrtf(ql2) : __int_as_float(0x7fc00000);
+      const float sum = fmaf(col[0], fabsf(h.x), fmaf(col[1], fabsf(h.y), col[2] * fabsf(h.z)));
+      m = fmaf(kUnitErr, sum * rq, kUnitErr0);
+      return ql2 * rq;
+    };
+    for (int c0 = 0; c0 < nh && !done; c0 += kHklChunk) {
+      const int cn = min(kHklChunk, nh - c0), words = (cn + 31) / 32;
+      for (int w = 0; w < words; w++) {  // energy = hc |q| / (4 pi s), s = -q_z / |q|
+        uint32_t bits = 0u;
+        for (int b = 0; b < 32 && w * 32 + b < cn; b++) {
+          const float e = g.hc * reflect(__ldg(hklf + c0 + w * 32 + b)), s = -qz * rq;
+          const bool out = s < -m || e * (1.f - 2.f * m) > g.ehif * (s + m) ||
+                           e * (1.f + 2.f * m) < g.elof * (s - m);
+          if (!out) bits |= 1u << b;
+        }
+        band[w * TB + t] = bits;
+      }
+      for (int w = 0; w < words; w++) {
+        uint32_t kept = 0u;
+        for (uint32_t bits = band[w * TB + t]; bits; bits &= bits - 1u) {
+          const int b = __ffs(bits) - 1;
+          const float4 h = __ldg(hklf + c0 + w * 32 + b);
+          reflect(h);
+          const float u0 = fmaf(U[0], h.x, fmaf(U[1], h.y, U[2] * h.z)) * rq;
+          const float u1 = fmaf(U[3], h.x, fmaf(U[4], h.y, U[5] * h.z)) * rq;
+          const float u2 = fmaf(U[6], h.x, fmaf(U[7], h.y, U[8] * h.z)) * rq;
+          if (!off_detector(qz * rq, u0, u1, u2, m)) kept |= 1u << b;
+        }
+        keep[w * TB + t] = kept;
+      }
+      int w = -1;
+      uint32_t bits = 0u;
+      while (!done) {
+        while (bits == 0u && ++w < words) bits = keep[w * TB + t];
+        if (w >= words) break;
+        const int i = c0 + w * 32 + __ffs(bits) - 1;
+        bits &= bits - 1u;
+        take(__ldg(hkl + i));
+      }
+    }
     done = true;
   }
   for (int c0 = 0, chunk = 0; !kExactAll && c0 < nseen; c0 += kHklChunk, chunk++) {
@@ -232,10 +303,7 @@ __global__ void __launch_bounds__(128, 6) dbbuild_kernel(const double *__restric
         const float u0 = fmaf(U[0], h.x, fmaf(U[1], h.y, U[2] * h.z));
         const float u1 = fmaf(U[3], h.x, fmaf(U[4], h.y, U[5] * h.z));
         const float u2 = fmaf(U[6], h.x, fmaf(U[7], h.y, U[8] * h.z));
-        const float x = fmaf(qz, u0, g.cx2), y = fmaf(qz, u1, g.cy2), z = fmaf(qz, u2, g.cz2);
-        const bool off = z < -m || fmaf(g.bx0, z, x) < -m || fmaf(g.bx1, z, x) > m ||
-                         fmaf(g.by0, z, y) < -m || fmaf(g.by1, z, y) > m;
-        if (off) continue;
+        if (off_detector(qz, u0, u1, u2, m)) continue;
         const bool either = !(fabsf(qz) > m);  // q_z may have either sign (or m is NaN)
         const uint32_t i = pos & 0xFFFFu, j = pos >> 16;
         if ((qz < 0.f || either) && i != 0xFFFFu) keep[(i >> 5) * TB + t] |= 1u << (i & 31u);
@@ -392,6 +460,9 @@ static BuildGeo make_build_geo(const lmb_geometry &geo) {
   g.bx1 = (float)((bx - g.W) / tolx);
   g.by0 = (float)((by + 1.0) / toly);
   g.by1 = (float)((by - g.H) / toly);
+  g.hc = (float)(kHcKeVnm / kFourPi);
+  g.elof = (float)g.elo;
+  g.ehif = (float)g.ehi;
   return g;
 }
 
@@ -522,7 +593,7 @@ static void build_units(const lmb_geometry &geo, const int4 *hkl, int nh, std::v
     float w;
     memcpy(&w, &band, 4);
     bu.hkl_band[nu] = make_float4((float)(h.x / len), (float)(h.y / len), (float)(h.z / len), w);
-    bu.eps[nu] = plain ? (float)(256.0 * ulp * sum / q + 4e-6 + kBandTol) : std::numeric_limits<float>::quiet_NaN();
+    bu.eps[nu] = plain ? (float)((double)kUnitErr * sum / q + (double)kUnitErr0 + kBandTol) : std::numeric_limits<float>::quiet_NaN();
     bu.pos[nu] = (uint32_t)i | 0xFFFF0000u;
     open[std::make_tuple(h.x, h.y, h.z)].push_back(nu);
     nu++;
@@ -546,6 +617,7 @@ static size_t dbbuild_smem_bytes(int S) {
 // The HKL list with its screens on the device, for the builds of one call.
 struct BuildTables {
   int4 *hkl = nullptr, *seen = nullptr;
+  float4 *hklf = nullptr;  // hkl as floats
   BuildUnits *units = nullptr;
   uint32_t *count = nullptr;
   BuildGeo g{};
@@ -577,7 +649,10 @@ int dbbuild_tables(const lmb_geometry &geo, const int32_t *hkls, int nh, bool ex
     std::copy_n(static_cast<const unsigned char *>(src), bytes, host.begin() + (ptrdiff_t)at);
     return at;
   };
+  std::vector<float4> hf(h.size());
+  for (size_t i = 0; i < h.size(); i++) hf[i] = make_float4((float)h[i].x, (float)h[i].y, (float)h[i].z, 0.f);
   const size_t oh = part(h.data(), h.size() * sizeof(int4));
+  const size_t of = part(hf.data(), hf.size() * sizeof(float4));
   const size_t os = part(seen.data(), seen.size() * sizeof(int4));
   const size_t ou = part(units.data(), units.size() * sizeof(BuildUnits));
   const size_t oc = part(count.data(), count.size() * sizeof(uint32_t));
@@ -595,6 +670,7 @@ int dbbuild_tables(const lmb_geometry &geo, const int32_t *hkls, int nh, bool ex
     return cuda_fail(ce, "DB build tables", __FILE__, __LINE__);
   }
   t->hkl = reinterpret_cast<int4 *>(d + oh);  // oh = 0: the allocation itself
+  t->hklf = reinterpret_cast<float4 *>(d + of);
   t->seen = reinterpret_cast<int4 *>(d + os);
   t->units = reinterpret_cast<BuildUnits *>(d + ou);
   t->count = reinterpret_cast<uint32_t *>(d + oc);
@@ -616,10 +692,10 @@ int dbbuild_launch(const double *d_om, uint64_t n, const BuildTables *t, uint16_
   const uint64_t blocks = (n + tb - 1) / tb;
   LMB_REQUIRE(blocks < (1ull << 31), "too many orientations (%llu)", (unsigned long long)n);
   if (t->all)
-    dbbuild_kernel<true><<<(unsigned)blocks, tb, smem, st>>>(d_om, n, t->hkl, t->nh, t->seen, t->nseen,
+    dbbuild_kernel<true><<<(unsigned)blocks, tb, smem, st>>>(d_om, n, t->hkl, t->hklf, t->nh, t->seen, t->nseen,
                                                              t->units, t->count, t->g, d_out);
   else
-    dbbuild_kernel<false><<<(unsigned)blocks, tb, smem, st>>>(d_om, n, t->hkl, t->nh, t->seen, t->nseen,
+    dbbuild_kernel<false><<<(unsigned)blocks, tb, smem, st>>>(d_om, n, t->hkl, t->hklf, t->nh, t->seen, t->nseen,
                                                               t->units, t->count, t->g, d_out);
   LMB_CUDA(cudaGetLastError());
   return LMB_OK;
