@@ -530,6 +530,7 @@ def tilted_leg(args, dev, K=64, n=None):
             runs[name] = {"compare_ms": round(cmp_ms, 4), "step_ms": round(step_ms, 4),
                           "images_per_s": round(K / (step_ms * 1e-3), 1),
                           "variant": e.get_tuning()["last_variant"],
+                          "form": e.get_tuning()["last_form"],
                           "identical_to_auto": same_survivors(sv, ref_surv)}
         lay = e.layout_info()
         surv = [int(ref_surv[k][0].shape[0]) for k in slots]
@@ -586,7 +587,7 @@ def tilted_leg(args, dev, K=64, n=None):
         # the filter reads the cell codes (2 B per spot) of the records that can pass
         # and the occupancy words (the mask's source)
         streamed = (round(2 * out["gathers"]["spots_per_record"] * n) + p.nr_px_x * p.nr_px_y * 8) \
-            if auto["variant"] == 5 else ref_bytes
+            if auto["form"] == 2 else ref_bytes
         out["roofline"] = {"bound": "hbm", "peak": peak, "peak_source": peak_src, "unit": "GB/s",
                            "reference_layout_bytes": ref_bytes,
                            "reference_layout_gbs": round(ref_bytes / t / 1e9, 1),
@@ -1390,21 +1391,24 @@ def run_ours(args, rank, world):
     # Algorithmic bytes of one pass: over the reference records, 122 B per
     # orientation plus the K uint8 frames; over the listed records, for each
     # orientation with MinNrSpots spots its place in the list, its count and spots,
-    # and an occupancy word (8 B) per spot (shares of the DB from its first records).
+    # and an occupancy word (8 B) per spot (shares of the DB from its first records);
+    # when they are filtered first, their cell codes (2 B per spot) and the occupancy
+    # words (the mask's source).
     lay, shape = lay_main, shape_main
-    listed = shape.get("last_variant") == 2 and shape.get("variant") == 3 and lay["tiles"] == 0
+    form = shape["last_form"]  # 0 every record, 1 listed, 2 filtered
     ref_bytes = N * REC_BYTES_PER_ORIENT + K * p.nr_px_x * p.nr_px_y
     cnt_head = rec_head[:, 0].astype(np.int64)
     can_pass = cnt_head[cnt_head >= p.min_nr_spots]
-    alg_bytes = int(N / len(cnt_head) * (6 * len(can_pass) + 12 * can_pass.sum())) if listed \
-        else ref_bytes
+    share = N / len(cnt_head)
+    alg_bytes = (ref_bytes, int(share * (6 * len(can_pass) + 12 * can_pass.sum())),
+                 int(share * 2 * can_pass.sum()) + p.nr_px_x * p.nr_px_y * 8)[form]
     cmp_avg = statistics.mean(cmp_ms)
     achieved = alg_bytes / (cmp_avg * 1e-3) / 1e9
-    tpo = None if listed else TRAFFIC_BYTES_PER_ORIENT["reference"]
-    roof = {"bound": "latency" if listed else "hbm", "achieved": round(achieved, 1), "peak": peak,
+    tpo = None if form else TRAFFIC_BYTES_PER_ORIENT["reference"]
+    roof = {"bound": "latency" if form == 1 else "hbm", "achieved": round(achieved, 1), "peak": peak,
             "unit": "GB/s", "frac": round(achieved / peak, 4), "peak_source": peak_src,
-            "kernel": "listed_kernel" if listed else "compare_ws_kernel",
-            "layout": "listed records" if listed else "reference",
+            "kernel": ("compare_ws_kernel", "listed_kernel", "group_filter_kernel")[form],
+            "layout": ("reference", "listed records", "listed records, filtered")[form],
             "algorithmic_bytes_per_launch": alg_bytes,
             "avg_launch_ms": round(cmp_avg, 4),
             "traffic": round(tpo * N) if tpo else None,
@@ -1413,8 +1417,8 @@ def run_ours(args, rank, world):
             "reference_layout_bytes_per_launch": ref_bytes,
             "reference_layout_equivalent_gbs": round(ref_bytes / (cmp_avg * 1e-3) / 1e9, 1),
             "tuning": shape}
-    if listed:
-        roof["records_that_can_pass"] = int(N / len(cnt_head) * len(can_pass))
+    if form:
+        roof["records_that_can_pass"] = int(share * len(can_pass))
         roof["layout_info"] = lay
 
     out = {
@@ -1450,8 +1454,9 @@ def run_ours(args, rank, world):
             # enqueue), match (enqueue), results_batch (wait for the pass + copy)
             "breakdown_ms_p50": {k: round(1e3 * float(np.median(v)), 3)
                                  for k, v in phase.items() if v}},
-        # per timed pass: compare, ordering (one graph replay)
-        "gpu_launches": 2 * args.steps,
+        # per timed pass (one graph replay): compare and ordering; before a filtered
+        # one's compare, group mask and filter
+        "gpu_launches": (4 if form == 2 else 2) * args.steps,
         "clocks": clk,
         "latency_ms": {"batched_p50": round(float(np.percentile(seq_lat, 50)), 3),
                        "batched_p99": round(float(np.percentile(seq_lat, 99)), 3),

@@ -130,7 +130,8 @@ int lmb_engine_set_tuning(lmb_engine *e, const int32_t *fields, int32_t n_fields
 /* get: fields 0-6 as set, 7: the variant the latest pass ran (of the automatic
  * one over grouped records: 2 while the records that can pass hold at most 3
  * spots per DB record, 5 beyond), 8: the test wait, 9-11: cell_consumers,
- * cell_stages, cell_queue. */
+ * cell_stages, cell_queue, 12: what the latest pass ran over (0 every record, 1 the
+ * listed records that can pass, 2 the listed ones that the filter kept). */
 int lmb_engine_get_tuning(lmb_engine *e, int32_t *fields, int32_t n_fields);
 
 /* The device layouts derived from the resident records (which stay): the records

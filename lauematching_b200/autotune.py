@@ -150,6 +150,7 @@ def main():
         bytes_pass = args.n_orient * R * 2 + kb * p.nr_px_x * p.nr_px_y
         shape = dict(best[1])
         shape.pop("last_variant", None)
+        shape.pop("last_form", None)
         if shape["variant"] == 2:  # engines pick the layout per pass (automatic variant 3)
             shape["variant"] = 3
         entries[f"R{R}_K{batch_bucket(kb)}" + ("_dense" if args.dense else "")] = {

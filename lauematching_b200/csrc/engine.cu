@@ -169,6 +169,7 @@ struct lmb_engine {
   // warps, 8 blocks per SM)
   CompareTuning tuning{3, 0, 2, 3, 1, 8, 0, 0, 0, 0, 0};
   int last_variant = -1;  // variant the latest pass ran
+  int last_form = 0;      // ... over: 0 all records, 1 those that can pass, 2 filtered ones
   std::vector<PassGraph> graphs;  // captured passes, most recent last
   bool use_graphs = true;
   bool sparse_uploads = true;               // frames cross the link as pairs when sparse
@@ -1438,6 +1439,7 @@ int lmb_match(lmb_engine *e, uint64_t slot_mask, int32_t min_nr_spots, double mi
       tun = CompareTuning{1, 0, 0, 0, 0, 0, tun.full_gather, tun.test_consumer_wait_us, 0, 0, 0};
   }
   e->last_variant = tun.variant;
+  e->last_form = listed ? (filter ? 2 : 1) : 0;
   ensure_lists(e);
   uint64_t waited = 0;
   for (int k = 0; k < LMB_MAX_SLOTS; k++) {
@@ -1709,11 +1711,12 @@ int lmb_engine_set_sparse_uploads(lmb_engine *e, int32_t enable) {
 int lmb_engine_get_tuning(lmb_engine *e, int32_t *fields, int32_t n_fields) {
   LMB_REQUIRE(e && (fields || n_fields == 0), "null argument");
   const CompareTuning c = compare_config(e->R, e->tuning);
-  const int32_t src[12] = {c.variant,        c.tile_sub,       c.stages,
+  const int32_t src[13] = {c.variant,        c.tile_sub,       c.stages,
                            c.consumers,      c.blocks_per_sm,  c.grid_mult,
                            c.full_gather,    e->last_variant,  c.test_consumer_wait_us,
-                           c.cell_consumers, c.cell_stages,    c.cell_queue};
-  for (int i = 0; i < n_fields && i < 12; i++) fields[i] = src[i];
+                           c.cell_consumers, c.cell_stages,    c.cell_queue,
+                           e->last_form};
+  for (int i = 0; i < n_fields && i < 13; i++) fields[i] = src[i];
   return LMB_OK;
 }
 

@@ -144,11 +144,12 @@ class Engine:
                 "tile_bytes": tb.value}
 
     def get_tuning(self) -> dict:
-        """The shape set (variant 3 = automatic) and ``last_variant``, the
-        variant the latest pass ran."""
-        vals = (C.c_int32 * 8)()
-        check(lib().lmb_engine_get_tuning(self._h, vals, 8))
-        return dict(zip(self.TUNING_FIELDS + ("last_variant",), list(vals)))
+        """The shape set (variant 3 = automatic), ``last_variant``, the variant
+        the latest pass ran, and ``last_form``, what it ran over: 0 every
+        record, 1 the listed records that can pass, 2 those the filter kept."""
+        vals = (C.c_int32 * 13)()
+        check(lib().lmb_engine_get_tuning(self._h, vals, 13))
+        return dict(zip(self.TUNING_FIELDS + ("last_variant",), list(vals))) | {"last_form": vals[12]}
 
     # ---- DB -------------------------------------------------------------------
     def upload_db(self, records: np.ndarray) -> None:

@@ -253,3 +253,20 @@ def test_components_are_found_once(fake, method, dtype, fractional_bg):
     radix = fractional_bg or dtype is np.float32  # the fake leaves the value path unset
     assert (fake.fake_launched(b"sel_hist_kernel") > 0) == bool(radix)
     h.close()
+
+
+@pytest.mark.parametrize("n,spots,variant,form", [(1000, 15, 5, 1), (1_000_000, 3, 2, 2),
+                                                  (1_000_000, 15, 5, 2), (1000, 2, 2, 1)])
+def test_the_form_of_the_pass_is_reported(fake, n, spots, variant, form):
+    """What a pass ran over goes by the number of spots to look at, ``last_variant`` by
+    the number per record."""
+    fake.fake_counts(spots, n)
+    with _engine(min_nr_spots=2) as e:
+        e.upload_db(_records(n))
+        e.load_image(0, np.ones(64 * 64))
+        e.match([0], 2, 1.0)
+        assert fake.fake_launched(b"group_filter_kernel") == form - 1
+        assert e.get_tuning()["last_variant"] == variant and e.get_tuning()["last_form"] == form
+        e.set_tuning(variant=1)
+        e.match([0], 2, 1.0)
+        assert e.get_tuning()["last_form"] == 0
