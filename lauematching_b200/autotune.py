@@ -5,13 +5,13 @@ layout), tile size, ring depth, consumer warps and grid size on the device for
 a DB of the given record size and batch width, checks that every shape
 returns the same survivors, and writes the fastest shape per (record words,
 batch bucket) to ``tuning.json`` next to this file.  With ``--dense`` it
-compares the grouped records' filter (variant 5) with the cell-mask pass
-(variant 4) on a DB of many spots per record and writes the ``_dense`` entries.
-Engines load the table before their first pass; the automatic variant over
-grouped records has no shape to choose, pinned variants take theirs from it.
+compares the grouped records' filter (variant 5, which has no shape to choose)
+with the cell-mask pass (variant 4) on a DB of many spots per record, and
+writes nothing.  Engines load the table before their first pass, for the passes
+over all records.
 
     python -m lauematching_b200.autotune --n-orient 100000000 --batches 1,64 --write
-    python -m lauematching_b200.autotune --dense --n-orient 100000000 --batches 64 --write
+    python -m lauematching_b200.autotune --dense --n-orient 100000000 --batches 64
 """
 from __future__ import annotations
 
@@ -44,11 +44,10 @@ def load_table() -> dict:
     return {}
 
 
-def lookup(R: int, k: int, dense: bool = False) -> dict | None:
-    """Best shape for records of R uint16 words and a pass of k images; with
-    ``dense``, that of a DB of many spots per record."""
+def lookup(R: int, k: int) -> dict | None:
+    """Best shape for records of R uint16 words and a pass of k images."""
     t = load_table().get("entries", {})
-    suffix = f"_K{batch_bucket(k)}" + ("_dense" if dense else "")
+    suffix = f"_K{batch_bucket(k)}"
     key = f"R{R}{suffix}"
     if key in t:
         return t[key]["shape"]
@@ -101,9 +100,8 @@ def main():
     ap.add_argument("--seed", type=int, default=1)
     ap.add_argument("--write", action="store_true", help="update tuning.json")
     ap.add_argument("--dense", action="store_true",
-                    help="tune the cell-mask pass (variant 4) on a DB of many spots per "
-                         "record (the reference's tilted 34-ID-E detector); stored as the "
-                         "table's _dense entries")
+                    help="compare the filter (variant 5) and the cell-mask pass (variant 4) on "
+                         "a DB of many spots per record (the reference's tilted 34-ID-E detector)")
     args = ap.parse_args()
     geo = dict(p=(0.028745, 0.002788, 0.513115),
                r=(-1.20131258, -1.21399082, -1.21881158)) if args.dense else {}
@@ -144,24 +142,24 @@ def main():
             results.append((ms, used, same))
             print(f"K={kb} {used} {ms:.4f} ms identical={same}", file=sys.stderr)
         ok = [r for r in results if r[2]]
-        # the dense entry shapes the pass the automatic variant runs there (5)
-        best = min([r for r in ok if not args.dense or r[1]["variant"] == 5] or ok,
-                   key=lambda r: r[0])
+        best = min(ok, key=lambda r: r[0])
         bytes_pass = args.n_orient * R * 2 + kb * p.nr_px_x * p.nr_px_y
         shape = dict(best[1])
         shape.pop("last_variant", None)
         shape.pop("last_form", None)
         if shape["variant"] == 2:  # engines pick the layout per pass (automatic variant 3)
             shape["variant"] = 3
-        entries[f"R{R}_K{batch_bucket(kb)}" + ("_dense" if args.dense else "")] = {
-            "shape": shape, "compare_ms": round(best[0], 4),
-            "gbs": round(bytes_pass / (best[0] * 1e-3) / 1e9, 1), "n_orient": args.n_orient,
-            "swept": len(results),
-            "all": [{"shape": r[1], "ms": round(r[0], 4)} for r in sorted(results, key=lambda r: r[0])],
-        }
+        if not args.dense:
+            entries[f"R{R}_K{batch_bucket(kb)}"] = {
+                "shape": shape, "compare_ms": round(best[0], 4),
+                "gbs": round(bytes_pass / (best[0] * 1e-3) / 1e9, 1), "n_orient": args.n_orient,
+                "swept": len(results),
+                "all": [{"shape": r[1], "ms": round(r[0], 4)}
+                        for r in sorted(results, key=lambda r: r[0])],
+            }
         print(json.dumps({"K": kb, "best": best[1], "ms": best[0]}))
     table["device"] = "NVIDIA B200"
-    if args.write:
+    if args.write and not args.dense:
         with open(TABLE, "w") as f:
             json.dump(table, f, indent=1)
     e.close()

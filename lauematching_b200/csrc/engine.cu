@@ -167,7 +167,8 @@ struct lmb_engine {
   uint64_t fresh_mask = 0;            // slots loaded since a pass waited for them
   // automatic variant with the compact pass's tuned shape (2 stages, 3 consumer
   // warps, 8 blocks per SM)
-  CompareTuning tuning{3, 0, 2, 3, 1, 8, 0, 0, 0, 0, 0};
+  CompareTuning tuning{3, 0, 2, 3, 1, 8, 0, 0, 0};
+  int cell_shape[2] = {0, 0};  // cell_consumers, cell_stages as set: no pass reads them
   int last_variant = -1;  // variant the latest pass ran
   int last_form = 0;      // ... over: 0 all records, 1 those that can pass, 2 filtered ones
   std::vector<PassGraph> graphs;  // captured passes, most recent last
@@ -584,8 +585,7 @@ int build_compact(lmb_engine *e, int min_spots) {
   const uint64_t avg_chunk = 36 + (4 * total_spots + nch - 1) / nch;
   uint64_t TB = std::min<uint64_t>(24 * 1024, std::max<uint64_t>(4096, round128(64 * avg_chunk)));
   if (gathered_per_record(e, e->cl_hist, min_spots) > kAutoGather) {
-    // the automatic variant will run the cell-mask filter over it: its tile
-    // size, whatever the tuning of this pass
+    // the cell-mask pass's tile size, for whichever pinned variant comes first
     TB = kCellTileBytes;
   } else {
     // room for the pass shape's blocks (three consumer warps, a two-stage
@@ -1436,7 +1436,7 @@ int lmb_match(lmb_engine *e, uint64_t slot_mask, int32_t min_nr_spots, double mi
       compact = gathered_per_record(e, e->cl_hist, tun.full_gather ? 0 : min_nr_spots) <= kAutoGather;
     }
     if (!compact)  // warp-specialised over the reference records
-      tun = CompareTuning{1, 0, 0, 0, 0, 0, tun.full_gather, tun.test_consumer_wait_us, 0, 0, 0};
+      tun = CompareTuning{1, 0, 0, 0, 0, 0, tun.full_gather, tun.test_consumer_wait_us, 0};
   }
   e->last_variant = tun.variant;
   e->last_form = listed ? (filter ? 2 : 1) : 0;
@@ -1665,22 +1665,23 @@ int lmb_last_pass_ms(lmb_engine *e, float *compare_ms, float *order_ms) {
 
 int lmb_engine_set_tuning(lmb_engine *e, const int32_t *fields, int32_t n_fields) {
   LMB_REQUIRE(e && (fields || n_fields == 0), "null argument");
-  CompareTuning t{1, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+  CompareTuning t{1, 0, 0, 0, 0, 0, 0, 0, 0};
+  int cell_shape[2] = {0, 0};
   int32_t *dst[11] = {&t.variant,     &t.tile_sub,      &t.stages,
                       &t.consumers,   &t.blocks_per_sm, &t.grid_mult,
-                      &t.full_gather, &t.test_consumer_wait_us, &t.cell_consumers,
-                      &t.cell_stages, &t.cell_queue};
+                      &t.full_gather, &t.test_consumer_wait_us, &cell_shape[0],
+                      &cell_shape[1], &t.cell_queue};
   for (int i = 0; i < n_fields && i < 11; i++) *dst[i] = fields[i];
   LMB_REQUIRE(t.cell_queue == 0 || t.cell_queue == 1, "cell_queue must be 0 or 1");
-  LMB_REQUIRE(t.cell_consumers >= 0 && t.cell_consumers <= 24 && t.cell_stages >= 0 &&
-                  t.cell_stages <= 16,
-              "cell-mask pass shape (%d consumers, %d stages) out of range", t.cell_consumers,
-              t.cell_stages);
+  LMB_REQUIRE(cell_shape[0] >= 0 && cell_shape[0] <= 24 && cell_shape[1] >= 0 && cell_shape[1] <= 16,
+              "cell-mask pass shape (%d consumers, %d stages) out of range", cell_shape[0],
+              cell_shape[1]);
   LMB_REQUIRE(t.full_gather == 0 || t.full_gather == 1, "full_gather must be 0 or 1");
   LMB_REQUIRE(t.test_consumer_wait_us >= 0 && t.test_consumer_wait_us <= 1000000,
               "test wait of %d us outside 0..1000000", t.test_consumer_wait_us);
   LMB_REQUIRE(t.variant >= 0 && t.variant <= 5, "unknown compare variant %d", t.variant);
   e->tuning = t;
+  for (int i = 0; i < 2; i++) e->cell_shape[i] = cell_shape[i];
   return LMB_OK;
 }
 
@@ -1714,7 +1715,7 @@ int lmb_engine_get_tuning(lmb_engine *e, int32_t *fields, int32_t n_fields) {
   const int32_t src[13] = {c.variant,        c.tile_sub,       c.stages,
                            c.consumers,      c.blocks_per_sm,  c.grid_mult,
                            c.full_gather,    e->last_variant,  c.test_consumer_wait_us,
-                           c.cell_consumers, c.cell_stages,    c.cell_queue,
+                           e->cell_shape[0], e->cell_shape[1], c.cell_queue,
                            e->last_form};
   for (int i = 0; i < n_fields && i < 13; i++) fields[i] = src[i];
   return LMB_OK;

@@ -76,10 +76,6 @@ struct CompareTuning {
   int grid_mult;      // grid = SMs * blocks_per_sm * grid_mult
   int full_gather;    // 1: gather every spot even of records that cannot pass
   int test_consumer_wait_us;  // test only: see CmpArgs::test_consumer_wait_ns
-  // shape of the cell-mask pass when the automatic variant picks it
-  // (0 = defaults): consumer warps, ring stages
-  int cell_consumers;
-  int cell_stages;
   int cell_queue;  // variant 4: see CmpArgs::cell_queue
 };
 CompareTuning compare_config(int R, const CompareTuning &req);

@@ -250,12 +250,8 @@ class Engine:
         b = batch_bucket(k)
         if b != self._shape_bucket:
             shape = lookup(self.R, b)
-            dense = lookup(self.R, b, dense=True) or {}
             if shape:
-                check(lib().lmb_engine_set_tuning(
-                    self._h, self._tuning_vals(shape, 0, dense.get("consumers", 0),
-                                               dense.get("stages", 0),
-                                               dense.get("cell_queue", 0)), 11))
+                check(lib().lmb_engine_set_tuning(self._h, self._tuning_vals(shape), 11))
             self._shape_bucket = b
 
     def match(self, slots, min_nr_spots: int, min_intensity: float, value_mode: int = 0) -> None:
