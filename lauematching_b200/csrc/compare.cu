@@ -5,21 +5,26 @@
 // (LaueMatchingGPU.cu:45-81, LaueMatchingGPUStream.cu:69-100); survivors are
 // delivered in ascending orientation ID like LaueMatchingCPU.c:781-788.
 //
-// Batched pass.  Up to 64 images ("slots") are matched in one pass over the
-// DB.  For every pixel the occupancy word holds bit k set when slot k's
+// Batched pass.  Up to 64 images ("slots") are matched in one pass.  For every pixel the occupancy word holds bit k set when slot k's
 // uint8 pixel is positive, so one 8-byte gather per spot gives the hit/miss
 // of that spot in every image at once; per-slot spot counts are kept as
 // bit-sliced counters (bit b of all 64 counters in one word).  Only an
 // orientation whose count reaches MinNrSpots in some slot ("candidate") goes
 // back over its spots to sum the intensity of that slot in FP64, in record
-// order, exactly as the reference does; candidates are rare, so the DB
-// stream and the 8-byte gathers are the cost.
+// order, exactly as the reference does.
 //
-// DB stream.  A persistent grid walks tiles of TILE consecutive records;
-// tile bytes are moved into shared memory by 1-D TMA bulk copies
-// (cp.async.bulk) through a STAGES-deep mbarrier ring, so the stream is
-// coalesced regardless of the 122-byte record stride.  Waits are bounded
-// (2 s of global time) and report through an error word.
+// Grouped records (the automatic pass, variants 3 and 5).  The DB is not
+// streamed: the records with at least MinNrSpots spots head a list by spot
+// count (glist.cu) and listed_kernel counts them; a long list first goes
+// through group_filter_kernel, which looks up 2-byte cell codes of the spots
+// in a mask of the frames in shared memory.
+//
+// Streamed records (pinned variants 0, 1, 2 and 4, and where the records cannot
+// be grouped).  A persistent grid walks tiles of consecutive records; tile
+// bytes are moved into shared memory by 1-D TMA bulk copies (cp.async.bulk)
+// through a STAGES-deep mbarrier ring, so the stream is coalesced regardless
+// of the 122-byte record stride.  Waits are bounded (2 s of global time) and
+// report through an error word.
 #include <climits>
 #include <mutex>
 #include <type_traits>
@@ -1624,9 +1629,10 @@ __device__ void bitonic_tiled(unsigned long long *g, uint32_t P, unsigned long l
   }
 }
 
-// One block per slot of the pass.  Short lists and the slot's counters also go to page-locked host memory from here, so that a caller who waits for the pass
-// has its results without another copy (a gather kernel, a copy and its
-// synchronisation; 20-25 us of a small pass, measured on B200).
+// One block per slot of the pass.  Short lists and the slot's counters also go to
+// page-locked host memory from here, so that a caller who waits for the pass has its
+// results without another copy (a gather kernel, a copy and its synchronisation; 20-25
+// us of a small pass, measured on B200).
 __global__ void __launch_bounds__(1024) order_kernel(const __grid_constant__ OrderArgs a) {
   extern __shared__ __align__(16) unsigned long long sk[];  // kSmemSortMax keys
   if (blockIdx.x == 0 && threadIdx.x == 0)

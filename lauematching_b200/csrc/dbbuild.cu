@@ -593,7 +593,8 @@ static void build_units(const lmb_geometry &geo, const int4 *hkl, int nh, std::v
     float w;
     memcpy(&w, &band, 4);
     bu.hkl_band[nu] = make_float4((float)(h.x / len), (float)(h.y / len), (float)(h.z / len), w);
-    bu.eps[nu] = plain ? (float)((double)kUnitErr * sum / q + (double)kUnitErr0 + kBandTol) : std::numeric_limits<float>::quiet_NaN();
+    bu.eps[nu] = plain ? (float)((double)kUnitErr * sum / q + (double)kUnitErr0 + kBandTol)
+                       : std::numeric_limits<float>::quiet_NaN();
     bu.pos[nu] = (uint32_t)i | 0xFFFF0000u;
     open[std::make_tuple(h.x, h.y, h.z)].push_back(nu);
     nu++;

@@ -37,8 +37,10 @@ using namespace lmb;
 // whatever other passes are in flight.
 static constexpr int kStatusWords = 2 * LMB_MAX_SLOTS + 1;
 static constexpr int kEventRing = 64;  // events of passes and loads
-// Survivor lists up to this long are written to host memory by the pass itself.
-static constexpr uint32_t kHostList = 4096;
+// Survivor lists up to this long are written to host memory by the pass itself: to
+// kShortList's room, made with the engine (512 KiB), until a slot has had a longer one.
+// Page-locking the 8 MiB for long ones takes 3 to 6 ms.
+static constexpr uint32_t kShortList = 256, kHostList = 4096;
 
 static constexpr int kSparseRing = 4;  // pinned staging buffers for sparse frames
 // Pairs of one frame up to this many bytes are not copied to the device first: the
@@ -148,8 +150,12 @@ struct lmb_engine {
   unsigned long long *d_scratch = nullptr;
   unsigned int *d_status = nullptr;
   unsigned int *h_status = nullptr;  // pinned, kStatusWords
-  lmb_survivor *h_list = nullptr;         // pinned: [64][kHostList], short lists of each slot
-  bool lists_tried = false;
+  // pinned: lists of each slot, [64][kShortList] and, once one has been longer,
+  // [64][kHostList]; and of each slot's last pass where its list lies and the room there
+  lmb_survivor *h_short = nullptr, *h_long = nullptr;
+  int long_state = 0;  // h_long: 0 not needed so far, 1 to be made, 2 made, -1 no memory
+  const lmb_survivor *slot_list[LMB_MAX_SLOTS] = {};
+  uint32_t slot_room[LMB_MAX_SLOTS] = {};
   uint64_t pass_seq = 0;                  // passes enqueued so far
   uint64_t done_mask = 0;                 // slots that have been in a pass
   cudaStream_t dl = nullptr;              // survivor downloads
@@ -259,18 +265,26 @@ int ensure_f64(lmb_engine *e, int slot) {
   return LMB_OK;
 }
 
-// Room for the passes' short lists (8 MiB), made for the first pass: an engine that
-// only builds records needs none.  Without it every list is fetched from the device.
+// Where the next pass writes its slots' lists, and the room for each.
+lmb_survivor *pass_lists(const lmb_engine *e) { return e->long_state == 2 ? e->h_long : e->h_short; }
+uint32_t pass_room(const lmb_engine *e) {
+  return std::min(e->long_state == 2 ? kHostList : kShortList, e->cap);
+}
+
+// A list that did not fit has been read: the next passes take the larger room.  Lists
+// of passes before stay where they are.
 void ensure_lists(lmb_engine *e) {
-  if (e->lists_tried) return;
-  e->lists_tried = true;
-  if (cudaHostAlloc(&e->h_list, (size_t)LMB_MAX_SLOTS * kHostList * sizeof(lmb_survivor),
-                    cudaHostAllocDefault) == cudaSuccess)
+  if (e->long_state != 1) return;
+  if (cudaHostAlloc(&e->h_long, (size_t)LMB_MAX_SLOTS * kHostList * sizeof(lmb_survivor),
+                    cudaHostAllocDefault) == cudaSuccess) {
+    e->long_state = 2;
+    drop_graphs(e);  // captured passes name the other room
     return;
-  e->h_list = nullptr;
+  }
+  e->h_long = nullptr;
+  e->long_state = -1;
   cudaGetLastError();
 }
-uint32_t host_list_cap(const lmb_engine *e) { return e->h_list ? std::min(kHostList, e->cap) : 0u; }
 
 // Slots about to be written on the load stream: after the last passes that read
 // them.
@@ -327,7 +341,8 @@ void free_engine(lmb_engine *e) {
   cudaFree(e->d_scratch);
   cudaFree(e->d_status);
   cudaFreeHost(e->h_status);
-  cudaFreeHost(e->h_list);
+  cudaFreeHost(e->h_short);
+  cudaFreeHost(e->h_long);
   if (e->dl) {
     cudaStreamSynchronize(e->dl);
     cudaStreamDestroy(e->dl);
@@ -863,8 +878,8 @@ int enqueue_pass(lmb_engine *e, const PassKey &k, bool capturing) {
   o.cap = e->cap;
   o.scratch = e->d_scratch;
   o.cap2 = e->cap2;
-  o.host_list = e->h_list;
-  o.host_cap = host_list_cap(e);
+  o.host_list = pass_lists(e);
+  o.host_cap = pass_room(e);
   o.host_status = e->h_status;
   o.status = e->d_status;
   for (int i = 0; i < LMB_MAX_SLOTS; i++)
@@ -964,6 +979,8 @@ int lmb_engine_create(int32_t device, const lmb_geometry *geo, uint64_t survivor
   TRY(cudaHostAlloc(&e->h_status, kStatusWords * sizeof(unsigned int),
                     cudaHostAllocDefault));
   memset(e->h_status, 0, kStatusWords * sizeof(unsigned int));
+  TRY(cudaHostAlloc(&e->h_short, (size_t)LMB_MAX_SLOTS * kShortList * sizeof(lmb_survivor),
+                    cudaHostAllocDefault));
 #undef TRY
   *out = e;
   return LMB_OK;
@@ -1496,7 +1513,11 @@ int lmb_match(lmb_engine *e, uint64_t slot_mask, int32_t min_nr_spots, double mi
   LMB_CUDA(cudaEventRecord(e->ev_pass[v], e->st));
   e->bytes_d2h += kStatusWords * sizeof(unsigned int);
   for (int k = 0; k < LMB_MAX_SLOTS; k++)
-    if (slot_mask >> k & 1) e->slot_pass[k] = v;
+    if (slot_mask >> k & 1) {
+      e->slot_pass[k] = v;
+      e->slot_list[k] = pass_lists(e) + (size_t)k * pass_room(e);
+      e->slot_room[k] = pass_room(e);
+    }
   e->done_mask |= slot_mask;
   e->pass_seq++;
   return LMB_OK;
@@ -1527,9 +1548,12 @@ int slot_status(lmb_engine *e, int slot, const unsigned int **st, uint64_t *wait
   return LMB_OK;
 }
 
-// A slot's list in host memory, when its pass wrote it there.
-const lmb_survivor *host_list(const lmb_engine *e, int slot) {
-  return e->h_list + (size_t)slot * host_list_cap(e);
+// A slot's list of cnt survivors in host memory; null when its pass did not write it
+// there.
+const lmb_survivor *host_list(lmb_engine *e, int slot, uint64_t cnt) {
+  if (cnt <= e->slot_room[slot]) return e->slot_list[slot];
+  if (cnt <= std::min(kHostList, e->cap) && e->long_state == 0) e->long_state = 1;
+  return nullptr;
 }
 
 }  // namespace
@@ -1558,8 +1582,8 @@ int lmb_results(lmb_engine *e, int32_t slot, lmb_survivor *out, uint64_t out_cap
               (unsigned long long)cnt, (unsigned long long)out_capacity);
     return LMB_ERR_OVERFLOW;
   }
-  if (cnt && cnt <= host_list_cap(e))
-    memcpy(out, host_list(e, slot), cnt * sizeof(lmb_survivor));
+  if (const lmb_survivor *l = cnt ? host_list(e, slot, cnt) : nullptr)
+    memcpy(out, l, cnt * sizeof(lmb_survivor));
   else if (cnt)
     LMB_CUDA(cudaMemcpy(out, e->d_sorted + (size_t)slot * e->cap, cnt * sizeof(lmb_survivor),
                         cudaMemcpyDeviceToHost));
@@ -1594,11 +1618,12 @@ int lmb_results_batch(lmb_engine *e, const int32_t *slots, int32_t nslots, lmb_s
     return LMB_ERR_OVERFLOW;
   }
   bool short_lists = true;
-  for (int i = 0; i < nslots; i++) short_lists &= counts[i] <= host_list_cap(e);
+  for (int i = 0; i < nslots; i++) short_lists &= host_list(e, slots[i], counts[i]) != nullptr;
   if (short_lists) {  // in host memory already
     uint64_t at = 0;
     for (int i = 0; i < nslots; i++) {
-      if (counts[i]) memcpy(out + at, host_list(e, slots[i]), counts[i] * sizeof(lmb_survivor));
+      if (counts[i])
+        memcpy(out + at, host_list(e, slots[i], counts[i]), counts[i] * sizeof(lmb_survivor));
       at += counts[i];
     }
     e->bytes_d2h += total * sizeof(lmb_survivor);
@@ -1744,7 +1769,8 @@ int engine_load_device_frame(lmb_engine *e, int slot, const void *d_img, int dty
   if ((rc = wait_released(e, 1ull << slot))) return rc;
   LMB_CUDA(cudaStreamWaitEvent(e->ld, ready, 0));
   rc = quantize_launch(d_img, dtype, e->npx, d_max_bits ? d_max_bits : e->d_max_bits,
-                       d_max_bits != nullptr, e->d_u8 + (size_t)slot * e->npx, nullptr, e->d_occ, slot, e->d_scale + slot, e->num_sms, e->ld);
+                       d_max_bits != nullptr, e->d_u8 + (size_t)slot * e->npx, nullptr, e->d_occ, slot,
+                       e->d_scale + slot, e->num_sms, e->ld);
   if (rc) return rc;
   LMB_CUDA(cudaEventRecord(consumed, e->ld));
   if ((rc = mark_loaded(e, 1ull << slot))) return rc;

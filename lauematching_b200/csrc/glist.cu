@@ -2,9 +2,10 @@
 //
 // A record can only pass when it has at least MinNrSpots spots on the detector
 // (LaueMatchingCPU.c:671-683), so a pass needs the records of the large counts
-// alone.  `perm` lists the record numbers by falling count (within one count in
-// tiles of kGlTile records, ascending in each), so the records with at least m
-// spots are its first entries whatever m is.  Each count starts at a multiple of 32
+// alone.  `perm` lists the record numbers by falling count (within one count tile by
+// tile of kGlTile records, in no order within a tile: its warps race for places, so
+// two builds of one DB may differ there; survivors are ordered by ID after the pass),
+// so the records with at least m spots are its first entries whatever m is.  Each count starts at a multiple of 32
 // (places without a record hold kNoRecord): a chunk of 32 places has one count.
 // 4 bytes per record, made once per DB by a counting sort on the device: 6 to 7 ms
 // to the end of the first pass at 1e8 records of 122 bytes on B200, where packing

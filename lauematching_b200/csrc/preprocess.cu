@@ -1970,7 +1970,8 @@ void free_pre(lmb_pre *p) {
   void *bufs[] = {p->d_raw, p->d_bg, p->d_sub, p->d_tmp, p->d_out, p->d_t16, p->d_filt, p->d_par,
                   p->d_cid, p->d_lab, p->d_flab, p->c.area, p->c.x0, p->c.y0, p->c.x1, p->c.y1,
                   p->c.fb, p->c.sw, p->c.swx, p->c.swy, p->c.label, p->c.keep, p->d_bits,
-                  p->d_sub16, p->d_bg16, p->d_bg_other, p->d_tiles, p->d_compact, p->d_centres, p->d_w, p->d_max, p->d_stats, p->d_head, p->d_next,
+                  p->d_sub16, p->d_bg16, p->d_bg_other, p->d_tiles, p->d_compact, p->d_centres, p->d_w,
+                  p->d_max, p->d_stats, p->d_head, p->d_next,
                   p->d_state, p->d_hist16, p->d_fg, p->m_keys, p->m_keys2, p->m_idx, p->m_idx2, p->m_flag,
                   p->m_incl, p->m_rank, p->m_nd, p->m_vals, p->m_img, p->m_cub,
                   p->m_v16[0], p->m_v16[1], p->m_flag16};

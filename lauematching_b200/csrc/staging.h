@@ -1,8 +1,9 @@
 // Copies between ordinary (pageable) host memory and the device through a small
 // ring of page-locked buffers: host threads copy one piece while the copy engine
 // moves the others.  cudaMemcpy alone does both on one thread, and touches the
-// pages of a fresh destination from it too.  Measured on B200 (16 host cores):
-// see Staging::upload and Staging::download.
+// pages of a fresh destination from it too.  Measured on B200 (16 host cores), results
+// into fresh arrays: 59 MB of a preprocessed frame, whole call 11.7 -> 3.9 ms; the 24
+// MB of 2e5 records, build and download 2.55 -> 1.99 ms.
 #pragma once
 
 #include <cuda_runtime.h>

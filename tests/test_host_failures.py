@@ -216,22 +216,25 @@ def test_large_copies_go_directly_without_page_locked_pieces(fake, pieces):
 
 
 @pytest.mark.parametrize("room", [True, False])
-def test_room_for_short_lists_comes_with_the_first_pass(fake, room):
-    """An engine that only builds locks no 8 MiB of host memory; without them a list
-    is fetched from the device."""
+def test_room_for_long_lists_comes_when_one_is_read(fake, room):
+    """An engine that only builds, and one whose passes find few survivors, lock no 8
+    MiB of host memory; without them a long list is fetched from the device."""
     fake.fake_counts(9, 1000)
     host = fake.fake_host_used()
     with _engine(min_nr_spots=5) as e:
         e.build_db(synth.shoemake_orientations(1000, 1), synth.hkls_cubic(2))
         e.download_db()
-        assert fake.fake_host_used() - host < MIB
         e.load_image(0, np.ones(64 * 64))
-        fake.fake_survivors(3)
-        if not room:
-            fake.fake_limits(1 << 50, fake.fake_host_used())
-        for _ in range(2):
-            e.match([0], 5, 1.0)
-            assert len(e.results(0)[0]) == 3 and len(e.results_batch([0])[0][0]) == 3
+        for need, n in enumerate((3, 256, 257, 4096, 4097, 30), 1):  # each pass eager
+            fake.fake_survivors(n)
+            if not room:
+                fake.fake_limits(1 << 50, fake.fake_host_used())
+            launched = fake.fake_launched(b"gather")
+            e.match([0], need, 1.0)
+            assert len(e.results(0)[0]) == n and len(e.results_batch([0])[0][0]) == n
+            fetched = n > (4096 if room and n > 257 else 256)
+            assert fake.fake_launched(b"gather") - launched == fetched
+            assert (fake.fake_host_used() - host > 8 * MIB) == (room and n in (4096, 4097, 30))
             fake.fake_limits(1 << 50, 1 << 50)
 
 
