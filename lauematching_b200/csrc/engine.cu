@@ -278,6 +278,7 @@ void ensure_lists(lmb_engine *e) {
   if (cudaHostAlloc(&e->h_long, (size_t)LMB_MAX_SLOTS * kHostList * sizeof(lmb_survivor),
                     cudaHostAllocDefault) == cudaSuccess) {
     e->long_state = 2;
+    cudaStreamSynchronize(e->st);
     drop_graphs(e);  // captured passes name the other room
     return;
   }

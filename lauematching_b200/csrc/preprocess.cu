@@ -2217,7 +2217,8 @@ int median_pass(lmb_pre *p, const double *d_in, double *d_out, int size) {
 }
 
 // All median passes of a frame of whole numbers; *done = false when it is none or a
-// tile was not resolved (the rank path then starts again from the frame).
+// tile was not resolved (the rank path then starts again from the frame).  The last
+// pass leaves the background as whole numbers too.
 int median_whole(lmb_pre *p, int dtype, int size, int passes, bool *done) {
   *done = false;
   if (size > kMedTileMaxS) return LMB_OK;
@@ -2249,7 +2250,7 @@ int median_whole(lmb_pre *p, int dtype, int size, int passes, bool *done) {
   LMB_CUDA(cudaEventRecord(p->ev[EV_MED_RANK], st));
   const dim3 tiles((p->nx + kMtX - 1) / kMtX, (p->ny + kMtY - 1) / kMtY);
   for (int i = 0; i < passes; ++i) {
-    uint16_t *to = p->m_v16[(i + 1) & 1];
+    uint16_t *to = i + 1 < passes ? p->m_v16[(i + 1) & 1] : p->d_bg16;  // the background as whole numbers
     median_tile_kernel<<<tiles, kMtThreads, smem, st>>>(in, p->ny, p->nx, size, p->d_bg, to,
                                                         p->m_flag16);
     in = to;
@@ -2398,10 +2399,10 @@ int lmb_pre_median(lmb_pre *p, const void *frame, int32_t dtype, int32_t size, i
       if ((rc = median_pass(p, p->m_img, p->d_bg, size))) return rc;
     }
   }
-  if ((rc = background_changed(p))) return rc;
+  if (!done && (rc = background_changed(p))) return rc;
   if (out && (rc = p->staging.download(out, p->d_bg, p->npx * sizeof(double), p->st))) return rc;
   LMB_CUDA(cudaStreamSynchronize(p->st));
-  p->bg_other = p->h_state->nonint;
+  p->bg_other = done ? 0u : p->h_state->nonint;
   if (size > 1 && passes > 0)
     return stage_times(p, EV_MED0, EV_MED_UP, 5) || stage_times(p, EV_MED_PASS, EV_MED_RANK, 6) ||
            stage_times(p, EV_MED_RANK, EV_MED_K, 7);
