@@ -1689,7 +1689,8 @@ __global__ void __launch_bounds__(kMedWarps * 32, 4)
 // the rank path (a steep background, s = 101; noise of standard deviation 1000, s = 31;
 // random words, s = 31, three passes), whole call: 5.89, 2.96, 15.2 ms there alone,
 // 7.34, 4.05, 18.4 with all 48 thresholds of every tile first, 6.02, 3.06, 15.4 as it
-// is.
+// is.  Values with gaps can look wilder than they are: multiples of 16, s = 31, are
+// given up (2.19 ms) where 48 thresholds would do (1.03; s = 101 is not).
 constexpr int kMtX = 64, kMtY = 32, kMtThreads = 256;
 constexpr int kMedTries = 48;
 constexpr int kMedLook = 5;   // the last threshold that the estimate is made from
